@@ -337,9 +337,9 @@ XKB_API int xkb_sched_set_grid(xkb_sched_t * sched, int ctas);
  * 16384^2 FP64 graph the register body moves 4.8 TB/s and the bulk-staged one 3.2 TB/s. Tiles
  * whose rows are not 16-byte aligned always use the register body. */
 XKB_API int xkb_sched_set_staging(xkb_sched_t * sched, int bulk);
-/* Warps that execute one task in the persistent kernel (1, 2, 4 or 8; default 2): each CTA
- * of 8 warps runs 8 / warps_per_task tasks at a time, each team taking and releasing tasks on
- * its own. */
+/* Warps that execute one task in the persistent kernel at least (1, 2, 4 or 8; default 1): a task
+ * is split into that many units, each run by one warp, or into more where the graph has too few
+ * tasks side by side to fill the device, or its axpby ranges are long. */
 XKB_API int xkb_sched_set_team(xkb_sched_t * sched, int warps_per_task);
 /* Distance, in columns, of the L2 bulk prefetch ahead of a heat tile's sweep (0 = off; default 4). */
 XKB_API int xkb_sched_set_prefetch(xkb_sched_t * sched, int columns);

@@ -185,3 +185,59 @@ def test_bulk_staged_body_matches_register_body(torch_cuda, nx, ny, ts, steps, f
         assert sch.wait() == len(descs)
         np.testing.assert_array_equal((a if steps % 2 == 0 else b).cpu().numpy(), want)
         sch.close(); res.close()
+
+
+@pytest.mark.parametrize("nx,ny,ts,steps,f32", [
+    (130, 70, 128, 7, False),       # 2 tiles (one a sliver): 32 units each, some without a column
+    (200, 136, 64, 9, True),        # 12 tiles: 32 units, several CTAs per tile
+    (1024, 640, 64, 5, False),      # 160 tiles: 8 units, one CTA per tile
+    (1152, 1152, 48, 4, True),      # 576 tiles: 8 units, warps take them one by one
+    (1700, 1500, 48, 3, False),     # 1152 tiles: 4 units
+    (3000, 3000, 48, 3, False)])    # 3969 tiles: not split
+@pytest.mark.parametrize("order", ["in order", "queue", "periodic"])
+def test_heat_units_and_orders(torch_cuda, nx, ny, ts, steps, f32, order):
+    """Every split of a tile task into units, taken in spawn order, through the ready queue (two
+    graphs spawned one after the other are not spawned level by level), and in order over the
+    windows of a periodic graph with a partial last window: the oracle's grids bit for bit."""
+    torch = torch_cuda
+    dt = np.float32 if f32 else np.float64
+    per_step = (-(-nx // ts)) * (-(-ny // ts))
+    graphs = 2 if order == "queue" else 1
+    window = 2 if order == "periodic" else steps
+    grids, recs, descs = [], [], []
+    for k in range(graphs):
+        g = O.heat_init(nx, ny, seed=60 + k).astype(dt)
+        a, b = torch.from_numpy(g).cuda(), torch.from_numpy(g).cuda()
+        r = xk.heat_access_records(nx, ny, ts, ts, 0, 6 if order == "periodic" else steps, a.data_ptr(), b.data_ptr(), esize=dt().itemsize)
+        r["task"] += k * steps * per_step
+        grids.append((g, a, b)); recs.append(r)
+        descs.append(xk.heat_task_descs((a.data_ptr(), b.data_ptr()), nx, ny, nx, ts, ts, window, C, f32=f32))
+    res = xk.Resolver(); res.add(np.concatenate(recs))
+    sch = xk.Scheduler(); sch.set_tasks(np.concatenate(descs))
+    if order == "periodic":
+        sch.run_periodic(res.periodic(2 * per_step), (steps + 1) // 2, per_step if steps % 2 else 2 * per_step)
+    else:
+        sch.run(res.graph())
+    assert sch.wait() == graphs * steps * per_step
+    for g, a, b in grids:
+        np.testing.assert_array_equal((a if steps % 2 == 0 else b).cpu().numpy(), O.heat_run(g, nx, ny, steps, C, dtype=dt))
+    sch.close(); res.close()
+
+
+@pytest.mark.parametrize("lo", [0, 1])
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 8191, 8192, 8193, 3 * 8192 + 5, 300_001])
+def test_axpby_units(torch_cuda, n, lo):
+    """One axpby task over n elements from an aligned and an unaligned start, split into pieces of
+    8192 elements: every element updated once, nothing outside the range touched."""
+    torch = torch_cuda
+    rng = np.random.default_rng(n)
+    x, y = rng.uniform(-1, 1, n + 4), rng.uniform(-1, 1, n + 4)
+    dx, dy = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    d = np.zeros(1, dtype=xk.axpby_desc_dtype())
+    d["kind"], d["x"], d["y"], d["lo"], d["hi"], d["a"], d["b"] = xk.TASK_AXPBY, dx.data_ptr(), dy.data_ptr(), lo, lo + n, 0.3, -1.7
+    res = xk.Resolver()
+    res.add(S.from_tuples([[("s", S.RW, dy.data_ptr() + 8 * lo, dy.data_ptr() + 8 * (lo + n))]]))
+    sch = xk.Scheduler(); sch.set_tasks(d); sch.run(res.graph())
+    assert sch.wait() == 1
+    y[lo:lo + n] = O.axpby(0.3, x[lo:lo + n], -1.7, y[lo:lo + n])
+    np.testing.assert_array_equal(dy.cpu().numpy(), y)

@@ -369,16 +369,17 @@ __device__ __forceinline__ void heat_strip_halo(const T * __restrict__ src, T * 
 // (first base = rx0 rounded down to a multiple of VEC) times column groups.
 template <int VEC>
 __host__ __device__ __forceinline__ void heat_tile_split(const TileBox & b, int nwarps, int64_t & rbase0,
-                                                         int & nrg, int & ncg, int64_t & cols_per)
+                                                         int & nrg, int & ncg, int & cols_per)
 {
+    // (tile sides fit 32 bits; 64-bit divisions here were a third of a small unit's time)
     rbase0 = b.rx0 - (b.rx0 % VEC);
-    const int64_t rows = b.rx1 - rbase0;
+    const uint32_t rows = (uint32_t) (b.rx1 - rbase0), cols = (uint32_t) (b.cy1 - b.cy0);
     nrg = (int) ((rows + 32 * VEC - 1) / (32 * VEC));
-    ncg = nwarps / (nrg > 0 ? nrg : 1);
-    if (ncg < 1) ncg = 1;
-    const int64_t cols = b.cy1 - b.cy0;
-    if (ncg > cols) ncg = (int) (cols > 0 ? cols : 1);
-    cols_per = (cols + ncg - 1) / ncg;
+    uint32_t n = (uint32_t) nwarps / (uint32_t) nrg;
+    if (n < 1) n = 1;
+    if (n > cols) n = cols;
+    ncg = (int) n;
+    cols_per = (int) ((cols + n - 1) / n);
 }
 
 // A team of `nwarps` warps (warp index `warp` within the team) executes one tile task: the
@@ -390,12 +391,12 @@ __device__ __forceinline__ void heat_tile_team(const T * src, T * dst, int64_t l
 {
     const TileBox b = heat_tile_box(nx, ny, x0, x1, y0, y1);
     if (b.rx0 >= b.rx1 || b.cy0 >= b.cy1) return;
-    int64_t rbase0, cols_per; int nrg, ncg;
+    int64_t rbase0; int nrg, ncg, cols_per;
     heat_tile_split<VEC>(b, nwarps, rbase0, nrg, ncg, cols_per);
     for (int s = warp; s < nrg * ncg; s += nwarps)
     {
-        const int rg = s % nrg, cg = s / nrg;
-        const int64_t cy0 = b.cy0 + cg * cols_per;
+        const int cg = (int) ((uint32_t) s / (uint32_t) nrg), rg = s - cg * nrg;
+        const int64_t cy0 = b.cy0 + (int64_t) cg * cols_per;
         int64_t cy1 = cy0 + cols_per; if (cy1 > b.cy1) cy1 = b.cy1;
         if (cy0 >= cy1) continue;
         heat_strip_halo<T, VEC, PF, CG>(src, dst, ld, nx, rbase0 + (int64_t) rg * 32 * VEC, b.rx0, b.rx1, cy0, cy1, c, vec_ok, pfd);

@@ -234,13 +234,13 @@ __device__ __forceinline__ bool heat_tile_team_bulk(const T * src, T * dst, int6
 {
     const TileBox b = heat_tile_box(nx, ny, x0, x1, y0, y1);
     if (b.rx0 >= b.rx1 || b.cy0 >= b.cy1) return true;
-    int64_t rbase0, cols_per; int nrg, ncg;
+    int64_t rbase0; int nrg, ncg, cols_per;
     heat_tile_split<VEC>(b, nwarps, rbase0, nrg, ncg, cols_per);
     bool ok = true;
     for (int s = warp; s < nrg * ncg && ok; s += nwarps)
     {
         const int rg = s % nrg, cg = s / nrg;
-        const int64_t cy0 = b.cy0 + cg * cols_per;
+        const int64_t cy0 = b.cy0 + (int64_t) cg * cols_per;
         int64_t cy1 = cy0 + cols_per; if (cy1 > b.cy1) cy1 = b.cy1;
         if (cy0 >= cy1) continue;
         ok = heat_strip_bulk<T, VEC, NBUF>(src, dst, ld, rbase0 + (int64_t) rg * 32 * VEC, b.rx0, b.rx1, cy0, cy1, c, ring, deadline);

@@ -97,20 +97,23 @@ struct XkbSrvSlot {
     const xkb_task_desc_t * tasks;       // the periodic window's `period` descriptors
     const uint32_t * succ_ptr, * succ, * xsucc_ptr, * xsucc, * npred_first, * npred_next;
     int * wc;                            // ntasks wait counters
+    int * units_done;                    // ntasks counts of the units that ended
     int * queue;                         // ntasks ready-queue slots
     const uint8_t * copy_src;            // the grid the host copied in ...
     uint8_t * copy_dst;                  //   ... duplicated here by the set-up chunks (second grid)
     uint64_t copy_bytes;
     uint32_t period, ntasks;
     uint32_t nchunks;                    // set-up chunks (wait counters, queue slots, grid copy)
+    uint32_t chunk_tasks;                // tasks whose counters one chunk sets up
     uint32_t gen;                        // admission number, reported back when the request ends
     uint32_t seed_later;                 // 1: some task of a later window has no predecessor
+    uint32_t units_log2;                 // a task is 2^units_log2 units, each run by one warp
     int32_t pfd;
 };
 // The slot's counters (device memory): state 0 idle, 1 admitted (set-up pending), 2 running,
-// 3 done; set-up chunks claimed / finished; ready-queue head and tail; tasks executed.
-// claimers: teams between their check that the slot runs (state 2) and their claim on `head`;
-// the team that ends the request waits for none to be left before the host may reuse the slot.
+// 3 done; set-up chunks claimed / finished; tickets taken (head) and tasks published (tail); tasks
+// executed. claimers: warps between their check that the slot runs (state 2) and their claim on `head`;
+// the warp that ends the request waits for none to be left before the host may reuse the slot.
 struct XkbSrvCtl { unsigned state, init_next, init_done, head, tail, executed, claimers, pad; };
 struct XkbSrvArgs {
     XkbSrvSlot * slots;
@@ -120,12 +123,17 @@ struct XkbSrvArgs {
     unsigned * status;                   // [0] first error (XKB_ETIMEDOUT), [1] tasks executed,
                                          // [2] set by the host: 1 once no request will come,
                                          //     2 to stop at once (the host gave up)
-    uint64_t run_ns;                     // how long a team may run before it gives up
+    uint64_t run_ns;                     // how long a warp may run before it gives up
     uint64_t timeout_ns;                 // longest wait for one published queue slot
 };
-// Tasks per set-up chunk of a served request, and at most this many bytes of its grid copy.
-constexpr uint32_t XKB_SRV_CHUNK = 16384;
-constexpr uint64_t XKB_SRV_COPY_CHUNK = uint64_t(256) << 10;
-// Launch the serving kernel (grid CTAs of 256 threads, warps_per_task 1, 2, 4 or 8).
-int xkb_internal_server_launch(const XkbSrvArgs & a, int grid, int warps_per_task, cudaStream_t stream);
-
+// At most this many tasks and bytes of the grid copy per set-up chunk of a served request; an idle
+// warp looks for work again after at most XKB_SRV_NAP_MAX ns.
+constexpr uint32_t XKB_SRV_CHUNK = 1024;
+constexpr uint64_t XKB_SRV_COPY_CHUNK = uint64_t(64) << 10;
+#ifndef XKB_SRV_NAP_MAX
+#define XKB_SRV_NAP_MAX 2048
+#endif
+// Launch the serving kernel (grid CTAs of 256 threads).
+int xkb_internal_server_launch(const XkbSrvArgs & a, int grid, cudaStream_t stream);
+// log2 of the units heat tile tasks are split into when `width` of them run side by side on `warps` warps.
+int xkb_internal_split_log2(uint64_t width, uint64_t warps);

@@ -6,13 +6,18 @@
 // completion decrements each successor's counter, queueing those that reach 0
 // (src/task.cc:160-247).
 //
-//  * PERSISTENT: one kernel, one CTA per resident slot. CTA thread 0 takes the next queue
-//    slot (atomicAdd on head) and waits, with a time limit, for a task id to be published
-//    there; the CTA runs the built-in tile body; after a fence and a barrier, warp 0 decrements
-//    the successors' counters with acq_rel atomics and publishes every successor that reaches
-//    zero with a release store. Every queue slot is written exactly once (a task is pushed
-//    once), so the queue is a plain array of ntasks slots. Tile data written inside the kernel
-//    is read back with L1-bypassing loads.
+//  * PERSISTENT: one kernel whose warps are the workers. A task is split into 2^k UNITS (column
+//    slabs of a heat tile, pieces of an axpby range; k is fixed for a run, see split_log2). A
+//    warp takes the next ticket (atomicAdd on head): unit (ticket mod 2^k) of task number
+//    (ticket / 2^k). Two orders, chosen on the device before the run (sched_plan_kernel):
+//      - IN ORDER, for graphs spawned level by level (the heat graphs): tasks are taken in spawn
+//        order; a warp waits, with a time limit, for its task's counter of unfinished
+//        predecessor units, runs the unit and decrements the successors' counters.
+//      - QUEUE, for any graph: tasks are taken in the order they became ready. A warp waits for
+//        a task id to be published in its queue slot; the warp that ends a task's last unit
+//        decrements the successors' counters and publishes those that reach zero. Every slot
+//        is written once (a task is pushed once): a plain array of ntasks slots.
+//    Tile data written inside the kernel is read back with L1-bypassing loads.
 //  * PLAIN: the host launches one kernel per task in spawn order (a topological order) on one
 //    stream -- the reference's one-launch-per-task device path.
 //  * GRAPH: the task graph becomes a CUDA graph (one kernel node per task, one edge per
@@ -49,7 +54,23 @@ __device__ __forceinline__ void axpby_team(int64_t lo, int64_t hi, double a, con
     const int64_t nv = (hi - head) / 2;
     const double2 * xv = (const double2 *) (x + head);
     double2 * yv = (double2 *) (y + head);
-    for (int64_t v = tid; v < nv; v += nth)
+    // Four vectors of each operand in flight per lane: with one (32 bytes per lane, 16 KB per SM
+    // at 16 warps) a team waited out a DRAM round trip per step of the loop.
+    int64_t v = tid;
+    for (; v + 3 * nth < nv; v += 4 * nth)
+    {
+        double2 xx[4], yy[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+        {
+            xx[k] = CG ? __ldcg(xv + v + k * nth) : __ldg(xv + v + k * nth);
+            yy[k] = CG ? __ldcg(yv + v + k * nth) : yv[v + k * nth];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            yv[v + k * nth] = make_double2(axpby1<CG>(a, xx[k].x, b, yy[k].x), axpby1<CG>(a, xx[k].y, b, yy[k].y));
+    }
+    for (; v < nv; v += nth)
     {
         const double2 xx = CG ? __ldcg(xv + v) : __ldg(xv + v);
         const double2 yy = CG ? __ldcg(yv + v) : yv[v];
@@ -60,6 +81,9 @@ __device__ __forceinline__ void axpby_team(int64_t lo, int64_t hi, double a, con
 }
 
 constexpr int SCHED_THREADS = 256;
+// log2 of the units of one task that the warps of one CTA run together (team runs).
+constexpr int TEAM_LOG2 = 3;
+static_assert((1 << TEAM_LOG2) * 32 == SCHED_THREADS, "a team is a CTA");
 
 constexpr int SCHED_BULK_NBUF = 8;       // staged columns in flight per warp (bulk tile body)
 #ifndef XKB_TILE_PF
@@ -74,36 +98,53 @@ constexpr int SCHED_BULK_NBUF = 8;       // staged columns in flight per warp (b
 #ifndef XKB_SCHED_MINB
 #define XKB_SCHED_MINB 2                 // persistent CTAs resident per SM (register budget)
 #endif
+constexpr unsigned SCHED_POLL_NS = 100;  // between two looks at a counter or slot (20 or 200: within 1 %)
 constexpr int SCHED_PFD_DEFAULT = 4;     // L2 prefetch distance of heat tiles in columns (3-5 measured best)
 constexpr double SCHED_TIMEOUT_MAX_S = 3600.0;   // longest device wait a caller may ask for
 
 // A device wait limit in seconds is usable when finite, positive and at most an hour.
 static inline bool timeout_ok(double s) { return std::isfinite(s) && s > 0 && s <= SCHED_TIMEOUT_MAX_S; }
 
-// Run one task with a team of `nwarps` warps; `warp` is the warp's index in the team.
-__device__ __forceinline__ void run_task_team(const xkb_task_desc_t & d, int warp, int nwarps, int pfd)
+constexpr int TEAM_PF = 4;               // columns a strip of a team run loads ahead: its units are 4 to 16 columns wide
+// Piece of an axpby range that unit `unit` of `nunits` runs: contiguous, a multiple of
+// AXPBY_PIECE elements (so every piece keeps the range's alignment phase; the last one ends the
+// range), empty for the units a short range does not need.
+constexpr int64_t AXPBY_PIECE = 8192;    // 192 KiB of traffic: 30 us for one warp of a full device
+__device__ __forceinline__ void axpby_piece(int64_t lo, int64_t hi, int unit, int nunits, int64_t & plo, int64_t & phi)
+{
+    const int64_t pieces = (hi - lo + AXPBY_PIECE - 1) / AXPBY_PIECE;
+    const int64_t per = (pieces + nunits - 1) / nunits * AXPBY_PIECE;
+    plo = lo + unit * per;
+    phi = plo + per < hi ? plo + per : hi;
+}
+
+// Run unit `unit` of the `nunits` (a power of two) a task is split into, with one warp. PF64, PF32:
+// columns a heat strip loads ahead into registers.
+template <int PF64, int PF32>
+__device__ __forceinline__ void run_unit(const xkb_task_desc_t & d, int unit, int nunits, int pfd)
 {
     switch (d.kind)
     {
         case XKB_TASK_HEAT_F64: {
             const auto & h = d.u.heat;
             const bool vok = (h.ld % 2 == 0) && (h.src % 16 == 0) && (h.dst % 16 == 0);
-            heat_tile_team<double, XKB_F64_VEC, XKB_F64_PF, true>((const double *) h.src, (double *) h.dst, h.ld, h.nx, h.ny,
-                                               h.x0, h.x1, h.y0, h.y1, h.c, vok, pfd, warp, nwarps);
+            heat_tile_team<double, XKB_F64_VEC, PF64, true>((const double *) h.src, (double *) h.dst, h.ld, h.nx, h.ny,
+                                               h.x0, h.x1, h.y0, h.y1, h.c, vok, pfd, unit, nunits);
             break;
         }
         case XKB_TASK_HEAT_F32: {
             const auto & h = d.u.heat;
             const bool vok = (h.ld % 4 == 0) && (h.src % 16 == 0) && (h.dst % 16 == 0);
             // an FP32 column is half the bytes of an FP64 one: prefetch twice as many columns ahead
-            heat_tile_team<float, 4, XKB_TILE_PF, true>((const float *) h.src, (float *) h.dst, h.ld, h.nx, h.ny,
-                                              h.x0, h.x1, h.y0, h.y1, h.c, vok, 2 * pfd, warp, nwarps);
+            heat_tile_team<float, 4, PF32, true>((const float *) h.src, (float *) h.dst, h.ld, h.nx, h.ny,
+                                              h.x0, h.x1, h.y0, h.y1, h.c, vok, 2 * pfd, unit, nunits);
             break;
         }
         case XKB_TASK_AXPBY: {
             const auto & a = d.u.axpby;
-            axpby_team<true>(a.lo, a.hi, a.a, (const double *) a.x, a.b, (double *) a.y,
-                             (int64_t) warp * 32 + (threadIdx.x & 31), (int64_t) nwarps * 32);
+            int64_t lo, hi;
+            axpby_piece(a.lo, a.hi, unit, nunits, lo, hi);
+            axpby_team<true>(lo, hi, a.a, (const double *) a.x, a.b, (double *) a.y, threadIdx.x & 31, 32);
             break;
         }
         default: break;   // XKB_TASK_NOOP (first-touch / placement tasks)
@@ -116,6 +157,13 @@ __device__ __forceinline__ int atom_add_acq_rel(int * p, int v)
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
     return old;
 }
+
+// Counters of a run (device memory): ready-queue tickets and tasks published, status, tasks
+// executed; then what the seed kernel learnt about the tasks that are ready at the start.
+// Head and tail have cache lines of their own: every warp's ticket and every release is an atomic there.
+// CTR_EXECUTED counts units of an in-order run, tasks of a queue run (executed_tasks).
+enum { CTR_HEAD = 0, CTR_TAIL = 32, CTR_STATUS = 48, CTR_EXECUTED, CTR_BAD_TASK, CTR_SEEDS, CTR_SEED_LAST, CTR_SEED_DEG, CTR_SEED_PIECES,
+       CTR_SEED_HEAT, CTR_QUEUE, CTR_SPLIT, CTR_TEAM, CTR_COUNT = 64 };
 
 // A run covers `ntasks` tasks numbered w * period + t (window w, task t of the window's
 // `period` descriptors). A plain graph is one window (period = ntasks); a periodic graph adds
@@ -130,11 +178,14 @@ struct SchedArgs {
     const uint32_t * xsucc;
     const uint32_t * npred_first;
     const uint32_t * npred_next;
-    int * wc;
+    int * wc;                  // wait counters
+    int * units_done;          // units of each task that ended (null: tasks are not split)
     int * queue;
-    unsigned * ctr;            // [0] head, [1] tail, [2] status, [3] executed
+    unsigned * ctr;            // CTR_*
     uint64_t timeout_ns;
     int pfd;                   // L2 prefetch distance of the tile bodies, in columns
+    int allow_team;            // narrow graphs may go to sched_team_kernel
+    int min_units;             // the caller's warps per task (xkb_sched_set_team): at least this many units
 };
 
 __global__ void sched_init_kernel(SchedArgs a)
@@ -142,6 +193,7 @@ __global__ void sched_init_kernel(SchedArgs a)
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= a.ntasks) return;
     a.queue[t] = -1;
+    if (a.units_done) a.units_done[t] = 0;
     const uint32_t w = t / a.period, l = t - w * a.period;
     a.wc[t] = (int) (w == 0 ? a.npred_first[l] : a.npred_next[l]);
 }
@@ -149,24 +201,256 @@ __global__ void sched_init_kernel(SchedArgs a)
 __global__ void sched_seed_kernel(SchedArgs a)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= a.ntasks) return;
-    if (*(volatile unsigned *) (a.ctr + 2) != 0) return;   // a check before the run failed: nothing becomes ready
+    const uint32_t lane = threadIdx.x & 31;
+    const bool ok = *(volatile unsigned *) (a.ctr + CTR_STATUS) == 0;   // a check before the run failed: nothing becomes ready
     const uint32_t w = t / a.period, l = t - w * a.period;
-    if ((w == 0 ? a.npred_first[l] : a.npred_next[l]) != 0) return;
-    const unsigned pos = atomicAdd(a.ctr + 1, 1u);
-    a.queue[pos] = (int) t;
+    const bool seed = ok && t < a.ntasks && (w == 0 ? a.npred_first[l] : a.npred_next[l]) == 0;
+    const unsigned m = __ballot_sync(0xffffffffu, seed);
+    if (!m) return;
+    unsigned deg = 0, pieces = 0;
+    bool heat = false;
+    if (seed)
+    {
+        deg = min(a.succ_ptr[l + 1] - a.succ_ptr[l], 1u << 16);
+        const xkb_task_desc_t & d = a.tasks[l];
+        heat = d.kind == XKB_TASK_HEAT_F64 || d.kind == XKB_TASK_HEAT_F32;
+        if (d.kind == XKB_TASK_AXPBY) pieces = (unsigned) min((d.u.axpby.hi - d.u.axpby.lo + AXPBY_PIECE - 1) / AXPBY_PIECE, (int64_t) 4096);
+    }
+    deg = __reduce_add_sync(0xffffffffu, deg);
+    pieces = __reduce_add_sync(0xffffffffu, pieces);
+    const unsigned last = __reduce_max_sync(0xffffffffu, seed ? t + 1 : 0u);
+    const unsigned nheat = __popc(__ballot_sync(0xffffffffu, heat));
+    unsigned pos = 0;
+    if (lane == 0)
+    {
+        pos = atomicAdd(a.ctr + CTR_TAIL, (unsigned) __popc(m));
+        atomicAdd(a.ctr + CTR_SEEDS, (unsigned) __popc(m));
+        atomicMax(a.ctr + CTR_SEED_LAST, last);
+        if (deg) atomicAdd(a.ctr + CTR_SEED_DEG, deg);
+        if (pieces) atomicAdd(a.ctr + CTR_SEED_PIECES, pieces);
+        if (nheat) atomicAdd(a.ctr + CTR_SEED_HEAT, nheat);
+    }
+    pos = __shfl_sync(0xffffffffu, pos, 0);
+    if (seed) a.queue[pos + __popc(m & ((1u << lane) - 1))] = (int) t;
 }
 
-__device__ __forceinline__ void team_sync(int id, int nthreads)
+// log2 of the units a run's tasks are split into, from `width` = how many tasks the graph runs side
+// by side, `heat` whether they are heat tiles, `pieces` the mean number of AXPBY_PIECE pieces per
+// task, `warps` the run's workers, and the caller's least.
+//  * heat tiles, few: as many units as there are warps, 32 at most (128^2 FP64 tiles, us per step:
+//    64 tiles, 32 units of 4 columns 5.4, 16 units 7.6, one warp per tile 59; 256 tiles, 8 units
+//    12.3, one warp 62);
+//  * heat tiles, more than an eighth of the warps: up to two units per warp, 8 per tile at most, as
+//    a warp alone does not keep its memory requests in flight (576 tiles: 28.5 with 8 units, 40.5
+//    with 4, 70 with one; 1024 tiles: 45.3 with 4, 49.3 with 2, 49.7 with 8); a tile per warp or
+//    more is not split (4096 tiles: 174 with one or two units);
+//  * axpby: units of about AXPBY_PIECE elements, twice as many as the mean task needs, so that the
+//    largest chunk of a mixed graph spreads too (10 passes over 2^26 elements in chunks of 64 KiB
+//    to 16 MiB: 2.5 ms against 142 ms with one warp per chunk).
+constexpr int SPLIT_MAX_HEAT = 5, SPLIT_MAX = 8;
+__host__ __device__ __forceinline__ int split_log2(unsigned width, bool heat, unsigned pieces, unsigned warps, int min_units)
 {
-    if (nthreads == SCHED_THREADS) __syncthreads();
-    else asm volatile("bar.sync %0, %1;" :: "r"(id), "r"(nthreads) : "memory");
+    int k = 0;
+    if (heat)
+    {
+        while (k < SPLIT_MAX_HEAT && ((uint64_t) width << (k + 1)) <= warps) ++k;
+        if (k < TEAM_LOG2) while (k < TEAM_LOG2 && ((uint64_t) width << (k + 1)) <= 2 * (uint64_t) warps) ++k;
+    }
+    if (pieces > 1)
+    {
+        int q = 0;
+        while (q < SPLIT_MAX && (1u << q) < 2 * pieces) ++q;
+        if (q > k) k = q;
+    }
+    while ((1 << k) < min_units) ++k;
+    return k;
 }
 
-// Each CTA holds 8 / TEAM_WARPS independent TEAMS of TEAM_WARPS warps. A team's first
-// thread takes the next queue slot and waits for it; the team runs the task, fences, syncs
-// on its own named barrier, and its first warp releases the successors. Teams never wait for
-// one another, so while one team takes or releases a task the others keep HBM busy.
+// The split of a run, from the seed kernel's counters. The width is the number of tasks ready at the
+// start, or what those release if that is more (a graph with one root and a wide second level; a
+// tile task has about eight successors that each wait for as many tasks).
+__device__ __forceinline__ int run_split_log2(const SchedArgs & a, unsigned warps)
+{
+    if (!a.units_done) return 0;
+    const unsigned seeds = a.ctr[CTR_SEEDS], deg = a.ctr[CTR_SEED_DEG];
+    const unsigned pieces = seeds ? (a.ctr[CTR_SEED_PIECES] + seeds - 1) / seeds : 0;
+    int k = split_log2(max(seeds, deg / 8), a.ctr[CTR_SEED_HEAT] > 0, pieces, warps, a.min_units);
+    while (k > 0 && ((uint64_t) a.ntasks << k) > 0xf0000000ull) --k;      // tickets are 32-bit
+    return k;
+}
+
+// Chooses the order of the run. Let W be the number of tasks ready at the start. The run goes in
+// order when those are tasks 0 .. W-1 and every edge leads from one block of W consecutive tasks to
+// a later one: then the tasks of a block are independent of one another, so taking them in spawn
+// order keeps W tasks runnable at a time and no warp waits behind a task that a later one could have
+// overtaken by more than a block. (A chain spawned before the next chain fails the test and takes
+// the queue.) In order, nothing is published, a warp knows its task -- descriptor and successors --
+// before it may run, and every unit decrements its successors itself, without waiting for the
+// answer: 15.6 us per step of the 2048^2 FP64 graph against 19.6 through the queue with the same
+// units, and 174 against 180 for 8192^2.
+// In order, a counter starts at the task's number of predecessors n and every one of their 2^k units
+// takes one off, so the task may run at n - n * 2^k.
+constexpr unsigned INORDER_MAX_NPRED = 1u << 20;      // keeps that inside an int
+
+__global__ void sched_plan_kernel(SchedArgs a, unsigned warps)
+{
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= a.period) return;
+    if (t == 0)
+    {
+        const int k = run_split_log2(a, warps);
+        a.ctr[CTR_SPLIT] = (unsigned) k;
+        a.ctr[CTR_TEAM] = a.allow_team && a.ctr[CTR_SEED_HEAT] > 0 && a.ctr[CTR_SEED_PIECES] == 0 && k >= TEAM_LOG2 &&
+                          ((uint64_t) a.ctr[CTR_SEEDS] << k) <= warps;
+    }
+    const uint32_t W = a.ctr[CTR_SEEDS];
+    bool ok = W > 0 && a.ctr[CTR_SEED_LAST] == W && (a.xsucc_ptr == nullptr || a.period % W == 0);
+    if (ok)
+    {
+        ok = a.npred_first[t] < INORDER_MAX_NPRED && a.npred_next[t] < INORDER_MAX_NPRED;
+        for (uint32_t i = a.succ_ptr[t], e = a.succ_ptr[t + 1], b = t / W; i < e; ++i) ok = ok && a.succ[i] / W > b;
+    }
+    if (!ok && *(volatile unsigned *) (a.ctr + CTR_QUEUE) == 0) atomicExch(a.ctr + CTR_QUEUE, 1u);
+}
+
+// Whether sched_team_kernel has the run.
+__device__ __forceinline__ bool team_run(const SchedArgs & a) { return a.ctr[CTR_TEAM] != 0 && a.ctr[CTR_QUEUE] == 0; }
+
+// Tasks run, from the counters of a run that ended.
+__host__ __device__ __forceinline__ unsigned executed_tasks(const unsigned * ctr)
+{
+    return ctr[CTR_QUEUE] ? ctr[CTR_EXECUTED] : ctr[CTR_EXECUTED] >> ctr[CTR_SPLIT];
+}
+
+__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+__device__ __forceinline__ int atom_add_relaxed(int * p, int v)
+{
+    int old;
+    asm volatile("atom.relaxed.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    return old;
+}
+
+__device__ __forceinline__ void red_add_relaxed(int * p, int v)
+{
+    asm volatile("red.relaxed.gpu.global.add.s32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
+}
+
+// The successor graph of a run (see SchedArgs) and the entry i of a task's successors: those of
+// its own window, then those of the next window. A successor at or beyond ntasks -- past the tail of
+// the last window -- is not part of the run.
+struct SuccGraph {
+    const uint32_t * succ_ptr, * succ, * xsucc_ptr, * xsucc;
+    uint32_t period, ntasks;
+
+    __device__ __forceinline__ uint32_t count(uint32_t l) const
+    {
+        return succ_ptr[l + 1] - succ_ptr[l] + (xsucc_ptr ? xsucc_ptr[l + 1] - xsucc_ptr[l] : 0u);
+    }
+    __device__ __forceinline__ uint32_t entry(uint32_t l, uint32_t base, uint32_t i) const
+    {
+        const uint32_t b = succ_ptr[l], n = succ_ptr[l + 1] - b;
+        return i < n ? base + succ[b + i] : base + period + xsucc[xsucc_ptr[l] + i - n];
+    }
+    // the lane's entry, loaded ahead (almost every task has at most 32 successors)
+    __device__ __forceinline__ uint32_t first(uint32_t l, uint32_t base, int lane, bool & more) const
+    {
+        const uint32_t n = count(l);
+        more = n > 32;
+        return (uint32_t) lane < n ? entry(l, base, (uint32_t) lane) : 0xffffffffu;
+    }
+};
+
+// One warp, after task t's last unit: decrement the successors' counters and publish those that
+// became ready. The caller's fence orders the task's writes before the counters; the fence here, the
+// writes of the other predecessors before the queue slot.
+__device__ __forceinline__ void release_successors(const SuccGraph & g, uint32_t t, uint32_t first, bool more, int * wc, int * queue,
+                                                   unsigned * tail, int lane)
+{
+    for (uint32_t i0 = 0;; i0 += 32)
+    {
+        uint32_t s = first;
+        if (i0)
+        {
+            const uint32_t w = t / g.period, l = t - w * g.period, n = g.count(l);
+            if (i0 >= n) break;
+            s = i0 + lane < n ? g.entry(l, w * g.period, i0 + lane) : 0xffffffffu;
+        }
+        const bool ready = s < g.ntasks && atom_add_relaxed(wc + s, -1) == 1;
+        const unsigned m = __ballot_sync(0xffffffffu, ready);
+        if (m)
+        {
+            if (ready) fence_acq_rel_gpu();
+            unsigned pos = 0;
+            if (lane == 0) pos = atomicAdd(tail, (unsigned) __popc(m));
+            pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(m & ((1u << lane) - 1));
+            if (ready) asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" :: "l"(queue + pos), "r"((int) s) : "memory");
+        }
+        if (!more) break;
+    }
+}
+
+// One warp, after a unit of task t of an in-order run.
+__device__ __forceinline__ void count_down_successors(const SuccGraph & g, uint32_t t, uint32_t first, bool more, int * wc, int lane)
+{
+    if (first < g.ntasks) red_add_relaxed(wc + first, -1);
+    if (!more) return;
+    const uint32_t w = t / g.period, l = t - w * g.period, n = g.count(l);
+    for (uint32_t i = 32 + lane; i < n; i += 32)
+    {
+        const uint32_t s = g.entry(l, w * g.period, i);
+        if (s < g.ntasks) red_add_relaxed(wc + s, -1);
+    }
+}
+
+// 64-byte descriptor as four independent 16-byte loads
+__device__ __forceinline__ xkb_task_desc_t load_desc(const xkb_task_desc_t * p)
+{
+    static_assert(sizeof(xkb_task_desc_t) == 64, "descriptor size");
+    union { int4 v[4]; xkb_task_desc_t d; } q;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q.v[k] = __ldg((const int4 *) p + k);
+    return q.d;
+}
+
+// Wait (one lane) until *p <= target, polling with acquire loads; false when the time limit ran out
+// here or anywhere (the status word, looked at now and then).
+__device__ __forceinline__ bool wait_at_most(const int * p, int target, unsigned * status, uint64_t timeout_ns)
+{
+    if (xkb_ld_acquire(p) <= target) return true;
+    const uint64_t t0 = xkb_globaltimer();
+    for (uint32_t spins = 1;; ++spins)
+    {
+        __nanosleep(SCHED_POLL_NS);
+        if (xkb_ld_acquire(p) <= target) return true;
+        if ((spins & 63) == 0)
+        {
+            if (*(volatile unsigned *) status != 0) return false;
+            if (xkb_globaltimer() - t0 > timeout_ns) { atomicCAS(status, 0u, (unsigned) -XKB_ETIMEDOUT); return false; }
+        }
+    }
+}
+
+// Wait (one lane) until queue slot *p holds a task id; -1 when the time limit ran out.
+__device__ __forceinline__ int wait_published(const int * p, unsigned * status, uint64_t timeout_ns)
+{
+    int t = xkb_ld_acquire(p);
+    if (t >= 0) return t;
+    const uint64_t t0 = xkb_globaltimer();
+    for (uint32_t spins = 1;; ++spins)
+    {
+        __nanosleep(SCHED_POLL_NS);
+        if ((t = xkb_ld_acquire(p)) >= 0) return t;
+        if ((spins & 63) == 0)
+        {
+            if (*(volatile unsigned *) status != 0) return -1;
+            if (xkb_globaltimer() - t0 > timeout_ns) { atomicCAS(status, 0u, (unsigned) -XKB_ETIMEDOUT); return -1; }
+        }
+    }
+}
+
+// Warps never wait for one another except through the counters or the queue, so while one takes or
+// releases a task the others keep HBM busy.
 //
 // BULK: heat tiles whose layout allows it run the bulk-staged body (heat_bulk.cuh): each warp
 // streams its strips' columns through its own ring of shared-memory slots; other tasks run the
@@ -174,17 +458,15 @@ __device__ __forceinline__ void team_sync(int id, int nthreads)
 // Dynamic shared memory of the BULK variant with NBUF slots per warp: the slots, then the mbarriers.
 constexpr size_t bulk_smem_bytes(int nbuf) { return (size_t) (SCHED_THREADS / 32) * nbuf * (BULK_SLOT_BYTES + 8); }
 
-template <int TEAM_WARPS, bool BULK = false, int NBUF = SCHED_BULK_NBUF>
+template <bool BULK, int NBUF = SCHED_BULK_NBUF>
 __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_persistent_kernel(SchedArgs a)
 {
-    constexpr int NTEAMS = (SCHED_THREADS / 32) / TEAM_WARPS;
-    constexpr int TEAM_THREADS = TEAM_WARPS * 32;
     constexpr int NWARPS = SCHED_THREADS / 32;
-    __shared__ int cur[NTEAMS];
     extern __shared__ __align__(128) unsigned char bulk_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int team = warp / TEAM_WARPS, twarp = warp % TEAM_WARPS;
-    const int bar = 1 + team;
+    const bool inorder = a.ctr[CTR_QUEUE] == 0;
+    const int k = (int) a.ctr[CTR_SPLIT];
+    const int nunits = 1 << k;
     unsigned executed = 0;
     BulkRing<NBUF> ring;
     if constexpr (BULK)
@@ -193,92 +475,136 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_persisten
         ring.bars = (uint64_t *) (bulk_smem + (size_t) NWARPS * NBUF * BULK_SLOT_BYTES) + warp * NBUF;
         bulk_ring_init(ring);
     }
+    // (a check before the run that failed left its status: nothing runs)
+    if (team_run(a) || *(volatile unsigned *) (a.ctr + CTR_STATUS) != 0) return;
+    unsigned ticket = 0;
+    if (lane == 0) ticket = atomicAdd(a.ctr + CTR_HEAD, 1u);
     for (;;)
     {
-        if (twarp == 0 && lane == 0)
+        ticket = __shfl_sync(0xffffffffu, ticket, 0);
+        const uint32_t slot = ticket >> k;
+        const int unit = (int) (ticket & (nunits - 1));
+        if (slot >= a.ntasks) break;
+        int t = (int) slot;
+        if (!inorder)
         {
-            int t = -1;
-            const unsigned slot = atomicAdd(a.ctr + 0, 1u);
-            if (slot < a.ntasks)
-            {
-                const uint64_t t0 = xkb_globaltimer();
-                uint32_t spins = 0;
-                while ((t = xkb_ld_acquire(a.queue + slot)) < 0)
-                {
-                    if (*(volatile unsigned *) (a.ctr + 2) != 0) { t = -2; break; }   // another team gave up
-                    if ((++spins & 63) == 0 && xkb_globaltimer() - t0 > a.timeout_ns)
-                    {
-                        atomicCAS(a.ctr + 2, 0u, (unsigned) -XKB_ETIMEDOUT);
-                        t = -2;
-                        break;
-                    }
-                    __nanosleep(64);
-                }
-            }
-            cur[team] = t;
+            if (lane == 0) t = wait_published(a.queue + slot, a.ctr + CTR_STATUS, a.timeout_ns);
+            t = __shfl_sync(0xffffffffu, t, 0);
+            if (t < 0) break;
         }
-        team_sync(bar, TEAM_THREADS);
-        const int t = cur[team];
-        if (t < 0) break;
         const uint32_t w = (uint32_t) t / a.period, l = (uint32_t) t - w * a.period;
+        const xkb_task_desc_t d = load_desc(a.tasks + l);
+        const SuccGraph g{a.succ_ptr, a.succ, a.xsucc_ptr, a.xsucc, a.period, a.ntasks};
+        bool more;
+        const uint32_t first = g.first(l, w * a.period, lane, more);
+        if (inorder)
+        {
+            int ok = 1;
+            if (lane == 0)
+            {
+                const int np = (int) (w == 0 ? a.npred_first[l] : a.npred_next[l]);
+                ok = wait_at_most(a.wc + t, np - np * nunits, a.ctr + CTR_STATUS, a.timeout_ns);
+            }
+            if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+        }
+        __syncwarp();
         if constexpr (BULK)
         {
-            const xkb_task_desc_t & d = a.tasks[l];
             const auto & h = d.u.heat;
             // once a wait has run out anywhere, the remaining tasks are passed over quickly
-            bool done = *(volatile unsigned *) (a.ctr + 2) != 0;
+            bool done = *(volatile unsigned *) (a.ctr + CTR_STATUS) != 0;
             if (d.kind == XKB_TASK_HEAT_F64 && bulk_ok<double, 2>((const double *) h.src, h.ld, h.nx) && h.dst % 16 == 0)
             {
                 done = true;
                 if (!heat_tile_team_bulk<double, 2, NBUF>((const double *) h.src, (double *) h.dst, h.ld, h.nx, h.ny, h.x0, h.x1,
-                                                          h.y0, h.y1, h.c, twarp, TEAM_WARPS, ring, xkb_globaltimer() + a.timeout_ns))
-                    atomicCAS(a.ctr + 2, 0u, (unsigned) -XKB_ETIMEDOUT);
+                                                          h.y0, h.y1, h.c, unit, nunits, ring, xkb_globaltimer() + a.timeout_ns))
+                    atomicCAS(a.ctr + CTR_STATUS, 0u, (unsigned) -XKB_ETIMEDOUT);
             }
             else if (d.kind == XKB_TASK_HEAT_F32 && bulk_ok<float, 4>((const float *) h.src, h.ld, h.nx) && h.dst % 16 == 0)
             {
                 done = true;
                 if (!heat_tile_team_bulk<float, 4, NBUF>((const float *) h.src, (float *) h.dst, h.ld, h.nx, h.ny, h.x0, h.x1,
-                                                         h.y0, h.y1, h.c, twarp, TEAM_WARPS, ring, xkb_globaltimer() + a.timeout_ns))
-                    atomicCAS(a.ctr + 2, 0u, (unsigned) -XKB_ETIMEDOUT);
+                                                         h.y0, h.y1, h.c, unit, nunits, ring, xkb_globaltimer() + a.timeout_ns))
+                    atomicCAS(a.ctr + CTR_STATUS, 0u, (unsigned) -XKB_ETIMEDOUT);
             }
-            if (!done) run_task_team(d, twarp, TEAM_WARPS, a.pfd);
+            if (!done) run_unit<XKB_F64_PF, XKB_TILE_PF>(d, unit, nunits, a.pfd);
         }
         else
-            run_task_team(a.tasks[l], twarp, TEAM_WARPS, a.pfd);
-        __threadfence();
-        team_sync(bar, TEAM_THREADS);
-        if (twarp == 0)
+            run_unit<XKB_F64_PF, XKB_TILE_PF>(d, unit, nunits, a.pfd);
+        // the next ticket arrives while the fence waits for the unit's stores
+        if (lane == 0) ticket = atomicAdd(a.ctr + CTR_HEAD, 1u);
+        __syncwarp();
+        fence_acq_rel_gpu();
+        if (inorder) count_down_successors(g, (uint32_t) t, first, more, a.wc, lane);
+        else
         {
-            const uint32_t base = w * a.period;
-            const uint32_t b = a.succ_ptr[l], e = a.succ_ptr[l + 1];
-            for (uint32_t i = b + lane; i < e; i += 32)
+            if (k > 0)
             {
-                const uint32_t s = base + a.succ[i];
-                if (s >= a.ntasks) continue;                 // beyond the tail of the last window
-                if (atom_add_acq_rel(a.wc + s, -1) == 1)
+                int last = 0;
+                if (lane == 0)
                 {
-                    const unsigned pos = atomicAdd(a.ctr + 1, 1u);
-                    xkb_st_release(a.queue + pos, (int) s);
+                    last = atom_add_relaxed(a.units_done + t, 1) == nunits - 1;
+                    fence_acq_rel_gpu();
                 }
+                if (!__shfl_sync(0xffffffffu, last, 0)) continue;
+                __syncwarp();
             }
-            if (a.xsucc_ptr)
-            {
-                const uint32_t xb = a.xsucc_ptr[l], xe = a.xsucc_ptr[l + 1];
-                for (uint32_t i = xb + lane; i < xe; i += 32)
-                {
-                    const uint32_t s = base + a.period + a.xsucc[i];
-                    if (s >= a.ntasks) continue;
-                    if (atom_add_acq_rel(a.wc + s, -1) == 1)
-                    {
-                        const unsigned pos = atomicAdd(a.ctr + 1, 1u);
-                        xkb_st_release(a.queue + pos, (int) s);
-                    }
-                }
-            }
-            ++executed;
+            release_successors(g, (uint32_t) t, first, more, a.wc, a.queue, a.ctr + CTR_TAIL, lane);
         }
+        ++executed;
     }
-    if (twarp == 0 && lane == 0 && executed) atomicAdd(a.ctr + 3, executed);
+    if (lane == 0 && executed) atomicAdd(a.ctr + CTR_EXECUTED, executed);
+}
+
+// In-order runs of narrow heat graphs: the 8 warps of a CTA run 8 units of one task together. One
+// thread takes the group's ticket and waits for the task's counter, one barrier before and one after
+// the units, one fence and one round of counter updates for the group: an eighth of the polling,
+// tickets and counter updates of one warp per unit, whose atomics are what bounds a step of a few
+// microseconds (1024^2 FP64, 64 tiles of 32 units: 5.4 us per step against 11.2). Every run launches
+// both kernels, and the one that does not have it returns at once.
+__global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_team_kernel(SchedArgs a)
+{
+    constexpr int NWARPS = SCHED_THREADS / 32;
+    if (!team_run(a) || *(volatile unsigned *) (a.ctr + CTR_STATUS) != 0) return;
+    __shared__ unsigned next_ticket;
+    __shared__ int ready;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k = (int) a.ctr[CTR_SPLIT];
+    const int nunits = 1 << k;
+    const SuccGraph g{a.succ_ptr, a.succ, a.xsucc_ptr, a.xsucc, a.period, a.ntasks};
+    unsigned executed = 0;
+    if (threadIdx.x == 0) next_ticket = atomicAdd(a.ctr + CTR_HEAD, (unsigned) NWARPS);
+    for (;;)
+    {
+        __syncthreads();                                       // the group's ticket
+        const unsigned ticket = next_ticket;
+        const uint32_t t = ticket >> k;
+        const int unit = (int) (ticket & (nunits - 1)) + warp;
+        if (t >= a.ntasks) break;
+        const uint32_t w = t / a.period, l = t - w * a.period;
+        const xkb_task_desc_t d = load_desc(a.tasks + l);
+        uint32_t first = 0xffffffffu;
+        bool more = false;
+        if (warp == 0)
+        {
+            first = g.first(l, w * a.period, lane, more);
+            if (lane == 0)
+            {
+                const int np = (int) (w == 0 ? a.npred_first[l] : a.npred_next[l]);
+                ready = wait_at_most(a.wc + t, np - np * (nunits / NWARPS), a.ctr + CTR_STATUS, a.timeout_ns);
+            }
+        }
+        __syncthreads();
+        if (!ready) break;
+        run_unit<TEAM_PF, TEAM_PF>(d, unit, nunits, 0);
+        __syncthreads();                                       // the group's units are done
+        ++executed;
+        if (warp != 0) continue;
+        if (lane == 0) next_ticket = atomicAdd(a.ctr + CTR_HEAD, (unsigned) NWARPS);
+        fence_acq_rel_gpu();
+        count_down_successors(g, t, first, more, a.wc, lane);
+    }
+    if (lane == 0 && executed) atomicAdd(a.ctr + CTR_EXECUTED, executed);
 }
 
 // per-task kernels (PLAIN and GRAPH forms)
@@ -350,7 +676,7 @@ struct xkb_sched {
     std::vector<xkb_task_desc_t> host_tasks;  // host copy for the per-task forms (empty: device only)
     size_t ntasks = 0;                        // descriptors set
     Dev<xkb_task_desc_t> tasks;
-    Dev<int> wc, queue;
+    Dev<int> wc, queue;                       // wc: wait counters, then the units done of each task
     Dev<unsigned> ctr;
     Dev<unsigned long long> wsum;             // windows run without waiting: [0] first status, [1] executed
     cudaGraphExec_t gexec = nullptr;
@@ -358,7 +684,7 @@ struct xkb_sched {
     const void * graph_key = nullptr;
     int last_form = -1;
     int grid = 0;
-    int team_warps = 1;                       // one warp per 128-row tile (FP64 and FP32 bodies)
+    int team_warps = 1;                       // at least this many units (warps) per task
     int bulk = 0;                             // 1: bulk-staged heat tile body (measured slower; opt-in)
     int pfd = SCHED_PFD_DEFAULT;              // L2 prefetch distance in columns
     uint64_t last_total = 0;                  // tasks of the last run
@@ -396,8 +722,7 @@ extern "C" int xkb_sched_create(xkb_sched_t ** out, void * stream)
     S->stream = (cudaStream_t) stream;
     int sms = 148, per = 2;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sched_persistent_kernel<2>, SCHED_THREADS, 0);
-    // (all team variants share the register budget fixed by __launch_bounds__(256, 2))
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sched_persistent_kernel<false>, SCHED_THREADS, 0);
     S->grid = sms * (per > 0 ? per : 1);
     *out = S;
     return XKB_OK;
@@ -481,46 +806,57 @@ extern "C" int xkb_sched_set_staging(xkb_sched_t * S, int bulk)
 
 static int launch_persistent(xkb_sched * S, SchedArgs & a);
 
-template <int TEAM, int NBUF>
-static int launch_bulk_n(xkb_sched * S, SchedArgs & a)
+static int launch_bulk(xkb_sched * S, SchedArgs & a)
 {
-    const size_t smem = bulk_smem_bytes(NBUF);
-    XKB_CUDA_TRY(cudaFuncSetAttribute(sched_persistent_kernel<TEAM, true, NBUF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-    sched_persistent_kernel<TEAM, true, NBUF><<<S->grid, SCHED_THREADS, smem, S->stream>>>(a);
+    const size_t smem = bulk_smem_bytes(SCHED_BULK_NBUF);
+    XKB_CUDA_TRY(cudaFuncSetAttribute(sched_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    sched_persistent_kernel<true><<<S->grid, SCHED_THREADS, smem, S->stream>>>(a);
     return XKB_OK;
 }
 
-static int launch_bulk(xkb_sched * S, SchedArgs & a)
+// Working memory of runs of up to n tasks: wait counters and units done, queue slots, counters.
+static int reserve_run(xkb_sched * S, size_t n)
 {
-    switch (S->team_warps)
-    {
-        case 1: return launch_bulk_n<1, SCHED_BULK_NBUF>(S, a);
-        case 2: return launch_bulk_n<2, SCHED_BULK_NBUF>(S, a);
-        case 4: return launch_bulk_n<4, SCHED_BULK_NBUF>(S, a);
-        default: return launch_bulk_n<8, SCHED_BULK_NBUF>(S, a);
-    }
+    if (n < 1) n = 1;
+    int rc;
+    if ((rc = S->wc.reserve(2 * n)) || (rc = S->queue.reserve(n)) || (rc = S->ctr.reserve(CTR_COUNT))) return rc;
+    return XKB_OK;
+}
+
+static SchedArgs run_args(xkb_sched * S, uint32_t ntasks, uint32_t period)
+{
+    SchedArgs a;
+    a.tasks = S->tasks.p; a.ntasks = ntasks; a.period = period;
+    a.wc = S->wc.p; a.units_done = S->wc.p + ntasks; a.queue = S->queue.p; a.ctr = S->ctr.p;
+    a.timeout_ns = S->timeout_ns; a.pfd = S->pfd; a.min_units = S->team_warps;
+    a.allow_team = !S->bulk;
+    return a;
+}
+
+static void plain_graph(SchedArgs & a, const xkb_task_graph_t * g)
+{
+    a.succ_ptr = g->succ_ptr; a.succ = g->succ; a.xsucc_ptr = nullptr; a.xsucc = nullptr;
+    a.npred_first = g->npred; a.npred_next = g->npred;
 }
 
 static int run_persistent(xkb_sched * S, const xkb_task_graph_t * g)
 {
     const uint32_t n = (uint32_t) g->ntasks;
-    int rc;
-    if ((rc = S->wc.reserve(n ? n : 1)) || (rc = S->queue.reserve(n ? n : 1)) || (rc = S->ctr.reserve(4))) return rc;
-    SchedArgs a;
-    a.tasks = S->tasks.p; a.ntasks = n; a.period = n ? n : 1; a.succ_ptr = g->succ_ptr; a.succ = g->succ;
-    a.xsucc_ptr = nullptr; a.xsucc = nullptr; a.npred_first = g->npred; a.npred_next = g->npred;
-    a.wc = S->wc.p; a.queue = S->queue.p; a.ctr = S->ctr.p; a.timeout_ns = S->timeout_ns; a.pfd = S->pfd;
+    if (int rc = reserve_run(S, n)) return rc;
+    SchedArgs a = run_args(S, n, n ? n : 1);
+    plain_graph(a, g);
     return launch_persistent(S, a);
 }
 
 static int launch_persistent(xkb_sched * S, SchedArgs & a)
 {
     const uint32_t n = a.ntasks;
-    XKB_CUDA_TRY(cudaMemsetAsync(S->ctr.p, 0, 4 * sizeof(unsigned), S->stream));
+    XKB_CUDA_TRY(cudaMemsetAsync(S->ctr.p, 0, CTR_COUNT * sizeof(unsigned), S->stream));
     if (n)
     {
         sched_init_kernel<<<(n + 255) / 256, 256, 0, S->stream>>>(a);
         sched_seed_kernel<<<(n + 255) / 256, 256, 0, S->stream>>>(a);
+        sched_plan_kernel<<<(a.period + 255) / 256, 256, 0, S->stream>>>(a, (unsigned) S->grid * (SCHED_THREADS / 32));
         if (!S->ev[0]) { XKB_CUDA_TRY(cudaEventCreate(&S->ev[0])); XKB_CUDA_TRY(cudaEventCreate(&S->ev[1])); }
         XKB_CUDA_TRY(cudaEventRecord(S->ev[0], S->stream));
         if (S->bulk)
@@ -529,13 +865,10 @@ static int launch_persistent(xkb_sched * S, SchedArgs & a)
             if (rc) return rc;
         }
         else
-            switch (S->team_warps)
-            {
-                case 1: sched_persistent_kernel<1><<<S->grid, SCHED_THREADS, 0, S->stream>>>(a); break;
-                case 2: sched_persistent_kernel<2><<<S->grid, SCHED_THREADS, 0, S->stream>>>(a); break;
-                case 4: sched_persistent_kernel<4><<<S->grid, SCHED_THREADS, 0, S->stream>>>(a); break;
-                default: sched_persistent_kernel<8><<<S->grid, SCHED_THREADS, 0, S->stream>>>(a); break;
-            }
+        {
+            sched_persistent_kernel<false><<<S->grid, SCHED_THREADS, 0, S->stream>>>(a);
+            sched_team_kernel<<<S->grid, SCHED_THREADS, 0, S->stream>>>(a);
+        }
         XKB_CUDA_TRY(cudaEventRecord(S->ev[1], S->stream));
     }
     XKB_CUDA_TRY(cudaGetLastError());
@@ -624,13 +957,10 @@ extern "C" int xkb_sched_run_periodic(xkb_sched_t * S, const xkb_periodic_graph_
                              (unsigned long long) g->period, S->ntasks);
     const uint64_t total = (uint64_t) (repeats - 1) * g->period + tail;
     if (total >= (1ull << 31)) return xkb_set_error(XKB_ERANGE, "sched_run_periodic: %llu tasks in one run", (unsigned long long) total);
-    int rc;
-    if ((rc = S->wc.reserve(total)) || (rc = S->queue.reserve(total)) || (rc = S->ctr.reserve(4))) return rc;
-    SchedArgs a;
-    a.tasks = S->tasks.p; a.ntasks = (uint32_t) total; a.period = (uint32_t) g->period;
+    if (int rc = reserve_run(S, total)) return rc;
+    SchedArgs a = run_args(S, (uint32_t) total, (uint32_t) g->period);
     a.succ_ptr = g->succ_ptr; a.succ = g->succ; a.xsucc_ptr = g->xsucc_ptr; a.xsucc = g->xsucc;
     a.npred_first = g->npred_first; a.npred_next = g->npred_next;
-    a.wc = S->wc.p; a.queue = S->queue.p; a.ctr = S->ctr.p; a.timeout_ns = S->timeout_ns; a.pfd = S->pfd;
     S->last_form = XKB_FORM_PERSISTENT;
     S->last_total = total;
     return launch_persistent(S, a);
@@ -640,16 +970,15 @@ extern "C" int xkb_sched_run_periodic(xkb_sched_t * S, const xkb_periodic_graph_
 __global__ void window_status_kernel(const unsigned * __restrict__ ctr, unsigned long long * sum)
 {
     if (threadIdx.x != 0) return;
-    if (sum[0] == 0 && ctr[2] != 0) sum[0] = ctr[2];
-    sum[1] += ctr[3];
+    if (sum[0] == 0 && ctr[CTR_STATUS] != 0) sum[0] = ctr[CTR_STATUS];
+    sum[1] += executed_tasks(ctr);
 }
 
 int xkb_internal_sched_reserve(xkb_sched_t * S, size_t ntasks)
 {
     if (!S) return xkb_set_error(XKB_EINVAL, "sched_reserve: null scheduler");
     int rc;
-    if ((rc = S->tasks.reserve(ntasks)) || (rc = S->wc.reserve(ntasks)) || (rc = S->queue.reserve(ntasks)) || (rc = S->ctr.reserve(4)))
-        return rc;
+    if ((rc = S->tasks.reserve(ntasks)) || (rc = reserve_run(S, ntasks))) return rc;
     if (!S->wsum.p)
     {
         if ((rc = S->wsum.reserve(2))) return rc;
@@ -662,12 +991,12 @@ int xkb_internal_sched_upload_window(xkb_sched_t * S, const xkb_task_desc_t * ta
 {
     if (!S || (ntasks && !tasks) || ntasks >= (size_t(1) << 31)) return xkb_set_error(XKB_EINVAL, "sched_upload_window: bad arguments");
     int rc;
-    if (ntasks > S->tasks.cap || ntasks > S->wc.cap || ntasks > S->queue.cap)
+    if (ntasks > S->tasks.cap || 2 * ntasks > S->wc.cap || ntasks > S->queue.cap)
     {
         // earlier windows may still be reading these buffers
         XKB_CUDA_TRY(cudaStreamSynchronize(S->stream));
         const size_t c = ntasks + ntasks / 2;
-        if ((rc = S->tasks.reserve(c)) || (rc = S->wc.reserve(c)) || (rc = S->queue.reserve(c))) return rc;
+        if ((rc = S->tasks.reserve(c)) || (rc = reserve_run(S, c))) return rc;
     }
     if (ntasks) XKB_CUDA_TRY(cudaMemcpyAsync(S->tasks.p, tasks, ntasks * sizeof(xkb_task_desc_t), cudaMemcpyHostToDevice, S->stream));
     S->host_tasks.clear();
@@ -687,11 +1016,9 @@ int xkb_internal_sched_launch_window(xkb_sched_t * S, const xkb_task_graph_t * g
     }
     const size_t ntasks = S->ntasks;
     if (ntasks == 0) return XKB_OK;
-    if ((rc = S->ctr.reserve(4))) return rc;
-    SchedArgs a;
-    a.tasks = S->tasks.p; a.ntasks = (uint32_t) ntasks; a.period = (uint32_t) ntasks; a.succ_ptr = g->succ_ptr; a.succ = g->succ;
-    a.xsucc_ptr = nullptr; a.xsucc = nullptr; a.npred_first = g->npred; a.npred_next = g->npred;
-    a.wc = S->wc.p; a.queue = S->queue.p; a.ctr = S->ctr.p; a.timeout_ns = S->timeout_ns; a.pfd = S->pfd;
+    if ((rc = reserve_run(S, ntasks))) return rc;      // (no-op: xkb_internal_sched_upload_window made room)
+    SchedArgs a = run_args(S, (uint32_t) ntasks, (uint32_t) ntasks);
+    plain_graph(a, g);
     if ((rc = launch_persistent(S, a))) return rc;
     window_status_kernel<<<1, 32, 0, S->stream>>>(S->ctr.p, S->wsum.p);
     XKB_CUDA_TRY(cudaGetLastError());
@@ -727,11 +1054,13 @@ extern "C" int xkb_sched_wait(xkb_sched_t * S, uint64_t * executed)
 {
     if (!S) return xkb_set_error(XKB_EINVAL, "sched_wait: null scheduler");
     XKB_CUDA_TRY(cudaStreamSynchronize(S->stream));
-    unsigned ctr[4] = {0, 0, 0, (unsigned) S->last_total};
+    unsigned ctr[CTR_COUNT] = {};
+    ctr[CTR_EXECUTED] = (unsigned) S->last_total;               // the other forms count nothing
     if (S->ctr.p && S->last_form == XKB_FORM_PERSISTENT) XKB_CUDA_TRY(cudaMemcpy(ctr, S->ctr.p, sizeof(ctr), cudaMemcpyDeviceToHost));
-    if (executed) *executed = ctr[3];
-    if (ctr[2] != 0)
-        return xkb_set_error(-(int) ctr[2], "sched: a device wait ran out of time (%u of %llu tasks were made ready)", ctr[1], (unsigned long long) S->last_total);
+    if (executed) *executed = executed_tasks(ctr);
+    if (ctr[CTR_STATUS] != 0)
+        return xkb_set_error(-(int) ctr[CTR_STATUS], "sched: a device wait ran out of time (%u of %llu tasks ran)", executed_tasks(ctr),
+                             (unsigned long long) S->last_total);
     return XKB_OK;
 }
 
@@ -760,9 +1089,8 @@ extern "C" int xkb_sched_kernel_ms(xkb_sched_t * S, double * ms)
 // every GPU that loads the library, until the process exits).
 static __device__ __align__(256) int g_sched_noalloc_scratch[2 * XKB_NOALLOC_MAX_TASKS + 64];   // + counters
 
-// Counters of a no-allocation run, after the wait counters and queue: [0] head, [1] tail,
-// [2] status, [3] executed, [4] the lowest task index whose descriptor failed the check.
-constexpr int NOALLOC_CTRS = 8;
+// (the counters CTR_* stand after the wait counters and the queue; CTR_BAD_TASK is the lowest task
+// index whose descriptor failed the check)
 
 // Every descriptor of a no-allocation run is checked on the device with the host checks of
 // xkb_sched_set_tasks before anything runs: a bad one sets the status to XKB_EINVAL, records
@@ -773,8 +1101,8 @@ __global__ void noalloc_check_kernel(const xkb_task_desc_t * __restrict__ tasks,
     if (t >= n) return;
     if (!xkb_internal_task_valid(tasks[t]))
     {
-        atomicCAS(ctr + 2, 0u, (unsigned) -XKB_EINVAL);
-        atomicMin(ctr + 4, t);
+        atomicCAS(ctr + CTR_STATUS, 0u, (unsigned) -XKB_EINVAL);
+        atomicMin(ctr + CTR_BAD_TASK, t);
     }
 }
 
@@ -818,9 +1146,8 @@ static int noalloc_scratch(int ** out)
         if (e != cudaSuccess) return xkb_set_cuda_error(e);
         cudaFuncAttributes fa;
         const void * kernels[] = {(const void *) noalloc_check_kernel, (const void *) sched_init_kernel,
-                                  (const void *) sched_seed_kernel, (const void *) sched_persistent_kernel<1>,
-                                  (const void *) sched_persistent_kernel<2>, (const void *) sched_persistent_kernel<4>,
-                                  (const void *) sched_persistent_kernel<8>};
+                                  (const void *) sched_seed_kernel, (const void *) sched_plan_kernel,
+                                  (const void *) sched_persistent_kernel<false>, (const void *) sched_team_kernel};
         for (const void * k : kernels)
             if ((e = cudaFuncGetAttributes(&fa, k)) != cudaSuccess) return xkb_set_cuda_error(e);
         sl.ctx = ctx;
@@ -850,54 +1177,55 @@ extern "C" int xkb_sched_run_noalloc(const xkb_task_desc_t * tasks, const xkb_ta
     SchedArgs a;
     a.tasks = tasks; a.ntasks = n; a.period = n ? n : 1; a.succ_ptr = graph->succ_ptr; a.succ = graph->succ;
     a.xsucc_ptr = nullptr; a.xsucc = nullptr; a.npred_first = graph->npred; a.npred_next = graph->npred;
+    // the units done stand behind the wait counters where these fill half of their room at most;
+    // a larger graph runs with one warp per task
     a.wc = scratch; a.queue = scratch + XKB_NOALLOC_MAX_TASKS;
+    a.units_done = n <= XKB_NOALLOC_MAX_TASKS / 2 ? scratch + n : nullptr;
+    a.min_units = warps_per_task;
+    a.allow_team = 1;
     a.ctr = (unsigned *) (scratch + 2 * XKB_NOALLOC_MAX_TASKS);
     a.timeout_ns = (uint64_t) (timeout_s * 1e9);
     a.pfd = SCHED_PFD_DEFAULT;
     // the array keeps the previous call's contents: the counters are cleared here (the lowest bad
     // index to all ones), and the init kernel rewrites every wait counter and queue slot this run uses
-    XKB_CUDA_TRY(cudaMemsetAsync(a.ctr, 0, 4 * sizeof(unsigned), st));
-    XKB_CUDA_TRY(cudaMemsetAsync(a.ctr + 4, 0xff, (NOALLOC_CTRS - 4) * sizeof(unsigned), st));
+    XKB_CUDA_TRY(cudaMemsetAsync(a.ctr, 0, CTR_COUNT * sizeof(unsigned), st));
+    XKB_CUDA_TRY(cudaMemsetAsync(a.ctr + CTR_BAD_TASK, 0xff, sizeof(unsigned), st));
     if (n)
     {
         int dev = 0, sms = 148, per = 2;
         XKB_CUDA_TRY(cudaGetDevice(&dev));
         XKB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        XKB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sched_persistent_kernel<2>, SCHED_THREADS, 0));
+        XKB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sched_persistent_kernel<false>, SCHED_THREADS, 0));
         const unsigned grid = (unsigned) (sms * (per > 0 ? per : 1));
         noalloc_check_kernel<<<(n + 255) / 256, 256, 0, st>>>(tasks, n, a.ctr);
         sched_init_kernel<<<(n + 255) / 256, 256, 0, st>>>(a);
         sched_seed_kernel<<<(n + 255) / 256, 256, 0, st>>>(a);
-        switch (warps_per_task)
-        {
-            case 1: sched_persistent_kernel<1><<<grid, SCHED_THREADS, 0, st>>>(a); break;
-            case 2: sched_persistent_kernel<2><<<grid, SCHED_THREADS, 0, st>>>(a); break;
-            case 4: sched_persistent_kernel<4><<<grid, SCHED_THREADS, 0, st>>>(a); break;
-            default: sched_persistent_kernel<8><<<grid, SCHED_THREADS, 0, st>>>(a); break;
-        }
+        sched_plan_kernel<<<(n + 255) / 256, 256, 0, st>>>(a, grid * (SCHED_THREADS / 32));
+        sched_persistent_kernel<false><<<grid, SCHED_THREADS, 0, st>>>(a);
+        sched_team_kernel<<<grid, SCHED_THREADS, 0, st>>>(a);
         XKB_CUDA_TRY(cudaGetLastError());
     }
-    unsigned ctr[NOALLOC_CTRS] = {};
+    unsigned ctr[CTR_COUNT] = {};
     XKB_CUDA_TRY(cudaMemcpyAsync(ctr, a.ctr, sizeof(ctr), cudaMemcpyDeviceToHost, st));
     XKB_CUDA_TRY(cudaStreamSynchronize(st));
-    if (executed) *executed = ctr[3];
-    if (ctr[2] == (unsigned) -XKB_EINVAL)
-        return xkb_set_error(XKB_EINVAL, "sched_run_noalloc: task %u: bad descriptor (unknown kind, bad heat tile or axpby range); nothing ran", ctr[4]);
-    if (ctr[2] != 0)
-        return xkb_set_error(-(int) ctr[2], "sched_run_noalloc: a device wait ran out of time (%u of %u tasks were made ready)", ctr[1], n);
+    if (executed) *executed = executed_tasks(ctr);
+    if (ctr[CTR_STATUS] == (unsigned) -XKB_EINVAL)
+        return xkb_set_error(XKB_EINVAL, "sched_run_noalloc: task %u: bad descriptor (unknown kind, bad heat tile or axpby range); nothing ran", ctr[CTR_BAD_TASK]);
+    if (ctr[CTR_STATUS] != 0)
+        return xkb_set_error(-(int) ctr[CTR_STATUS], "sched_run_noalloc: a device wait ran out of time (%u of %u tasks ran)", executed_tasks(ctr), n);
     return XKB_OK;
 }
 
 // ------------------------------------------------------------------------------------------
 // Device-resident serving loop: ONE persistent kernel runs the tile tasks of every admitted
 // request. The host admits a request by writing its slot record (descriptors, periodic graph,
-// counter and queue arrays, the grid to duplicate) and then the slot's state word; any idle team
+// counter and queue arrays, the grid to duplicate) and then the slot's state word; any idle warp
 // of the kernel then takes the slot's set-up chunks (wait counters, queue slots, second grid),
-// the team that finishes the last chunk publishes the request's first ready tasks, and from then
-// on teams take ready tasks from whichever slot has some -- a small request does not hold SMs it
-// cannot use, and requests admitted while others run share the device at once. The team that
-// executes a request's last task marks the slot done and reports the admission number to mapped
-// host memory; the host copies the result out. Teams stop when the host has said no request will
+// the warp that finishes the last chunk publishes the request's first ready tasks, and from then
+// on warps take units of ready tasks from whichever slot has some -- a small request does not hold
+// SMs it cannot use, and requests admitted while others run share the device at once. The warp
+// that ends a request's last task marks the slot done and reports the admission number to mapped
+// host memory; the host copies the result out. Warps stop when the host has said no request will
 // come and every slot is idle or done, on an error, or at the time limit; every wait is bounded.
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned * p)
@@ -918,64 +1246,60 @@ __device__ __forceinline__ void srv_publish(const XkbSrvSlot & S, XkbSrvCtl * c,
     xkb_st_release(S.queue + pos, (int) t);
 }
 
-template <int TEAM_WARPS>
 __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) server_kernel(XkbSrvArgs a)
 {
-    constexpr int NTEAMS = (SCHED_THREADS / 32) / TEAM_WARPS;
-    constexpr int TEAM_THREADS = TEAM_WARPS * 32;
-    __shared__ int job_kind[NTEAMS];           // 0 stop, 1 task, 2 set-up chunk, -1 nothing yet
-    __shared__ int job_slot[NTEAMS];
-    __shared__ int job_idx[NTEAMS];            // task id, or chunk index
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int team = warp / TEAM_WARPS, twarp = warp % TEAM_WARPS;
-    const int bar = 1 + team, tthread = twarp * 32 + lane;
-    const int gteam = blockIdx.x * NTEAMS + team;
+    const int lane = threadIdx.x & 31;
+    const int gwarp = blockIdx.x * (SCHED_THREADS / 32) + (threadIdx.x >> 5);
     unsigned executed = 0;
     uint32_t nap = 32;
     const uint64_t t_start = xkb_globaltimer();
     for (;;)
     {
-        if (tthread == 0)
+        // kind: 0 stop, 1 unit of a task, 2 set-up chunk, -1 nothing yet
+        int kind = -1, sl = -1, idx = -1, unit = 0;
+        if (lane == 0)
         {
-            int kind = -1, slot = -1, idx = -1;
             if (*(volatile unsigned *) (a.status + 2) >= 2) kind = 0;     // the host gave up: stop now
             for (int k = 0; k < a.nslots && kind < 0; ++k)
             {
-                const int sl = (gteam + k) % a.nslots;
-                XkbSrvCtl * c = a.ctl + sl;
+                const int q = (gwarp + k) % a.nslots;
+                XkbSrvCtl * c = a.ctl + q;
                 const unsigned st = ld_acquire_u32(&c->state);
                 if (st == 1)
                 {
-                    if (*(volatile unsigned *) &c->init_next < a.slots[sl].nchunks)
+                    if (*(volatile unsigned *) &c->init_next < a.slots[q].nchunks)
                     {
                         const unsigned ch = atomicAdd(&c->init_next, 1u);
-                        if (ch < a.slots[sl].nchunks) { kind = 2; slot = sl; idx = (int) ch; }
+                        if (ch < a.slots[q].nchunks) { kind = 2; sl = q; idx = (int) ch; }
                     }
                 }
-                else if (st == 2 && *(volatile unsigned *) &c->head < *(volatile unsigned *) &c->tail)
+                else if (st == 2)
                 {
-                    // claim the next queue position with one atomicAdd (a compare-and-swap loop on
-                    // `head` serialises the teams on it); the position may be published a little
-                    // later, which the wait below covers. The claim counts in `claimers` while the
-                    // state is re-checked, so the team ending the request can tell when no claim
-                    // on this request's counters is left.
+                    if (*(volatile unsigned *) &c->head >= *(volatile unsigned *) &c->tail << a.slots[q].units_log2) continue;
+                    // claim the next ticket with one atomicAdd (a compare-and-swap loop on `head`
+                    // serialises the warps on it); the position may be published a little later,
+                    // which the wait below covers. The claim counts in `claimers` while the state
+                    // is re-checked, so the warp ending the request can tell when no claim on this
+                    // request's counters is left.
                     atomicAdd(&c->claimers, 1u);
                     __threadfence();
                     unsigned h = 0;
                     if (ld_acquire_u32(&c->state) == 2)
                     {
-                        h = atomicAdd(&c->head, 1u);
-                        if (h < a.slots[sl].ntasks) { kind = 1; slot = sl; }
+                        const uint32_t lg = a.slots[q].units_log2;       // this request's: the slot is not reused under a claim
+                        const unsigned ticket = atomicAdd(&c->head, 1u);
+                        h = ticket >> lg;
+                        unit = (int) (ticket & ((1u << lg) - 1));
+                        if (h < a.slots[q].ntasks) { kind = 1; sl = q; }
                     }
                     atomicSub(&c->claimers, 1u);
                     if (kind == 1)
                     {
                         // the id at that position was published (tail counts it) or is about to be
-                        const int * q = a.slots[sl].queue + h;
+                        const int * pq = a.slots[q].queue + h;
                         const uint64_t t0 = xkb_globaltimer();
                         uint32_t spins = 0;
-                        int t;
-                        while ((t = xkb_ld_acquire(q)) < 0)
+                        while ((idx = xkb_ld_acquire(pq)) < 0)
                         {
                             if ((++spins & 63) == 0 && xkb_globaltimer() - t0 > a.timeout_ns)
                             {
@@ -983,7 +1307,7 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) server_kernel(X
                                 break;
                             }
                         }
-                        if (t < 0) kind = 0; else idx = t;
+                        if (idx < 0) kind = 0;
                     }
                 }
             }
@@ -994,30 +1318,34 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) server_kernel(X
                 else if (*(volatile unsigned *) (a.status + 2))
                 {
                     bool busy = false;
-                    for (int sl = 0; sl < a.nslots && !busy; ++sl)
+                    for (int q = 0; q < a.nslots && !busy; ++q)
                     {
-                        const unsigned st = ld_acquire_u32(&a.ctl[sl].state);
+                        const unsigned st = ld_acquire_u32(&a.ctl[q].state);
                         busy = st == 1 || st == 2;
                     }
                     if (!busy) kind = 0;
                 }
-                if (kind < 0) { __nanosleep(nap); if (nap < 8192) nap *= 2; }
+                if (kind < 0) { __nanosleep(nap); if (nap < XKB_SRV_NAP_MAX) nap *= 2; }
             }
             else nap = 32;
-            job_kind[team] = kind; job_slot[team] = slot; job_idx[team] = idx;
         }
-        team_sync(bar, TEAM_THREADS);
-        const int kind = job_kind[team], sl = job_slot[team], idx = job_idx[team];
+        kind = __shfl_sync(0xffffffffu, kind, 0);
+        if (kind < 0) continue;
         if (kind == 0) break;
+        sl = __shfl_sync(0xffffffffu, sl, 0);
+        idx = __shfl_sync(0xffffffffu, idx, 0);
+        unit = __shfl_sync(0xffffffffu, unit, 0);
+        __syncwarp();
         if (kind == 2)
         {
-            // set-up chunk: wait counters and empty queue slots of its tasks, and its share of the
-            // second grid (a copy of the first, which the host copied in)
+            // set-up chunk: wait counters, unit counts and empty queue slots of its tasks, and its
+            // share of the second grid (a copy of the first, which the host copied in)
             const XkbSrvSlot & S = a.slots[sl];
-            const uint32_t t0 = (uint32_t) idx * XKB_SRV_CHUNK, t1 = min(S.ntasks, t0 + XKB_SRV_CHUNK);
-            for (uint32_t t = t0 + tthread; t < t1; t += TEAM_THREADS)
+            const uint32_t t0 = (uint32_t) idx * S.chunk_tasks, t1 = min(S.ntasks, t0 + S.chunk_tasks);
+            for (uint32_t t = t0 + lane; t < t1; t += 32)
             {
                 S.queue[t] = -1;
+                if (S.units_done) S.units_done[t] = 0;
                 const uint32_t w = t / S.period, l = t - w * S.period;
                 S.wc[t] = (int) (w == 0 ? S.npred_first[l] : S.npred_next[l]);
             }
@@ -1026,96 +1354,95 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) server_kernel(X
             const uint4 * src = (const uint4 *) (S.copy_src + b0);
             uint4 * dst = (uint4 *) (S.copy_dst + b0);
             const uint64_t nv = (b1 - b0) / 16;
-            uint64_t k = tthread;
-            for (; k + 3 * TEAM_THREADS < nv; k += 4 * TEAM_THREADS)     // four 16-byte loads in flight per lane
+            uint64_t k = lane;
+            for (; k + 3 * 32 < nv; k += 4 * 32)                         // four 16-byte loads in flight per lane
             {
-                const uint4 v0 = __ldcg(src + k), v1 = __ldcg(src + k + TEAM_THREADS), v2 = __ldcg(src + k + 2 * TEAM_THREADS),
-                            v3 = __ldcg(src + k + 3 * TEAM_THREADS);
-                dst[k] = v0; dst[k + TEAM_THREADS] = v1; dst[k + 2 * TEAM_THREADS] = v2; dst[k + 3 * TEAM_THREADS] = v3;
+                const uint4 v0 = __ldcg(src + k), v1 = __ldcg(src + k + 32), v2 = __ldcg(src + k + 64), v3 = __ldcg(src + k + 96);
+                dst[k] = v0; dst[k + 32] = v1; dst[k + 64] = v2; dst[k + 96] = v3;
             }
-            for (; k < nv; k += TEAM_THREADS) dst[k] = __ldcg(src + k);
-            for (uint64_t r = ((b1 - b0) & ~(uint64_t) 15) + tthread; r < b1 - b0; r += TEAM_THREADS)
+            for (; k < nv; k += 32) dst[k] = __ldcg(src + k);
+            for (uint64_t r = ((b1 - b0) & ~(uint64_t) 15) + lane; r < b1 - b0; r += 32)
                 S.copy_dst[b0 + r] = S.copy_src[b0 + r];
             __threadfence();
-            team_sync(bar, TEAM_THREADS);
-            if (tthread == 0)
+            __syncwarp();
+            XkbSrvCtl * c = a.ctl + sl;
+            int last = 0;
+            if (lane == 0) last = atom_add_acq_rel((int *) &c->init_done, 1) + 1 == (int) S.nchunks;
+            if (__shfl_sync(0xffffffffu, last, 0))
             {
-                XkbSrvCtl * c = a.ctl + sl;
-                if (atomicAdd(&c->init_done, 1u) + 1 == S.nchunks)
-                {
-                    // every chunk is done: publish the tasks with no predecessor, then run
-                    for (uint32_t l = 0; l < S.period && l < S.ntasks; ++l)
-                        if (S.npred_first[l] == 0) srv_publish(S, c, l);
-                    if (S.seed_later)
-                        for (uint32_t t = S.period; t < S.ntasks; ++t)
-                            if (S.npred_next[t % S.period] == 0) srv_publish(S, c, t);
-                    st_release_u32(&c->state, 2u);
-                }
-            }
-        }
-        else if (kind == 1)
-        {
-            const XkbSrvSlot & S = a.slots[sl];
-            const uint32_t t = (uint32_t) idx, w = t / S.period, l = t - w * S.period;
-            run_task_team(S.tasks[l], twarp, TEAM_WARPS, S.pfd);
-            __threadfence();
-            team_sync(bar, TEAM_THREADS);
-            if (twarp == 0)
-            {
-                XkbSrvCtl * c = a.ctl + sl;
-                const uint32_t base = w * S.period;
-                for (uint32_t i = S.succ_ptr[l] + lane; i < S.succ_ptr[l + 1]; i += 32)
-                {
-                    const uint32_t u = base + S.succ[i];
-                    if (u < S.ntasks && atom_add_acq_rel(S.wc + u, -1) == 1) srv_publish(S, c, u);
-                }
-                if (S.xsucc_ptr)
-                    for (uint32_t i = S.xsucc_ptr[l] + lane; i < S.xsucc_ptr[l + 1]; i += 32)
-                    {
-                        const uint32_t u = base + S.period + S.xsucc[i];
-                        if (u < S.ntasks && atom_add_acq_rel(S.wc + u, -1) == 1) srv_publish(S, c, u);
-                    }
+                // every chunk is done: publish the tasks with no predecessor, then run
+                for (uint32_t l = lane; l < S.period && l < S.ntasks; l += 32)
+                    if (S.npred_first[l] == 0) srv_publish(S, c, l);
+                if (S.seed_later)
+                    for (uint32_t t = S.period + lane; t < S.ntasks; t += 32)
+                        if (S.npred_next[t % S.period] == 0) srv_publish(S, c, t);
+                __threadfence();
                 __syncwarp();
-                if (lane == 0)
-                {
-                    ++executed;
-                    if (atomicAdd(&c->executed, 1u) + 1 == S.ntasks)
+                if (lane == 0) st_release_u32(&c->state, 2u);
+            }
+            __syncwarp();
+            continue;
+        }
+        const XkbSrvSlot & S = a.slots[sl];
+        XkbSrvCtl * c = a.ctl + sl;
+        const uint32_t t = (uint32_t) idx, w = t / S.period, l = t - w * S.period, base = w * S.period;
+        const int nunits = 1 << S.units_log2;
+        const xkb_task_desc_t d = load_desc(S.tasks + l);
+        const SuccGraph g{S.succ_ptr, S.succ, S.xsucc_ptr, S.xsucc, S.period, S.ntasks};
+        bool more;
+        const uint32_t first = g.first(l, base, lane, more);
+        run_unit<XKB_F64_PF, XKB_TILE_PF>(d, unit, nunits, S.pfd);
+        __syncwarp();
+        fence_acq_rel_gpu();
+        if (nunits > 1)
+        {
+            int last = 0;
+            if (lane == 0)
+            {
+                last = atom_add_relaxed(S.units_done + t, 1) == nunits - 1;
+                fence_acq_rel_gpu();
+            }
+            if (!__shfl_sync(0xffffffffu, last, 0)) continue;
+            __syncwarp();
+        }
+        release_successors(g, t, first, more, S.wc, S.queue, &c->tail, lane);
+        __syncwarp();
+        if (lane == 0)
+        {
+            ++executed;
+            if (atomicAdd(&c->executed, 1u) + 1 == S.ntasks)
+            {
+                st_release_u32(&c->state, 3u);
+                __threadfence();
+                // warps that saw state 2 before the store above claim past the last task and leave;
+                // wait (bounded) until none is between its check and its claim
+                const uint64_t tw = xkb_globaltimer();
+                uint32_t spins = 0;
+                while (*(volatile unsigned *) &c->claimers != 0)
+                    if ((++spins & 63) == 0 && xkb_globaltimer() - tw > a.timeout_ns)
                     {
-                        st_release_u32(&c->state, 3u);
-                        __threadfence();
-                        // teams that saw state 2 before the store above claim past the last task
-                        // and leave; wait (bounded) until none is between its check and its claim
-                        const uint64_t tw = xkb_globaltimer();
-                        uint32_t spins = 0;
-                        while (*(volatile unsigned *) &c->claimers != 0)
-                            if ((++spins & 63) == 0 && xkb_globaltimer() - tw > a.timeout_ns)
-                            {
-                                atomicCAS(a.status, 0u, (unsigned) -XKB_ETIMEDOUT);
-                                break;
-                            }
-                        __threadfence_system();
-                        a.host_done[sl] = S.gen;
+                        atomicCAS(a.status, 0u, (unsigned) -XKB_ETIMEDOUT);
+                        break;
                     }
-                }
+                __threadfence_system();
+                a.host_done[sl] = S.gen;
             }
         }
-        team_sync(bar, TEAM_THREADS);           // job_* are rewritten only after every thread read them
+        __syncwarp();
     }
-    if (tthread == 0 && executed) atomicAdd(a.status + 1, executed);
+    if (lane == 0 && executed) atomicAdd(a.status + 1, executed);
 }
 
-int xkb_internal_server_launch(const XkbSrvArgs & a, int grid, int warps_per_task, cudaStream_t stream)
+int xkb_internal_server_launch(const XkbSrvArgs & a, int grid, cudaStream_t stream)
 {
-    switch (warps_per_task)
-    {
-        case 1: server_kernel<1><<<grid, SCHED_THREADS, 0, stream>>>(a); break;
-        case 2: server_kernel<2><<<grid, SCHED_THREADS, 0, stream>>>(a); break;
-        case 4: server_kernel<4><<<grid, SCHED_THREADS, 0, stream>>>(a); break;
-        case 8: server_kernel<8><<<grid, SCHED_THREADS, 0, stream>>>(a); break;
-        default: return xkb_set_error(XKB_EINVAL, "server: warps per task must be 1, 2, 4 or 8");
-    }
+    server_kernel<<<grid, SCHED_THREADS, 0, stream>>>(a);
     XKB_CUDA_TRY(cudaGetLastError());
     return XKB_OK;
+}
+
+int xkb_internal_split_log2(uint64_t width, uint64_t warps)
+{
+    return split_log2((unsigned) std::min<uint64_t>(width, 1u << 30), true, 0, (unsigned) warps, 1);
 }
 
 int xkb_internal_launch_task(const xkb_task_desc_t * d, cudaStream_t stream)

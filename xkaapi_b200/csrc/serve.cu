@@ -203,6 +203,8 @@ struct xkb_server {
     unsigned * h_stop = nullptr;
     cudaStream_t kstream = nullptr;
     uint32_t gen = 0;
+    uint64_t kernel_warps = 0;             // warps of the serving kernel
+    uint64_t active_width = 0;             // tasks per step of the requests on the device
 };
 
 static int get_window(xkb_server * S, const Shape & s, Window ** out)
@@ -425,12 +427,16 @@ static int server_run_launches(xkb_server * S, xkb_request_t * reqs, size_t n)
 
 // ---- the device-resident loop ---------------------------------------------------------------
 
-// Device bytes of a request: two grids, the window's descriptors, wait counters and queue slots.
-static uint64_t device_need(const xkb_request_t & q, uint64_t per_step)
+// Device bytes of a request: two grids, the window's descriptors, wait counters, unit counts and queue slots.
+// The unit counts are left out (tasks are not split) where the request only fits without them.
+static uint64_t device_need(const xkb_request_t & q, uint64_t per_step, uint64_t budget, bool & split)
 {
     const uint64_t esz = q.f32 ? 4 : 8, grid = ((uint64_t) q.nx * q.ny * esz + 255) & ~(uint64_t) 255;
     const uint64_t ntasks = (uint64_t) q.steps * per_step;
-    return 2 * grid + ((2 * per_step * sizeof(xkb_task_desc_t) + 255) & ~(uint64_t) 255) + 2 * ((ntasks * 4 + 255) & ~(uint64_t) 255);
+    const uint64_t words = (ntasks * 4 + 255) & ~(uint64_t) 255;
+    const uint64_t need = 2 * grid + ((2 * per_step * sizeof(xkb_task_desc_t) + 255) & ~(uint64_t) 255) + 2 * words;
+    split = need + words <= budget;
+    return split ? need + words : need;
 }
 
 template <typename T>
@@ -445,7 +451,7 @@ static int grow_pinned(T *& p, size_t & cap, size_t bytes)
 
 // Admit request q into slot k: its input in, its descriptors and slot record, then the state
 // word -- all copies on the slot's stream, in that order; the kernel does the rest.
-static int admit(xkb_server * S, int k, xkb_request_t & q, uint8_t * mem, Window * w)
+static int admit(xkb_server * S, int k, xkb_request_t & q, uint8_t * mem, Window * w, bool split)
 {
     Slot & sl = S->slots[k];
     const uint64_t esz = q.f32 ? 4 : 8, bytes = (uint64_t) q.nx * q.ny * esz, grid = (bytes + 255) & ~(uint64_t) 255;
@@ -472,6 +478,7 @@ static int admit(xkb_server * S, int k, xkb_request_t & q, uint8_t * mem, Window
     uint8_t * desc = b + grid;
     int * wc = (int *) (desc + ((period * sizeof(xkb_task_desc_t) + 255) & ~(uint64_t) 255));
     int * queue = (int *) ((uint8_t *) wc + ((ntasks * 4 + 255) & ~(uint64_t) 255));
+    int * units_done = split ? (int *) ((uint8_t *) queue + ((ntasks * 4 + 255) & ~(uint64_t) 255)) : nullptr;
     std::vector<xkb_task_desc_t> d;
     heat_descs(sh, 2, (uint64_t) a, (uint64_t) b, q.c, d);
     if (sl.hdesc_cap < d.size() * sizeof(xkb_task_desc_t)) return xkb_set_error(XKB_EINVAL, "server_run: descriptor staging was not sized for the trace");
@@ -481,11 +488,17 @@ static int admit(xkb_server * S, int k, xkb_request_t & q, uint8_t * mem, Window
     r.tasks = (const xkb_task_desc_t *) desc;
     r.succ_ptr = w->g.succ_ptr; r.succ = w->g.succ; r.xsucc_ptr = w->g.xsucc_ptr; r.xsucc = w->g.xsucc;
     r.npred_first = w->g.npred_first; r.npred_next = w->g.npred_next;
-    r.wc = wc; r.queue = queue;
+    r.wc = wc; r.units_done = units_done; r.queue = queue;
     r.copy_src = a; r.copy_dst = b; r.copy_bytes = bytes;
     r.period = (uint32_t) period; r.ntasks = (uint32_t) ntasks;
     r.nchunks = (uint32_t) std::max<uint64_t>({1, (ntasks + XKB_SRV_CHUNK - 1) / XKB_SRV_CHUNK,
                                               (bytes + XKB_SRV_COPY_CHUNK - 1) / XKB_SRV_COPY_CHUNK});
+    r.chunk_tasks = (uint32_t) ((ntasks + r.nchunks - 1) / r.nchunks);
+    // tiles of every request in flight share the warps; a request admitted into a quiet server
+    // splits its tiles over more of them (tickets are 32-bit)
+    int lg = split ? xkb_internal_split_log2(S->active_width + w->per_step, S->kernel_warps) : 0;
+    while (lg > 0 && (ntasks << lg) > 0xf0000000ull) --lg;
+    r.units_log2 = (uint32_t) lg;
     r.gen = sl.gen = ++S->gen;
     r.seed_later = w->seed_later ? 1u : 0u;
     r.pfd = XKB_SERVE_PFD;
@@ -508,9 +521,12 @@ static int server_run_device(xkb_server * S, xkb_request_t * reqs, size_t n)
         if (reqs[i].steps > 0 && (rc = get_window(S, Shape{reqs[i].nx, reqs[i].ny, reqs[i].ts, reqs[i].f32}, &win[i]))) return rc;
     XKB_CUDA_TRY(cudaStreamSynchronize(S->aux));
     std::vector<uint64_t> need(n);
+    std::vector<char> split(n, 0);
     for (size_t i = 0; i < n; ++i)
     {
-        need[i] = device_need(reqs[i], win[i] ? win[i]->per_step : 0);
+        bool sp = false;
+        need[i] = device_need(reqs[i], win[i] ? win[i]->per_step : 0, S->cfg.budget_bytes, sp);
+        split[i] = sp;
         if (need[i] > S->cfg.budget_bytes)
             return xkb_set_error(XKB_ERANGE, "server_run: request %zu needs %llu bytes, over the budget", i, (unsigned long long) need[i]);
     }
@@ -563,7 +579,9 @@ static int server_run_device(xkb_server * S, xkb_request_t * reqs, size_t n)
     int sms = 148, per = 2;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S->dev);
     const int grid = S->cfg.ctas_per_graph > 0 ? S->cfg.ctas_per_graph : sms * per;
-    if ((rc = xkb_internal_server_launch(ka, grid, XKB_SERVE_TEAM, S->kstream))) return rc;
+    S->kernel_warps = (uint64_t) grid * 8;
+    S->active_width = 0;
+    if ((rc = xkb_internal_server_launch(ka, grid, S->kstream))) return rc;
 
     // (4) admissions and completions
     std::vector<uint8_t *> mem(n, nullptr);
@@ -588,6 +606,7 @@ static int server_run_device(xkb_server * S, xkb_request_t * reqs, size_t n)
                     rc = xkb_set_cuda_error(cudaGetLastError());
                 else if (cudaEventRecord(sl.done, sl.stream) != cudaSuccess) rc = xkb_set_cuda_error(cudaGetLastError());
                 sl.phase = 2;
+                S->active_width -= win[sl.req]->per_step;
                 progressed = true;
             }
             if (sl.phase == 2)
@@ -610,7 +629,8 @@ static int server_run_device(xkb_server * S, xkb_request_t * reqs, size_t n)
             mem[next] = m;
             S->slots[k].req = (long) next;
             reqs[next].start_s = now();
-            rc = admit(S, k, reqs[next], m, win[next]);
+            rc = admit(S, k, reqs[next], m, win[next], split[next] != 0);
+            if (S->slots[k].phase == 1) S->active_width += win[next]->per_step;
             ++next; progressed = true;
         }
         if (rc == XKB_OK && now() > limit) rc = xkb_set_error(XKB_ETIMEDOUT, "server_run: %zu of %zu requests done after %.0f s", done, n, limit);
