@@ -241,3 +241,27 @@ def test_axpby_units(torch_cuda, n, lo):
     assert sch.wait() == 1
     y[lo:lo + n] = O.axpby(0.3, x[lo:lo + n], -1.7, y[lo:lo + n])
     np.testing.assert_array_equal(dy.cpu().numpy(), y)
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("nx,ny,ld,ts,steps", [(131, 77, 131, 40, 5), (260, 150, 261, 64, 5), (1027, 300, 1027, 64, 4),
+                                               (130, 90, 132, 32, 5), (2310, 2500, 2310, 48, 3)])
+def test_heat_grids_of_any_alignment(torch_cuda, nx, ny, ld, ts, steps, f32):
+    """Graphs on grids with odd leading dimensions (the row-by-row kernels), with a last vector past
+    the last row, and one wide enough to take its tiles column by column: bit-exact, padding intact."""
+    torch = torch_cuda
+    dt = np.float32 if f32 else np.float64
+    g = np.full((ny, ld), 7.0, dtype=dt)
+    g[:, :nx] = O.heat_init(nx, ny, seed=nx).astype(dt)
+    a, b = torch.from_numpy(g).cuda(), torch.from_numpy(g).cuda()
+    res = xk.Resolver()
+    res.add(xk.heat_access_records(nx, ny, ts, ts, 0, steps, a.data_ptr(), b.data_ptr(), esize=dt().itemsize, ld=ld))
+    sch = xk.Scheduler()
+    sch.set_tasks(xk.heat_task_descs((a.data_ptr(), b.data_ptr()), nx, ny, ld, ts, ts, steps, C, f32=f32))
+    sch.run(res.graph())
+    sch.wait()
+    out = (a if steps % 2 == 0 else b).cpu().numpy()
+    want = O.heat_run(np.ascontiguousarray(g[:, :nx]), nx, ny, steps, C, dtype=dt)
+    np.testing.assert_array_equal(out[:, :nx], want.reshape(ny, nx))
+    assert (out[:, nx:] == 7.0).all()
+    sch.close(); res.close()

@@ -219,10 +219,10 @@ __host__ __device__ __forceinline__ TileBox heat_tile_box(int64_t nx, int64_t ny
 // Tile tasks use HALO strips: a strip based at rbase (multiple of VEC) writes the rows
 // [rbase, rbase + 32*VEC) it loads; lanes 0 and 31 fetch the north/south halo cell of each
 // column. A 128-row FP64 tile is then exactly two strips (overlapping strips would need three).
-template <typename T, int VEC, int PF, bool CG, bool FAST>
+template <typename T, int VEC, int PF, bool CG>
 __device__ __forceinline__ void heat_strip_halo_impl(const T * __restrict__ src, T * __restrict__ dst, int64_t ld,
                                                      int64_t nx, int64_t rbase, int64_t rx0, int64_t rx1,
-                                                     int64_t cy0, int64_t cy1, double c, bool vec_ok, int pfd)
+                                                     int64_t cy0, int64_t cy1, double c, int pfd)
 {
     const int lane = threadIdx.x & 31;
     const int64_t r = rbase + (int64_t) lane * VEC;
@@ -241,34 +241,32 @@ __device__ __forceinline__ void heat_strip_halo_impl(const T * __restrict__ src,
     const bool h_row_ok = h_south ? rs < nx : rn >= 0;
     const int64_t h_row = h_south ? rs : rn;
     const bool lane_rows = (r + VEC > rx0) && (r < rx1);
-    const bool full_store = vec_ok && r >= rx0 && r + VEC <= rx1;
+    const bool full_store = r >= rx0 && r + VEC <= rx1;
+    // lanes past the grid's last rows load the last vector of the column again
+    const int64_t r_last = ((nx - 1) / VEC) * VEC, r_load = r < r_last ? r : r_last;
     // the L2 prefetch of a column covers the strip AND its halo rows (VEC rows on each side keep
     // the 16-byte alignment), so the lanes' halo loads hit L2 like the strip's own loads
     const int64_t pf_lo = rbase >= VEC ? rbase - VEC : 0;
     int64_t pf_hi = rbase + 33 * VEC; if (pf_hi > nx) pf_hi = nx;
     const uint32_t pf_bytes = (uint32_t) (((pf_hi - pf_lo) * (int64_t) sizeof(T)) & ~(int64_t) 15);
-    const bool pf_on = pfd > 0 && vec_ok && pf_hi > pf_lo && pf_bytes > 0;
-    const T * __restrict__ sp = src + r;
+    const bool pf_on = pfd > 0 && pf_hi > pf_lo && pf_bytes > 0;
+    const T * __restrict__ sp = src + r_load;
     T * __restrict__ dp = dst + r;
     auto load = [&](int64_t j) -> Cells<T, VEC> {
-        if constexpr (FAST) {
-            Cells<T, VEC> q;
-            const T * p = sp + j * ld;
-            if constexpr (VEC == 2 && sizeof(T) == 8) {
-                double2 v = CG ? __ldcg((const double2 *) p) : __ldg((const double2 *) p);
-                q.v[0] = v.x; q.v[1] = v.y;
-            } else if constexpr (VEC == 4 && sizeof(T) == 8) {
-                double2 a = CG ? __ldcg((const double2 *) p) : __ldg((const double2 *) p);
-                double2 b = CG ? __ldcg((const double2 *) p + 1) : __ldg((const double2 *) p + 1);
-                q.v[0] = a.x; q.v[1] = a.y; q.v[2] = b.x; q.v[3] = b.y;
-            } else {
-                float4 v = CG ? __ldcg((const float4 *) p) : __ldg((const float4 *) p);
-                q.v[0] = v.x; q.v[1] = v.y; q.v[2] = v.z; q.v[3] = v.w;
-            }
-            return q;
+        Cells<T, VEC> q;
+        const T * p = sp + j * ld;
+        if constexpr (VEC == 2 && sizeof(T) == 8) {
+            double2 v = CG ? __ldcg((const double2 *) p) : __ldg((const double2 *) p);
+            q.v[0] = v.x; q.v[1] = v.y;
+        } else if constexpr (VEC == 4 && sizeof(T) == 8) {
+            double2 a = CG ? __ldcg((const double2 *) p) : __ldg((const double2 *) p);
+            double2 b = CG ? __ldcg((const double2 *) p + 1) : __ldg((const double2 *) p + 1);
+            q.v[0] = a.x; q.v[1] = a.y; q.v[2] = b.x; q.v[3] = b.y;
         } else {
-            return ld_cells<T, VEC, CG>(src, ld, nx, r, j, vec_ok);
+            float4 v = CG ? __ldcg((const float4 *) p) : __ldg((const float4 *) p);
+            q.v[0] = v.x; q.v[1] = v.y; q.v[2] = v.z; q.v[3] = v.w;
         }
+        return q;
     };
     Cells<T, VEC> west = load(cy0 - 1);
     Cells<T, VEC> cur  = load(cy0);
@@ -346,23 +344,72 @@ __device__ __forceinline__ void heat_strip_halo_impl(const T * __restrict__ src,
     if (j0 < cy1) block(j0, std::false_type{});
 }
 
-template <typename T, int VEC, int PF, bool CG>
-__device__ __noinline__ void heat_strip_halo_edge(const T * __restrict__ src, T * __restrict__ dst, int64_t ld,
-                                                  int64_t nx, int64_t rbase, int64_t rx0, int64_t rx1,
-                                                  int64_t cy0, int64_t cy1, double c, bool vec_ok, int pfd)
+// The strip of a grid whose rows do not start on 16-byte boundaries (or whose last vector is
+// unsafe to load, see Strips): lane l holds rows rbase + 32 e + l, e < E, so that a warp's
+// load or store of one e is 32 consecutive elements whatever the alignment. (Four consecutive rows
+// per lane, loaded element by element, made four requests of every 512 bytes: 8191 x 4001 FP32 graph
+// 126 us per step against 68.) Neighbours come by rotating each e through the warp: lane 0's north is the previous e's
+// lane 31, lane 31's south the next e's lane 0; rows rbase - 1 and rbase + 32 E are loaded by lanes 0
+// and 31. Rows past the grid load its last row and are not written.
+template <typename T, int E, int PF, bool CG>
+__device__ __forceinline__ void heat_strip_rows(const T * __restrict__ src, T * __restrict__ dst, int64_t ld, int64_t nx, int64_t rbase,
+                                             int64_t rx0, int64_t rx1, int64_t cy0, int64_t cy1, double c)
 {
-    heat_strip_halo_impl<T, VEC, 2, CG, false>(src, dst, ld, nx, rbase, rx0, rx1, cy0, cy1, c, vec_ok, pfd);
-}
-
-template <typename T, int VEC, int PF, bool CG>
-__device__ __forceinline__ void heat_strip_halo(const T * __restrict__ src, T * __restrict__ dst, int64_t ld,
-                                                int64_t nx, int64_t rbase, int64_t rx0, int64_t rx1,
-                                                int64_t cy0, int64_t cy1, double c, bool vec_ok, int pfd)
-{
-    if (vec_ok && rbase >= 0 && rbase + 32 * VEC <= nx)
-        heat_strip_halo_impl<T, VEC, PF, CG, true>(src, dst, ld, nx, rbase, rx0, rx1, cy0, cy1, c, vec_ok, pfd);
-    else
-        heat_strip_halo_edge<T, VEC, PF, CG>(src, dst, ld, nx, rbase, rx0, rx1, cy0, cy1, c, vec_ok, pfd);
+    const int lane = threadIdx.x & 31;
+    int off[E];                                          // row offsets from rbase
+    unsigned wmask = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+    {
+        const int64_t r = rbase + e * 32 + lane;
+        off[e] = (int) ((r < nx - 1 ? r : nx - 1) - rbase);
+        if (r >= rx0 && r < rx1) wmask |= 1u << e;
+    }
+    const bool has_h = (lane == 0 && rbase > 0) || (lane == 31 && rbase + 32 * E < nx);
+    const int hoff = lane == 0 ? -1 : 32 * E;
+    const T * __restrict__ sp = src + rbase;
+    T * __restrict__ dp = dst + rbase;
+    struct Col { T v[E]; T h; };
+    auto load = [&](int64_t j) -> Col {
+        Col q;
+        const T * p = sp + j * ld;
+#pragma unroll
+        for (int e = 0; e < E; ++e) q.v[e] = ld_scalar<CG>(p + off[e]);
+        q.h = has_h ? ld_scalar<CG>(p + hoff) : T(0);
+        return q;
+    };
+    Col west = load(cy0 - 1), cur = load(cy0);
+    for (int64_t j0 = cy0; j0 < cy1; j0 += PF)
+    {
+        Col nxt[PF];
+#pragma unroll
+        for (int k = 0; k < PF; ++k)
+            if (j0 + k + 1 <= cy1) nxt[k] = load(j0 + k + 1);
+#pragma unroll
+        for (int k = 0; k < PF; ++k)
+        {
+            const int64_t jc = j0 + k;
+            if (jc >= cy1) break;                        // warp-uniform
+            T up[E], dn[E];
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+            {
+                up[e] = __shfl_sync(0xffffffffu, cur.v[e], (lane + 31) & 31);
+                dn[e] = __shfl_sync(0xffffffffu, cur.v[e], (lane + 1) & 31);
+            }
+            T * q = dp + jc * ld;
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+            {
+                const T n = lane == 0 ? (e == 0 ? cur.h : up[e > 0 ? e - 1 : 0]) : up[e];
+                const T s = lane == 31 ? (e == E - 1 ? cur.h : dn[e < E - 1 ? e + 1 : E - 1]) : dn[e];
+                const T out = (T) heat_update((double) cur.v[e], (double) n, (double) s, (double) west.v[e], (double) nxt[k].v[e], c);
+                if (wmask >> e & 1u) q[off[e]] = out;
+            }
+            west = cur;
+            cur = nxt[k];
+        }
+    }
 }
 
 // Strips a tile box splits into when `nwarps` warps share it: row groups of 32*VEC rows
@@ -382,15 +429,10 @@ __host__ __device__ __forceinline__ void heat_tile_split(const TileBox & b, int 
     cols_per = (int) ((cols + n - 1) / n);
 }
 
-// A team of `nwarps` warps (warp index `warp` within the team) executes one tile task: the
-// warps take the tile's strips round-robin.
-template <typename T, int VEC, int PF, bool CG>
-__device__ __forceinline__ void heat_tile_team(const T * src, T * dst, int64_t ld, int64_t nx, int64_t ny,
-                                               int64_t x0, int64_t x1, int64_t y0, int64_t y1, double c, bool vec_ok,
-                                               int pfd, int warp, int nwarps)
+// The strips of warp `warp` of `nwarps` that share a tile box, taken round-robin: strip(rbase, cy0, cy1).
+template <int VEC, typename Strip>
+__device__ __forceinline__ void heat_tile_strips(const TileBox & b, int warp, int nwarps, Strip && strip)
 {
-    const TileBox b = heat_tile_box(nx, ny, x0, x1, y0, y1);
-    if (b.rx0 >= b.rx1 || b.cy0 >= b.cy1) return;
     int64_t rbase0; int nrg, ncg, cols_per;
     heat_tile_split<VEC>(b, nwarps, rbase0, nrg, ncg, cols_per);
     for (int s = warp; s < nrg * ncg; s += nwarps)
@@ -398,9 +440,46 @@ __device__ __forceinline__ void heat_tile_team(const T * src, T * dst, int64_t l
         const int cg = (int) ((uint32_t) s / (uint32_t) nrg), rg = s - cg * nrg;
         const int64_t cy0 = b.cy0 + (int64_t) cg * cols_per;
         int64_t cy1 = cy0 + cols_per; if (cy1 > b.cy1) cy1 = b.cy1;
-        if (cy0 >= cy1) continue;
-        heat_strip_halo<T, VEC, PF, CG>(src, dst, ld, nx, rbase0 + (int64_t) rg * 32 * VEC, b.rx0, b.rx1, cy0, cy1, c, vec_ok, pfd);
+        if (cy0 < cy1) strip(rbase0 + (int64_t) rg * 32 * VEC, cy0, cy1);
     }
+}
+
+// The same strip in its own frame, few columns ahead: for the rare strips of a kernel built around
+// the vector strips (a callee with many registers makes the caller spill around every call).
+template <typename T, int E, bool CG>
+__device__ __noinline__ void heat_strip_rows_call(const T * __restrict__ src, T * __restrict__ dst, int64_t ld, int64_t nx, int64_t rbase,
+                                                  int64_t rx0, int64_t rx1, int64_t cy0, int64_t cy1, double c)
+{
+    heat_strip_rows<T, E, sizeof(T) == 8 ? 1 : 2, CG>(src, dst, ld, nx, rbase, rx0, rx1, cy0, cy1, c);
+}
+
+// Columns ahead of a strip in a kernel that holds nothing but heat_strip_rows.
+// (8191 x 4001 graph, us per step: FP64 2 / 3 / 4 columns 105 / 99 / 145, FP32 3 / 4 / 5 / 6 columns
+// 74 / 69 / 68 / 66, but 1027 x 1030 7.3 / 7.0 / 7.0 / 7.2)
+template <typename T> constexpr int ROWS_PF = sizeof(T) == 8 ? 3 : 5;
+
+// Which strips a kernel holds: VECTOR, the vector strips, with a call to the others (vec_ok: ld and
+// both base pointers allow aligned 16-byte accesses; a strip's last vector may run past row nx - 1 into
+// the column's padding, except in the grid's last column, which may end the allocation); ROWS, the
+// row-by-row strips alone, for any grid.
+enum class Strips { VECTOR, ROWS };
+
+// A team of `nwarps` warps (warp index `warp` within the team) executes one tile task.
+template <typename T, int VEC, int PF, bool CG, Strips K = Strips::VECTOR>
+__device__ __forceinline__ void heat_tile_team(const T * src, T * dst, int64_t ld, int64_t nx, int64_t ny,
+                                               int64_t x0, int64_t x1, int64_t y0, int64_t y1, double c, bool vec_ok,
+                                               int pfd, int warp, int nwarps)
+{
+    const TileBox b = heat_tile_box(nx, ny, x0, x1, y0, y1);
+    if (b.rx0 >= b.rx1 || b.cy0 >= b.cy1) return;
+    heat_tile_strips<VEC>(b, warp, nwarps, [&](int64_t rbase, int64_t cy0, int64_t cy1) {
+        if constexpr (K == Strips::ROWS)
+            heat_strip_rows<T, VEC, PF, CG>(src, dst, ld, nx, rbase, b.rx0, b.rx1, cy0, cy1, c);
+        else if (vec_ok && (rbase + 32 * VEC <= nx || nx % VEC == 0 || cy1 < ny - 1))
+            heat_strip_halo_impl<T, VEC, PF, CG>(src, dst, ld, nx, rbase, b.rx0, b.rx1, cy0, cy1, c, pfd);
+        else
+            heat_strip_rows_call<T, VEC, CG>(src, dst, ld, nx, rbase, b.rx0, b.rx1, cy0, cy1, c);
+    });
 }
 
 // A whole CTA executes one tile task.

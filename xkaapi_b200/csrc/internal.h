@@ -16,9 +16,10 @@ uint64_t xkb_internal_issued_host_copies();
 int xkb_internal_plan_execute_cut(const xkb_copy_t * copies, size_t n, void * const * alloc_ptrs, size_t nallocs,
                                   cudaStream_t stream, const uint64_t * cuts, size_t ncuts);
 
-// Set a scheduler's descriptors on the device only (persistent forms only; no host copy).
-// checked: the caller validated every descriptor with xkb_internal_task_valid.
-int xkb_internal_sched_set_tasks_device(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks, bool checked);
+// Set a scheduler's descriptors on the device only (persistent forms only; no host copy). The
+// caller validated every descriptor with xkb_internal_task_valid; bodies: every task's
+// xkb_internal_body_of, or-ed.
+int xkb_internal_sched_set_tasks_device(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks, unsigned bodies);
 
 #ifdef __CUDACC__
 #define XKB_HD __host__ __device__
@@ -42,6 +43,23 @@ static inline XKB_HD bool xkb_internal_task_valid(const xkb_task_desc_t & d)
         return a.lo >= 0 && a.lo <= a.hi && (a.hi == a.lo || (a.x && a.y));
     }
     return d.kind == XKB_TASK_NOOP;
+}
+
+// The body a task needs in the persistent kernels: FP64 or FP32 heat tiles of grids that allow aligned
+// 16-byte accesses or of any grid (row by row), axpby; 0 for a task without a body. The scheduler runs
+// a kernel built for the bodies its tasks need.
+constexpr unsigned XKB_BODY_F64 = 1, XKB_BODY_F32 = 2, XKB_BODY_ROWS64 = 4, XKB_BODY_ROWS32 = 8, XKB_BODY_AXPBY = 16, XKB_BODY_ALL = 31;
+static inline unsigned xkb_internal_body_of(const xkb_task_desc_t & d)
+{
+    const auto & h = d.u.heat;
+    const bool aligned = h.src % 16 == 0 && h.dst % 16 == 0;
+    switch (d.kind)
+    {
+        case XKB_TASK_HEAT_F64: return aligned && h.ld % 2 == 0 ? XKB_BODY_F64 : XKB_BODY_ROWS64;
+        case XKB_TASK_HEAT_F32: return aligned && h.ld % 4 == 0 ? XKB_BODY_F32 : XKB_BODY_ROWS32;
+        case XKB_TASK_AXPBY: return XKB_BODY_AXPBY;
+        default: return 0;
+    }
 }
 
 // Host threads for the parallel passes of background work (resolution, coherency, descriptor
@@ -77,10 +95,10 @@ int xkb_internal_resolver_window_graph(xkb_resolver_t * R, const xkb_edge_mark_t
 // descriptors are copied in stream order (host memory may be pageable), the launch's status and
 // executed count are added to the scheduler's running totals, read and cleared by
 // xkb_internal_sched_windows_wait.
-int xkb_internal_sched_run_window(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks, const xkb_task_graph_t * g);
+int xkb_internal_sched_run_window(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks, unsigned bodies, const xkb_task_graph_t * g);
 // The two halves of a window run: the descriptors' copy (queued now, so that it can go ahead of
 // the window's graph), then the launch on the graph of the same ntasks tasks.
-int xkb_internal_sched_upload_window(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks);
+int xkb_internal_sched_upload_window(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks, unsigned bodies);
 int xkb_internal_sched_launch_window(xkb_sched_t * S, const xkb_task_graph_t * g);
 int xkb_internal_sched_windows_wait(xkb_sched_t * S, uint64_t * executed);
 

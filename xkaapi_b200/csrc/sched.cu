@@ -87,7 +87,7 @@ static_assert((1 << TEAM_LOG2) * 32 == SCHED_THREADS, "a team is a CTA");
 
 constexpr int SCHED_BULK_NBUF = 8;       // staged columns in flight per warp (bulk tile body)
 #ifndef XKB_TILE_PF
-#define XKB_TILE_PF 6                    // east columns an FP32 tile strip loads ahead into registers
+#define XKB_TILE_PF 5                    // (4, 6, 8: 111, 108, 111 us per step of the 8192^2 graph; 5: 107) east columns an FP32 tile strip loads ahead into registers
 #endif
 #ifndef XKB_F64_VEC
 #define XKB_F64_VEC 4                    // rows per lane of the FP64 tile body: one warp covers 128 rows
@@ -118,37 +118,67 @@ __device__ __forceinline__ void axpby_piece(int64_t lo, int64_t hi, int unit, in
     phi = plo + per < hi ? plo + per : hi;
 }
 
+// Which task bodies a kernel holds. A kernel of one body keeps all of the SM's registers for it: with
+// both heat bodies and the row-by-row strips in one kernel every tile pays for what the others spill:
+// with the row-by-row strips of 3 and 4 columns ahead called from one kernel for all, the 8192^2 FP32
+// graph took 132 us per step, alone 107; 8191 x 4001 (odd ld) FP32 123 against 68, FP64 135 against 99.
+enum class Body { ANY, F64, F32, ROWS64, ROWS32, AXPBY };
+
+// The kernel for tasks that need the bodies `seen` (XKB_BODY_*).
+static inline Body body_for(unsigned seen)
+{
+    switch (seen)
+    {
+        case 0: case XKB_BODY_F64: return Body::F64;
+        case XKB_BODY_F32: return Body::F32;
+        case XKB_BODY_ROWS64: return Body::ROWS64;
+        case XKB_BODY_ROWS32: return Body::ROWS32;
+        case XKB_BODY_AXPBY: return Body::AXPBY;
+        default: return Body::ANY;
+    }
+}
+
 // Run unit `unit` of the `nunits` (a power of two) a task is split into, with one warp. PF64, PF32:
-// columns a heat strip loads ahead into registers.
-template <int PF64, int PF32>
+// columns a heat strip loads ahead into registers. A kernel of one body passes the other kinds by:
+// the host chose it for tasks that have none.
+template <Body B, int PF64, int PF32>
 __device__ __forceinline__ void run_unit(const xkb_task_desc_t & d, int unit, int nunits, int pfd)
 {
-    switch (d.kind)
-    {
-        case XKB_TASK_HEAT_F64: {
-            const auto & h = d.u.heat;
+    const auto & h = d.u.heat;
+    if constexpr (B == Body::ANY || B == Body::F64)
+        if (d.kind == XKB_TASK_HEAT_F64)
+        {
             const bool vok = (h.ld % 2 == 0) && (h.src % 16 == 0) && (h.dst % 16 == 0);
             heat_tile_team<double, XKB_F64_VEC, PF64, true>((const double *) h.src, (double *) h.dst, h.ld, h.nx, h.ny,
                                                h.x0, h.x1, h.y0, h.y1, h.c, vok, pfd, unit, nunits);
-            break;
+            return;
         }
-        case XKB_TASK_HEAT_F32: {
-            const auto & h = d.u.heat;
+    if constexpr (B == Body::ROWS64)
+        if (d.kind == XKB_TASK_HEAT_F64)
+            heat_tile_team<double, XKB_F64_VEC, ROWS_PF<double>, true, Strips::ROWS>((const double *) h.src, (double *) h.dst, h.ld, h.nx, h.ny,
+                                               h.x0, h.x1, h.y0, h.y1, h.c, false, 0, unit, nunits);
+    if constexpr (B == Body::ANY || B == Body::F32)
+        if (d.kind == XKB_TASK_HEAT_F32)
+        {
             const bool vok = (h.ld % 4 == 0) && (h.src % 16 == 0) && (h.dst % 16 == 0);
             // an FP32 column is half the bytes of an FP64 one: prefetch twice as many columns ahead
             heat_tile_team<float, 4, PF32, true>((const float *) h.src, (float *) h.dst, h.ld, h.nx, h.ny,
                                               h.x0, h.x1, h.y0, h.y1, h.c, vok, 2 * pfd, unit, nunits);
-            break;
+            return;
         }
-        case XKB_TASK_AXPBY: {
+    if constexpr (B == Body::ROWS32)
+        if (d.kind == XKB_TASK_HEAT_F32)
+            heat_tile_team<float, 4, ROWS_PF<float>, true, Strips::ROWS>((const float *) h.src, (float *) h.dst, h.ld, h.nx, h.ny,
+                                              h.x0, h.x1, h.y0, h.y1, h.c, false, 0, unit, nunits);
+    if constexpr (B == Body::ANY || B == Body::AXPBY)
+        if (d.kind == XKB_TASK_AXPBY)
+        {
             const auto & a = d.u.axpby;
             int64_t lo, hi;
             axpby_piece(a.lo, a.hi, unit, nunits, lo, hi);
             axpby_team<true>(lo, hi, a.a, (const double *) a.x, a.b, (double *) a.y, threadIdx.x & 31, 32);
-            break;
         }
-        default: break;   // XKB_TASK_NOOP (first-touch / placement tasks)
-    }
+    // (XKB_TASK_NOOP: first-touch / placement tasks)
 }
 
 __device__ __forceinline__ int atom_add_acq_rel(int * p, int v)
@@ -163,7 +193,7 @@ __device__ __forceinline__ int atom_add_acq_rel(int * p, int v)
 // Head and tail have cache lines of their own: every warp's ticket and every release is an atomic there.
 // CTR_EXECUTED counts units of an in-order run, tasks of a queue run (executed_tasks).
 enum { CTR_HEAD = 0, CTR_TAIL = 32, CTR_STATUS = 48, CTR_EXECUTED, CTR_BAD_TASK, CTR_SEEDS, CTR_SEED_LAST, CTR_SEED_DEG, CTR_SEED_PIECES,
-       CTR_SEED_HEAT, CTR_QUEUE, CTR_SPLIT, CTR_TEAM, CTR_COUNT = 64 };
+       CTR_SEED_HEAT, CTR_QUEUE, CTR_SPLIT, CTR_TEAM, CTR_RUN, CTR_COUNT = 64 };
 
 // A run covers `ntasks` tasks numbered w * period + t (window w, task t of the window's
 // `period` descriptors). A plain graph is one window (period = ntasks); a periodic graph adds
@@ -311,7 +341,35 @@ __global__ void sched_plan_kernel(SchedArgs a, unsigned warps)
         for (uint32_t i = a.succ_ptr[t], e = a.succ_ptr[t + 1], b = t / W; i < e; ++i) ok = ok && a.succ[i] / W > b;
     }
     if (!ok && *(volatile unsigned *) (a.ctr + CTR_QUEUE) == 0) atomicExch(a.ctr + CTR_QUEUE, 1u);
+    // the first place among the ready tasks where the tiles' rows change (block_order); ~ so that 0 is none
+    if (ok && t + 1 < W && a.ctr[CTR_SEED_HEAT] == W && a.tasks[t].u.heat.x0 != a.tasks[t + 1].u.heat.x0)
+        atomicMax(a.ctr + CTR_RUN, ~(t + 1));
 }
+
+// Order of the tasks of a block in an in-order run. Tiles spawned column by column within a row of
+// tiles (the examples' loop: consecutive tasks work on the same 1 KB of every column) are taken row by
+// row within a column of tiles instead, so that the tasks in flight read and write whole columns,
+// which are contiguous (16384^2 FP64 graph 698 -> 658 us per step, 6.53 TB/s; 8192^2 175 -> 168). Any order of a block is valid, its tasks are
+// independent; a part of a block keeps spawn order.
+struct BlockOrder {
+    uint32_t W, rows, cols, whole;         // tiles: rows x cols per block; tasks in whole blocks
+
+    __device__ __forceinline__ BlockOrder(const SchedArgs & a)
+    {
+        W = a.ctr[CTR_SEEDS];
+        const uint32_t run = a.ctr[CTR_RUN] ? ~a.ctr[CTR_RUN] : 0u;
+        const bool grid = run > 1 && W % run == 0;
+        cols = grid ? run : 1u;
+        rows = grid ? W / run : 1u;
+        whole = grid ? a.ntasks - a.ntasks % W : 0u;
+    }
+    __device__ __forceinline__ uint32_t task(uint32_t slot) const
+    {
+        if (slot >= whole) return slot;
+        const uint32_t b = slot / W, p = slot - b * W, c = p / rows, r = p - c * rows;
+        return b * W + r * cols + c;
+    }
+};
 
 // Whether sched_team_kernel has the run.
 __device__ __forceinline__ bool team_run(const SchedArgs & a) { return a.ctr[CTR_TEAM] != 0 && a.ctr[CTR_QUEUE] == 0; }
@@ -458,7 +516,7 @@ __device__ __forceinline__ int wait_published(const int * p, unsigned * status, 
 // Dynamic shared memory of the BULK variant with NBUF slots per warp: the slots, then the mbarriers.
 constexpr size_t bulk_smem_bytes(int nbuf) { return (size_t) (SCHED_THREADS / 32) * nbuf * (BULK_SLOT_BYTES + 8); }
 
-template <bool BULK, int NBUF = SCHED_BULK_NBUF>
+template <Body B, bool BULK = false, int NBUF = SCHED_BULK_NBUF>
 __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_persistent_kernel(SchedArgs a)
 {
     constexpr int NWARPS = SCHED_THREADS / 32;
@@ -477,6 +535,7 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_persisten
     }
     // (a check before the run that failed left its status: nothing runs)
     if (team_run(a) || *(volatile unsigned *) (a.ctr + CTR_STATUS) != 0) return;
+    const BlockOrder order(a);
     unsigned ticket = 0;
     if (lane == 0) ticket = atomicAdd(a.ctr + CTR_HEAD, 1u);
     for (;;)
@@ -485,7 +544,7 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_persisten
         const uint32_t slot = ticket >> k;
         const int unit = (int) (ticket & (nunits - 1));
         if (slot >= a.ntasks) break;
-        int t = (int) slot;
+        int t = (int) order.task(slot);
         if (!inorder)
         {
             if (lane == 0) t = wait_published(a.queue + slot, a.ctr + CTR_STATUS, a.timeout_ns);
@@ -527,10 +586,10 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_persisten
                                                          h.y0, h.y1, h.c, unit, nunits, ring, xkb_globaltimer() + a.timeout_ns))
                     atomicCAS(a.ctr + CTR_STATUS, 0u, (unsigned) -XKB_ETIMEDOUT);
             }
-            if (!done) run_unit<XKB_F64_PF, XKB_TILE_PF>(d, unit, nunits, a.pfd);
+            if (!done) run_unit<B, XKB_F64_PF, XKB_TILE_PF>(d, unit, nunits, a.pfd);
         }
         else
-            run_unit<XKB_F64_PF, XKB_TILE_PF>(d, unit, nunits, a.pfd);
+            run_unit<B, XKB_F64_PF, XKB_TILE_PF>(d, unit, nunits, a.pfd);
         // the next ticket arrives while the fence waits for the unit's stores
         if (lane == 0) ticket = atomicAdd(a.ctr + CTR_HEAD, 1u);
         __syncwarp();
@@ -562,6 +621,7 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_persisten
 // tickets and counter updates of one warp per unit, whose atomics are what bounds a step of a few
 // microseconds (1024^2 FP64, 64 tiles of 32 units: 5.4 us per step against 11.2). Every run launches
 // both kernels, and the one that does not have it returns at once.
+template <Body B>
 __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_team_kernel(SchedArgs a)
 {
     constexpr int NWARPS = SCHED_THREADS / 32;
@@ -596,7 +656,7 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_team_kern
         }
         __syncthreads();
         if (!ready) break;
-        run_unit<TEAM_PF, TEAM_PF>(d, unit, nunits, 0);
+        run_unit<B, TEAM_PF, TEAM_PF>(d, unit, nunits, 0);
         __syncthreads();                                       // the group's units are done
         ++executed;
         if (warp != 0) continue;
@@ -605,6 +665,14 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_team_kern
         count_down_successors(g, t, first, more, a.wc, lane);
     }
     if (lane == 0 && executed) atomicAdd(a.ctr + CTR_EXECUTED, executed);
+}
+
+// Both kernels of a run (see sched_team_kernel); teams are of heat tiles only.
+template <Body B>
+static void launch_run(const SchedArgs & a, unsigned grid, cudaStream_t stream)
+{
+    sched_persistent_kernel<B><<<grid, SCHED_THREADS, 0, stream>>>(a);
+    if constexpr (B != Body::AXPBY) sched_team_kernel<B><<<grid, SCHED_THREADS, 0, stream>>>(a);
 }
 
 // per-task kernels (PLAIN and GRAPH forms)
@@ -675,6 +743,7 @@ struct xkb_sched {
     cudaStream_t stream = nullptr;
     std::vector<xkb_task_desc_t> host_tasks;  // host copy for the per-task forms (empty: device only)
     size_t ntasks = 0;                        // descriptors set
+    unsigned bodies = XKB_BODY_ALL;           // the bodies they need
     Dev<xkb_task_desc_t> tasks;
     Dev<int> wc, queue;                       // wc: wait counters, then the units done of each task
     Dev<unsigned> ctr;
@@ -698,9 +767,11 @@ struct xkb_sched {
     }
 };
 
-static int check_tasks(const xkb_task_desc_t * t, size_t n)
+static int check_tasks(const xkb_task_desc_t * t, size_t n, unsigned & bodies)
 {
+    bodies = 0;
     for (size_t i = 0; i < n; ++i)
+    {
         if (!xkb_internal_task_valid(t[i]))
         {
             const uint32_t k = t[i].kind;
@@ -708,6 +779,8 @@ static int check_tasks(const xkb_task_desc_t * t, size_t n)
             if (k == XKB_TASK_AXPBY) return xkb_set_error(XKB_EINVAL, "sched: task %zu: bad axpby range", i);
             return xkb_set_error(XKB_EINVAL, "sched: task %zu: unknown kind %u", i, k);
         }
+        bodies |= xkb_internal_body_of(t[i]);
+    }
     return XKB_OK;
 }
 
@@ -722,7 +795,7 @@ extern "C" int xkb_sched_create(xkb_sched_t ** out, void * stream)
     S->stream = (cudaStream_t) stream;
     int sms = 148, per = 2;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sched_persistent_kernel<false>, SCHED_THREADS, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sched_persistent_kernel<Body::ANY>, SCHED_THREADS, 0);
     S->grid = sms * (per > 0 ? per : 1);
     *out = S;
     return XKB_OK;
@@ -737,8 +810,10 @@ extern "C" int xkb_sched_destroy(xkb_sched_t * S)
 extern "C" int xkb_sched_set_tasks(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks)
 {
     if (!S || (ntasks && !tasks)) return xkb_set_error(XKB_EINVAL, "sched_set_tasks: bad arguments");
-    int rc = check_tasks(tasks, ntasks);
+    unsigned bodies;
+    int rc = check_tasks(tasks, ntasks, bodies);
     if (rc) return rc;
+    S->bodies = bodies;
     S->host_tasks.assign(tasks, tasks + ntasks);
     S->ntasks = ntasks;
     if ((rc = S->tasks.reserve(ntasks ? ntasks : 1))) return rc;
@@ -752,11 +827,11 @@ extern "C" int xkb_sched_set_tasks(xkb_sched_t * S, const xkb_task_desc_t * task
 
 // Library-internal: the descriptors go to the device only (no host copy, so only the persistent
 // forms can run them); for callers that hand over millions of descriptors for one run.
-int xkb_internal_sched_set_tasks_device(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks, bool checked)
+int xkb_internal_sched_set_tasks_device(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks, unsigned bodies)
 {
     if (!S || (ntasks && !tasks)) return xkb_set_error(XKB_EINVAL, "sched_set_tasks: bad arguments");
-    int rc = checked ? XKB_OK : check_tasks(tasks, ntasks);
-    if (rc) return rc;
+    int rc;
+    S->bodies = bodies;
     S->host_tasks.clear(); S->host_tasks.shrink_to_fit();
     S->ntasks = ntasks;
     if ((rc = S->tasks.reserve(ntasks ? ntasks : 1))) return rc;
@@ -809,8 +884,8 @@ static int launch_persistent(xkb_sched * S, SchedArgs & a);
 static int launch_bulk(xkb_sched * S, SchedArgs & a)
 {
     const size_t smem = bulk_smem_bytes(SCHED_BULK_NBUF);
-    XKB_CUDA_TRY(cudaFuncSetAttribute(sched_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-    sched_persistent_kernel<true><<<S->grid, SCHED_THREADS, smem, S->stream>>>(a);
+    XKB_CUDA_TRY(cudaFuncSetAttribute(sched_persistent_kernel<Body::ANY, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    sched_persistent_kernel<Body::ANY, true><<<S->grid, SCHED_THREADS, smem, S->stream>>>(a);
     return XKB_OK;
 }
 
@@ -865,10 +940,15 @@ static int launch_persistent(xkb_sched * S, SchedArgs & a)
             if (rc) return rc;
         }
         else
-        {
-            sched_persistent_kernel<false><<<S->grid, SCHED_THREADS, 0, S->stream>>>(a);
-            sched_team_kernel<<<S->grid, SCHED_THREADS, 0, S->stream>>>(a);
-        }
+            switch (body_for(S->bodies))
+            {
+                case Body::F64: launch_run<Body::F64>(a, S->grid, S->stream); break;
+                case Body::F32: launch_run<Body::F32>(a, S->grid, S->stream); break;
+                case Body::ROWS64: launch_run<Body::ROWS64>(a, S->grid, S->stream); break;
+                case Body::ROWS32: launch_run<Body::ROWS32>(a, S->grid, S->stream); break;
+                case Body::AXPBY: launch_run<Body::AXPBY>(a, S->grid, S->stream); break;
+                default: launch_run<Body::ANY>(a, S->grid, S->stream);
+            }
         XKB_CUDA_TRY(cudaEventRecord(S->ev[1], S->stream));
     }
     XKB_CUDA_TRY(cudaGetLastError());
@@ -987,7 +1067,7 @@ int xkb_internal_sched_reserve(xkb_sched_t * S, size_t ntasks)
     return XKB_OK;
 }
 
-int xkb_internal_sched_upload_window(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks)
+int xkb_internal_sched_upload_window(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks, unsigned bodies)
 {
     if (!S || (ntasks && !tasks) || ntasks >= (size_t(1) << 31)) return xkb_set_error(XKB_EINVAL, "sched_upload_window: bad arguments");
     int rc;
@@ -1001,6 +1081,7 @@ int xkb_internal_sched_upload_window(xkb_sched_t * S, const xkb_task_desc_t * ta
     if (ntasks) XKB_CUDA_TRY(cudaMemcpyAsync(S->tasks.p, tasks, ntasks * sizeof(xkb_task_desc_t), cudaMemcpyHostToDevice, S->stream));
     S->host_tasks.clear();
     S->ntasks = ntasks;
+    S->bodies = bodies;
     S->graph_key = nullptr;
     return XKB_OK;
 }
@@ -1027,11 +1108,11 @@ int xkb_internal_sched_launch_window(xkb_sched_t * S, const xkb_task_graph_t * g
     return XKB_OK;
 }
 
-int xkb_internal_sched_run_window(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks, const xkb_task_graph_t * g)
+int xkb_internal_sched_run_window(xkb_sched_t * S, const xkb_task_desc_t * tasks, size_t ntasks, unsigned bodies, const xkb_task_graph_t * g)
 {
     if (!S || (ntasks && !tasks) || !g || g->ntasks != ntasks || ntasks >= (size_t(1) << 31))
         return xkb_set_error(XKB_EINVAL, "sched_run_window: bad arguments");
-    int rc = xkb_internal_sched_upload_window(S, tasks, ntasks);
+    int rc = xkb_internal_sched_upload_window(S, tasks, ntasks, bodies);
     return rc ? rc : xkb_internal_sched_launch_window(S, g);
 }
 
@@ -1147,7 +1228,7 @@ static int noalloc_scratch(int ** out)
         cudaFuncAttributes fa;
         const void * kernels[] = {(const void *) noalloc_check_kernel, (const void *) sched_init_kernel,
                                   (const void *) sched_seed_kernel, (const void *) sched_plan_kernel,
-                                  (const void *) sched_persistent_kernel<false>, (const void *) sched_team_kernel};
+                                  (const void *) sched_persistent_kernel<Body::ANY>, (const void *) sched_team_kernel<Body::ANY>};
         for (const void * k : kernels)
             if ((e = cudaFuncGetAttributes(&fa, k)) != cudaSuccess) return xkb_set_cuda_error(e);
         sl.ctx = ctx;
@@ -1195,14 +1276,13 @@ extern "C" int xkb_sched_run_noalloc(const xkb_task_desc_t * tasks, const xkb_ta
         int dev = 0, sms = 148, per = 2;
         XKB_CUDA_TRY(cudaGetDevice(&dev));
         XKB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        XKB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sched_persistent_kernel<false>, SCHED_THREADS, 0));
+        XKB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sched_persistent_kernel<Body::ANY>, SCHED_THREADS, 0));
         const unsigned grid = (unsigned) (sms * (per > 0 ? per : 1));
         noalloc_check_kernel<<<(n + 255) / 256, 256, 0, st>>>(tasks, n, a.ctr);
         sched_init_kernel<<<(n + 255) / 256, 256, 0, st>>>(a);
         sched_seed_kernel<<<(n + 255) / 256, 256, 0, st>>>(a);
         sched_plan_kernel<<<(n + 255) / 256, 256, 0, st>>>(a, grid * (SCHED_THREADS / 32));
-        sched_persistent_kernel<false><<<grid, SCHED_THREADS, 0, st>>>(a);
-        sched_team_kernel<<<grid, SCHED_THREADS, 0, st>>>(a);
+        launch_run<Body::ANY>(a, grid, st);
         XKB_CUDA_TRY(cudaGetLastError());
     }
     unsigned ctr[CTR_COUNT] = {};
@@ -1391,7 +1471,7 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) server_kernel(X
         const SuccGraph g{S.succ_ptr, S.succ, S.xsucc_ptr, S.xsucc, S.period, S.ntasks};
         bool more;
         const uint32_t first = g.first(l, base, lane, more);
-        run_unit<XKB_F64_PF, XKB_TILE_PF>(d, unit, nunits, S.pfd);
+        run_unit<Body::ANY, XKB_F64_PF, XKB_TILE_PF>(d, unit, nunits, S.pfd);
         __syncwarp();
         fence_acq_rel_gpu();
         if (nunits > 1)

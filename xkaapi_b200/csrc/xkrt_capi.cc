@@ -2163,9 +2163,10 @@ static void pin_args(xkb_runtime * R, size_t bytes)
 // vector pointers to the mirrors), into `out` when given. Otherwise dense args (one descriptor
 // per task, back to back) are rewritten in place (nothing reads them as args after that), or
 // `copy` receives them.
-// *descs points at the result; *long_axpby tells whether some axpby task must be split.
+// *descs points at the result; *long_axpby tells whether some axpby task must be split, *bodies
+// which bodies the tasks need (xkb_internal_body_of).
 static int translate_descs(xkb_runtime * R, size_t t0, size_t t1, std::vector<xkb_task_desc_t> & copy, xkb_task_desc_t ** descs,
-                           bool * long_axpby, xkb_task_desc_t * out = nullptr)
+                           bool * long_axpby, unsigned * bodies, xkb_task_desc_t * out = nullptr)
 {
     const size_t nt = t1 - t0;
     const bool dense_args = R->args_dense && !out;
@@ -2174,8 +2175,10 @@ static int translate_descs(xkb_runtime * R, size_t t0, size_t t1, std::vector<xk
     else if (!dense_args) { copy.resize(nt); d = copy.data(); }
     std::atomic<size_t> bad_args(SIZE_MAX), bad_ptr(SIZE_MAX);     // first failing task, if any
     std::atomic<bool> longa(false);
+    std::atomic<unsigned> seen(0);
     parallel_chunks(nt, [&](size_t b, size_t e) {
         RegionHint h;
+        unsigned mine = 0;
         for (size_t k = b; k < e; ++k)
         {
             const size_t t = t0 + k;
@@ -2190,10 +2193,13 @@ static int translate_descs(xkb_runtime * R, size_t t0, size_t t1, std::vector<xk
             { size_t x = bad_ptr; while (t < x && !bad_ptr.compare_exchange_weak(x, t)) {} }
             if (d[k].kind == XKB_TASK_AXPBY && d[k].u.axpby.hi - d[k].u.axpby.lo > AXPBY_SPLIT && !longa)
                 longa.store(true, std::memory_order_relaxed);
+            mine |= xkb_internal_body_of(d[k]);
         }
+        seen.fetch_or(mine, std::memory_order_relaxed);
     });
     *descs = d;
     *long_axpby = longa;
+    *bodies = seen;
     if (bad_args != SIZE_MAX) return xkb_set_error(XKB_EINVAL, "built-in task %zu: args are not an xkb_task_desc_t", (size_t) bad_args);
     if (bad_ptr != SIZE_MAX)
         return xkb_set_error(XKB_EINVAL, "built-in task %zu: a grid or vector lies outside every registered region, or the "
@@ -2284,10 +2290,11 @@ static int stream_prepare(xkb_runtime * R, size_t t0, size_t t1, size_t a0, size
     std::vector<xkb_task_desc_t> copy;
     xkb_task_desc_t * descs = nullptr;
     bool longa = false;
-    if (rc == XKB_OK) rc = translate_descs(R, t0, t1, copy, &descs, &longa, sl.p);
+    unsigned bodies = 0;
+    if (rc == XKB_OK) rc = translate_descs(R, t0, t1, copy, &descs, &longa, &bodies, sl.p);
     const double d_ms = ms_since(w0) - f_ms;
     if (rc == XKB_OK) rc = team_for(R, descs, n);
-    if (rc == XKB_OK) rc = xkb_internal_sched_upload_window(R->sched, descs, n);
+    if (rc == XKB_OK) rc = xkb_internal_sched_upload_window(R->sched, descs, n, bodies);
     if (rc == XKB_OK && cudaEventRecord(sl.ev, R->stream) != cudaSuccess) rc = xkb_set_error(XKB_ECUDA, "xkrt: event");
     if (trace)
         fprintf(stderr, "  window: coherency %.1f ms, descriptors %.1f ms, upload %.1f ms\n", f_ms, d_ms, ms_since(w0) - f_ms - d_ms);
@@ -2369,8 +2376,9 @@ static int wait_batch(xkb_runtime * R)
         std::vector<xkb_task_desc_t> copy;
         xkb_task_desc_t * descs = nullptr;
         bool long_axpby = false;
+        unsigned bodies = 0;
         const size_t nt = ntasks - P;
-        if (rc == XKB_OK) rc = translate_descs(R, P, ntasks, copy, &descs, &long_axpby);
+        if (rc == XKB_OK) rc = translate_descs(R, P, ntasks, copy, &descs, &long_axpby, &bodies);
         if (pinner.joinable()) pinner.join();
         const double desc_ms = ms_since(t0) - fetch_ms;
         SplitGraph sg;
@@ -2382,7 +2390,7 @@ static int wait_batch(xkb_runtime * R)
         if (rc == XKB_OK) rc = team_for(R, run_d, run_n);
         if (P == 0)
         {
-            if (rc == XKB_OK) rc = xkb_internal_sched_set_tasks_device(R->sched, run_d, run_n, true);
+            if (rc == XKB_OK) rc = xkb_internal_sched_set_tasks_device(R->sched, run_d, run_n, bodies);
             if (getenv("XKB_TRACE_WAIT"))
                 fprintf(stderr, "xkrt_task_wait: fetches + copies %.1f ms, descriptors %.1f ms, upload %.1f ms\n", fetch_ms, desc_ms,
                         ms_since(t0) - fetch_ms - desc_ms);
@@ -2396,7 +2404,7 @@ static int wait_batch(xkb_runtime * R)
         else
         {
             // the rest of a streamed batch: one more window behind the streamed ones
-            if (rc == XKB_OK) rc = xkb_internal_sched_run_window(R->sched, run_d, run_n, &run_g);
+            if (rc == XKB_OK) rc = xkb_internal_sched_run_window(R->sched, run_d, run_n, bodies, &run_g);
             R->last_ms[1] = ms_since(t0);
             t0 = std::chrono::steady_clock::now();
             uint64_t ran = 0;
