@@ -138,3 +138,27 @@ def test_heat_norms_fp64_checks(torch_cuda, dtype):
         assert res == 0.0
     else:
         assert 0 < res <= 2.0 ** -24 * n["interior_max_abs"]
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("nx,ny,ld,shift", [
+    (3, 3, 4, 0), (4, 5, 4, 0), (5, 9, 8, 0),          # less than a lane's rows
+    (127, 40, 128, 0), (128, 40, 128, 0), (129, 40, 132, 0), (130, 40, 130, 0), (131, 40, 132, 0),   # around a strip
+    (258, 21, 258, 1), (257, 300, 257, 0), (260, 300, 261, 0),      # unaligned base, odd leading dimensions
+    (1030, 1500, 1032, 0), (2050, 1300, 2050, 0)])                  # wide strips, last vector past the last row
+def test_step_strips_bit_exact(torch_cuda, dtype, nx, ny, ld, shift):
+    """One whole step over grids whose rows end inside, at and past a lane's vector and a strip's
+    128 rows, with aligned and unaligned columns: the oracle's grid bit for bit, and nothing
+    written outside the interior (padding rows included)."""
+    torch = torch_cuda
+    dt = np.float64 if dtype == "f64" else np.float32
+    rng = np.random.default_rng(nx * 31 + ny)
+    src = rng.random(shift + ny * ld).astype(dt)
+    dst = rng.random(shift + ny * ld).astype(dt)
+    s, d = torch.from_numpy(src).cuda(), torch.from_numpy(dst).cuda()
+    xk.heat_step(s[shift:], d[shift:], nx, ny, ld, C)
+    want = dst.copy()
+    want[shift:].reshape(ny, ld)[:, :nx] = O.heat_step(np.ascontiguousarray(src[shift:].reshape(ny, ld)[:, :nx]),
+                                                       np.ascontiguousarray(want[shift:].reshape(ny, ld)[:, :nx]), nx, ny, C)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(d.cpu().numpy(), want)

@@ -5,21 +5,37 @@
 namespace xkb {
 
 constexpr int HEAT_THREADS = 256;   // 8 warps per CTA
-constexpr int HEAT_PF = 6;          // east columns in flight per lane
-constexpr int STEP_COLS = 64;       // columns per warp strip in the whole-step kernel
 
-template <typename T, int VEC>
+constexpr int HEAT_VEC = 4;         // rows per lane of the box kernel: a warp strip is 128 rows
+constexpr int BOX_COLS_F64 = 48, BOX_COLS_F32 = 96;   // columns of a strip of a large box
+constexpr int BOX_PFD_F64 = 3, BOX_PFD_F32 = 6;       // its L2 prefetch distance in columns
+constexpr int HEAT_NARROW = 16;     // columns of a strip up to which all of them are loaded 4 ahead, without L2 prefetch
+
+// The cells of a box (a tile, or the whole interior), split into strips of 128 rows x `cols` columns,
+// one warp each, consecutive warps down a column chunk so that the warps in flight read and write
+// whole columns (across the columns of a row of strips instead: 16384^2 FP64 701 us against 662). The
+// strips are the tile bodies' of the persistent scheduler (heat.cuh): four rows per lane, twice the
+// bytes per request of the two-row overlapping strips of heat_step_kernel, which this replaces as
+// the default. A step, us: 16384^2 FP64 762 -> 651 (6.6 TB/s), 8192^2 197 -> 172, 8192^2 FP32
+// 118 -> 113, 1024^2 FP64 29 -> 6, 5003 x 4001 (odd ld) FP32 78 -> 47, FP64 106 -> 62.
+template <typename T, int PF, Strips K>
 __global__ void __launch_bounds__(HEAT_THREADS, 2)
-heat_tile_kernel(const T * __restrict__ src, T * __restrict__ dst, int64_t ld, int64_t nx, int64_t ny,
-                 int64_t x0, int64_t x1, int64_t y0, int64_t y1, double c, bool vec_ok)
+heat_box_kernel(const T * __restrict__ src, T * __restrict__ dst, int64_t ld, int64_t nx, int64_t ny, TileBox b,
+                int64_t rbase0, int nrg, int ncg, int cols, double c, int pfd)
 {
-    // blockIdx.x selects a column slab of the tile so one task can still use several SMs.
-    const int64_t cols = y1 - y0;
-    const int64_t per = (cols + gridDim.x - 1) / gridDim.x;
-    const int64_t a = y0 + (int64_t) blockIdx.x * per;
-    int64_t b = a + per; if (b > y1) b = y1;
-    if (a >= b) return;
-    heat_tile_cta<T, VEC, HEAT_PF, false>(src, dst, ld, nx, ny, x0, x1, a, b, c, vec_ok, 8);
+    const int s = (int) blockIdx.x * (HEAT_THREADS / 32) + (int) (threadIdx.x >> 5);
+    if (s < nrg * ncg)
+    {
+        const int cg = (int) ((uint32_t) s / (uint32_t) nrg), rg = s - cg * nrg;
+        const int64_t cy0 = b.cy0 + (int64_t) cg * cols, rbase = rbase0 + (int64_t) rg * 32 * HEAT_VEC;
+        int64_t cy1 = cy0 + cols; if (cy1 > b.cy1) cy1 = b.cy1;
+        if constexpr (K == Strips::ROWS)
+            heat_strip_rows<T, HEAT_VEC, PF, false>(src, dst, ld, nx, rbase, b.rx0, b.rx1, cy0, cy1, c);
+        else if (rbase + 32 * HEAT_VEC <= nx || nx % HEAT_VEC == 0 || cy1 < ny - 1)
+            heat_strip_halo_impl<T, HEAT_VEC, PF, false>(src, dst, ld, nx, rbase, b.rx0, b.rx1, cy0, cy1, c, pfd);
+        else
+            heat_strip_rows_call<T, HEAT_VEC, false>(src, dst, ld, nx, rbase, b.rx0, b.rx1, cy0, cy1, c);
+    }
 }
 
 template <typename T, int VEC, int PF, int MINB>
@@ -47,22 +63,6 @@ static bool vec_ok_for(const void * src, const void * dst, int64_t ld)
     return (ld % VEC == 0) && ((uintptr_t) src % 16 == 0) && ((uintptr_t) dst % 16 == 0);
 }
 
-template <typename T>
-static int launch_tile(const void * src, void * dst, int64_t ld, int64_t nx, int64_t ny,
-                       int64_t x0, int64_t x1, int64_t y0, int64_t y1, double c, cudaStream_t st)
-{
-    constexpr int VEC = HeatVec<T>::N;
-    const TileBox b = heat_tile_box(nx, ny, x0, x1, y0, y1);
-    if (b.rx0 >= b.rx1 || b.cy0 >= b.cy1) return XKB_OK;
-    // one CTA per 32 columns of the tile (a 128x128 tile runs on 4 SMs)
-    const int64_t cols = b.cy1 - b.cy0;
-    int grid = (int) ((cols + 31) / 32); if (grid < 1) grid = 1;
-    heat_tile_kernel<T, VEC><<<grid, HEAT_THREADS, 0, st>>>((const T *) src, (T *) dst, ld, nx, ny,
-                                                           b.rx0, b.rx1, b.cy0, b.cy1, c, vec_ok_for<T>(src, dst, ld));
-    XKB_CUDA_TRY(cudaGetLastError());
-    return XKB_OK;
-}
-
 static int sm_count()
 {
     static int sms = 0;
@@ -72,6 +72,35 @@ static int sm_count()
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     }
     return sms;
+}
+
+// Launch the box kernel, a CTA per 8 strips (CTAs are handed out as others end: with the strips dealt
+// to resident warps in advance the slowest warp made 16384^2 FP64 767 us). Strips of about BOX_COLS
+// columns, their number rounded to whole waves of the device's warps; a box of less than a wave gets a
+// strip per warp, of 4 columns at least. (FP64 strips of 32 / 48 / 64 / 96 / 128 columns: 649 / 651 /
+// 654 / 659 / 767 us at 16384^2, 170 / 172 / 178 / 189 / 204 at 8192^2; FP32 strips of 32 / 64 / 96:
+// 119 / 114 / 113 at 8192^2.)
+template <typename T>
+static int launch_box(const void * src, void * dst, int64_t ld, int64_t nx, int64_t ny, const TileBox & b, double c, cudaStream_t st)
+{
+    if (b.rx0 >= b.rx1 || b.cy0 >= b.cy1) return XKB_OK;
+    const int64_t rbase0 = b.rx0 - b.rx0 % HEAT_VEC, width = b.cy1 - b.cy0, warps = (int64_t) sm_count() * 2 * (HEAT_THREADS / 32);
+    const int64_t nrg = (b.rx1 - rbase0 + 32 * HEAT_VEC - 1) / (32 * HEAT_VEC);
+    const int64_t target = sizeof(T) == 8 && vec_ok_for<T>(src, dst, ld) ? BOX_COLS_F64 : BOX_COLS_F32;
+    const int64_t waves = std::max<int64_t>(1, (nrg * width + target / 2 * warps) / (target * warps));
+    int64_t ncg = std::max<int64_t>(1, waves * warps / nrg);
+    const int64_t cols = std::max<int64_t>(4, (width + ncg - 1) / ncg);
+    ncg = (width + cols - 1) / cols;
+    if (nrg > INT32_MAX / ncg - 8 || cols > INT32_MAX) return xkb_set_error(XKB_EINVAL, "heat: grid too large");
+    const unsigned grid = (unsigned) ((nrg * ncg + HEAT_THREADS / 32 - 1) / (HEAT_THREADS / 32));
+    auto run = [&](auto kernel, int pfd) {
+        kernel<<<grid, HEAT_THREADS, 0, st>>>((const T *) src, (T *) dst, ld, nx, ny, b, rbase0, (int) nrg, (int) ncg, (int) cols, c, pfd);
+    };
+    if (!vec_ok_for<T>(src, dst, ld)) run(heat_box_kernel<T, ROWS_PF<T>, Strips::ROWS>, 0);
+    else if (cols <= HEAT_NARROW) run(heat_box_kernel<T, 4, Strips::VECTOR>, 0);
+    else run(heat_box_kernel<T, sizeof(T) == 8 ? 2 : 5, Strips::VECTOR>, sizeof(T) == 8 ? BOX_PFD_F64 : BOX_PFD_F32);
+    XKB_CUDA_TRY(cudaGetLastError());
+    return XKB_OK;
 }
 
 template <typename T, int PF, int MINB>
@@ -132,16 +161,15 @@ extern "C" int xkb_heat_tile(int dtype, const void * src, void * dst, int64_t ld
     if (tsx <= 0 || tsy <= 0 || tile_x < 0 || tile_y < 0) return xkb_set_error(XKB_EINVAL, "heat_tile: bad tile");
     const int64_t x0 = tile_x * tsx, y0 = tile_y * tsy;
     const int64_t x1 = x0 + tsx, y1 = y0 + tsy;
-    return dtype == XKB_F64 ? launch_tile<double>(src, dst, ld, nx, ny, x0, x1, y0, y1, c, xkb_stream(stream))
-                            : launch_tile<float>(src, dst, ld, nx, ny, x0, x1, y0, y1, c, xkb_stream(stream));
+    const TileBox b = heat_tile_box(nx, ny, x0, x1, y0, y1);
+    return dtype == XKB_F64 ? launch_box<double>(src, dst, ld, nx, ny, b, c, xkb_stream(stream))
+                            : launch_box<float>(src, dst, ld, nx, ny, b, c, xkb_stream(stream));
 }
-
-static const xkb_heat_cfg_t kDefaultStepCfg = {4, 2, 8, 8, 64};
 
 extern "C" int xkb_heat_step(int dtype, const void * src, void * dst, int64_t ld, int64_t nx, int64_t ny,
                              double c, void * stream)
 {
-    return xkb_heat_step_cfg(dtype, src, dst, ld, nx, ny, c, &kDefaultStepCfg, stream);
+    return xkb_heat_step_cfg(dtype, src, dst, ld, nx, ny, c, nullptr, stream);
 }
 
 extern "C" int xkb_heat_step_cfg(int dtype, const void * src, void * dst, int64_t ld, int64_t nx, int64_t ny,
@@ -149,7 +177,13 @@ extern "C" int xkb_heat_step_cfg(int dtype, const void * src, void * dst, int64_
 {
     int rc = heat_check(dtype, src, dst, ld, nx, ny);
     if (rc) return rc;
-    const xkb_heat_cfg_t & k = cfg ? *cfg : kDefaultStepCfg;
+    if (!cfg)
+    {
+        const TileBox b = heat_tile_box(nx, ny, 0, nx, 0, ny);
+        return dtype == XKB_F64 ? launch_box<double>(src, dst, ld, nx, ny, b, c, xkb_stream(stream))
+                                : launch_box<float>(src, dst, ld, nx, ny, b, c, xkb_stream(stream));
+    }
+    const xkb_heat_cfg_t & k = *cfg;
     if (k.l2_prefetch_cols < 0 || k.l2_prefetch_cols > 256 || k.cols_per_strip < 0)
         return xkb_set_error(XKB_EINVAL, "heat_step: bad configuration");
     return dtype == XKB_F64 ? launch_step<double>(src, dst, ld, nx, ny, c, k, xkb_stream(stream))
