@@ -216,3 +216,37 @@ def test_time_split_resolution_same_edges(torch_cuda, monkeypatch, nseg, global_
     for nreaders, batches in ((100, 1), (3000, 1), (3000, 4)):
         recs = _readers_stream(nreaders)
         np.testing.assert_array_equal(gpu_edges(recs, batches, seed=7), U.oracle_edges(recs), err_msg=f"{nreaders} readers")
+
+
+@pytest.mark.parametrize("nseg", [1, 5, 24])
+@pytest.mark.parametrize("writers", [0, 3, 60])
+def test_segments_look_back(torch_cuda, monkeypatch, nseg, writers):
+    """Segments find each cell's last write by looking back from their cut: streams whose cells are
+    never written, written a few times far back, and often, over two batches, give the oracle's edges."""
+    monkeypatch.setenv("XKB_RESOLVE_SEGMENTS", str(nseg))
+    rng = np.random.default_rng(10 * nseg + writers)
+    tasks = []
+    for t in range(1200):
+        x, y, m, n = (int(v) for v in (rng.integers(0, 12) * 16, rng.integers(0, 12) * 16, rng.integers(1, 5) * 16, rng.integers(1, 5) * 16))
+        w = writers and t % (1200 // writers) == 0
+        tasks.append([("m", S.RW if w and t % 2 else S.W if w else S.R, 1 << 20, 256, x, y, m, n, 8)])
+    recs = S.from_tuples(tasks)
+    want = U.oracle_edges(recs)
+    for batches in (1, 2):
+        np.testing.assert_array_equal(gpu_edges(recs, batches, seed=5), want)
+
+
+@pytest.mark.parametrize("nreaders", [1, 31, 32, 33, 511, 512, 513, 1500])
+def test_successor_lists_ascending(torch_cuda, nreaders):
+    """A writer followed by nreaders readers of its cells: its successor list comes back in ascending
+    order whatever sorts it (one warp's registers, shared memory, global memory)."""
+    torch = torch_cuda
+    recs = S.from_tuples([[("m", S.W, 1 << 20, 256, 0, 0, 64, 8, 8)]] +
+                         [[("m", S.R, 1 << 20, 256, 8 * (k % 8), 0, 8, 8, 8)] for k in range(nreaders)])
+    r = xk.Resolver()
+    r.add(recs)
+    g = r.graph()
+    assert g.nedges == nreaders
+    succ = torch.as_tensor(_DevView(g.succ, g.nedges), device="cuda").cpu().numpy()
+    np.testing.assert_array_equal(succ, np.arange(1, nreaders + 1))
+    r.close()

@@ -22,10 +22,10 @@
 //
 // Method (B200): the host turns the accesses of a batch into each domain's ordered op list
 // and keeps a coordinate compression of the domain (elementary cells between all rect
-// boundaries seen so far). On the GPU one CTA owns a region of RX x RY cells: it streams the
-// batch's ops, keeps those overlapping its region with a ballot + block prefix sum (order
-// preserving), and each thread then applies the ops to its own cell's writer/readers state,
-// emitting (pred, succ) pairs; lanes emitting the same pred for the same op are merged with
+// boundaries seen so far). On the GPU the ops are binned to regions of RX x RY cells, in op order; a
+// CTA takes a segment of a region's list, finds each cell's state at the segment's start by looking
+// back for its last write, and each thread then applies the ops to its own cell's writer/readers
+// state, emitting (pred, succ) pairs; lanes emitting the same pred for the same op are merged with
 // __match_any_sync. A GPU hash set keeps the unique pairs; finalising counts predecessors,
 // scans and scatters the pairs into a successor CSR. Cell state stays in HBM between batches.
 #include "common.cuh"
@@ -116,160 +116,21 @@ __device__ __forceinline__ void emit_flush(const ResolveArgs & a, const unsigned
     __syncwarp();
 }
 
-// BINNED: the CTA's ops come from its region's list (op indices in op order, built by the
-// binning kernels below) instead of a scan of every op of the batch.
-template <int RX, int RY, bool BINNED>
-__global__ void __launch_bounds__(RX * RY)
-resolve_region_kernel(ResolveArgs a, const unsigned * __restrict__ roff, const int * __restrict__ rlist)
-{
-    constexpr int NT = RX * RY;
-    constexpr int NW = NT / 32;
-    constexpr int CHUNK = NT * RES_CHUNK_PER_THREAD;
-    extern __shared__ int rd[];                  // readers: rd[k * NT + tid]
-    __shared__ DOp list[CHUNK];
-    __shared__ int wcount[NW];
-    __shared__ int nlist_s;
-    __shared__ unsigned long long ebuf[NW][EMIT_BUF];   // each warp's pairs not yet in a.emit
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int rx = blockIdx.x % a.nrx, ry = blockIdx.x / a.nrx;
-    const int gx0 = rx * RX, gy0 = ry * RY;
-    const int gx1 = min(gx0 + RX, a.ncx), gy1 = min(gy0 + RY, a.ncy);
-    const int cx = gx0 + tid % RX, cy = gy0 + tid / RX;
-    const bool valid = cx < a.ncx && cy < a.ncy;
-    const size_t cell = valid ? (size_t) cy * a.ncx + cx : 0;
-
-    int writer = -1, nr = 0, head = -1, tail = -1;
-    int nbuf = 0;                                // pairs in this warp's ebuf (same in every lane)
-    if (valid)
-    {
-        const int * st = a.state_in + cell * STRIDE;
-        writer = st[0]; nr = st[1]; head = st[2]; tail = st[3];
-        for (int k = 0; k < nr && k < RCAP; ++k) rd[k * NT + tid] = st[SHDR + k];
-    }
-
-    const int lo = BINNED ? (int) roff[blockIdx.x] : 0, hi = BINNED ? (int) roff[blockIdx.x + 1] : a.nops;
-    for (int base = lo; base < hi; base += CHUNK)
-    {
-        if constexpr (BINNED)
-        {
-            // ---- gather the next CHUNK ops of this region's list (already in op order) -----
-            for (int j = tid; j < CHUNK && base + j < hi; j += NT) list[j] = a.ops[rlist[base + j]];
-            if (tid == 0) nlist_s = min(CHUNK, hi - base);
-            __syncthreads();
-        }
-        else
-        {
-        // ---- compact the ops of this chunk that overlap the region, in op order ----------
-        if (tid == 0) nlist_s = 0;
-        __syncthreads();
-        for (int j = 0; j < RES_CHUNK_PER_THREAD; ++j)
-        {
-            const int idx = base + j * NT + tid;
-            DOp op;
-            bool hit = false;
-            if (idx < a.nops)
-            {
-                op = a.ops[idx];
-                hit = op.cx0 < gx1 && gx0 < op.cx1 && op.cy0 < gy1 && gy0 < op.cy1;
-            }
-            const unsigned bal = __ballot_sync(0xffffffffu, hit);
-            if (lane == 0) wcount[warp] = __popc(bal);
-            __syncthreads();
-            int off = nlist_s;
-            for (int w = 0; w < warp; ++w) off += wcount[w];
-            if (hit) list[off + __popc(bal & ((1u << lane) - 1))] = op;
-            __syncthreads();
-            if (tid == 0) { int t = 0; for (int w = 0; w < NW; ++w) t += wcount[w]; nlist_s += t; }
-            __syncthreads();
-        }
-        }
-        const int nlist = nlist_s;
-
-        // ---- apply them to this thread's cell -----------------------------------------------
-        for (int k = 0; k < nlist; ++k)
-        {
-            const DOp op = list[k];
-            const bool in = valid && op.cx0 <= cx && cx < op.cx1 && op.cy0 <= cy && cy < op.cy1;
-            if (op.link)
-            {
-                const bool from_readers = in && (op.mode & M_W) && nr > 0;
-                const int cnt = from_readers ? nr : ((in && writer >= 0) ? 1 : 0);
-                const int maxcnt = __reduce_max_sync(0xffffffffu, cnt);
-                int chunk = head, ci = 0;                // walk of the spill chain past RCAP
-                for (int q = 0; q < maxcnt; ++q)
-                {
-                    int p = -1;
-                    if (q < cnt)
-                    {
-                        if (!from_readers) p = writer;
-                        else if (q < RCAP) p = rd[q * NT + tid];
-                        else
-                        {
-                            if (ci == SPILL_R) { chunk = chunk >= 0 ? a.spill[(size_t) chunk * SPILL] : -1; ci = 0; }
-                            p = chunk >= 0 ? a.spill[(size_t) chunk * SPILL + 1 + ci] : -1;   // -1: pool ran out, batch redone
-                            ++ci;
-                        }
-                    }
-                    const unsigned peers = __match_any_sync(0xffffffffu, p);
-                    const bool leader = p >= 0 && lane == __ffs(peers) - 1;
-                    const unsigned em = __ballot_sync(0xffffffffu, leader);
-                    if (leader)
-                        ebuf[warp][nbuf + __popc(em & ((1u << lane) - 1))] = ((unsigned long long) (uint32_t) p << 32) | (uint32_t) op.task;
-                    nbuf += __popc(em);
-                    if (nbuf > EMIT_BUF - 32) { emit_flush(a, ebuf[warp], nbuf, lane); nbuf = 0; }
-                }
-            }
-            else if (in)
-            {
-                if (op.mode & M_W) { writer = op.task; nr = 0; head = tail = -1; }
-                else if (op.mode == M_R)
-                {
-                    if (nr < RCAP) rd[nr * NT + tid] = op.task;
-                    else
-                    {
-                        const int slot = (nr - RCAP) % SPILL_R;
-                        if (slot == 0)
-                        {
-                            const int c = spill_alloc(a.spill, a.spill_ctr, a.spill_cap);
-                            if (c >= 0) { if (tail >= 0) a.spill[(size_t) tail * SPILL] = c; else head = c; }
-                            tail = c;
-                        }
-                        if (tail >= 0) a.spill[(size_t) tail * SPILL + 1 + slot] = op.task;
-                    }
-                    ++nr;
-                }
-            }
-        }
-        __syncthreads();
-    }
-
-    if (nbuf) emit_flush(a, ebuf[warp], nbuf, lane);
-    if (valid)
-    {
-        int * st = a.state_out + cell * STRIDE;
-        st[0] = writer; st[1] = nr; st[2] = head; st[3] = tail;
-        for (int k = 0; k < nr && k < RCAP; ++k) st[SHDR + k] = rd[k * NT + tid];
-    }
-}
-
-// ---- time-split resolution of a region ---------------------------------------------------------
-// A region's op list is cut into nseg segments (cut s at lo + (hi - lo) * s / nseg). The cell
-// state before each cut is all a segment needs to emit its edges, and only PUT ops change the
-// state, so:
-//  * resolve_puts_kernel (one CTA per region) applies the PUT ops of the whole list -- the
-//    cheap half of the work -- writing the state before every cut to `snap` and the final state
-//    to state_out; it owns the reader spill chains, exactly as resolve_region_kernel does;
-//  * resolve_links_kernel (one CTA per region and segment, nseg times the CTAs) replays its
-//    segment from that state: PUT ops update a private copy of the state and LINK ops emit
-//    the edges. Readers past RCAP that were in the state at the cut are read from the chain the
-//    snapshot names (resolve_puts_kernel only ever appends to a chain past the snapshot's count,
-//    and a write drops a chain without reusing it, so the first nr entries stay as they were);
-//    readers the segment itself adds past RCAP go to a private chain (chunks from the same pool,
-//    never linked into the kept state).
-// The edges are those of resolve_region_kernel over the whole list (the same LINK ops see the
-// same states); only the order in which pairs reach a.emit differs, which the dedupe ignores.
-
+// ---- a region's ops applied to its cells, cut in time -----------------------------------------
+// One CTA per region (RX x RY cells, a thread per cell) and SEGMENT of the region's op list (cut s at
+// lo + (hi - lo) * s / nseg), so that a batch of few regions still fills the device. A segment
+// applies its ops in order: PUT ops update the cell's state, LINK ops emit the edges from it.
+// The state at its cut is not handed over by the segment before: a cell's state is its last write and
+// the reads since, so the CTA looks back from the cut for each cell's last write (a handful of ops
+// where tasks write what they read) and applies the PUT ops from there on; a cell without one starts
+// from the state before the batch. (One CTA per region applying all PUT ops first, to leave a snapshot
+// at every cut, was 2.06 of 2.65 ms on the 65,536-task stream of 128 x 128 cells; this is 0.66.) The readers matter
+// to LINK ops that write only, so a segment without one skips them, unless it is the region's last
+// segment, whose state is the batch's final one.
+//  * Readers past RCAP: a cell that starts from the state before the batch finds the first of them on
+//    that state's spill chain, which only the last segment appends to (past the count the others
+//    use; a write drops a chain without reusing its chunks); the readers a segment adds go to a chain
+//    of its own. The last segment's chain is kept.
 __device__ __forceinline__ int seg_cut(int lo, int hi, int s, int nseg)
 {
     return lo + (int) ((long long) (hi - lo) * s / nseg);
@@ -277,110 +138,77 @@ __device__ __forceinline__ int seg_cut(int lo, int hi, int s, int nseg)
 
 template <int RX, int RY>
 __global__ void __launch_bounds__(RX * RY)
-resolve_puts_kernel(ResolveArgs a, const unsigned * __restrict__ roff, const int * __restrict__ rlist, int nseg,
-                    int * __restrict__ snap, size_t ncells)
-{
-    constexpr int NT = RX * RY;
-    constexpr int CHUNK = NT * RES_CHUNK_PER_THREAD;
-    extern __shared__ int rd[];                  // readers: rd[k * NT + tid]
-    __shared__ DOp list[CHUNK];
-
-    const int tid = threadIdx.x;
-    const int rx = blockIdx.x % a.nrx, ry = blockIdx.x / a.nrx;
-    const int cx = rx * RX + tid % RX, cy = ry * RY + tid / RX;
-    const bool valid = cx < a.ncx && cy < a.ncy;
-    const size_t cell = valid ? (size_t) cy * a.ncx + cx : 0;
-
-    int writer = -1, nr = 0, head = -1, tail = -1;
-    if (valid)
-    {
-        const int * st = a.state_in + cell * STRIDE;
-        writer = st[0]; nr = st[1]; head = st[2]; tail = st[3];
-        for (int k = 0; k < nr && k < RCAP; ++k) rd[k * NT + tid] = st[SHDR + k];
-    }
-    auto snapshot = [&](int s) {
-        if (!valid) return;
-        int * st = snap + ((size_t) (s - 1) * ncells + cell) * STRIDE;
-        st[0] = writer; st[1] = nr; st[2] = head; st[3] = tail;
-        for (int k = 0; k < nr && k < RCAP; ++k) st[SHDR + k] = rd[k * NT + tid];
-    };
-
-    const int lo = (int) roff[blockIdx.x], hi = (int) roff[blockIdx.x + 1];
-    int seg = 1, cut = nseg > 1 ? seg_cut(lo, hi, 1, nseg) : INT_MAX;
-    for (int base = lo; base < hi; base += CHUNK)
-    {
-        const int n = min(CHUNK, hi - base);
-        for (int j = tid; j < n; j += NT) list[j] = a.ops[rlist[base + j]];
-        __syncthreads();
-        for (int k = 0; k < n; ++k)
-        {
-            while (base + k == cut) { snapshot(seg); ++seg; cut = seg < nseg ? seg_cut(lo, hi, seg, nseg) : INT_MAX; }
-            const DOp op = list[k];
-            if (op.link) continue;
-            const bool in = valid && op.cx0 <= cx && cx < op.cx1 && op.cy0 <= cy && cy < op.cy1;
-            if (!in) continue;
-            if (op.mode & M_W) { writer = op.task; nr = 0; head = tail = -1; }
-            else if (op.mode == M_R)
-            {
-                if (nr < RCAP) rd[nr * NT + tid] = op.task;
-                else
-                {
-                    const int slot = (nr - RCAP) % SPILL_R;
-                    if (slot == 0)
-                    {
-                        const int c = spill_alloc(a.spill, a.spill_ctr, a.spill_cap);
-                        if (c >= 0) { if (tail >= 0) a.spill[(size_t) tail * SPILL] = c; else head = c; }
-                        tail = c;
-                    }
-                    if (tail >= 0) a.spill[(size_t) tail * SPILL + 1 + slot] = op.task;
-                }
-                ++nr;
-            }
-        }
-        __syncthreads();
-    }
-    while (seg < nseg) { snapshot(seg); ++seg; }          // cuts at the end of the list
-    if (valid)
-    {
-        int * st = a.state_out + cell * STRIDE;
-        st[0] = writer; st[1] = nr; st[2] = head; st[3] = tail;
-        for (int k = 0; k < nr && k < RCAP; ++k) st[SHDR + k] = rd[k * NT + tid];
-    }
-}
-
-template <int RX, int RY>
-__global__ void __launch_bounds__(RX * RY)
-resolve_links_kernel(ResolveArgs a, const unsigned * __restrict__ roff, const int * __restrict__ rlist, int nseg,
-                     const int * __restrict__ snap, size_t ncells)
+resolve_segment_kernel(ResolveArgs a, const unsigned * __restrict__ roff, const int * __restrict__ rlist, int nseg)
 {
     constexpr int NT = RX * RY;
     constexpr int NW = NT / 32;
     constexpr int CHUNK = NT * RES_CHUNK_PER_THREAD;
-    extern __shared__ int rd[];
+    extern __shared__ int rd[];                  // readers: rd[k * NT + tid]
     __shared__ DOp list[CHUNK];
-    __shared__ unsigned long long ebuf[NW][EMIT_BUF];
+    __shared__ unsigned long long ebuf[NW][EMIT_BUF];   // each warp's pairs not yet in a.emit
+    __shared__ int first_s;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int region = blockIdx.x / nseg, s = blockIdx.x % nseg;
+    const bool last = s == nseg - 1;
     const int rx = region % a.nrx, ry = region / a.nrx;
     const int cx = rx * RX + tid % RX, cy = ry * RY + tid / RX;
     const bool valid = cx < a.ncx && cy < a.ncy;
     const size_t cell = valid ? (size_t) cy * a.ncx + cx : 0;
-
-    int writer = -1, nr = 0, shead = -1;
-    if (valid)
-    {
-        const int * st = s == 0 ? a.state_in + cell * STRIDE : snap + ((size_t) (s - 1) * ncells + cell) * STRIDE;
-        writer = st[0]; nr = st[1]; shead = st[2];
-        for (int k = 0; k < nr && k < RCAP; ++k) rd[k * NT + tid] = st[SHDR + k];
-    }
-    int nsnap = nr;                              // readers [RCAP, nsnap) are on the snapshot's chain
-    int phead = -1, ptail = -1;                  // readers the segment adds past RCAP
-    int nbuf = 0;
-
     const int lo = (int) roff[region], hi = (int) roff[region + 1];
     const int from = seg_cut(lo, hi, s, nseg), to = seg_cut(lo, hi, s + 1, nseg);
-    for (int base = from; base < to; base += CHUNK)
+    auto covers = [&](const DOp & op) { return valid && op.cx0 <= cx && cx < op.cx1 && op.cy0 <= cy && cy < op.cy1; };
+
+    // the cell's last write before the cut
+    int wpos = -1;
+    int start = from;
+    bool readers = true;
+    if (from > lo)
+    {
+        for (int e = from; e > lo;)
+        {
+            const int b = max(lo, e - NT), n = e - b;
+            if (tid < n) list[tid] = a.ops[rlist[b + tid]];
+            __syncthreads();
+            for (int k = n - 1; k >= 0 && wpos < 0; --k)
+            {
+                const DOp op = list[k];
+                if (!op.link && (op.mode & M_W) && covers(op)) wpos = b + k;
+            }
+            e = b;
+            if (__syncthreads_and(wpos >= 0 || !valid)) break;
+        }
+        if (!last)
+        {
+            int w = 0;
+            for (int i = from + tid; i < to; i += NT) { const DOp op = a.ops[rlist[i]]; w |= op.link && (op.mode & M_W); }
+            readers = __syncthreads_or(w) != 0;
+        }
+        if (readers)
+        {
+            if (tid == 0) first_s = from;
+            __syncthreads();
+            const int mine = !valid ? from : wpos >= 0 ? wpos : lo;
+            atomicMin(&first_s, mine);
+            __syncthreads();
+            start = first_s;
+        }
+    }
+
+    int writer = -1, nr = 0;
+    int shead = -1, nsnap = 0;                   // readers [RCAP, nsnap) are on the chain of the state before the batch
+    int phead = -1, ptail = -1;                  // readers from max(RCAP, nsnap) on
+    if (valid && wpos < 0)
+    {
+        const int * st = a.state_in + cell * STRIDE;
+        writer = st[0]; nr = st[1]; shead = st[2];
+        for (int k = 0; k < nr && k < RCAP; ++k) rd[k * NT + tid] = st[SHDR + k];
+        if (last) { phead = shead; ptail = st[3]; } else nsnap = nr;
+    }
+    if (valid && wpos >= 0 && !readers) writer = a.ops[rlist[wpos]].task;
+    int nbuf = 0;                                // pairs in this warp's ebuf (same in every lane)
+
+    for (int base = start; base < to; base += CHUNK)
     {
         const int n = min(CHUNK, to - base);
         for (int j = tid; j < n; j += NT) list[j] = a.ops[rlist[base + j]];
@@ -388,14 +216,15 @@ resolve_links_kernel(ResolveArgs a, const unsigned * __restrict__ roff, const in
         for (int k = 0; k < n; ++k)
         {
             const DOp op = list[k];
-            const bool in = valid && op.cx0 <= cx && cx < op.cx1 && op.cy0 <= cy && cy < op.cy1;
-            const int pbase = max(RCAP, nsnap);  // first reader position on the private chain
+            const bool in = covers(op) && base + k >= wpos;
+            const int pbase = max(RCAP, nsnap);
             if (op.link)
             {
+                if (base + k < from) continue;
                 const bool from_readers = in && (op.mode & M_W) && nr > 0;
                 const int cnt = from_readers ? nr : ((in && writer >= 0) ? 1 : 0);
                 const int maxcnt = __reduce_max_sync(0xffffffffu, cnt);
-                int chunk = shead, ci = 0;
+                int chunk = shead, ci = 0;                // walk of the spill chain past RCAP
                 for (int q = 0; q < maxcnt; ++q)
                 {
                     int p = -1;
@@ -423,7 +252,7 @@ resolve_links_kernel(ResolveArgs a, const unsigned * __restrict__ roff, const in
             else if (in)
             {
                 if (op.mode & M_W) { writer = op.task; nr = 0; nsnap = 0; phead = ptail = -1; }
-                else if (op.mode == M_R)
+                else if (op.mode == M_R && readers)
                 {
                     if (nr < RCAP) rd[nr * NT + tid] = op.task;
                     else
@@ -443,7 +272,14 @@ resolve_links_kernel(ResolveArgs a, const unsigned * __restrict__ roff, const in
         }
         __syncthreads();
     }
+
     if (nbuf) emit_flush(a, ebuf[warp], nbuf, lane);
+    if (valid && last)
+    {
+        int * st = a.state_out + cell * STRIDE;
+        st[0] = writer; st[1] = nr; st[2] = nr > RCAP ? phead : -1; st[3] = nr > RCAP ? ptail : -1;
+        for (int k = 0; k < nr && k < RCAP; ++k) st[SHDR + k] = rd[k * NT + tid];
+    }
 }
 
 // ---- binning of ops to regions ----------------------------------------------------------------
@@ -536,39 +372,70 @@ __global__ void bin_fill_smem_kernel(const DOp * __restrict__ ops, int nops, int
     }
 }
 
-constexpr int MAX_SEGMENTS = 8;              // time-split segments per region (resolve_links_kernel)
+constexpr int MAX_SEGMENTS = 24;             // segments per region at most
+constexpr int SEGMENT_OPS = 512;             // ops per segment aimed at (12 or 32 segments, 256 ops: within 3 %)
 constexpr int BIN_SORT_THREADS = 1024;
-constexpr int BIN_SORT_CAP = 16384;          // ops of one region sortable in one CTA (64 KB of shared memory)
+constexpr int BIN_SORT_SHORT = 1024;         // a list of up to this many ops is sorted as keys
+constexpr int BIN_SORT_WORDS = 40960;        // words of the bitmap of a longer one at most (160 KB: 1.3 M ops a pass)
 
-// Put each region's list back in op order (the fill appends in arbitrary order): bitonic sort of
-// the region's segment in shared memory. A region holding more than BIN_SORT_CAP ops sets
-// *too_long and the batch falls back to the unbinned scan.
-__global__ void __launch_bounds__(BIN_SORT_THREADS) bin_sort_kernel(const unsigned * __restrict__ roff, int * list, int * too_long)
+// Put each region's list back in op order (the fill appends in arbitrary order), from `in` to `out`.
+// A short list: bitonic sort in shared memory. A longer one: its ops set their bits in a bitmap of the
+// batch's ops, whose set bits are then written out in order -- the list is a set of distinct numbers
+// below nops -- `words` words of it at a time. (Bitonic sorts of 12,800 ops per region took 264 us; this
+// 24.)
+__global__ void __launch_bounds__(BIN_SORT_THREADS) bin_sort_kernel(const unsigned * __restrict__ roff, const int * __restrict__ in,
+                                                                    int * __restrict__ out, int nops, int words)
 {
-    extern __shared__ int keys[];
+    extern __shared__ unsigned bits[];
+    __shared__ uint32_t wt[32];
     const unsigned b = roff[blockIdx.x], e = roff[blockIdx.x + 1];
     const int n = (int) (e - b);
-    if (n <= 1) return;
-    if (n > BIN_SORT_CAP) { if (threadIdx.x == 0) atomicExch(too_long, 1); return; }
-    int p2 = 1;
-    while (p2 < n) p2 <<= 1;
-    for (int i = threadIdx.x; i < p2; i += blockDim.x) keys[i] = i < n ? list[b + i] : 0x7fffffff;
-    __syncthreads();
-    for (int k = 2; k <= p2; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1)
-        {
-            for (int i = threadIdx.x; i < p2; i += blockDim.x)
+    if (n == 0) return;
+    if (n <= BIN_SORT_SHORT)
+    {
+        int * keys = (int *) bits;
+        int p2 = 1;
+        while (p2 < n) p2 <<= 1;
+        const int i = threadIdx.x;
+        if (i < p2) keys[i] = i < n ? in[b + i] : 0x7fffffff;
+        __syncthreads();
+        for (int k = 2; k <= p2; k <<= 1)
+            for (int j = k >> 1; j > 0; j >>= 1)
             {
                 const int l = i ^ j;
-                if (l > i)
+                if (i < p2 && l > i)
                 {
                     const int x = keys[i], y = keys[l];
                     if (((i & k) == 0) == (x > y)) { keys[i] = y; keys[l] = x; }
                 }
+                __syncthreads();
             }
-            __syncthreads();
+        if (i < n) out[b + i] = keys[i];
+        return;
+    }
+    unsigned pos = b;
+    for (int w0 = 0; w0 * 32 < nops; w0 += words)
+    {
+        for (int w = threadIdx.x; w < words; w += BIN_SORT_THREADS) bits[w] = 0;
+        __syncthreads();
+        const int op0 = w0 * 32, op1 = op0 + words * 32;         // (nops is an int: the last window may end past it)
+        for (int i = threadIdx.x; i < n; i += BIN_SORT_THREADS)
+        {
+            const int op = in[b + i];
+            if (op >= op0 && (op < op1 || op1 < op0)) atomicOr(bits + ((op - op0) >> 5), 1u << ((op - op0) & 31));
         }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) list[b + i] = keys[i];
+        __syncthreads();
+        const int used = min(words, (nops - op0 + 31) / 32);
+        for (int w = threadIdx.x; w < ((used + BIN_SORT_THREADS - 1) / BIN_SORT_THREADS) * BIN_SORT_THREADS; w += BIN_SORT_THREADS)
+        {
+            unsigned m = w < used ? bits[w] : 0u;
+            uint32_t total;
+            unsigned at = pos + block_exclusive_scan((uint32_t) __popc(m), wt, total);
+            pos += total;
+            for (; m; m &= m - 1) out[at++] = op0 + w * 32 + __ffs(m) - 1;
+        }
+        __syncthreads();
+    }
 }
 
 // New compression refines the old one: every new cell lies inside exactly one old cell (or
@@ -615,34 +482,53 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long k)
     return k;
 }
 
-__global__ void dedupe_kernel(const unsigned long long * __restrict__ emit, size_t n, unsigned long long * table,
-                              unsigned long long mask, unsigned long long * uniq, unsigned long long * nuniq,
-                              unsigned long long uniq_cap)
+// Results of a batch's device work, read back together: pairs emitted, unique pairs stored so far in
+// the segment, and whether the hash set or the segment had no room.
+enum { CNT_EMIT, CNT_UNIQ, CNT_FULL, CNT_COUNT };
+
+// Unique the emitted pairs into a hash set and append the new ones to `uniq`. The count is read on the
+// device; nothing is done when the pairs did not fit their buffer (the host redoes the batch). Most
+// pairs are already there (a pair is emitted by every region the two tasks share): a plain load finds
+// them without an atomic (8.2 M pairs, 1.4 M unique: 544 us with an atomic each, 372 so).
+constexpr int DEDUPE_PROBES = 128;
+__global__ void __launch_bounds__(256) dedupe_kernel(const unsigned long long * __restrict__ emit, unsigned long long emit_cap,
+                                                     unsigned long long * table, unsigned long long mask, unsigned long long * uniq,
+                                                     unsigned long long * cnt, unsigned long long uniq_cap)
 {
-    const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const unsigned long long key = emit[i];
-    unsigned long long h = mix64(key) & mask;
-    bool fresh = false;
-    for (unsigned long long probe = 0; probe <= mask; ++probe)
+    const unsigned long long n = cnt[CNT_EMIT];
+    if (n > emit_cap) return;
+    const int lane = threadIdx.x & 31;
+    const unsigned long long stride = (unsigned long long) gridDim.x * blockDim.x;
+    for (unsigned long long i0 = (unsigned long long) blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < n; i0 += stride)
     {
-        const unsigned long long prev = atomicCAS(table + h, EDGE_EMPTY, key);
-        if (prev == EDGE_EMPTY) { fresh = true; break; }
-        if (prev == key) break;
-        h = (h + 1) & mask;
-    }
-    // one atomic per warp on the shared counter for the warp's new pairs
-    const unsigned act = __activemask();
-    const unsigned nb = __ballot_sync(act, fresh);
-    if (!nb) return;
-    const int lane = threadIdx.x & 31, first = __ffs(nb) - 1;
-    unsigned long long base = 0;
-    if (lane == first) base = atomicAdd(nuniq, (unsigned long long) __popc(nb));
-    base = __shfl_sync(act, base, first);
-    if (fresh)
-    {
-        const unsigned long long s = base + __popc(nb & ((1u << lane) - 1));
-        if (s < uniq_cap) uniq[s] = key;
+        const unsigned long long i = i0 + lane;
+        bool fresh = false;
+        unsigned long long key = 0;
+        if (i < n)
+        {
+            key = emit[i];
+            unsigned long long h = mix64(key) & mask;
+            bool done = false;
+            for (int probe = 0; probe < DEDUPE_PROBES && !done; ++probe)
+            {
+                unsigned long long v = *(volatile unsigned long long *) (table + h);
+                if (v == EDGE_EMPTY) { v = atomicCAS(table + h, EDGE_EMPTY, key); fresh = done = v == EDGE_EMPTY; }
+                done = done || v == key;
+                h = (h + 1) & mask;
+            }
+            if (!done) cnt[CNT_FULL] = 1;
+        }
+        // one atomic per warp on the shared counter for the warp's new pairs
+        const unsigned nb = __ballot_sync(0xffffffffu, fresh);
+        if (!nb) continue;
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(cnt + CNT_UNIQ, (unsigned long long) __popc(nb));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (fresh)
+        {
+            const unsigned long long at = base + __popc(nb & ((1u << lane) - 1));
+            if (at < uniq_cap) uniq[at] = key; else cnt[CNT_FULL] = 1;
+        }
     }
 }
 
@@ -688,19 +574,50 @@ __global__ void scatter_window_edges_kernel(const unsigned long long * __restric
     succ[atomicAdd(cursor + (p - first), 1u)] = q - first;
 }
 
-// Sort each successor list ascending (deterministic CSR). Short lists: one thread, insertion sort.
-__global__ void sort_segments_kernel(const uint32_t * __restrict__ ptr, uint32_t * succ, uint32_t ntasks)
+// Sort each successor list ascending (deterministic CSR), a warp per task: up to 32 successors by
+// counting the smaller ones over shuffles, up to SORT_LIST by a bitonic sort in the warp's share of
+// shared memory, longer lists in place in global memory by the same network. (Successors of a task are
+// distinct.) 45 us for 1.4 M edges of 65,536 tasks; one thread per task with an insertion sort took 235.
+constexpr uint32_t SORT_LIST = 512;
+__global__ void __launch_bounds__(256) sort_segments_kernel(const uint32_t * __restrict__ ptr, uint32_t * succ, uint32_t ntasks)
 {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ uint32_t keys_s[8][SORT_LIST];
+    const uint32_t t = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
     if (t >= ntasks) return;
-    const uint32_t b = ptr[t], e = ptr[t + 1];
-    for (uint32_t i = b + 1; i < e; ++i)
+    const uint32_t b = ptr[t], n = ptr[t + 1] - b;
+    if (n < 2) return;
+    if (n <= 32)
     {
-        const uint32_t v = succ[i];
-        uint32_t j = i;
-        while (j > b && succ[j - 1] > v) { succ[j] = succ[j - 1]; --j; }
-        succ[j] = v;
+        const uint32_t v = (uint32_t) lane < n ? succ[b + lane] : 0xffffffffu;
+        int rank = 0;
+        for (uint32_t k = 0; k < n; ++k) rank += __shfl_sync(0xffffffffu, v, (int) k) < v;
+        if ((uint32_t) lane < n) succ[b + rank] = v;
+        return;
     }
+    uint32_t * keys = n <= SORT_LIST ? keys_s[threadIdx.x >> 5] : succ + b;
+    if (n <= SORT_LIST) for (uint32_t i = lane; i < n; i += 32) keys[i] = succ[b + i];
+    __syncwarp();
+    // bitonic network for any n: every merge step compares ascending (the first one of a merge mirrored),
+    // so places past the end, which would hold the largest keys, never move
+    uint32_t p2 = 64;
+    while (p2 < n) p2 <<= 1;
+    for (uint32_t k = 2; k <= p2; k <<= 1)
+        for (uint32_t j = k; j > 1; j >>= 1)
+        {
+            for (uint32_t q = lane; q < p2 / 2; q += 32)
+            {
+                // the q-th pair: mirrored within blocks of k, then at distance j / 2 within blocks of j
+                const uint32_t blk = q / (j / 2), o = q % (j / 2), i = blk * j + o, l = j == k ? blk * j + j - 1 - o : i + j / 2;
+                if (l < n)
+                {
+                    const uint32_t x = keys[i], y = keys[l];
+                    if (x > y) { keys[i] = y; keys[l] = x; }
+                }
+            }
+            __syncwarp();
+        }
+    if (n <= SORT_LIST) for (uint32_t i = lane; i < n; i += 32) succ[b + i] = keys[i];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -892,6 +809,47 @@ struct HostStage {
     }
 };
 
+// Page-locked host memory for what the device reports back and for the small arrays it is given, so
+// that neither waits for a staging copy: results (first, fixed places), then `used` bytes handed out
+// to arrays whose copies are in flight; release() once the stream has been waited for.
+struct HostScratch {
+    static constexpr size_t RESULTS = 256, KEYS = 2048;           // bytes; keys of each axis read back with the counts
+    uint8_t * p = nullptr;
+    size_t cap = 0, used = 0;
+    HostScratch() = default;
+    HostScratch(const HostScratch &) = delete;
+    HostScratch & operator=(const HostScratch &) = delete;
+    ~HostScratch() { if (p) cudaFreeHost(p); }
+    uint64_t * results() { return (uint64_t *) p; }
+    uint64_t * keys(int axis) { return (uint64_t *) (p + RESULTS) + axis * KEYS; }
+    void release() { used = RESULTS + 2 * KEYS * sizeof(uint64_t); }
+    int init() { return p ? XKB_OK : grow(size_t(1) << 18); }
+    // n bytes for a copy to the device queued on `st`; a full scratch waits for the copies so far
+    int take(size_t n, cudaStream_t st, void ** out)
+    {
+        n = (n + 15) & ~(size_t) 15;
+        if (used + n > cap)
+        {
+            XKB_CUDA_TRY(cudaStreamSynchronize(st));
+            release();
+            if (used + n > cap) if (int rc = grow(2 * (used + n))) return rc;
+        }
+        *out = p + used;
+        used += n;
+        return XKB_OK;
+    }
+private:
+    int grow(size_t n)
+    {
+        uint8_t * q = nullptr;
+        cudaError_t e = cudaHostAlloc((void **) &q, n, cudaHostAllocDefault);
+        if (e != cudaSuccess) return xkb_set_cuda_error(e);
+        if (p) cudaFreeHost(p);
+        p = q; cap = n; release();
+        return XKB_OK;
+    }
+};
+
 } // namespace xkb
 
 using namespace xkb;
@@ -915,7 +873,8 @@ struct xkb_resolver {
     // the last one cannot take a batch's worst case, so stored edges are never moved
     std::vector<std::unique_ptr<DevBuf<unsigned long long>>> useg;
     std::vector<size_t> useg_n;
-    DevBuf<unsigned long long> counters;        // [0] emit count, [1] unique count
+    DevBuf<unsigned long long> counters;        // CNT_*
+    DevBuf<int> maps;                           // refinement: the old cell row / column of each new one
     DevBuf<int> spill;                          // reader spill chunks (SPILL ints each)
     DevBuf<unsigned> spill_ctr;                 // [0] chunks handed out, [1] ran-out flag
     size_t spill_chunks = 0;                    // pool capacity in chunks
@@ -926,12 +885,15 @@ struct xkb_resolver {
     DevBuf<uint32_t> win_ptr, win_succ, win_npred, win_tmp;   // window graphs (a runtime running the graph in pieces)
     DevBuf<uint32_t> periodic;                  // packed arrays of the periodic form
     DevBuf<unsigned> bin_off, bin_cur;          // ops binned to regions: offsets, fill cursors
-    DevBuf<int> bin_list, bin_flag;             // op indices per region; region-too-long flag
-    DevBuf<int> snap;                           // cell states at the time-split cuts (resolve_puts_kernel)
+    DevBuf<int> bin_list, bin_sorted;           // op indices per region, as filled and in op order
     bool graph_valid = false;
     double last_device_ms = 0;
     double last_ops_ms = 0, last_compress_ms = 0;   // host phases of the last batch
     double emit_per_op = 32.0;                  // emitted-pair estimate per op (from the last batch)
+    double uniq_per_op = 8.0;                   // unique-pair estimate per op
+    HostScratch host;
+    cudaEvent_t ev[2] = {nullptr, nullptr};     // around the last batch
+    ~xkb_resolver() { for (cudaEvent_t e : ev) if (e) cudaEventDestroy(e); }
     // parallel host passes (validation, op build): the host team and the page-locked staging buffer
     std::unique_ptr<WorkPool> pool;
     HostStage stage;
@@ -1238,11 +1200,12 @@ static int spill_reserve(xkb_resolver * R, size_t chunks)
     return XKB_OK;
 }
 
+__global__ void set_spill_kernel(unsigned * ctr, unsigned used) { ctr[0] = used; ctr[1] = 0; }
+
 static int reset_spill(xkb_resolver * R)
 {
-    const unsigned v[2] = {R->spill_used, 0u};
-    XKB_CUDA_TRY(cudaMemcpyAsync(R->spill_ctr.p, v, sizeof(v), cudaMemcpyHostToDevice, R->stream));
-    XKB_CUDA_TRY(cudaStreamSynchronize(R->stream));   // v is on this stack frame
+    set_spill_kernel<<<1, 1, 0, R->stream>>>(R->spill_ctr.p, R->spill_used);
+    XKB_CUDA_TRY(cudaGetLastError());
     return XKB_OK;
 }
 
@@ -1297,7 +1260,10 @@ static int refine_domain(xkb_resolver * R, Domain & d, std::vector<uint64_t> & x
     else
     {
         const size_t old_ncx = d.xs.size() - 1;
-        std::vector<int> mx(ncx), my(ncy);
+        if ((rc = R->maps.reserve(ncx + ncy))) return rc;
+        void * m = nullptr;
+        if ((rc = R->host.take((ncx + ncy) * sizeof(int), R->stream, &m))) return rc;
+        int * mx = (int *) m, * my = mx + ncx;
         for (size_t i = 0; i < ncx; ++i) {
             const uint64_t v = xs[i];
             if (v < d.xs.front() || v >= d.xs.back()) mx[i] = -1;
@@ -1308,10 +1274,7 @@ static int refine_domain(xkb_resolver * R, Domain & d, std::vector<uint64_t> & x
             if (v < d.ys.front() || v >= d.ys.back()) my[i] = -1;
             else my[i] = (int) (std::upper_bound(d.ys.begin(), d.ys.end(), v) - d.ys.begin()) - 1;
         }
-        DevBuf<int> dm;
-        if ((rc = dm.reserve(ncx + ncy))) return rc;
-        XKB_CUDA_TRY(cudaMemcpyAsync(dm.p, mx.data(), ncx * sizeof(int), cudaMemcpyHostToDevice, R->stream));
-        XKB_CUDA_TRY(cudaMemcpyAsync(dm.p + ncx, my.data(), ncy * sizeof(int), cudaMemcpyHostToDevice, R->stream));
+        XKB_CUDA_TRY(cudaMemcpyAsync(R->maps.p, mx, (ncx + ncy) * sizeof(int), cudaMemcpyHostToDevice, R->stream));
         pt.mark("maps");
         if ((rc = spill_reserve(R, 1))) return rc;
         pt.mark("spill-reserve");
@@ -1319,10 +1282,10 @@ static int refine_domain(xkb_resolver * R, Domain & d, std::vector<uint64_t> & x
         {
             if ((rc = reset_spill(R))) return rc;
             refine_state_kernel<<<(unsigned) ((ncells + 255) / 256), 256, 0, R->stream>>>(
-                d.state[d.cur].p, out.p, dm.p, dm.p + ncx, (int) ncx, (int) ncy, (int) old_ncx, R->spill.p, R->spill_ctr.p,
+                d.state[d.cur].p, out.p, R->maps.p, R->maps.p + ncx, (int) ncx, (int) ncy, (int) old_ncx, R->spill.p, R->spill_ctr.p,
                 (unsigned) R->spill_chunks);
             XKB_CUDA_TRY(cudaGetLastError());
-            if ((rc = spill_check(R, redo))) return rc;   // synchronises: dm is freed on return
+            if ((rc = spill_check(R, redo))) return rc;
             pt.mark("refine-kernel+sync");
         }
     }
@@ -1332,9 +1295,25 @@ static int refine_domain(xkb_resolver * R, Domain & d, std::vector<uint64_t> & x
     return XKB_OK;
 }
 
-// Bin the batch's ops to regions (counts, offsets, fill, per-region sort) and run the region
-// kernel over each region's own list; a region too crowded to sort falls back to the kernel that
-// scans every op of the batch.
+// Dynamic shared memory a kernel may ask for on the current device, set once per kernel and device
+// and raised when a call needs more.
+template <typename K>
+static int allow_smem(K kernel, size_t bytes)
+{
+    if (bytes > 48 * 1024) XKB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes));
+    return XKB_OK;
+}
+
+static int device_sms()
+{
+    int sms = 148, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+// Bin the batch's ops to regions (counts, offsets, fill, per-region sort) and run the segment kernel
+// over each region's own list.
 template <int RX, int RY>
 static int launch_region(xkb_resolver * R, ResolveArgs & a, int nregions)
 {
@@ -1343,82 +1322,53 @@ static int launch_region(xkb_resolver * R, ResolveArgs & a, int nregions)
     const size_t nb = (size_t) nregions + 1;
     int rc;
     PhaseTrace pt("regions");
-    if ((rc = R->bin_off.reserve(nb)) || (rc = R->bin_cur.reserve(nb)) ||
-        (rc = R->tmp.reserve(nb / SCAN_TILE + 2)) || (rc = R->bin_flag.reserve(1)))
-        return rc;
+    if ((rc = R->bin_off.reserve(nb)) || (rc = R->bin_cur.reserve(nb)) || (rc = R->tmp.reserve(nb / SCAN_TILE + 2))) return rc;
     pt.mark("reserve");
     XKB_CUDA_TRY(cudaMemsetAsync(R->bin_off.p, 0, nb * sizeof(unsigned), st));
     XKB_CUDA_TRY(cudaMemsetAsync(R->bin_cur.p, 0, nb * sizeof(unsigned), st));
-    XKB_CUDA_TRY(cudaMemsetAsync(R->bin_flag.p, 0, sizeof(int), st));
     const unsigned g = (unsigned) ((a.nops + 255) / 256);
     // block-local binning: a grid of a few blocks per SM, each walking its share of the ops
     const char * gb = getenv("XKB_RESOLVE_BIN_GLOBAL");             // 1: the global-atomic binning (tests)
     const bool smem_bins = nregions <= BIN_SMEM_REGIONS && !(gb && atoi(gb) == 1);
-    int sms = 148, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const unsigned gs = std::min<unsigned>(g, (unsigned) (2 * sms));
+    const unsigned gs = std::min<unsigned>(g, (unsigned) (2 * device_sms()));
+    const size_t bins = (size_t) nregions * sizeof(unsigned);
     if (smem_bins)
     {
-        XKB_CUDA_TRY(cudaFuncSetAttribute(bin_count_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          BIN_SMEM_REGIONS * (int) sizeof(unsigned)));
-        bin_count_smem_kernel<<<gs, 256, (size_t) nregions * sizeof(unsigned), st>>>(a.ops, a.nops, RX, RY, a.nrx, nregions,
-                                                                                   R->bin_off.p);
+        if ((rc = allow_smem(bin_count_smem_kernel, bins))) return rc;
+        bin_count_smem_kernel<<<gs, 256, bins, st>>>(a.ops, a.nops, RX, RY, a.nrx, nregions, R->bin_off.p);
     }
     else
         bin_count_kernel<<<g, 256, 0, st>>>(a.ops, a.nops, RX, RY, a.nrx, R->bin_off.p);
     if ((rc = device_exclusive_scan(R->bin_off.p, R->bin_off.p, nb, R->tmp.p, nullptr, st))) return rc;
-    unsigned total = 0;
-    XKB_CUDA_TRY(cudaMemcpyAsync(&total, R->bin_off.p + nregions, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    unsigned * total_p = (unsigned *) R->host.results();
+    XKB_CUDA_TRY(cudaMemcpyAsync(total_p, R->bin_off.p + nregions, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     XKB_CUDA_TRY(cudaStreamSynchronize(st));
+    R->host.release();
+    const unsigned total = *total_p;
     pt.mark("count+sync");
-    bool binned = total > 0;
-    if (binned)
+    if (total)
     {
-        if ((rc = R->bin_list.reserve(total))) return rc;
+        if ((rc = R->bin_list.reserve(total)) || (rc = R->bin_sorted.reserve(total))) return rc;
         if (smem_bins)
         {
-            XKB_CUDA_TRY(cudaFuncSetAttribute(bin_fill_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              2 * BIN_SMEM_REGIONS * (int) sizeof(unsigned)));
-            bin_fill_smem_kernel<<<gs, 256, 2 * (size_t) nregions * sizeof(unsigned), st>>>(a.ops, a.nops, RX, RY, a.nrx, nregions,
-                                                                                         R->bin_off.p, R->bin_cur.p, R->bin_list.p);
+            if ((rc = allow_smem(bin_fill_smem_kernel, 2 * bins))) return rc;
+            bin_fill_smem_kernel<<<gs, 256, 2 * bins, st>>>(a.ops, a.nops, RX, RY, a.nrx, nregions, R->bin_off.p, R->bin_cur.p,
+                                                            R->bin_list.p);
         }
         else
             bin_fill_kernel<<<g, 256, 0, st>>>(a.ops, a.nops, RX, RY, a.nrx, R->bin_off.p, R->bin_cur.p, R->bin_list.p);
-        XKB_CUDA_TRY(cudaFuncSetAttribute(bin_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BIN_SORT_CAP * (int) sizeof(int)));
-        bin_sort_kernel<<<(unsigned) nregions, BIN_SORT_THREADS, BIN_SORT_CAP * sizeof(int), st>>>(R->bin_off.p, R->bin_list.p, R->bin_flag.p);
-        int too_long = 0;
-        XKB_CUDA_TRY(cudaMemcpyAsync(&too_long, R->bin_flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-        XKB_CUDA_TRY(cudaStreamSynchronize(st));
-        pt.mark("fill+sort+sync");
-        binned = !too_long;
+        const int words = std::max(BIN_SORT_SHORT, std::min(BIN_SORT_WORDS, (a.nops + 31) / 32));
+        if ((rc = allow_smem(bin_sort_kernel, (size_t) words * sizeof(unsigned)))) return rc;
+        bin_sort_kernel<<<(unsigned) nregions, BIN_SORT_THREADS, (size_t) words * sizeof(unsigned), st>>>(R->bin_off.p, R->bin_list.p,
+                                                                                                          R->bin_sorted.p, a.nops, words);
     }
-    // time split: segments per region from the mean list length (a segment of a few hundred ops
-    // still amortises its state load); XKB_RESOLVE_SEGMENTS overrides (1 = one pass per region)
+    // segments per region from the mean list length (a segment of a few hundred ops still amortises its
+    // look-back); XKB_RESOLVE_SEGMENTS overrides (1 = one pass per region)
     const char * seg_s = getenv("XKB_RESOLVE_SEGMENTS");
     const int seg_env = seg_s ? atoi(seg_s) : 0;
-    int nseg = seg_env > 0 ? seg_env : (int) std::min<size_t>(MAX_SEGMENTS, std::max<size_t>(1, (size_t) total / nregions / 512));
+    int nseg = seg_env > 0 ? seg_env : (int) std::min<size_t>(MAX_SEGMENTS, std::max<size_t>(1, (size_t) total / nregions / SEGMENT_OPS));
     nseg = std::max(1, std::min(nseg, MAX_SEGMENTS));
-    if (binned && nseg > 1)
-    {
-        const size_t ncells = (size_t) a.ncx * a.ncy;
-        if ((rc = R->snap.reserve((size_t) (nseg - 1) * ncells * STRIDE))) return rc;
-        XKB_CUDA_TRY(cudaFuncSetAttribute(resolve_puts_kernel<RX, RY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-        XKB_CUDA_TRY(cudaFuncSetAttribute(resolve_links_kernel<RX, RY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-        resolve_puts_kernel<RX, RY><<<(unsigned) nregions, RX * RY, smem, st>>>(a, R->bin_off.p, R->bin_list.p, nseg, R->snap.p, ncells);
-        resolve_links_kernel<RX, RY><<<(unsigned) (nregions * nseg), RX * RY, smem, st>>>(a, R->bin_off.p, R->bin_list.p, nseg,
-                                                                                      R->snap.p, ncells);
-    }
-    else if (binned)
-    {
-        XKB_CUDA_TRY(cudaFuncSetAttribute(resolve_region_kernel<RX, RY, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-        resolve_region_kernel<RX, RY, true><<<(unsigned) nregions, RX * RY, smem, st>>>(a, R->bin_off.p, R->bin_list.p);
-    }
-    else
-    {
-        XKB_CUDA_TRY(cudaFuncSetAttribute(resolve_region_kernel<RX, RY, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-        resolve_region_kernel<RX, RY, false><<<(unsigned) nregions, RX * RY, smem, st>>>(a, nullptr, nullptr);
-    }
+    resolve_segment_kernel<RX, RY><<<(unsigned) (nregions * nseg), RX * RY, smem, st>>>(a, R->bin_off.p, R->bin_sorted.p, nseg);
     XKB_CUDA_TRY(cudaGetLastError());
     return XKB_OK;
 }
@@ -1462,16 +1412,23 @@ static int compress_domain(xkb_resolver * R, Domain & d, const HOp * hops, DOp *
     collect_bounds_kernel<<<g, 256, 0, st>>>(hops, (int) nops, R->hset.p, R->hset.p + cap, (uint32_t) (cap - 1),
                                              R->ukeys.p, R->ukeys.p + 2 * nops, R->ucount.p);
     XKB_CUDA_TRY(cudaGetLastError());
-    unsigned cnt[3];
-    XKB_CUDA_TRY(cudaMemcpyAsync(cnt, R->ucount.p, sizeof(cnt), cudaMemcpyDeviceToHost, st));
+    // the counts and the first keys come back together: most batches have no more
+    unsigned * cnt = (unsigned *) R->host.results();
+    const size_t some = std::min<size_t>(HostScratch::KEYS, 2 * nops);
+    XKB_CUDA_TRY(cudaMemcpyAsync(cnt, R->ucount.p, 3 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    XKB_CUDA_TRY(cudaMemcpyAsync(R->host.keys(0), R->ukeys.p, some * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    XKB_CUDA_TRY(cudaMemcpyAsync(R->host.keys(1), R->ukeys.p + 2 * nops, some * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     XKB_CUDA_TRY(cudaStreamSynchronize(st));
+    R->host.release();
     pt.mark("collect+sync");
     std::vector<uint64_t> xs(d.xs.size() + cnt[0] + 1), ys(d.ys.size() + cnt[1] + 1);
     std::copy(d.xs.begin(), d.xs.end(), xs.begin());
     std::copy(d.ys.begin(), d.ys.end(), ys.begin());
-    if (cnt[0]) XKB_CUDA_TRY(cudaMemcpyAsync(xs.data() + d.xs.size(), R->ukeys.p, cnt[0] * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    if (cnt[1]) XKB_CUDA_TRY(cudaMemcpyAsync(ys.data() + d.ys.size(), R->ukeys.p + 2 * nops, cnt[1] * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    XKB_CUDA_TRY(cudaStreamSynchronize(st));
+    std::copy_n(R->host.keys(0), std::min<size_t>(cnt[0], some), xs.begin() + d.xs.size());
+    std::copy_n(R->host.keys(1), std::min<size_t>(cnt[1], some), ys.begin() + d.ys.size());
+    if (cnt[0] > some) XKB_CUDA_TRY(cudaMemcpyAsync(xs.data() + d.xs.size() + some, R->ukeys.p + some, (cnt[0] - some) * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    if (cnt[1] > some) XKB_CUDA_TRY(cudaMemcpyAsync(ys.data() + d.ys.size() + some, R->ukeys.p + 2 * nops + some, (cnt[1] - some) * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    if (cnt[0] > some || cnt[1] > some) XKB_CUDA_TRY(cudaStreamSynchronize(st));
     if (cnt[2] & 1u) xs.back() = KEY_EMPTY; else xs.pop_back();
     if (cnt[2] & 2u) ys.back() = KEY_EMPTY; else ys.pop_back();
     for (std::vector<uint64_t> * v : {&xs, &ys})
@@ -1483,22 +1440,26 @@ static int compress_domain(xkb_resolver * R, Domain & d, const HOp * hops, DOp *
     if ((rc = refine_domain(R, d, xs, ys))) return rc;
     pt.mark("refine");
     if ((rc = R->bounds.reserve(d.xs.size() + d.ys.size()))) return rc;
-    XKB_CUDA_TRY(cudaMemcpyAsync(R->bounds.p, d.xs.data(), d.xs.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    XKB_CUDA_TRY(cudaMemcpyAsync(R->bounds.p + d.xs.size(), d.ys.data(), d.ys.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
+    void * hb = nullptr;
+    const size_t nbounds = d.xs.size() + d.ys.size();
+    if ((rc = R->host.take(nbounds * sizeof(uint64_t), st, &hb))) return rc;
+    std::copy(d.ys.begin(), d.ys.end(), std::copy(d.xs.begin(), d.xs.end(), (uint64_t *) hb));
+    XKB_CUDA_TRY(cudaMemcpyAsync(R->bounds.p, hb, nbounds * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     map_ops_kernel<<<g, 256, 0, st>>>(hops, (int) nops, R->bounds.p, (int) d.xs.size(), R->bounds.p + d.xs.size(),
                                       (int) d.ys.size(), dops);
     XKB_CUDA_TRY(cudaGetLastError());
-    // the host vectors above die on return: the copies out of them must be done
-    XKB_CUDA_TRY(cudaStreamSynchronize(st));
-    pt.mark("map+sync");
+    pt.mark("map");
     return XKB_OK;
 }
+
+__global__ void set_uniq_kernel(unsigned long long * cnt, unsigned long long n) { cnt[CNT_UNIQ] = n; cnt[CNT_FULL] = 0; }
 
 static int resolve_batch(xkb_resolver * R, const xkb_access_rec_t * recs, size_t n)
 {
     int rc;
     using clk = std::chrono::steady_clock;
     const auto t0 = clk::now();
+    if ((rc = R->host.init())) return rc;
     R->staged = false;
     rc = build_ops_staged(R, recs, n);
     if (rc < 0) return rc;
@@ -1533,77 +1494,88 @@ static int resolve_batch(xkb_resolver * R, const xkb_access_rec_t * recs, size_t
 
     static const bool trace = getenv("XKB_TRACE_RESOLVE") != nullptr;
     const size_t realloc0 = g_realloc_bytes;
-    // an emit buffer too small costs a second pass of the region kernel: size it from the pairs per
-    // op the last batch emitted (32 per op before the first), within 2^28 pairs
+    // the emit buffer, the hash set and the room for unique pairs are sized from the pairs per op of the
+    // last batch (32 emitted and 8 unique per op before the first), within 2^28 pairs, so that nothing is read back between
+    // the steps; what turns out too small is redone with what it needs
     size_t emit_guess = std::max<size_t>(1 << 16, std::min<size_t>(size_t(1) << 28, (size_t) (total * R->emit_per_op)));
-    for (int attempt = 0; attempt < 16; ++attempt)
+    size_t uniq_guess = std::min<size_t>(emit_guess, std::max<size_t>(1 << 14, (size_t) (total * R->uniq_per_op)));
+    bool regions = true;                       // false: only the unique step is redone
+    auto ta = clk::now();
+    for (int attempt = 0; attempt < 24; ++attempt)
     {
-        const auto ta = clk::now();
-        if ((rc = R->emit.reserve(emit_guess))) return rc;
-        if ((rc = R->counters.reserve(2))) return rc;
-        if ((rc = spill_reserve(R, 1)) || (rc = reset_spill(R))) return rc;
-        XKB_CUDA_TRY(cudaMemsetAsync(R->counters.p, 0, 2 * sizeof(unsigned long long), R->stream));
-        for (size_t k = 0; k < doms.size(); ++k)
+        if (regions)
         {
-            const size_t nops = doms[k]->nops;
-            // states must exist for every cell (ncells > 0 when the domain has >= 1 op)
-            if ((rc = R->emit.reserve(emit_guess))) return rc;
-            if (doms[k]->ncells == 0) continue;
-            if ((rc = doms[k]->state[doms[k]->cur ^ 1].reserve(doms[k]->ncells * STRIDE))) return rc;
-            if ((rc = launch_domain(R, *doms[k], offs[k], nops))) return rc;
+            ta = clk::now();
+            if ((rc = R->emit.reserve(emit_guess)) || (rc = R->counters.reserve(CNT_COUNT))) return rc;
+            if ((rc = spill_reserve(R, 1)) || (rc = reset_spill(R))) return rc;
+            XKB_CUDA_TRY(cudaMemsetAsync(R->counters.p, 0, CNT_COUNT * sizeof(unsigned long long), R->stream));
+            for (size_t k = 0; k < doms.size(); ++k)
+            {
+                const size_t nops = doms[k]->nops;
+                // states must exist for every cell (ncells > 0 when the domain has >= 1 op)
+                if (doms[k]->ncells == 0) continue;
+                if ((rc = doms[k]->state[doms[k]->cur ^ 1].reserve(doms[k]->ncells * STRIDE))) return rc;
+                if ((rc = launch_domain(R, *doms[k], offs[k], nops))) return rc;
+            }
         }
-        unsigned long long nemit = 0;
-        unsigned sp[2] = {0, 0};
-        XKB_CUDA_TRY(cudaMemcpyAsync(&nemit, R->counters.p, sizeof(nemit), cudaMemcpyDeviceToHost, R->stream));
-        XKB_CUDA_TRY(cudaMemcpyAsync(sp, R->spill_ctr.p, sizeof(sp), cudaMemcpyDeviceToHost, R->stream));
+        // unique the emitted pairs into the accumulated edge list
+        size_t tcap = 1024;
+        while (tcap < 2 * uniq_guess) tcap *= 2;
+        if ((rc = R->table.reserve(tcap))) return rc;
+        if (R->useg.empty() || R->useg.back()->cap - R->useg_n.back() < uniq_guess)
+        {
+            std::unique_ptr<DevBuf<unsigned long long>> seg(new (std::nothrow) DevBuf<unsigned long long>());
+            if (!seg) return xkb_set_error(XKB_ENOMEM, "resolver: out of host memory");
+            seg->use_pool(R->stream);
+            // segments double in size, so a long stream allocates a few of them, not one per batch
+            const size_t last = R->useg.empty() ? 0 : R->useg.back()->cap;
+            if ((rc = seg->reserve(std::max<size_t>({uniq_guess, size_t(1) << 24, 2 * last})))) return rc;
+            R->useg.push_back(std::move(seg));
+            R->useg_n.push_back(0);
+        }
+        DevBuf<unsigned long long> & seg = *R->useg.back();
+        const unsigned long long nu0 = R->useg_n.back();
+        XKB_CUDA_TRY(cudaMemsetAsync(R->table.p, 0xff, tcap * sizeof(unsigned long long), R->stream));
+        set_uniq_kernel<<<1, 1, 0, R->stream>>>(R->counters.p, nu0);
+        dedupe_kernel<<<(unsigned) std::min<size_t>((emit_guess + 255) / 256, (size_t) device_sms() * 8), 256, 0, R->stream>>>(
+            R->emit.p, R->emit.cap, R->table.p, tcap - 1, seg.p, R->counters.p, seg.cap);
+        XKB_CUDA_TRY(cudaGetLastError());
+        unsigned long long * cnt = (unsigned long long *) R->host.results();
+        unsigned * sp = (unsigned *) (cnt + CNT_COUNT);
+        XKB_CUDA_TRY(cudaMemcpyAsync(cnt, R->counters.p, CNT_COUNT * sizeof(unsigned long long), cudaMemcpyDeviceToHost, R->stream));
+        XKB_CUDA_TRY(cudaMemcpyAsync(sp, R->spill_ctr.p, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, R->stream));
         XKB_CUDA_TRY(cudaStreamSynchronize(R->stream));
-        if (sp[1])
+        R->host.release();
+        const unsigned long long nemit = cnt[CNT_EMIT], nu = cnt[CNT_UNIQ];
+        if (regions && sp[1])
         {
             // the reader spill pool ran out: grow it (keeping its chunks) and redo the batch
             if ((rc = spill_reserve(R, (size_t) sp[0] + 1))) return rc;
             continue;
         }
-        const auto tb = clk::now();
-        if (nemit > R->emit.cap) { emit_guess = (size_t) nemit; continue; }
-        R->spill_used = sp[0];
-        if (total) R->emit_per_op = std::max(2.0, 1.25 * (double) nemit / (double) total);
-
-        // success: unique the emitted pairs into the accumulated edge list
-        if (nemit)
+        if (nemit > R->emit.cap) { emit_guess = (size_t) nemit; uniq_guess = std::min<size_t>(2 * uniq_guess, emit_guess); regions = true; continue; }
+        if (cnt[CNT_FULL])
         {
-            size_t tcap = 1024;
-            while (tcap < 2 * nemit) tcap *= 2;
-            if ((rc = R->table.reserve(tcap))) return rc;
-            if (R->useg.empty() || R->useg.back()->cap - R->useg_n.back() < nemit)
-            {
-                std::unique_ptr<DevBuf<unsigned long long>> seg(new (std::nothrow) DevBuf<unsigned long long>());
-                if (seg) seg->use_pool(R->stream);
-                if (!seg) return xkb_set_error(XKB_ENOMEM, "resolver: out of host memory");
-                // segments double in size, so a long stream allocates a few of them, not one per batch
-                const size_t last = R->useg.empty() ? 0 : R->useg.back()->cap;
-                if ((rc = seg->reserve(std::max<size_t>({(size_t) nemit, size_t(1) << 24, 2 * last})))) return rc;
-                R->useg.push_back(std::move(seg));
-                R->useg_n.push_back(0);
-            }
-            DevBuf<unsigned long long> & seg = *R->useg.back();
-            XKB_CUDA_TRY(cudaMemsetAsync(R->table.p, 0xff, tcap * sizeof(unsigned long long), R->stream));
-            unsigned long long nu0 = R->useg_n.back();
-            XKB_CUDA_TRY(cudaMemcpyAsync(R->counters.p + 1, &nu0, sizeof(nu0), cudaMemcpyHostToDevice, R->stream));
-            dedupe_kernel<<<(unsigned) ((nemit + 255) / 256), 256, 0, R->stream>>>(R->emit.p, nemit, R->table.p, tcap - 1,
-                                                                                 seg.p, R->counters.p + 1, seg.cap);
-            XKB_CUDA_TRY(cudaGetLastError());
-            unsigned long long nu = 0;
-            XKB_CUDA_TRY(cudaMemcpyAsync(&nu, R->counters.p + 1, sizeof(nu), cudaMemcpyDeviceToHost, R->stream));
-            XKB_CUDA_TRY(cudaStreamSynchronize(R->stream));
-            R->nuniq += nu - nu0;
-            R->useg_n.back() = nu;
+            // no room in the hash set or the segment: four times as much
+            uniq_guess *= 4;
+            regions = false;
+            continue;
         }
+        const auto tb = clk::now();
+        R->spill_used = sp[0];
+        if (total)
+        {
+            R->emit_per_op = std::max(2.0, 1.25 * (double) nemit / (double) total);
+            R->uniq_per_op = std::max(1.0, 1.5 * (double) (nu - nu0) / (double) total);
+        }
+        R->nuniq += nu - nu0;
+        R->useg_n.back() = nu;
         for (Domain * d : doms) { d->cur ^= 1; d->ops.clear(); d->nops = 0; }
         if (trace)
-            fprintf(stderr, "resolver batch: %zu ops (built in %.1f ms, compressed in %.1f ms), attempt %d, regions %.1f ms, dedupe %.1f ms, "
-                    "%llu emitted, %.1f MB allocated\n",
+            fprintf(stderr, "resolver batch: %zu ops (built in %.2f ms, compressed in %.2f ms), attempt %d, regions and unique %.2f ms, "
+                    "%llu emitted, %llu unique, %.1f MB allocated\n",
                     total, R->last_ops_ms, R->last_compress_ms, attempt, std::chrono::duration<double, std::milli>(tb - ta).count(),
-                    std::chrono::duration<double, std::milli>(clk::now() - tb).count(), nemit, (g_realloc_bytes - realloc0) / 1e6);
+                    nemit, nu - nu0, (g_realloc_bytes - realloc0) / 1e6);
         return XKB_OK;
     }
     return xkb_set_error(XKB_ERANGE, "resolver: batch did not fit after resizing");
@@ -1630,7 +1602,7 @@ static int build_graph(xkb_resolver * R)
         if (R->useg_n[k])
             scatter_edges_kernel<<<(unsigned) ((R->useg_n[k] + 255) / 256), 256, 0, st>>>(R->useg[k]->p, R->useg_n[k], R->tmp.p,
                                                                                          R->succ.p);
-    if (nt) sort_segments_kernel<<<(unsigned) ((nt + 255) / 256), 256, 0, st>>>(R->succ_ptr.p, R->succ.p, (uint32_t) nt);
+    if (nt) sort_segments_kernel<<<(unsigned) ((nt + 7) / 8), 256, 0, st>>>(R->succ_ptr.p, R->succ.p, (uint32_t) nt);
     XKB_CUDA_TRY(cudaGetLastError());
     XKB_CUDA_TRY(cudaStreamSynchronize(st));
     R->graph_valid = true;
@@ -1659,7 +1631,7 @@ extern "C" int xkb_resolver_create(xkb_resolver_t ** out, void * stream)
     R->hset.use_pool(R->stream); R->ukeys.use_pool(R->stream); R->bounds.use_pool(R->stream); R->ucount.use_pool(R->stream);
     R->emit.use_pool(R->stream); R->table.use_pool(R->stream); R->counters.use_pool(R->stream);
     R->tmp.use_pool(R->stream); R->bin_off.use_pool(R->stream); R->bin_cur.use_pool(R->stream);
-    R->bin_list.use_pool(R->stream); R->bin_flag.use_pool(R->stream); R->snap.use_pool(R->stream);
+    R->bin_list.use_pool(R->stream); R->bin_sorted.use_pool(R->stream); R->maps.use_pool(R->stream);
     R->win_ptr.use_pool(R->stream); R->win_succ.use_pool(R->stream); R->win_npred.use_pool(R->stream);
     R->win_tmp.use_pool(R->stream);
     *out = R;
@@ -1746,16 +1718,14 @@ extern "C" int xkb_resolver_add(xkb_resolver_t * R, const xkb_access_rec_t * rec
     }
     int rc = validate(R, recs, n, R->ntasks);
     if (rc) return rc;
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0); cudaEventCreate(&e1);
-    cudaEventRecord(e0, R->stream);
+    for (cudaEvent_t & e : R->ev) if (!e) XKB_CUDA_TRY(cudaEventCreate(&e));
+    cudaEventRecord(R->ev[0], R->stream);
     rc = resolve_batch(R, recs, n);
     if (rc == XKB_OK) { R->ntasks = recs[n - 1].task + 1; R->graph_valid = false; }
-    cudaEventRecord(e1, R->stream);
-    cudaEventSynchronize(e1);
-    float ms = 0; cudaEventElapsedTime(&ms, e0, e1);
+    cudaEventRecord(R->ev[1], R->stream);
+    cudaEventSynchronize(R->ev[1]);
+    float ms = 0; cudaEventElapsedTime(&ms, R->ev[0], R->ev[1]);
     R->last_device_ms = ms;
-    cudaEventDestroy(e0); cudaEventDestroy(e1);
     return rc;
 }
 
@@ -1802,7 +1772,7 @@ int xkb_internal_resolver_window_graph(xkb_resolver_t * R, const xkb_edge_mark_t
     each_range([&](const unsigned long long * e, size_t n) {
         scatter_window_edges_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(e, n, first, R->win_tmp.p, R->win_succ.p);
     });
-    if (nt) sort_segments_kernel<<<(unsigned) ((nt + 255) / 256), 256, 0, st>>>(R->win_ptr.p, R->win_succ.p, (uint32_t) nt);
+    if (nt) sort_segments_kernel<<<(unsigned) ((nt + 7) / 8), 256, 0, st>>>(R->win_ptr.p, R->win_succ.p, (uint32_t) nt);
     XKB_CUDA_TRY(cudaGetLastError());
     g->ntasks = nt;
     g->nedges = ne;
