@@ -33,6 +33,10 @@
 #include "scan.cuh"
 #include "workpool.h"
 
+#if defined(__x86_64__)
+#include <emmintrin.h>
+#endif
+
 #include <algorithm>
 #include <climits>
 #include <chrono>
@@ -624,7 +628,29 @@ __global__ void __launch_bounds__(256) sort_segments_kernel(const uint32_t * __r
 // host side
 
 struct HRect { uint64_t x0, x1, y0, y1; };
+// An op in byte coordinates. PAIRED ops (staged batches) stand for a LINK and a PUT op each.
 struct HOp { uint32_t task; uint8_t link; uint8_t mode; HRect r; };
+
+// Store an op past the caches: the page-locked staging buffer is read by the GPU next, and reading
+// lines that lie modified in the caches of a dozen cores ran at 5 GB/s instead of 53 (13 MB: 2.3 ms
+// against 0.26). stream_fence() before the copy is queued.
+static inline void stream_op(HOp * p, const HOp & op)
+{
+#if defined(__x86_64__)
+    static_assert(sizeof(HOp) == 40, "five 8-byte stores");
+    long long w[5];
+    memcpy(w, &op, sizeof(op));
+    for (int k = 0; k < 5; ++k) _mm_stream_si64((long long *) p + k, w[k]);
+#else
+    *p = op;
+#endif
+}
+static inline void stream_fence()
+{
+#if defined(__x86_64__)
+    _mm_sfence();
+#endif
+}
 
 static size_t g_realloc_bytes = 0;               // device bytes allocated by reserve (trace)
 
@@ -661,6 +687,52 @@ static cudaMemPool_t resolver_pool()
     }
     return pools[dev];
 }
+
+// Page-locked host memory the resolvers of the process share: a batch takes blocks for its staging and
+// its read-backs and gives them back when it has been waited for, so a resolver holds none between
+// batches and a new one finds them there (page-locking costs about 0.5 ms per MB and waits for the
+// device; a server keeps a resolver per graph shape). Given-back blocks are kept up to PINNED_KEEP
+// bytes (XKB_POOL_CACHE=0: none); a block in use belongs to one batch.
+class PinnedBlocks {
+public:
+    static constexpr size_t PINNED_KEEP = size_t(128) << 20, MIN_BLOCK = size_t(1) << 18;
+
+    static int take(size_t bytes, void ** p, size_t * cap)
+    {
+        size_t c = MIN_BLOCK;
+        while (c < bytes) c *= 2;
+        {
+            std::lock_guard<std::mutex> lk(mu());
+            auto it = free_blocks().find(c);
+            if (it != free_blocks().end())
+            {
+                *p = it->second; *cap = c;
+                free_blocks().erase(it);
+                kept() -= c;
+                return XKB_OK;
+            }
+        }
+        cudaError_t e = cudaHostAlloc(p, c, cudaHostAllocPortable);
+        if (e != cudaSuccess) { *p = nullptr; return xkb_set_cuda_error(e); }
+        *cap = c;
+        return XKB_OK;
+    }
+    static void give(void * p, size_t cap)
+    {
+        if (!p) return;
+        static const bool none = getenv("XKB_POOL_CACHE") && atoi(getenv("XKB_POOL_CACHE")) == 0;
+        {
+            std::lock_guard<std::mutex> lk(mu());
+            if (!none && kept() + cap <= PINNED_KEEP) { free_blocks().emplace(cap, p); kept() += cap; return; }
+        }
+        cudaFreeHost(p);
+    }
+
+private:                                        // (never destroyed: resolvers may outlive static objects)
+    static std::mutex & mu() { static std::mutex * m = new std::mutex; return *m; }
+    static std::multimap<size_t, void *> & free_blocks() { static auto * f = new std::multimap<size_t, void *>; return *f; }
+    static size_t & kept() { static size_t k = 0; return k; }
+};
 
 template <typename T>
 struct DevBuf {
@@ -760,7 +832,10 @@ __device__ __forceinline__ int32_t lower_index(const uint64_t * __restrict__ v, 
     return lo;
 }
 
-// Ops in cell coordinates: each boundary's index in the domain's sorted boundary lists.
+// Ops in cell coordinates: each boundary's index in the domain's sorted boundary lists. PAIRED: op e
+// of a task's ops [b, f) (ops are in task order) becomes the LINK op b + e and the PUT op f + e -- all
+// of a task's LINK ops before its PUT ops.
+template <bool PAIRED>
 __global__ void map_ops_kernel(const HOp * __restrict__ ops, int n, const uint64_t * __restrict__ xs, int nxs,
                                const uint64_t * __restrict__ ys, int nys, DOp * out)
 {
@@ -768,10 +843,31 @@ __global__ void map_ops_kernel(const HOp * __restrict__ ops, int n, const uint64
     if (i >= n) return;
     const HOp o = ops[i];
     DOp q;
-    q.task = (int32_t) o.task; q.link = o.link; q.mode = o.mode; q.pad = 0;
+    q.task = (int32_t) o.task; q.link = PAIRED ? 1 : o.link; q.mode = o.mode; q.pad = 0;
     q.cx0 = lower_index(xs, nxs, o.r.x0); q.cx1 = lower_index(xs, nxs, o.r.x1);
     q.cy0 = lower_index(ys, nys, o.r.y0); q.cy1 = lower_index(ys, nys, o.r.y1);
-    out[i] = q;
+    if constexpr (!PAIRED) { out[i] = q; return; }
+    // the task's first and one past its last op: most tasks have a few, others are bisected for
+    auto edge = [&](int dir) {
+        int k = i;
+        for (int step = 1; step <= 8; ++step)
+        {
+            const int m = i + dir * step;
+            if (m < 0 || m >= n || ops[m].task != o.task) return k;
+            k = m;
+        }
+        int in = k, outside = dir < 0 ? -1 : n;
+        while (in - outside > 1 || outside - in > 1)
+        {
+            const int m = in + (outside - in) / 2;
+            if (ops[m].task == o.task) in = m; else outside = m;
+        }
+        return in;
+    };
+    const int b = edge(-1), f = edge(1) + 1;
+    out[b + i] = q;
+    q.link = 0;
+    out[f + i] = q;
 }
 
 struct Domain {
@@ -782,36 +878,26 @@ struct Domain {
     int cur = 0;
     size_t ncells = 0;
     std::vector<HOp> ops;               // ops of the batch being resolved (sequential build)
-    size_t nops = 0;                    // ops of the batch (in `ops`, or in the staging buffer)
-    size_t stage_off = 0;               // where they start in the staging buffer
+    size_t nops = 0;                    // ops of the batch
+    size_t nhops = 0;                   // as they are uploaded: nops, or half of them (staged: PAIRED)
 };
 
-// Page-locked host memory the parallel build writes the batch's ops into, reused batch after
-// batch, so their upload runs at DMA speed.
+// Page-locked host memory the staged build writes the batch's ops into, so that their upload runs at
+// DMA speed. Held during a batch.
 struct HostStage {
     HOp * p = nullptr;
-    size_t cap = 0;
+    size_t bytes = 0;
     HostStage() = default;
     HostStage(const HostStage &) = delete;
     HostStage & operator=(const HostStage &) = delete;
-    ~HostStage() { if (p) cudaFreeHost(p); }
-    int reserve(size_t n)
-    {
-        if (n <= cap) return XKB_OK;
-        size_t c = cap ? cap : size_t(1) << 20;
-        while (c < n) c *= 2;
-        HOp * q = nullptr;
-        cudaError_t e = cudaHostAlloc((void **) &q, c * sizeof(HOp), cudaHostAllocDefault);
-        if (e != cudaSuccess) return xkb_set_cuda_error(e);
-        if (p) cudaFreeHost(p);
-        p = q; cap = c;
-        return XKB_OK;
-    }
+    ~HostStage() { give(); }
+    int take(size_t n) { give(); return PinnedBlocks::take(n * sizeof(HOp), (void **) &p, &bytes); }
+    void give() { PinnedBlocks::give(p, bytes); p = nullptr; bytes = 0; }
 };
 
 // Page-locked host memory for what the device reports back and for the small arrays it is given, so
 // that neither waits for a staging copy: results (first, fixed places), then `used` bytes handed out
-// to arrays whose copies are in flight; release() once the stream has been waited for.
+// to arrays whose copies are in flight; release() once the stream has been waited for. Held during a batch.
 struct HostScratch {
     static constexpr size_t RESULTS = 256, KEYS = 2048;           // bytes; keys of each axis read back with the counts
     uint8_t * p = nullptr;
@@ -819,11 +905,12 @@ struct HostScratch {
     HostScratch() = default;
     HostScratch(const HostScratch &) = delete;
     HostScratch & operator=(const HostScratch &) = delete;
-    ~HostScratch() { if (p) cudaFreeHost(p); }
+    ~HostScratch() { give(); }
+    void give() { PinnedBlocks::give(p, cap); p = nullptr; cap = 0; }
     uint64_t * results() { return (uint64_t *) p; }
     uint64_t * keys(int axis) { return (uint64_t *) (p + RESULTS) + axis * KEYS; }
     void release() { used = RESULTS + 2 * KEYS * sizeof(uint64_t); }
-    int init() { return p ? XKB_OK : grow(size_t(1) << 18); }
+    int init() { return p ? XKB_OK : grow(size_t(1) << 17); }
     // n bytes for a copy to the device queued on `st`; a full scratch waits for the copies so far
     int take(size_t n, cudaStream_t st, void ** out)
     {
@@ -841,11 +928,11 @@ struct HostScratch {
 private:
     int grow(size_t n)
     {
-        uint8_t * q = nullptr;
-        cudaError_t e = cudaHostAlloc((void **) &q, n, cudaHostAllocDefault);
-        if (e != cudaSuccess) return xkb_set_cuda_error(e);
-        if (p) cudaFreeHost(p);
-        p = q; cap = n; release();
+        void * q = nullptr;
+        size_t c = 0;
+        if (int rc = PinnedBlocks::take(n, &q, &c)) return rc;
+        give();
+        p = (uint8_t *) q; cap = c; release();
         return XKB_OK;
     }
 };
@@ -1009,23 +1096,25 @@ static inline int mat_nrects(const xkb_access_rec_t & r)
 
 // Matrix-only batches whose every (ld, sizeof) already has a domain: each record's ops go to its
 // own domain only (LINK ops of a task's records, then their PUT ops), so chunks of whole tasks
-// are built by the host team: a counting pass, then every chunk writes its ops straight into the
-// page-locked staging buffer, domain after domain and chunks in order within a domain -- the
-// order of the sequential build. Counters and cursors live on each member's own stack while it
-// runs (members sharing cache lines would serialise on them). Returns 1 (built), 0 (the batch
-// needs the sequential path: a segment or handle, a matrix key seen for the first time -- a new
-// domain replays earlier segments at that point of the stream -- or a small batch), or an error.
+// are built on their own -- by the host team when the batch is large: a counting pass, then every
+// chunk writes its ops straight into the page-locked staging buffer, domain after domain and chunks
+// in order within a domain, one per rect: the device makes the LINK and the PUT op of it
+// (map_ops_kernel). Counters and cursors live on each member's own stack while it runs (members
+// sharing cache lines would serialise on them). Returns 1 (built), 0 (the batch needs the
+// sequential path: a segment or handle, or a matrix key seen for the first time after a segment -- a
+// new domain replays earlier segments at that point of the stream), or an error.
+constexpr size_t TEAM_RECORDS = 16384;      // records from which the host team pays (waking it: about 20 us a pass)
+
 static int build_ops_staged(xkb_resolver * R, const xkb_access_rec_t * recs, size_t n)
 {
-    if (n < 65536 || !R->pool) return 0;
-    const unsigned nc = R->pool->size();
-    if (nc < 2) return 0;
+    const unsigned nc = n >= TEAM_RECORDS && R->pool ? R->pool->size() : 1;
+    auto team = [&](const std::function<void(unsigned)> & fn) { if (nc > 1) R->pool->run(fn); else fn(0); };
     if (R->segments.empty())
     {
         // no segment seen yet, so a new matrix domain replays nothing: create the batch's new
         // ones up front, in the order the sequential build would meet them
         std::vector<char> other(nc, 0), fresh(nc, 0);
-        R->pool->run([&](unsigned c) {
+        team([&](unsigned c) {
             uint64_t lk = ~0ull, ls = ~0ull;
             for (size_t i = n * c / nc; i < n * (c + 1) / nc; ++i)
             {
@@ -1074,7 +1163,7 @@ static int build_ops_staged(xkb_resolver * R, const xkb_access_rec_t * recs, siz
     }
     std::vector<size_t> cnt(nc * nd, 0);
     std::vector<char> ok(nc, 1);
-    R->pool->run([&](unsigned c) {
+    team([&](unsigned c) {
         uint64_t lk = ~0ull, ls = ~0ull;
         size_t li = 0;
         std::vector<size_t> my(nd, 0);
@@ -1082,7 +1171,7 @@ static int build_ops_staged(xkb_resolver * R, const xkb_access_rec_t * recs, siz
         {
             const xkb_access_rec_t & r = recs[i];
             if (r.type != XKB_ACCESS_TYPE_BLAS_MATRIX || !dom_of(r, lk, ls, li)) { ok[c] = 0; return; }
-            my[li] += 2 * (size_t) mat_nrects(r);
+            my[li] += (size_t) mat_nrects(r);
         }
         std::copy(my.begin(), my.end(), cnt.begin() + c * nd);
     });
@@ -1091,30 +1180,25 @@ static int build_ops_staged(xkb_resolver * R, const xkb_access_rec_t * recs, siz
     size_t total = 0;
     for (size_t k = 0; k < nd; ++k)
     {
-        R->blas[k]->stage_off = total;
+        const size_t first = total;
         for (unsigned c = 0; c < nc; ++c) { pos[c * nd + k] = total; total += cnt[c * nd + k]; }
-        R->blas[k]->nops = total - R->blas[k]->stage_off;
+        R->blas[k]->nhops = total - first;
+        R->blas[k]->nops = 2 * R->blas[k]->nhops;
     }
-    if (int rc = R->stage.reserve(total ? total : 1)) return rc;
+    if (int rc = R->stage.take(total ? total : 1)) return rc;
     HOp * out = R->stage.p;
-    R->pool->run([&](unsigned c) {
+    team([&](unsigned c) {
         uint64_t lk = ~0ull, ls = ~0ull;
         size_t li = 0;
         std::vector<size_t> p(pos.begin() + c * nd, pos.begin() + (c + 1) * nd);
-        for (size_t i = cut[c]; i < cut[c + 1];)
+        for (size_t i = cut[c]; i < cut[c + 1]; ++i)
         {
-            size_t j = i;
-            while (j < cut[c + 1] && recs[j].task == recs[i].task) ++j;
-            for (int pass = 0; pass < 2; ++pass)                 // LINK ops, then PUT ops
-                for (size_t a = i; a < j; ++a)
-                {
-                    dom_of(recs[a], lk, ls, li);
-                    HRect rr[2];
-                    const int nr = mat_rects(recs[a], rr);
-                    for (int q = 0; q < nr; ++q) out[p[li]++] = HOp{recs[a].task, (uint8_t) (pass == 0), recs[a].mode, rr[q]};
-                }
-            i = j;
+            dom_of(recs[i], lk, ls, li);
+            HRect rr[2];
+            const int nr = mat_rects(recs[i], rr);
+            for (int q = 0; q < nr; ++q) stream_op(out + p[li]++, HOp{recs[i].task, 1, recs[i].mode, rr[q]});
         }
+        stream_fence();
     });
     R->staged = true;
     return 1;
@@ -1396,8 +1480,8 @@ static int launch_domain(xkb_resolver * R, Domain & d, size_t op_offset, size_t 
 
 // Compress the domain's coordinates with the batch's boundaries (found on the device, merged with
 // the domain's earlier ones on the host), refine the cell state, and write the batch's ops in cell
-// coordinates to dops. hops / dops: this domain's nops ops on the device.
-static int compress_domain(xkb_resolver * R, Domain & d, const HOp * hops, DOp * dops, size_t nops)
+// coordinates to dops. hops: this domain's nops uploaded ops on the device, each two of dops if paired.
+static int compress_domain(xkb_resolver * R, Domain & d, const HOp * hops, DOp * dops, size_t nops, bool paired)
 {
     cudaStream_t st = R->stream;
     size_t cap = 1024;
@@ -1445,8 +1529,8 @@ static int compress_domain(xkb_resolver * R, Domain & d, const HOp * hops, DOp *
     if ((rc = R->host.take(nbounds * sizeof(uint64_t), st, &hb))) return rc;
     std::copy(d.ys.begin(), d.ys.end(), std::copy(d.xs.begin(), d.xs.end(), (uint64_t *) hb));
     XKB_CUDA_TRY(cudaMemcpyAsync(R->bounds.p, hb, nbounds * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    map_ops_kernel<<<g, 256, 0, st>>>(hops, (int) nops, R->bounds.p, (int) d.xs.size(), R->bounds.p + d.xs.size(),
-                                      (int) d.ys.size(), dops);
+    (paired ? map_ops_kernel<true> : map_ops_kernel<false>)<<<g, 256, 0, st>>>(hops, (int) nops, R->bounds.p, (int) d.xs.size(),
+                                                                               R->bounds.p + d.xs.size(), (int) d.ys.size(), dops);
     XKB_CUDA_TRY(cudaGetLastError());
     pt.mark("map");
     return XKB_OK;
@@ -1466,8 +1550,9 @@ static int resolve_batch(xkb_resolver * R, const xkb_access_rec_t * recs, size_t
     if (!R->staged)
     {
         build_ops(R, recs, n);
-        R->interval.nops = R->interval.ops.size(); R->handles.nops = R->handles.ops.size();
-        for (auto & d : R->blas) d->nops = d->ops.size();
+        R->interval.nops = R->interval.nhops = R->interval.ops.size();
+        R->handles.nops = R->handles.nhops = R->handles.ops.size();
+        for (auto & d : R->blas) d->nops = d->nhops = d->ops.size();
     }
     const auto t1 = clk::now();
     std::vector<Domain *> doms;
@@ -1475,20 +1560,20 @@ static int resolve_batch(xkb_resolver * R, const xkb_access_rec_t * recs, size_t
     if (R->handles.nops) doms.push_back(&R->handles);
     for (auto & d : R->blas) if (d->nops) doms.push_back(d.get());
 
-    std::vector<size_t> offs;
-    size_t total = 0;
-    for (Domain * d : doms) { offs.push_back(total); total += d->nops; }
-    if ((rc = R->hops.reserve(total ? total : 1)) || (rc = R->dops.reserve(total ? total : 1))) return rc;
+    std::vector<size_t> offs, hoffs;            // each domain's first op, and first uploaded op
+    size_t total = 0, htotal = 0;
+    for (Domain * d : doms) { offs.push_back(total); hoffs.push_back(htotal); total += d->nops; htotal += d->nhops; }
+    if ((rc = R->hops.reserve(htotal ? htotal : 1)) || (rc = R->dops.reserve(total ? total : 1))) return rc;
     if (R->staged)          // domain-major in the staging buffer, in the order of `doms`
     {
-        if (total) XKB_CUDA_TRY(cudaMemcpyAsync(R->hops.p, R->stage.p, total * sizeof(HOp), cudaMemcpyHostToDevice, R->stream));
+        if (htotal) XKB_CUDA_TRY(cudaMemcpyAsync(R->hops.p, R->stage.p, htotal * sizeof(HOp), cudaMemcpyHostToDevice, R->stream));
     }
     else
         for (size_t k = 0; k < doms.size(); ++k)
-            XKB_CUDA_TRY(cudaMemcpyAsync(R->hops.p + offs[k], doms[k]->ops.data(), doms[k]->nops * sizeof(HOp),
+            XKB_CUDA_TRY(cudaMemcpyAsync(R->hops.p + hoffs[k], doms[k]->ops.data(), doms[k]->nhops * sizeof(HOp),
                                          cudaMemcpyHostToDevice, R->stream));
     for (size_t k = 0; k < doms.size(); ++k)
-        if ((rc = compress_domain(R, *doms[k], R->hops.p + offs[k], R->dops.p + offs[k], doms[k]->nops))) return rc;
+        if ((rc = compress_domain(R, *doms[k], R->hops.p + hoffs[k], R->dops.p + offs[k], doms[k]->nhops, R->staged))) return rc;
     R->last_ops_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
     R->last_compress_ms = std::chrono::duration<double, std::milli>(clk::now() - t1).count();
 
@@ -1570,7 +1655,7 @@ static int resolve_batch(xkb_resolver * R, const xkb_access_rec_t * recs, size_t
         }
         R->nuniq += nu - nu0;
         R->useg_n.back() = nu;
-        for (Domain * d : doms) { d->cur ^= 1; d->ops.clear(); d->nops = 0; }
+        for (Domain * d : doms) { d->cur ^= 1; d->ops.clear(); d->nops = d->nhops = 0; }
         if (trace)
             fprintf(stderr, "resolver batch: %zu ops (built in %.2f ms, compressed in %.2f ms), attempt %d, regions and unique %.2f ms, "
                     "%llu emitted, %llu unique, %.1f MB allocated\n",
@@ -1666,8 +1751,9 @@ int xkb_internal_resolver_prepare(xkb_resolver_t * R, size_t nops)
     int rc;
     if ((rc = R->hops.reserve(nops)) || (rc = R->dops.reserve(nops)) || (rc = R->hset.reserve(2 * cap)) ||
         (rc = R->ukeys.reserve(4 * nops)) || (rc = R->ucount.reserve(3)) || (rc = R->emit.reserve(emit)) ||
-        (rc = R->counters.reserve(2)) || (rc = R->table.reserve(tcap)) || (rc = R->stage.reserve(nops)) || (rc = spill_reserve(R, 1)))
+        (rc = R->counters.reserve(CNT_COUNT)) || (rc = R->table.reserve(tcap)) || (rc = R->stage.take(nops)) || (rc = spill_reserve(R, 1)))
         return rc;
+    R->stage.give();                            // (kept for the batches to come)
     if (R->useg.empty())
     {
         std::unique_ptr<DevBuf<unsigned long long>> seg(new (std::nothrow) DevBuf<unsigned long long>());
@@ -1712,7 +1798,7 @@ extern "C" int xkb_resolver_add(xkb_resolver_t * R, const xkb_access_rec_t * rec
 {
     if (!R || (n && !recs)) return xkb_set_error(XKB_EINVAL, "resolver_add: bad arguments");
     if (n == 0) return XKB_OK;
-    if (!R->pool)
+    if (!R->pool && n >= TEAM_RECORDS)
     {
         R->pool.reset(new (std::nothrow) WorkPool(xkb_internal_helpers()));
     }
@@ -1724,6 +1810,8 @@ extern "C" int xkb_resolver_add(xkb_resolver_t * R, const xkb_access_rec_t * rec
     if (rc == XKB_OK) { R->ntasks = recs[n - 1].task + 1; R->graph_valid = false; }
     cudaEventRecord(R->ev[1], R->stream);
     cudaEventSynchronize(R->ev[1]);
+    R->host.give();                             // no copy of the batch is in flight any more
+    R->stage.give();
     float ms = 0; cudaEventElapsedTime(&ms, R->ev[0], R->ev[1]);
     R->last_device_ms = ms;
     return rc;
