@@ -421,9 +421,9 @@ typedef struct xkb_request_t {
  * free and their memory fits in the budget (best-fit allocation with split/merge, as the
  * reference's device allocator, src/driver/device.cc:49-280). ONE persistent kernel, launched
  * for the whole trace, runs the tile tasks of every admitted request: the host copies a request's
- * input grid in and writes its slot record; the kernel's idle teams set the request up (wait
- * counters, queue, second grid) and then take ready tasks from whichever request has some; the
- * host copies each result out as its last task ends. The graph of every request shape is
+ * input grid in and writes its slot record; the kernel's idle CTAs set the request up (wait
+ * counters, second grid) and then work on the requests, as many on each as its steps keep busy or
+ * its share of the device; the host copies each result out as its last task ends. The graph of every request shape is
  * resolved (two-step windows, periodic form) before the loop starts. XKB_SERVE_MODE=launch in
  * the environment runs each request as its own persistent launch on its slot's stream instead. */
 XKB_API int xkb_server_create(xkb_server_t ** server, const xkb_server_cfg_t * cfg);

@@ -107,3 +107,24 @@ def test_tile_sides_of_a_stream_equal_the_oracle(torch_cuda):
     for (t, n, steps, f32, seed), buf in zip(specs, bufs):
         dt = np.float32 if f32 else np.float64
         np.testing.assert_array_equal(buf, O.heat_run(O.serve_init(n, n, seed, dt), n, n, steps, 0.2, dtype=dt))
+
+
+@pytest.mark.parametrize("slots,ctas", [(1, 0), (5, 3), (16, 0), (40, 24)])
+def test_shares_and_units_match_oracle(torch_cuda, slots, ctas):
+    """Requests of one tile to hundreds, some admitted into a quiet server (their tiles split over
+    many warps) and some into a crowded one, with more requests than CTAs and more CTAs than
+    requests need: every result is the oracle's."""
+    rng = np.random.default_rng(slots)
+    specs, tiles = [], []
+    for k in range(30):
+        n = int(rng.choice([40, 64, 129, 257, 384, 700]))
+        specs.append((0.0 if k % 3 else 0.001 * k, n, int(rng.integers(1, 30)), int(rng.integers(0, 2)), 500 + k))
+        tiles.append(int(rng.choice([32, 64, 128])) if n != 129 and n != 257 else 50)
+    specs.sort(key=lambda q: q[0])
+    srv = xk.Server(budget_bytes=64 << 20, slots=slots, ctas_per_graph=ctas, max_seconds=60.0)
+    reqs, bufs = make_requests(specs, tiles)
+    srv.run(reqs)
+    srv.close()
+    for (t, n, steps, f32, seed), buf in zip(specs, bufs):
+        dt = np.float32 if f32 else np.float64
+        np.testing.assert_array_equal(buf, O.heat_run(O.serve_init(n, n, seed, dt), n, n, steps, 0.2, dtype=dt))

@@ -115,8 +115,6 @@ struct XkbSrvSlot {
     const xkb_task_desc_t * tasks;       // the periodic window's `period` descriptors
     const uint32_t * succ_ptr, * succ, * xsucc_ptr, * xsucc, * npred_first, * npred_next;
     int * wc;                            // ntasks wait counters
-    int * units_done;                    // ntasks counts of the units that ended
-    int * queue;                         // ntasks ready-queue slots
     const uint8_t * copy_src;            // the grid the host copied in ...
     uint8_t * copy_dst;                  //   ... duplicated here by the set-up chunks (second grid)
     uint64_t copy_bytes;
@@ -124,15 +122,24 @@ struct XkbSrvSlot {
     uint32_t nchunks;                    // set-up chunks (wait counters, queue slots, grid copy)
     uint32_t chunk_tasks;                // tasks whose counters one chunk sets up
     uint32_t gen;                        // admission number, reported back when the request ends
-    uint32_t seed_later;                 // 1: some task of a later window has no predecessor
     uint32_t units_log2;                 // a task is 2^units_log2 units, each run by one warp
+    uint32_t rows, cols;                 // tiles of a step (rows x cols tasks, row by row)
+    uint32_t ctas;                       // CTAs its steps keep busy: units per step / warps per CTA, at least 1
     int32_t pfd;
 };
-// The slot's counters (device memory): state 0 idle, 1 admitted (set-up pending), 2 running,
-// 3 done; set-up chunks claimed / finished; tickets taken (head) and tasks published (tail); tasks
-// executed. claimers: warps between their check that the slot runs (state 2) and their claim on `head`;
-// the warp that ends the request waits for none to be left before the host may reuse the slot.
-struct XkbSrvCtl { unsigned state, init_next, init_done, head, tail, executed, claimers, pad; };
+// The slot's counters (device memory), one cache line for each kind of traffic. state: 0 idle, 1 admitted
+// (set-up pending), 2 running, 3 done; set-up chunks claimed / finished; tickets taken; units executed;
+// CTAs that work on the request, or are about to find that they cannot. The host writes what stands
+// before `attached` when it admits a request; `attached` counts up and down over the whole run, as a CTA
+// may look at a slot while the host refills it.
+struct XkbSrvCtl {
+    alignas(128) unsigned state;
+    alignas(128) unsigned init_next;
+    unsigned init_done;
+    alignas(128) unsigned head;
+    alignas(128) unsigned executed;
+    alignas(128) unsigned attached;
+};
 struct XkbSrvArgs {
     XkbSrvSlot * slots;
     XkbSrvCtl * ctl;
@@ -141,16 +148,12 @@ struct XkbSrvArgs {
     unsigned * status;                   // [0] first error (XKB_ETIMEDOUT), [1] tasks executed,
                                          // [2] set by the host: 1 once no request will come,
                                          //     2 to stop at once (the host gave up)
-    uint64_t run_ns;                     // how long a warp may run before it gives up
-    uint64_t timeout_ns;                 // longest wait for one published queue slot
+    uint64_t run_ns;                     // how long a CTA may run before it gives up
+    uint64_t timeout_ns;                 // longest wait for one task's predecessors
 };
-// At most this many tasks and bytes of the grid copy per set-up chunk of a served request; an idle
-// warp looks for work again after at most XKB_SRV_NAP_MAX ns.
-constexpr uint32_t XKB_SRV_CHUNK = 1024;
-constexpr uint64_t XKB_SRV_COPY_CHUNK = uint64_t(64) << 10;
-#ifndef XKB_SRV_NAP_MAX
-#define XKB_SRV_NAP_MAX 2048
-#endif
+// At most this many tasks and bytes of the grid copy per set-up chunk (one CTA) of a served request.
+constexpr uint32_t XKB_SRV_CHUNK = 8192;
+constexpr uint64_t XKB_SRV_COPY_CHUNK = uint64_t(128) << 10;
 // Launch the serving kernel (grid CTAs of 256 threads).
 int xkb_internal_server_launch(const XkbSrvArgs & a, int grid, cudaStream_t stream);
 // log2 of the units heat tile tasks are split into when `width` of them run side by side on `warps` warps.

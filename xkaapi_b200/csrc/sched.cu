@@ -354,6 +354,8 @@ __global__ void sched_plan_kernel(SchedArgs a, unsigned warps)
 struct BlockOrder {
     uint32_t W, rows, cols, whole;         // tiles: rows x cols per block; tasks in whole blocks
 
+    // blocks of rows x cols tiles spawned row of tiles by row of tiles, ntasks in whole blocks
+    __device__ __forceinline__ BlockOrder(uint32_t rows_, uint32_t cols_, uint32_t ntasks) : W(rows_ * cols_), rows(rows_), cols(cols_), whole(ntasks) {}
     __device__ __forceinline__ BlockOrder(const SchedArgs & a)
     {
         W = a.ctr[CTR_SEEDS];
@@ -1299,14 +1301,19 @@ extern "C" int xkb_sched_run_noalloc(const xkb_task_desc_t * tasks, const xkb_ta
 // ------------------------------------------------------------------------------------------
 // Device-resident serving loop: ONE persistent kernel runs the tile tasks of every admitted
 // request. The host admits a request by writing its slot record (descriptors, periodic graph,
-// counter and queue arrays, the grid to duplicate) and then the slot's state word; any idle warp
-// of the kernel then takes the slot's set-up chunks (wait counters, queue slots, second grid),
-// the warp that finishes the last chunk publishes the request's first ready tasks, and from then
-// on warps take units of ready tasks from whichever slot has some -- a small request does not hold
-// SMs it cannot use, and requests admitted while others run share the device at once. The warp
-// that ends a request's last task marks the slot done and reports the admission number to mapped
-// host memory; the host copies the result out. Warps stop when the host has said no request will
-// come and every slot is idle or done, on an error, or at the time limit; every wait is bounded.
+// counter array, the grid to duplicate) and then the slot's state word. Idle CTAs take the slot's
+// set-up chunks (wait counters, second grid), and the one that finishes the last chunk starts the
+// request. From then on idle CTAs ATTACH to it, as many as its steps can keep busy or its share of the
+// device when requests compete, and run it like an in-order batch run (the heat graph is spawned level
+// by level): tickets from the slot's counter, a wait for the task's predecessors, the unit, the
+// successors' counters -- a CTA at a time where a task has 8 units or more, else warp by warp. A CTA
+// leaves when the tickets run out, or between tickets when its request holds more than its share (a
+// look every SRV_LOOK_NS); the one that counts the last unit marks the slot done and reports the
+// admission number to mapped host memory, and the host copies the result out. CTAs stop when the host
+// has said no request will come and every slot is idle or done, on an error, or at the time limit;
+// every wait is bounded. (Warps that each looked for their next unit through every slot's queue kept
+// the counters' lines busy: 24 requests of 256^2 to 2048^2, 8 in flight, 10.1 ms
+// against 6.3; one 1024^2 request of 40 steps 1.27 ms against 0.83.)
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned * p)
 {
@@ -1320,112 +1327,126 @@ __device__ __forceinline__ void st_release_u32(unsigned * p, unsigned v)
     asm volatile("st.release.gpu.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
 }
 
-__device__ __forceinline__ void srv_publish(const XkbSrvSlot & S, XkbSrvCtl * c, uint32_t t)
+constexpr uint64_t SRV_LOOK_NS = 50000;      // between two looks of an attached CTA at its share
+constexpr int SRV_PF32 = 4;                  // columns an FP32 strip loads ahead beside the FP64 body (5 spills: 4.71 against 4.75 TB/s)
+constexpr unsigned SRV_NAP_MAX = 1024;       // longest nap of an idle CTA, ns
+constexpr unsigned SRV_LEAVE = 0xffffffffu;  // a ticket past every task
+
+// One warp, the slots spread over its lanes: the most CTAs any one request may hold now. Requests that
+// keep fewer busy take what they need, the others share the rest of the grid evenly (a few rounds of
+// water-filling; rounded up, so that no CTA is left without a request).
+__device__ __forceinline__ unsigned srv_share(const XkbSrvArgs & a, int lane)
 {
-    const unsigned pos = atomicAdd(&c->tail, 1u);
-    xkb_st_release(S.queue + pos, (int) t);
+    unsigned need[2] = {0, 0};                 // at most 64 slots
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+    {
+        const int q = lane + 32 * h;
+        if (q >= a.nslots) continue;
+        const unsigned w = *(volatile uint32_t *) &a.slots[q].ctas, st = ld_acquire_u32(&a.ctl[q].state);
+        if (st == 1 || st == 2) need[h] = w;
+    }
+    unsigned share = 0;
+    for (int round = 0; round < 4; ++round)
+    {
+        unsigned few = 0, many = 0;            // CTAs of the requests content with the share, number of the others
+#pragma unroll
+        for (int h = 0; h < 2; ++h) { if (need[h] > share) ++many; else few += need[h]; }
+        few = __reduce_add_sync(0xffffffffu, few);
+        many = __reduce_add_sync(0xffffffffu, many);
+        if (many == 0) return gridDim.x;
+        share = max(share, (gridDim.x - min(few, gridDim.x) + many - 1) / many);
+    }
+    return share;
+}
+
+// One thread: whether the kernel has to end (an error, the host gave up, the time limit), recorded in the
+// status word, which every wait looks at.
+__device__ __forceinline__ bool srv_ended(const XkbSrvArgs & a, uint64_t t_start)
+{
+    if (*(volatile unsigned *) a.status != 0) return true;
+    if (*(volatile unsigned *) (a.status + 2) < 2 && xkb_globaltimer() - t_start <= a.run_ns) return false;
+    atomicCAS(a.status, 0u, (unsigned) -XKB_ETIMEDOUT);
+    return true;
 }
 
 __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) server_kernel(XkbSrvArgs a)
 {
-    const int lane = threadIdx.x & 31;
-    const int gwarp = blockIdx.x * (SCHED_THREADS / 32) + (threadIdx.x >> 5);
-    unsigned executed = 0;
-    uint32_t nap = 32;
-    const uint64_t t_start = xkb_globaltimer();
+    constexpr int NWARPS = SCHED_THREADS / 32;
+    enum { STOP, SETUP, ATTACH, NAP };
+    __shared__ int job, job_slot, job_idx, ready;
+    __shared__ volatile int leave;
+    __shared__ unsigned next_ticket, units_run;
+    __shared__ XkbSrvSlot S;                   // the record of the request worked on
+    __shared__ XkbSrvCtl * c;                  // ... and its counters
+    // state that lasts over a tile stands here too: every register it took would be spilled in the body
+    __shared__ uint64_t t_start, looked;       // start of the kernel, last look at the share
+    __shared__ unsigned counted;               // this CTA counts in `attached`
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint32_t nap = 64;
+    if (tid == 0) t_start = xkb_globaltimer();
     for (;;)
     {
-        // kind: 0 stop, 1 unit of a task, 2 set-up chunk, -1 nothing yet
-        int kind = -1, sl = -1, idx = -1, unit = 0;
-        if (lane == 0)
+        if (warp == 0)
         {
-            if (*(volatile unsigned *) (a.status + 2) >= 2) kind = 0;     // the host gave up: stop now
-            for (int k = 0; k < a.nslots && kind < 0; ++k)
+            // every lane looks at its slots; the first in turn (a different one for each CTA) that has
+            // something to do is tried
+            const unsigned share = srv_share(a, lane);
+            unsigned best = 0xffffffffu;
+            bool busy = false;
+            for (int q = lane; q < a.nslots; q += 32)
             {
-                const int q = (gwarp + k) % a.nslots;
-                XkbSrvCtl * c = a.ctl + q;
-                const unsigned st = ld_acquire_u32(&c->state);
-                if (st == 1)
+                const unsigned st = ld_acquire_u32(&a.ctl[q].state);
+                busy = busy || st == 1 || st == 2;
+                const bool chunk = st == 1 && *(volatile unsigned *) &a.ctl[q].init_next < *(volatile uint32_t *) &a.slots[q].nchunks;
+                const bool run = st == 2 && *(volatile unsigned *) &a.ctl[q].attached < min(share, *(volatile uint32_t *) &a.slots[q].ctas);
+                if (chunk || run) best = min(best, (unsigned) ((q + a.nslots - (int) (blockIdx.x % a.nslots)) % a.nslots) << 8 | (unsigned) q);
+            }
+            best = __reduce_min_sync(0xffffffffu, best);
+            busy = __any_sync(0xffffffffu, busy);
+            if (lane == 0)
+            {
+                int kind = NAP, sl = -1, idx = -1;
+                if (srv_ended(a, t_start)) kind = STOP;
+                else if (best != 0xffffffffu)
                 {
-                    if (*(volatile unsigned *) &c->init_next < a.slots[q].nchunks)
+                    const int q = (int) (best & 0xff);
+                    XkbSrvCtl * c = a.ctl + q;
+                    const unsigned st = ld_acquire_u32(&c->state);
+                    if (st == 1)
                     {
                         const unsigned ch = atomicAdd(&c->init_next, 1u);
-                        if (ch < a.slots[q].nchunks) { kind = 2; sl = q; idx = (int) ch; }
+                        if (ch < a.slots[q].nchunks) { kind = SETUP; sl = q; idx = (int) ch; }
+                    }
+                    else if (st == 2)
+                    {
+                        // attached before the state is looked at again: the slot is not reused while it counts
+                        const unsigned n = atomicAdd(&c->attached, 1u);
+                        fence_acq_rel_gpu();
+                        if (ld_acquire_u32(&c->state) == 2 && n < a.slots[q].ctas) { kind = ATTACH; sl = q; }
+                        else atomicSub(&c->attached, 1u);
                     }
                 }
-                else if (st == 2)
-                {
-                    if (*(volatile unsigned *) &c->head >= *(volatile unsigned *) &c->tail << a.slots[q].units_log2) continue;
-                    // claim the next ticket with one atomicAdd (a compare-and-swap loop on `head`
-                    // serialises the warps on it); the position may be published a little later,
-                    // which the wait below covers. The claim counts in `claimers` while the state
-                    // is re-checked, so the warp ending the request can tell when no claim on this
-                    // request's counters is left.
-                    atomicAdd(&c->claimers, 1u);
-                    __threadfence();
-                    unsigned h = 0;
-                    if (ld_acquire_u32(&c->state) == 2)
-                    {
-                        const uint32_t lg = a.slots[q].units_log2;       // this request's: the slot is not reused under a claim
-                        const unsigned ticket = atomicAdd(&c->head, 1u);
-                        h = ticket >> lg;
-                        unit = (int) (ticket & ((1u << lg) - 1));
-                        if (h < a.slots[q].ntasks) { kind = 1; sl = q; }
-                    }
-                    atomicSub(&c->claimers, 1u);
-                    if (kind == 1)
-                    {
-                        // the id at that position was published (tail counts it) or is about to be
-                        const int * pq = a.slots[q].queue + h;
-                        const uint64_t t0 = xkb_globaltimer();
-                        uint32_t spins = 0;
-                        while ((idx = xkb_ld_acquire(pq)) < 0)
-                        {
-                            if ((++spins & 63) == 0 && xkb_globaltimer() - t0 > a.timeout_ns)
-                            {
-                                atomicCAS(a.status, 0u, (unsigned) -XKB_ETIMEDOUT);
-                                break;
-                            }
-                        }
-                        if (idx < 0) kind = 0;
-                    }
-                }
+                else if (!busy && *(volatile unsigned *) (a.status + 2) != 0) kind = STOP;
+                if (kind == NAP) { __nanosleep(nap); if (nap < SRV_NAP_MAX) nap *= 2; } else nap = 64;
+                job = kind; job_slot = sl; job_idx = idx; leave = 0; units_run = 0;
+                c = a.ctl + sl; counted = 1; looked = xkb_globaltimer();
             }
-            if (kind < 0)
-            {
-                if (*(volatile unsigned *) a.status != 0) kind = 0;
-                else if (xkb_globaltimer() - t_start > a.run_ns) { atomicCAS(a.status, 0u, (unsigned) -XKB_ETIMEDOUT); kind = 0; }
-                else if (*(volatile unsigned *) (a.status + 2))
-                {
-                    bool busy = false;
-                    for (int q = 0; q < a.nslots && !busy; ++q)
-                    {
-                        const unsigned st = ld_acquire_u32(&a.ctl[q].state);
-                        busy = st == 1 || st == 2;
-                    }
-                    if (!busy) kind = 0;
-                }
-                if (kind < 0) { __nanosleep(nap); if (nap < XKB_SRV_NAP_MAX) nap *= 2; }
-            }
-            else nap = 32;
         }
-        kind = __shfl_sync(0xffffffffu, kind, 0);
-        if (kind < 0) continue;
-        if (kind == 0) break;
-        sl = __shfl_sync(0xffffffffu, sl, 0);
-        idx = __shfl_sync(0xffffffffu, idx, 0);
-        unit = __shfl_sync(0xffffffffu, unit, 0);
-        __syncwarp();
-        if (kind == 2)
+        __syncthreads();
+        const int kind = job;
+        if (kind == STOP) break;
+        if (kind == NAP) { __syncthreads(); continue; }
+        for (int k = tid; k < (int) (sizeof(XkbSrvSlot) / 4); k += SCHED_THREADS)
+            ((uint32_t *) &S)[k] = __ldcg((const uint32_t *) (a.slots + job_slot) + k);
+        __syncthreads();
+        if (kind == SETUP)
         {
-            // set-up chunk: wait counters, unit counts and empty queue slots of its tasks, and its
-            // share of the second grid (a copy of the first, which the host copied in)
-            const XkbSrvSlot & S = a.slots[sl];
-            const uint32_t t0 = (uint32_t) idx * S.chunk_tasks, t1 = min(S.ntasks, t0 + S.chunk_tasks);
-            for (uint32_t t = t0 + lane; t < t1; t += 32)
+            // set-up chunk: wait counters of its tasks, and its share of the second grid (a copy of the
+            // first, which the host copied in)
+            const uint32_t idx = (uint32_t) job_idx, t0 = idx * S.chunk_tasks, t1 = min(S.ntasks, t0 + S.chunk_tasks);
+            for (uint32_t t = t0 + tid; t < t1; t += SCHED_THREADS)
             {
-                S.queue[t] = -1;
-                if (S.units_done) S.units_done[t] = 0;
                 const uint32_t w = t / S.period, l = t - w * S.period;
                 S.wc[t] = (int) (w == 0 ? S.npred_first[l] : S.npred_next[l]);
             }
@@ -1434,83 +1455,121 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) server_kernel(X
             const uint4 * src = (const uint4 *) (S.copy_src + b0);
             uint4 * dst = (uint4 *) (S.copy_dst + b0);
             const uint64_t nv = (b1 - b0) / 16;
-            uint64_t k = lane;
-            for (; k + 3 * 32 < nv; k += 4 * 32)                         // four 16-byte loads in flight per lane
+            uint64_t k = tid;
+            for (; k + 3 * SCHED_THREADS < nv; k += 4 * SCHED_THREADS)   // four 16-byte loads in flight per lane
             {
-                const uint4 v0 = __ldcg(src + k), v1 = __ldcg(src + k + 32), v2 = __ldcg(src + k + 64), v3 = __ldcg(src + k + 96);
-                dst[k] = v0; dst[k + 32] = v1; dst[k + 64] = v2; dst[k + 96] = v3;
+                const uint4 v0 = __ldcg(src + k), v1 = __ldcg(src + k + SCHED_THREADS), v2 = __ldcg(src + k + 2 * SCHED_THREADS),
+                            v3 = __ldcg(src + k + 3 * SCHED_THREADS);
+                dst[k] = v0; dst[k + SCHED_THREADS] = v1; dst[k + 2 * SCHED_THREADS] = v2; dst[k + 3 * SCHED_THREADS] = v3;
             }
-            for (; k < nv; k += 32) dst[k] = __ldcg(src + k);
-            for (uint64_t r = ((b1 - b0) & ~(uint64_t) 15) + lane; r < b1 - b0; r += 32)
-                S.copy_dst[b0 + r] = S.copy_src[b0 + r];
-            __threadfence();
-            __syncwarp();
-            XkbSrvCtl * c = a.ctl + sl;
-            int last = 0;
-            if (lane == 0) last = atom_add_acq_rel((int *) &c->init_done, 1) + 1 == (int) S.nchunks;
-            if (__shfl_sync(0xffffffffu, last, 0))
+            for (; k < nv; k += SCHED_THREADS) dst[k] = __ldcg(src + k);
+            for (uint64_t r = ((b1 - b0) & ~(uint64_t) 15) + tid; r < b1 - b0; r += SCHED_THREADS)
+                S.copy_dst[b0 + r] = __ldcg(S.copy_src + b0 + r);
+            __syncthreads();
+            if (tid == 0)
             {
-                // every chunk is done: publish the tasks with no predecessor, then run
-                for (uint32_t l = lane; l < S.period && l < S.ntasks; l += 32)
-                    if (S.npred_first[l] == 0) srv_publish(S, c, l);
-                if (S.seed_later)
-                    for (uint32_t t = S.period + lane; t < S.ntasks; t += 32)
-                        if (S.npred_next[t % S.period] == 0) srv_publish(S, c, t);
-                __threadfence();
-                __syncwarp();
-                if (lane == 0) st_release_u32(&c->state, 2u);
+                fence_acq_rel_gpu();
+                if (atomicAdd(&c->init_done, 1u) + 1 == S.nchunks)
+                {
+                    fence_acq_rel_gpu();
+                    st_release_u32(&c->state, 2u);
+                }
             }
-            __syncwarp();
-            continue;
+            continue;                                          // (the smem record is rewritten after the next barrier)
         }
-        const XkbSrvSlot & S = a.slots[sl];
-        XkbSrvCtl * c = a.ctl + sl;
-        const uint32_t t = (uint32_t) idx, w = t / S.period, l = t - w * S.period, base = w * S.period;
-        const int nunits = 1 << S.units_log2;
-        const xkb_task_desc_t d = load_desc(S.tasks + l);
+        // attached: an in-order run of the request's tasks
+        const int k = (int) S.units_log2, nunits = 1 << k;
+        const bool team = k >= TEAM_LOG2;
         const SuccGraph g{S.succ_ptr, S.succ, S.xsucc_ptr, S.xsucc, S.period, S.ntasks};
-        bool more;
-        const uint32_t first = g.first(l, base, lane, more);
-        run_unit<Body::ANY, XKB_F64_PF, XKB_TILE_PF>(d, unit, nunits, S.pfd);
-        __syncwarp();
-        fence_acq_rel_gpu();
-        if (nunits > 1)
-        {
-            int last = 0;
+        // warp 0, between two tickets: whether the CTA has to leave
+        auto look = [&]() -> bool {
+            if (!__shfl_sync(0xffffffffu, (int) (xkb_globaltimer() - looked >= SRV_LOOK_NS), 0)) return false;
+            const unsigned share = srv_share(a, lane);
+            int out = 0;
             if (lane == 0)
             {
-                last = atom_add_relaxed(S.units_done + t, 1) == nunits - 1;
-                fence_acq_rel_gpu();
+                looked = xkb_globaltimer();
+                const unsigned keep = share + share / 8;
+                if (srv_ended(a, t_start)) out = 1;
+                else if (*(volatile unsigned *) &c->attached > keep)
+                {
+                    // counted out at once, so that no more leave than have to; the slot stays this
+                    // request's until the units this CTA has run are counted
+                    if (atomicSub(&c->attached, 1u) > keep) { out = 1; counted = 0; }
+                    else atomicAdd(&c->attached, 1u);
+                }
             }
-            if (!__shfl_sync(0xffffffffu, last, 0)) continue;
-            __syncwarp();
-        }
-        release_successors(g, t, first, more, S.wc, S.queue, &c->tail, lane);
-        __syncwarp();
-        if (lane == 0)
+            return __shfl_sync(0xffffffffu, out, 0) != 0;
+        };
+        unsigned ticket = 0;
+        if (team) { if (tid == 0) next_ticket = atomicAdd(&c->head, (unsigned) NWARPS); }
+        else if (lane == 0) ticket = atomicAdd(&c->head, 1u);
+        for (;;)
         {
-            ++executed;
-            if (atomicAdd(&c->executed, 1u) + 1 == S.ntasks)
+            if (team) { __syncthreads(); ticket = next_ticket == SRV_LEAVE ? SRV_LEAVE : next_ticket + warp; }
+            else ticket = __shfl_sync(0xffffffffu, ticket, 0);
+            if ((ticket >> k) >= S.ntasks) break;
+            const uint32_t t = team ? ticket >> k : BlockOrder(S.rows, S.cols, S.ntasks).task(ticket >> k);
+            const int unit = (int) (ticket & (nunits - 1));
+            const uint32_t w = t / S.period, l = t - w * S.period;
+            const xkb_task_desc_t d = load_desc(S.tasks + l);
+            uint32_t first = 0xffffffffu;
+            bool more = false;
+            if (!team || warp == 0) first = g.first(l, w * S.period, lane, more);
+            int ok = 1;
+            if (lane == 0 && (!team || warp == 0))
             {
+                const int np = (int) (w == 0 ? S.npred_first[l] : S.npred_next[l]);
+                ok = wait_at_most(S.wc + t, np - np * (team ? nunits / NWARPS : nunits), a.status, a.timeout_ns);
+                if (team) ready = ok;
+            }
+            if (team) { __syncthreads(); ok = ready; }
+            else ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) break;
+            __syncwarp();
+            run_unit<Body::ANY, XKB_F64_PF, SRV_PF32>(d, unit, nunits, team ? 0 : S.pfd);
+            if (lane == 0) atomicAdd(&units_run, 1u);
+            if (team) { __syncthreads(); if (warp != 0) continue; }        // the group's units are done
+            const bool out = warp == 0 && look();
+            if (lane == 0)
+            {
+                if (out) { leave = 1; ticket = SRV_LEAVE; }
+                else if (!team && leave) ticket = SRV_LEAVE;
+                else ticket = atomicAdd(&c->head, team ? (unsigned) NWARPS : 1u);
+                if (team) next_ticket = ticket;
+            }
+            __syncwarp();
+            fence_acq_rel_gpu();
+            count_down_successors(g, t, first, more, S.wc, lane);
+        }
+        // the last writes of this CTA come before its count, and the count of the request's last unit
+        // before the slot is reported done
+        __syncthreads();
+        if (tid == 0)
+        {
+            fence_acq_rel_gpu();
+            const unsigned all = S.ntasks << k, mine = units_run;
+            if (mine && atomicAdd(&c->executed, mine) + mine == all)
+            {
+                fence_acq_rel_gpu();
                 st_release_u32(&c->state, 3u);
-                __threadfence();
-                // warps that saw state 2 before the store above claim past the last task and leave;
-                // wait (bounded) until none is between its check and its claim
+                // CTAs that saw state 2 before the store above find no ticket, or the new state, and
+                // leave; wait (bounded) until none but this one counts
                 const uint64_t tw = xkb_globaltimer();
-                uint32_t spins = 0;
-                while (*(volatile unsigned *) &c->claimers != 0)
-                    if ((++spins & 63) == 0 && xkb_globaltimer() - tw > a.timeout_ns)
+                for (uint32_t spins = 1; ld_acquire_u32(&c->attached) != counted; ++spins)
+                    if ((spins & 63) == 0 && xkb_globaltimer() - tw > a.timeout_ns)
                     {
                         atomicCAS(a.status, 0u, (unsigned) -XKB_ETIMEDOUT);
                         break;
                     }
+                atomicAdd(a.status + 1, S.ntasks);
                 __threadfence_system();
-                a.host_done[sl] = S.gen;
+                a.host_done[job_slot] = S.gen;
             }
+            if (counted) atomicSub(&c->attached, 1u);
         }
-        __syncwarp();
+        __syncthreads();
     }
-    if (lane == 0 && executed) atomicAdd(a.status + 1, executed);
 }
 
 int xkb_internal_server_launch(const XkbSrvArgs & a, int grid, cudaStream_t stream)

@@ -117,7 +117,6 @@ struct Window {                 // the periodic form of a shape's graph (window 
     xkb_resolver_t * res = nullptr;
     xkb_periodic_graph_t g{};
     uint64_t per_step = 0;
-    bool seed_later = false;    // a task of a later window has no predecessor
     ~Window() { if (res) xkb_resolver_destroy(res); }
 };
 
@@ -224,11 +223,6 @@ static int get_window(xkb_server * S, const Shape & s, Window ** out)
     w->per_step = (uint64_t) ((s.nx + s.ts - 1) / s.ts) * ((s.ny + s.ts - 1) / s.ts);
     if ((rc = xkb_resolver_add(w->res, recs.data(), recs.size()))) return rc;
     if ((rc = xkb_resolver_periodic(w->res, 2 * w->per_step, &w->g))) return rc;
-    {
-        std::vector<uint32_t> nn(2 * w->per_step);
-        XKB_CUDA_TRY(cudaMemcpy(nn.data(), w->g.npred_next, nn.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-        w->seed_later = std::find(nn.begin(), nn.end(), 0u) != nn.end();
-    }
     *out = w.get();
     S->windows[s] = std::move(w);
     return XKB_OK;
@@ -281,7 +275,7 @@ extern "C" int xkb_server_destroy(xkb_server_t * S)
     {
         if (sl.stream) cudaStreamDestroy(sl.stream);
         if (sl.hdesc) cudaFreeHost(sl.hdesc);
-        if (sl.hslot) cudaFreeHost(sl.hslot);
+        if (sl.hctl) cudaFreeHost(sl.hctl);
         if (sl.hinput) cudaFreeHost(sl.hinput);
     }
     if (S->d_slots) cudaFree(S->d_slots);
@@ -427,16 +421,12 @@ static int server_run_launches(xkb_server * S, xkb_request_t * reqs, size_t n)
 
 // ---- the device-resident loop ---------------------------------------------------------------
 
-// Device bytes of a request: two grids, the window's descriptors, wait counters, unit counts and queue slots.
-// The unit counts are left out (tasks are not split) where the request only fits without them.
-static uint64_t device_need(const xkb_request_t & q, uint64_t per_step, uint64_t budget, bool & split)
+// Device bytes of a request: two grids, the window's descriptors, wait counters.
+static uint64_t device_need(const xkb_request_t & q, uint64_t per_step)
 {
     const uint64_t esz = q.f32 ? 4 : 8, grid = ((uint64_t) q.nx * q.ny * esz + 255) & ~(uint64_t) 255;
     const uint64_t ntasks = (uint64_t) q.steps * per_step;
-    const uint64_t words = (ntasks * 4 + 255) & ~(uint64_t) 255;
-    const uint64_t need = 2 * grid + ((2 * per_step * sizeof(xkb_task_desc_t) + 255) & ~(uint64_t) 255) + 2 * words;
-    split = need + words <= budget;
-    return split ? need + words : need;
+    return 2 * grid + ((2 * per_step * sizeof(xkb_task_desc_t) + 255) & ~(uint64_t) 255) + ((ntasks * 4 + 255) & ~(uint64_t) 255);
 }
 
 template <typename T>
@@ -451,7 +441,7 @@ static int grow_pinned(T *& p, size_t & cap, size_t bytes)
 
 // Admit request q into slot k: its input in, its descriptors and slot record, then the state
 // word -- all copies on the slot's stream, in that order; the kernel does the rest.
-static int admit(xkb_server * S, int k, xkb_request_t & q, uint8_t * mem, Window * w, bool split)
+static int admit(xkb_server * S, int k, xkb_request_t & q, uint8_t * mem, Window * w)
 {
     Slot & sl = S->slots[k];
     const uint64_t esz = q.f32 ? 4 : 8, bytes = (uint64_t) q.nx * q.ny * esz, grid = (bytes + 255) & ~(uint64_t) 255;
@@ -477,8 +467,6 @@ static int admit(xkb_server * S, int k, xkb_request_t & q, uint8_t * mem, Window
     const uint64_t period = 2 * w->per_step, ntasks = (uint64_t) q.steps * w->per_step;
     uint8_t * desc = b + grid;
     int * wc = (int *) (desc + ((period * sizeof(xkb_task_desc_t) + 255) & ~(uint64_t) 255));
-    int * queue = (int *) ((uint8_t *) wc + ((ntasks * 4 + 255) & ~(uint64_t) 255));
-    int * units_done = split ? (int *) ((uint8_t *) queue + ((ntasks * 4 + 255) & ~(uint64_t) 255)) : nullptr;
     std::vector<xkb_task_desc_t> d;
     heat_descs(sh, 2, (uint64_t) a, (uint64_t) b, q.c, d);
     if (sl.hdesc_cap < d.size() * sizeof(xkb_task_desc_t)) return xkb_set_error(XKB_EINVAL, "server_run: descriptor staging was not sized for the trace");
@@ -488,24 +476,30 @@ static int admit(xkb_server * S, int k, xkb_request_t & q, uint8_t * mem, Window
     r.tasks = (const xkb_task_desc_t *) desc;
     r.succ_ptr = w->g.succ_ptr; r.succ = w->g.succ; r.xsucc_ptr = w->g.xsucc_ptr; r.xsucc = w->g.xsucc;
     r.npred_first = w->g.npred_first; r.npred_next = w->g.npred_next;
-    r.wc = wc; r.units_done = units_done; r.queue = queue;
+    r.wc = wc;
     r.copy_src = a; r.copy_dst = b; r.copy_bytes = bytes;
     r.period = (uint32_t) period; r.ntasks = (uint32_t) ntasks;
     r.nchunks = (uint32_t) std::max<uint64_t>({1, (ntasks + XKB_SRV_CHUNK - 1) / XKB_SRV_CHUNK,
                                               (bytes + XKB_SRV_COPY_CHUNK - 1) / XKB_SRV_COPY_CHUNK});
     r.chunk_tasks = (uint32_t) ((ntasks + r.nchunks - 1) / r.nchunks);
-    // tiles of every request in flight share the warps; a request admitted into a quiet server
-    // splits its tiles over more of them (tickets are 32-bit)
-    int lg = split ? xkb_internal_split_log2(S->active_width + w->per_step, S->kernel_warps) : 0;
+    // tiles of every request in flight share the warps; a request admitted into a quiet server splits
+    // its tiles over more of them (tickets are 32-bit). A request of few tiles is split into 8 units
+    // at least, so that it can take up the CTAs that others leave (24 requests of 256^2 to 2048^2:
+    // 6.4 ms against 7.1 without); a wide one is not, nor any where the tiles of the requests in flight
+    // fill the warps (16 requests of 2048^2 to 4096^2: 34.9 ms against 37.2 with it)
+    const int own = xkb_internal_split_log2(w->per_step, S->kernel_warps);
+    int lg = std::max(xkb_internal_split_log2(S->active_width + w->per_step, S->kernel_warps),
+                      w->per_step * 8 <= S->kernel_warps && S->active_width <= S->kernel_warps ? std::min(own, 3) : 0);
     while (lg > 0 && (ntasks << lg) > 0xf0000000ull) --lg;
     r.units_log2 = (uint32_t) lg;
+    r.rows = (uint32_t) ((q.nx + q.ts - 1) / q.ts); r.cols = (uint32_t) ((q.ny + q.ts - 1) / q.ts);
+    r.ctas = (uint32_t) std::max<uint64_t>(1, std::min<uint64_t>((w->per_step << lg) / 8 + 1, S->kernel_warps / 8));
     r.gen = sl.gen = ++S->gen;
-    r.seed_later = w->seed_later ? 1u : 0u;
     r.pfd = XKB_SERVE_PFD;
     *sl.hctl = XkbSrvCtl{};                                       // state 0 until the word below
     *sl.hstate = 1u;
     XKB_CUDA_TRY(cudaMemcpyAsync(S->d_slots + k, sl.hslot, sizeof(XkbSrvSlot), cudaMemcpyHostToDevice, sl.stream));
-    XKB_CUDA_TRY(cudaMemcpyAsync(S->d_ctl + k, sl.hctl, sizeof(XkbSrvCtl), cudaMemcpyHostToDevice, sl.stream));
+    XKB_CUDA_TRY(cudaMemcpyAsync(S->d_ctl + k, sl.hctl, offsetof(XkbSrvCtl, attached), cudaMemcpyHostToDevice, sl.stream));
     XKB_CUDA_TRY(cudaMemcpyAsync(&S->d_ctl[k].state, sl.hstate, sizeof(unsigned), cudaMemcpyHostToDevice, sl.stream));
     sl.phase = 1;
     return XKB_OK;
@@ -521,12 +515,9 @@ static int server_run_device(xkb_server * S, xkb_request_t * reqs, size_t n)
         if (reqs[i].steps > 0 && (rc = get_window(S, Shape{reqs[i].nx, reqs[i].ny, reqs[i].ts, reqs[i].f32}, &win[i]))) return rc;
     XKB_CUDA_TRY(cudaStreamSynchronize(S->aux));
     std::vector<uint64_t> need(n);
-    std::vector<char> split(n, 0);
     for (size_t i = 0; i < n; ++i)
     {
-        bool sp = false;
-        need[i] = device_need(reqs[i], win[i] ? win[i]->per_step : 0, S->cfg.budget_bytes, sp);
-        split[i] = sp;
+        need[i] = device_need(reqs[i], win[i] ? win[i]->per_step : 0);
         if (need[i] > S->cfg.budget_bytes)
             return xkb_set_error(XKB_ERANGE, "server_run: request %zu needs %llu bytes, over the budget", i, (unsigned long long) need[i]);
     }
@@ -541,9 +532,9 @@ static int server_run_device(xkb_server * S, xkb_request_t * reqs, size_t n)
         XKB_CUDA_TRY(cudaStreamCreateWithFlags(&S->kstream, cudaStreamNonBlocking));
         for (Slot & sl : S->slots)
         {
-            XKB_CUDA_TRY(cudaHostAlloc((void **) &sl.hslot, sizeof(XkbSrvSlot) + sizeof(XkbSrvCtl) + 64, cudaHostAllocDefault));
-            sl.hctl = (XkbSrvCtl *) (sl.hslot + 1);
-            sl.hstate = (unsigned *) (sl.hctl + 1);
+            XKB_CUDA_TRY(cudaHostAlloc((void **) &sl.hctl, sizeof(XkbSrvCtl) + sizeof(XkbSrvSlot) + 64, cudaHostAllocDefault));
+            sl.hslot = (XkbSrvSlot *) (sl.hctl + 1);
+            sl.hstate = (unsigned *) (sl.hslot + 1);
         }
     }
     // page-locked staging sized for the whole trace up front: no host allocation or release runs
@@ -629,7 +620,7 @@ static int server_run_device(xkb_server * S, xkb_request_t * reqs, size_t n)
             mem[next] = m;
             S->slots[k].req = (long) next;
             reqs[next].start_s = now();
-            rc = admit(S, k, reqs[next], m, win[next], split[next] != 0);
+            rc = admit(S, k, reqs[next], m, win[next]);
             if (S->slots[k].phase == 1) S->active_width += win[next]->per_step;
             ++next; progressed = true;
         }
@@ -647,8 +638,8 @@ static int server_run_device(xkb_server * S, xkb_request_t * reqs, size_t n)
             std::this_thread::sleep_for(std::chrono::microseconds(20));
         }
     }
-    // (5) no more requests: the kernel's teams stop (the word goes to device memory through a
-    // copy on the control stream, so idle teams poll L2, not host memory)
+    // (5) no more requests: the kernel's CTAs stop (the word goes to device memory through a
+    // copy on the control stream, so idle CTAs poll L2, not host memory)
     *S->h_stop = rc == XKB_OK ? 1u : 2u;
     if (cudaMemcpyAsync(S->d_status + 2, S->h_stop, sizeof(unsigned), cudaMemcpyHostToDevice, S->aux) == cudaSuccess)
         cudaStreamSynchronize(S->aux);
