@@ -33,3 +33,18 @@ def test_axpby_mismatched_alignment(torch_cuda):
     xk.axpby(0.5, dx[:n], 3.0, dy[1:n + 1])
     torch.cuda.synchronize()
     np.testing.assert_array_equal(dy.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("xo,yo", [(0, 0), (1, 1), (0, 1), (1, 0)])
+@pytest.mark.parametrize("n", [1, 2, 3, 255, 2047, 2048, 2049, 6145])
+def test_axpby_cta_edges(torch_cuda, n, xo, yo):
+    """Lengths around a CTA's share, operands aligned together, both one element off, and against
+    each other: every element once, none outside."""
+    torch = torch_cuda
+    rng = np.random.default_rng(n)
+    x, y = rng.uniform(-1, 1, n + 4), rng.uniform(-1, 1, n + 4)
+    dx, dy = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    xk.axpby(0.3, dx[xo:xo + n], -1.7, dy[yo:yo + n])
+    y[yo:yo + n] = O.axpby(0.3, x[xo:xo + n], -1.7, y[yo:yo + n])
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(dy.cpu().numpy(), y)

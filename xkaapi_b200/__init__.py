@@ -148,20 +148,40 @@ def check(rc):
     return rc
 
 
+_raw_stream = None               # torch's current-stream handle of a device index, and its current device
+_raw_device = None
+_dtype_codes = None              # torch dtype -> storage code
+
+
+def _bind_torch():
+    """Look torch's pieces up once: a launch pays for them on every call otherwise (building a Stream
+    object to read its handle is 3.3 us of a 9 us tile launch)."""
+    global _raw_stream, _raw_device
+    import torch
+    torch.cuda.current_stream()                    # the first use of CUDA initialises it, or raises
+    raw, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if raw is None or dev is None:
+        raw, dev = (lambda _: torch.cuda.current_stream().cuda_stream), (lambda: 0)
+    _raw_device, _raw_stream = dev, raw
+
+
 def _stream(stream):
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        if _raw_stream is None:
+            _bind_torch()
+        return _raw_stream(_raw_device())
     return getattr(stream, "cuda_stream", stream)
 
 
 def _dtype_code(t):
-    import torch
-    if t.dtype == torch.float64:
-        return F64
-    if t.dtype == torch.float32:
-        return F32
-    raise XkbError(XKB_EINVAL, f"unsupported grid dtype {t.dtype}")
+    global _dtype_codes
+    if _dtype_codes is None:
+        import torch
+        _dtype_codes = {torch.float64: F64, torch.float32: F32}
+    code = _dtype_codes.get(t.dtype)
+    if code is None:
+        raise XkbError(XKB_EINVAL, f"unsupported grid dtype {t.dtype}")
+    return code
 
 
 def heat_tile(src, dst, nx, ny, ld, tile_x, tile_y, tsx, tsy, c, stream=None):
