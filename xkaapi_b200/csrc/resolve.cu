@@ -692,10 +692,14 @@ static cudaMemPool_t resolver_pool()
 // its read-backs and gives them back when it has been waited for, so a resolver holds none between
 // batches and a new one finds them there (page-locking costs about 0.5 ms per MB and waits for the
 // device; a server keeps a resolver per graph shape). Given-back blocks are kept up to PINNED_KEEP
-// bytes (XKB_POOL_CACHE=0: none); a block in use belongs to one batch.
+// bytes (XKB_POOL_CACHE=0: none); a block in use belongs to one batch. A block up to four times the size
+// asked for will do, and a block given back displaces larger ones rather than being unlocked, so a
+// stream of batches finds its blocks again whatever an earlier one left: unlocking and locking 64 MB
+// behind a running window costs 35 to 90 ms a batch (16384^2 x 500 heat graph spawned through the C API:
+// 1.6 to 2.7 s to the end of the wait when a 128 MB block no batch asked for filled the room, 0.63 s now).
 class PinnedBlocks {
 public:
-    static constexpr size_t PINNED_KEEP = size_t(128) << 20, MIN_BLOCK = size_t(1) << 18;
+    static constexpr size_t PINNED_KEEP = size_t(256) << 20, MIN_BLOCK = size_t(1) << 18;
 
     static int take(size_t bytes, void ** p, size_t * cap)
     {
@@ -703,12 +707,12 @@ public:
         while (c < bytes) c *= 2;
         {
             std::lock_guard<std::mutex> lk(mu());
-            auto it = free_blocks().find(c);
-            if (it != free_blocks().end())
+            auto it = free_blocks().lower_bound(c);
+            if (it != free_blocks().end() && it->first <= 4 * c)
             {
-                *p = it->second; *cap = c;
+                *p = it->second; *cap = it->first;
+                kept() -= it->first;
                 free_blocks().erase(it);
-                kept() -= c;
                 return XKB_OK;
             }
         }
@@ -721,11 +725,23 @@ public:
     {
         if (!p) return;
         static const bool none = getenv("XKB_POOL_CACHE") && atoi(getenv("XKB_POOL_CACHE")) == 0;
+        std::vector<void *> out;
+        if (none || cap > PINNED_KEEP) out.push_back(p);
+        else
         {
             std::lock_guard<std::mutex> lk(mu());
-            if (!none && kept() + cap <= PINNED_KEEP) { free_blocks().emplace(cap, p); kept() += cap; return; }
+            free_blocks().emplace(cap, p);
+            kept() += cap;
+            while (kept() > PINNED_KEEP)                         // (the block just given is the last to go)
+            {
+                auto it = std::prev(free_blocks().end());
+                if (it->second == p) --it;
+                kept() -= it->first;
+                out.push_back(it->second);
+                free_blocks().erase(it);
+            }
         }
-        cudaFreeHost(p);
+        for (void * q : out) cudaFreeHost(q);
     }
 
 private:                                        // (never destroyed: resolvers may outlive static objects)
@@ -1751,9 +1767,9 @@ int xkb_internal_resolver_prepare(xkb_resolver_t * R, size_t nops)
     int rc;
     if ((rc = R->hops.reserve(nops)) || (rc = R->dops.reserve(nops)) || (rc = R->hset.reserve(2 * cap)) ||
         (rc = R->ukeys.reserve(4 * nops)) || (rc = R->ucount.reserve(3)) || (rc = R->emit.reserve(emit)) ||
-        (rc = R->counters.reserve(CNT_COUNT)) || (rc = R->table.reserve(tcap)) || (rc = R->stage.take(nops)) || (rc = spill_reserve(R, 1)))
+        (rc = R->counters.reserve(CNT_COUNT)) || (rc = R->table.reserve(tcap)) || (rc = R->stage.take((nops + 1) / 2)) || (rc = spill_reserve(R, 1)))
         return rc;
-    R->stage.give();                            // (kept for the batches to come)
+    R->stage.give();                            // (kept for the batches to come; one op per LINK and PUT pair is staged)
     if (R->useg.empty())
     {
         std::unique_ptr<DevBuf<unsigned long long>> seg(new (std::nothrow) DevBuf<unsigned long long>());
@@ -1763,7 +1779,7 @@ int xkb_internal_resolver_prepare(xkb_resolver_t * R, size_t nops)
         R->useg.push_back(std::move(seg));
         R->useg_n.push_back(0);
     }
-    // the buffers still to come (cell states of each domain, region bins, time-split snapshots,
+    // the buffers still to come (cell states of each domain, region bins,
     // window graphs) grow from the pool: give it room now rather than while batches run
     if (cudaMemPool_t pool = resolver_pool())
     {
