@@ -980,7 +980,7 @@ def main():
                            "d2h_bytes_per_step": bytes_grid, "ms_per_step": round(e2e_ms / args.steps, 3),
                            "what": "the resolved graph re-run by xkb_sched_run, the grid copied in from pinned host memory "
                                    "and the result copied out every step"},
-            "gpu_launches": 3 * args.steps,
+            "gpu_launches": 5 * args.steps,      # init, seed, plan, persistent and team kernel of each run
             "clocks": clk,
             "forms_first_2_steps": forms,
             "runs_ms": runs_ms,

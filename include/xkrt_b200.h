@@ -334,7 +334,7 @@ XKB_API int xkb_sched_set_grid(xkb_sched_t * sched, int ctas);
  * into registers, PF columns ahead, bulk L2 prefetch further ahead); 1 = bulk-staged body (per
  * warp, source columns stream into a ring of 8 shared-memory slots by asynchronous bulk copies,
  * cp.async.bulk with mbarrier completion, halo rows included). Same results either way; on the
- * 16384^2 FP64 graph the register body moves 4.8 TB/s and the bulk-staged one 3.2 TB/s. Tiles
+ * 16384^2 FP64 graph the register body moves 6.5 TB/s and the bulk-staged one 4.1 TB/s. Tiles
  * whose rows are not 16-byte aligned always use the register body. */
 XKB_API int xkb_sched_set_staging(xkb_sched_t * sched, int bulk);
 /* Warps that execute one task in the persistent kernel at least (1, 2, 4 or 8; default 1): a task

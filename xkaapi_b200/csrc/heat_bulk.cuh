@@ -13,9 +13,9 @@
 // Compared with the register body the halo rows arrive in the same copy as the strip (no
 // scalar halo loads), the bytes in flight cost shared memory instead of registers, and one
 // instruction moves a whole column. The arithmetic is the register body's (heat_update), so
-// results are identical. Measured on the 16384^2 FP64 graph (128^2 tiles) it moves 3.2 TB/s
-// against the register body's 4.8 TB/s, with 8 or 16 slots per warp alike: one 544-byte copy
-// per column is too small a unit; the scheduler keeps it as an opt-in body.
+// results are identical. Measured on the 16384^2 graph (128^2 tiles) it moves 4.1 TB/s against the
+// register body's 6.5 TB/s (FP32: 3.2 against 5.6): one 544-byte copy per column is too small a
+// unit; the scheduler keeps it as an opt-in body.
 //
 // Ordering: bulk copies read global memory through the async proxy. Tile data written by other
 // tasks is published by their release / this task's acquire in the generic proxy, so lane 0

@@ -119,7 +119,7 @@ struct XkbSrvSlot {
     uint8_t * copy_dst;                  //   ... duplicated here by the set-up chunks (second grid)
     uint64_t copy_bytes;
     uint32_t period, ntasks;
-    uint32_t nchunks;                    // set-up chunks (wait counters, queue slots, grid copy)
+    uint32_t nchunks;                    // set-up chunks (wait counters, grid copy)
     uint32_t chunk_tasks;                // tasks whose counters one chunk sets up
     uint32_t gen;                        // admission number, reported back when the request ends
     uint32_t units_log2;                 // a task is 2^units_log2 units, each run by one warp

@@ -10,9 +10,10 @@
 //  * graph: the heat graph repeats every two steps (the grids swap back), so the server resolves
 //    three two-step windows once per grid shape with the GPU resolver, keeps the periodic form
 //    (one window's CSR plus its edges into the next window) and runs every request of that shape
-//    as ONE persistent-scheduler launch over all its windows (a half window at the end for an odd
-//    step count) -- its tiles and counters stay on the device from its first step to its last,
-//    and consecutive steps overlap on the device;
+//    over all its windows at once (a half window at the end for an odd step count), in the
+//    persistent kernel that serves the whole trace (server_kernel) or, XKB_SERVE_MODE=launch, as a
+//    launch of its own -- its tiles and counters stay on the device from its first step to its
+//    last, and consecutive steps overlap on the device;
 //  * latency: from the request's arrival time to the host observing its completion event.
 // The initial grid is a seeded pseudo-random U[0,1) interior with a zero boundary, produced on
 // the device from (seed, cell index), so a request computes the same grid alone or in a mix.
@@ -31,13 +32,13 @@
 
 
 #ifndef XKB_SERVE_TEAM
-#define XKB_SERVE_TEAM 1                 // warps per tile task of a served graph
+#define XKB_SERVE_TEAM 1                 // warps per tile task of a served graph (launch mode: at least)
 #endif
 #ifndef XKB_SERVE_PFD
 #define XKB_SERVE_PFD 4                  // L2 prefetch distance (columns) of a served graph
 #endif
 #ifndef XKB_SERVE_TASKS_PER_CTA
-#define XKB_SERVE_TASKS_PER_CTA 2        // a graph gets one CTA per this many tasks of a step
+#define XKB_SERVE_TASKS_PER_CTA 2        // launch mode: a graph gets one CTA per this many tasks of a step
 #endif
 namespace {
 
