@@ -265,3 +265,38 @@ def test_heat_grids_of_any_alignment(torch_cuda, nx, ny, ld, ts, steps, f32):
     np.testing.assert_array_equal(out[:, :nx], want.reshape(ny, nx))
     assert (out[:, nx:] == 7.0).all()
     sch.close(); res.close()
+
+
+@pytest.mark.parametrize("fan", [3, 40, 100])
+def test_split_task_releases_successors_behind_all_its_units(torch_cuda, fan):
+    """Queue runs of split tasks with more successors than one lane, or one warp, decrements: a
+    producer of 64 pieces, `fan` consumers that wait for all of it, a producer that waits for theirs,
+    and so on. Two such graphs one after the other are not spawned level by level, so they take the queue."""
+    torch = torch_cuda
+    n, levels = 64 * 8192, 6
+    rng = np.random.default_rng(fan)
+    cuts = np.linspace(0, n, fan + 1).astype(np.int64)
+    tasks, descs, checks = [], [], []
+    for _ in range(2):
+        y, z = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+        dy, dz = torch.from_numpy(y).cuda(), torch.from_numpy(z).cuda()
+        for level in range(levels):
+            a, b = rng.uniform(-1, 1, 2)
+            whole = level % 2 == 0
+            src, dst, hs, hd = (dz, dy, z, y) if whole else (dy, dz, y, z)
+            for lo, hi in [(0, n)] if whole else zip(cuts[:-1], cuts[1:]):
+                tasks.append([("s", S.R, src.data_ptr(), src.data_ptr() + 8 * n),
+                              ("s", S.RW, dst.data_ptr() + 8 * int(lo), dst.data_ptr() + 8 * int(hi))])
+                descs.append((src.data_ptr(), dst.data_ptr(), int(lo), int(hi), a, b))
+                hd[lo:hi] = O.axpby(a, hs[lo:hi], b, hd[lo:hi])
+        checks += [(dy, y), (dz, z)]
+    d = np.zeros(len(descs), dtype=xk.axpby_desc_dtype())
+    d["kind"] = xk.TASK_AXPBY
+    for k, f in enumerate(("x", "y", "lo", "hi", "a", "b")):
+        d[f] = [t[k] for t in descs]
+    res = xk.Resolver(); res.add(S.from_tuples(tasks))
+    sch = xk.Scheduler(); sch.set_tasks(d); sch.run(res.graph())
+    assert sch.wait() == len(d)
+    for got, want in checks:
+        np.testing.assert_array_equal(got.cpu().numpy(), want)
+    sch.close(); res.close()

@@ -422,8 +422,8 @@ struct SuccGraph {
 };
 
 // One warp, after task t's last unit: decrement the successors' counters and publish those that
-// became ready. The caller's fence orders the task's writes before the counters; the fence here, the
-// writes of the other predecessors before the queue slot.
+// became ready. The caller's fence, by every lane, orders the writes of all of the task's units before the
+// counters; the fence here, the writes of the other predecessors before the queue slot.
 __device__ __forceinline__ void release_successors(const SuccGraph & g, uint32_t t, uint32_t first, bool more, int * wc, int * queue,
                                                    unsigned * tail, int lane)
 {
@@ -602,13 +602,12 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_persisten
             if (k > 0)
             {
                 int last = 0;
-                if (lane == 0)
-                {
-                    last = atom_add_relaxed(a.units_done + t, 1) == nunits - 1;
-                    fence_acq_rel_gpu();
-                }
+                if (lane == 0) last = atom_add_relaxed(a.units_done + t, 1) == nunits - 1;
                 if (!__shfl_sync(0xffffffffu, last, 0)) continue;
                 __syncwarp();
+                // every lane decrements counters below, so every lane fences: the other units' writes, which
+                // the count has shown to be done, come before its decrements too
+                fence_acq_rel_gpu();
             }
             release_successors(g, (uint32_t) t, first, more, a.wc, a.queue, a.ctr + CTR_TAIL, lane);
         }
