@@ -128,3 +128,23 @@ def test_shares_and_units_match_oracle(torch_cuda, slots, ctas):
     for (t, n, steps, f32, seed), buf in zip(specs, bufs):
         dt = np.float32 if f32 else np.float64
         np.testing.assert_array_equal(buf, O.heat_run(O.serve_init(n, n, seed, dt), n, n, steps, 0.2, dtype=dt))
+
+
+@pytest.mark.parametrize("slots", [1, 2])
+def test_slots_reused_by_short_requests(torch_cuda, slots):
+    """Hundreds of requests of a step or two, of several shapes, through one or two slots while every
+    CTA of the device looks for work in them: each slot changes hands as CTAs still arrive at the
+    request before, and every result is the oracle's."""
+    rng = np.random.default_rng(slots)
+    specs, tiles = [], []
+    for k in range(300):
+        n = int(rng.choice([34, 64, 130, 200]))
+        specs.append((0.0, n, int(rng.integers(1, 3)), int(k % 2), 900 + k))
+        tiles.append(int(rng.choice([16, 32, 64])))
+    srv = xk.Server(budget_bytes=16 << 20, slots=slots, max_seconds=60.0)
+    reqs, bufs = make_requests(specs, tiles)
+    srv.run(reqs)
+    srv.close()
+    for (t, n, steps, f32, seed), buf in zip(specs, bufs):
+        dt = np.float32 if f32 else np.float64
+        np.testing.assert_array_equal(buf, O.heat_run(O.serve_init(n, n, seed, dt), n, n, steps, 0.2, dtype=dt))

@@ -1411,19 +1411,22 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) server_kernel(X
                 {
                     const int q = (int) (best & 0xff);
                     XkbSrvCtl * c = a.ctl + q;
+                    // counted before the state is looked at (again): the slot is not reused while this CTA
+                    // counts. Whoever ends the request stores state 3 and then looks at the count; the
+                    // sequentially consistent fence between the two on either side makes one see the other.
+                    const unsigned n = atomicAdd(&c->attached, 1u);
+                    __threadfence();
                     const unsigned st = ld_acquire_u32(&c->state);
-                    if (st == 1)
+                    if (st == 2 && n < a.slots[q].ctas) { kind = ATTACH; sl = q; }
+                    else
                     {
-                        const unsigned ch = atomicAdd(&c->init_next, 1u);
-                        if (ch < a.slots[q].nchunks) { kind = SETUP; sl = q; idx = (int) ch; }
-                    }
-                    else if (st == 2)
-                    {
-                        // attached before the state is looked at again: the slot is not reused while it counts
-                        const unsigned n = atomicAdd(&c->attached, 1u);
-                        fence_acq_rel_gpu();
-                        if (ld_acquire_u32(&c->state) == 2 && n < a.slots[q].ctas) { kind = ATTACH; sl = q; }
-                        else atomicSub(&c->attached, 1u);
+                        if (st == 1)
+                        {
+                            // (a claimed chunk holds the request in state 1 by itself)
+                            const unsigned ch = atomicAdd(&c->init_next, 1u);
+                            if (ch < a.slots[q].nchunks) { kind = SETUP; sl = q; idx = (int) ch; }
+                        }
+                        atomicSub(&c->attached, 1u);
                     }
                 }
                 else if (!busy && *(volatile unsigned *) (a.status + 2) != 0) kind = STOP;
@@ -1552,6 +1555,7 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) server_kernel(X
             {
                 fence_acq_rel_gpu();
                 st_release_u32(&c->state, 3u);
+                __threadfence();                               // (see where a CTA counts itself in)
                 // CTAs that saw state 2 before the store above find no ticket, or the new state, and
                 // leave; wait (bounded) until none but this one counts
                 const uint64_t tw = xkb_globaltimer();
