@@ -1,6 +1,8 @@
 """GPU dependency resolver: bit-exact unique edge sets against the reference's own trees
 (golden fixtures) and against the oracle restatement on larger seeded streams."""
 import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -250,3 +252,46 @@ def test_successor_lists_ascending(torch_cuda, nreaders):
     succ = torch.as_tensor(_DevView(g.succ, g.nedges), device="cuda").cpu().numpy()
     np.testing.assert_array_equal(succ, np.arange(1, nreaders + 1))
     r.close()
+
+
+def diagonal(cells, first_task, count, passes=1):
+    """Write accesses to the first `count` of the `cells` 64 x 64 blocks on the diagonal of a matrix, a
+    task each, `passes` times over: 64 (cells / 8)^2 regions in the domain once all blocks were named."""
+    k = np.tile(np.arange(count, dtype=np.uint64), passes)
+    r = np.zeros(len(k), dtype=S.REC)
+    r["task"] = first_task + np.arange(len(k))
+    r["type"], r["mode"], r["ld"], r["sizeof_type"], r["m"], r["n"] = S.MATRIX, S.RW, 64 * cells, 8, 64, 64
+    r["offset_m"] = r["offset_n"] = 64 * k
+    return r
+
+
+def run_logged(tmp_path, body, **env):
+    """Run `body` (Python, with diagonal() and mark(text) at hand) in a process whose calls of the CUDA
+    runtime are logged (tests/cpp/cudart_log.c); the log's lines, split."""
+    tests = os.path.dirname(os.path.abspath(__file__))
+    shim, log = str(tmp_path / "cudart_log.so"), str(tmp_path / "log.txt")
+    subprocess.run(["gcc", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", os.path.join(tests, "cpp", "cudart_log.c"), "-o", shim, "-ldl"],
+                   check=True)
+    code = (f"import sys, ctypes; sys.path[:0] = [{tests!r}, {U.REPO!r}]\n"
+            "import numpy as np, xkaapi_b200 as xk\nfrom test_resolver_gpu import diagonal\n"
+            f"mark = lambda text: ctypes.CDLL({shim!r}).cudart_log_mark(text.encode())\n" + body)
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, LD_PRELOAD=shim, CUDART_LOG=log, **env),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    return [ln.split() for ln in open(log).read().splitlines()]
+
+
+def test_shared_memory_limits_are_never_lowered(torch_cuda, tmp_path):
+    """A kernel's shared-memory limit belongs to the process: a batch that needs less must not lower it
+    below what another thread's batch is about to launch with."""
+    log = run_logged(tmp_path, """
+big, small = xk.Resolver(), xk.Resolver()
+big.add(diagonal(870, 0, 870, 800))        # 11,881 regions, 1.4 M ops: more than one bitmap of 160 KB
+small.add(diagonal(640, 0, 640, 320))      # 6,400 regions, 410,000 ops
+""")
+    limits = {}
+    for ln in log:
+        if ln[0] == "smem":
+            assert int(ln[2]) >= limits.get(ln[1], 0), log
+            limits[ln[1]] = int(ln[2])
+    assert len(limits) >= 2

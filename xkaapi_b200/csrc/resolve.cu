@@ -1395,12 +1395,13 @@ static int refine_domain(xkb_resolver * R, Domain & d, std::vector<uint64_t> & x
     return XKB_OK;
 }
 
-// Dynamic shared memory a kernel may ask for on the current device, set once per kernel and device
-// and raised when a call needs more.
+// Let a launch on the current device ask for `bytes` of dynamic shared memory. The limit is the
+// kernel's, for every host thread, so it is always set to `most`, what the kernel may ever need: a
+// limit of just this call's bytes would take it from another thread's batch before its launch.
 template <typename K>
-static int allow_smem(K kernel, size_t bytes)
+static int allow_smem(K kernel, size_t bytes, size_t most)
 {
-    if (bytes > 48 * 1024) XKB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes));
+    if (bytes > 48 * 1024) XKB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) most));
     return XKB_OK;
 }
 
@@ -1431,10 +1432,10 @@ static int launch_region(xkb_resolver * R, ResolveArgs & a, int nregions)
     const char * gb = getenv("XKB_RESOLVE_BIN_GLOBAL");             // 1: the global-atomic binning (tests)
     const bool smem_bins = nregions <= BIN_SMEM_REGIONS && !(gb && atoi(gb) == 1);
     const unsigned gs = std::min<unsigned>(g, (unsigned) (2 * device_sms()));
-    const size_t bins = (size_t) nregions * sizeof(unsigned);
+    const size_t bins = (size_t) nregions * sizeof(unsigned), bins_most = BIN_SMEM_REGIONS * sizeof(unsigned);
     if (smem_bins)
     {
-        if ((rc = allow_smem(bin_count_smem_kernel, bins))) return rc;
+        if ((rc = allow_smem(bin_count_smem_kernel, bins, bins_most))) return rc;
         bin_count_smem_kernel<<<gs, 256, bins, st>>>(a.ops, a.nops, RX, RY, a.nrx, nregions, R->bin_off.p);
     }
     else
@@ -1451,14 +1452,14 @@ static int launch_region(xkb_resolver * R, ResolveArgs & a, int nregions)
         if ((rc = R->bin_list.reserve(total)) || (rc = R->bin_sorted.reserve(total))) return rc;
         if (smem_bins)
         {
-            if ((rc = allow_smem(bin_fill_smem_kernel, 2 * bins))) return rc;
+            if ((rc = allow_smem(bin_fill_smem_kernel, 2 * bins, 2 * bins_most))) return rc;
             bin_fill_smem_kernel<<<gs, 256, 2 * bins, st>>>(a.ops, a.nops, RX, RY, a.nrx, nregions, R->bin_off.p, R->bin_cur.p,
                                                             R->bin_list.p);
         }
         else
             bin_fill_kernel<<<g, 256, 0, st>>>(a.ops, a.nops, RX, RY, a.nrx, R->bin_off.p, R->bin_cur.p, R->bin_list.p);
         const int words = std::max(BIN_SORT_SHORT, std::min(BIN_SORT_WORDS, (a.nops + 31) / 32));
-        if ((rc = allow_smem(bin_sort_kernel, (size_t) words * sizeof(unsigned)))) return rc;
+        if ((rc = allow_smem(bin_sort_kernel, (size_t) words * sizeof(unsigned), BIN_SORT_WORDS * sizeof(unsigned)))) return rc;
         bin_sort_kernel<<<(unsigned) nregions, BIN_SORT_THREADS, (size_t) words * sizeof(unsigned), st>>>(R->bin_off.p, R->bin_list.p,
                                                                                                           R->bin_sorted.p, a.nops, words);
     }
