@@ -295,3 +295,11 @@ small.add(diagonal(640, 0, 640, 320))      # 6,400 regions, 410,000 ops
             assert int(ln[2]) >= limits.get(ln[1], 0), log
             limits[ln[1]] = int(ln[2])
     assert len(limits) >= 2
+
+
+def test_region_lists_sorted_over_several_bitmaps(torch_cuda):
+    """1.4 M ops, more than one bitmap of the list sort holds, in lists of 12,800: every block's writes
+    follow one another."""
+    n = 870 * 800
+    t = np.arange(n - 870)
+    np.testing.assert_array_equal(gpu_edges(diagonal(870, 0, 870, 800)), np.stack([t, t + 870], axis=1))

@@ -31,3 +31,13 @@ def test_pool_arrays_and_parked_reservations(tmp_path):
                     "-o", exe], check=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stderr
+
+
+def test_op_windows_up_to_the_last_int(tmp_path):
+    """The op numbers of a batch and the windows of the bitmap sort (xkaapi_b200/csrc/op_windows.h),
+    with signed overflow trapped."""
+    exe = str(tmp_path / "op_windows_test")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-Wall", "-Werror", "-fsanitize=undefined", "-fno-sanitize-recover=all",
+                    os.path.join(REPO, "tests", "cpp", "op_windows_test.cc"), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stderr

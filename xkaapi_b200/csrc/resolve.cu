@@ -30,6 +30,7 @@
 // scans and scatters the pairs into a successor CSR. Cell state stays in HBM between batches.
 #include "common.cuh"
 #include "internal.h"
+#include "op_windows.h"
 #include "scan.cuh"
 #include "workpool.h"
 
@@ -418,27 +419,28 @@ __global__ void __launch_bounds__(BIN_SORT_THREADS) bin_sort_kernel(const unsign
         return;
     }
     unsigned pos = b;
-    for (int w0 = 0; w0 * 32 < nops; w0 += words)
+    for (int at = 0; at < nops;)
     {
+        const OpWindow win = OpWindow::from(at, words, nops);
         for (int w = threadIdx.x; w < words; w += BIN_SORT_THREADS) bits[w] = 0;
         __syncthreads();
-        const int op0 = w0 * 32, op1 = op0 + words * 32;         // (nops is an int: the last window may end past it)
         for (int i = threadIdx.x; i < n; i += BIN_SORT_THREADS)
         {
             const int op = in[b + i];
-            if (op >= op0 && (op < op1 || op1 < op0)) atomicOr(bits + ((op - op0) >> 5), 1u << ((op - op0) & 31));
+            if (win.holds(op)) atomicOr(bits + ((op - win.first) >> 5), 1u << ((op - win.first) & 31));
         }
         __syncthreads();
-        const int used = min(words, (nops - op0 + 31) / 32);
+        const int used = (win.last - win.first + 31) / 32;
         for (int w = threadIdx.x; w < ((used + BIN_SORT_THREADS - 1) / BIN_SORT_THREADS) * BIN_SORT_THREADS; w += BIN_SORT_THREADS)
         {
             unsigned m = w < used ? bits[w] : 0u;
             uint32_t total;
-            unsigned at = pos + block_exclusive_scan((uint32_t) __popc(m), wt, total);
+            unsigned to = pos + block_exclusive_scan((uint32_t) __popc(m), wt, total);
             pos += total;
-            for (; m; m &= m - 1) out[at++] = op0 + w * 32 + __ffs(m) - 1;
+            for (; m; m &= m - 1) out[to++] = win.first + w * 32 + __ffs(m) - 1;
         }
         __syncthreads();
+        at = win.last;
     }
 }
 
@@ -1110,6 +1112,19 @@ static inline int mat_nrects(const xkb_access_rec_t & r)
     return (A % LDs) + r.m * r.sizeof_type <= LDs ? 1 : 2;
 }
 
+// Refuse a batch with more ops in one domain than the kernels can number; none of its ops is kept.
+static int check_ops(xkb_resolver * R)
+{
+    uint64_t most = std::max<uint64_t>(R->interval.nops, R->handles.nops);
+    for (auto & d : R->blas) most = std::max<uint64_t>(most, d->nops);
+    if (most <= RESOLVE_MAX_OPS) return XKB_OK;
+    auto drop = [](Domain & d) { d.ops.clear(); d.nops = d.nhops = 0; };
+    drop(R->interval); drop(R->handles);
+    for (auto & d : R->blas) drop(*d);
+    return xkb_set_error(XKB_ERANGE, "resolver: %llu ops of one domain in a batch (at most %llu): add it in smaller batches",
+                         (unsigned long long) most, (unsigned long long) RESOLVE_MAX_OPS);
+}
+
 // Matrix-only batches whose every (ld, sizeof) already has a domain: each record's ops go to its
 // own domain only (LINK ops of a task's records, then their PUT ops), so chunks of whole tasks
 // are built on their own -- by the host team when the batch is large: a counting pass, then every
@@ -1201,6 +1216,7 @@ static int build_ops_staged(xkb_resolver * R, const xkb_access_rec_t * recs, siz
         R->blas[k]->nhops = total - first;
         R->blas[k]->nops = 2 * R->blas[k]->nhops;
     }
+    if (int rc = check_ops(R)) return rc;
     if (int rc = R->stage.take(total ? total : 1)) return rc;
     HOp * out = R->stage.p;
     team([&](unsigned c) {
@@ -1570,6 +1586,7 @@ static int resolve_batch(xkb_resolver * R, const xkb_access_rec_t * recs, size_t
         R->interval.nops = R->interval.nhops = R->interval.ops.size();
         R->handles.nops = R->handles.nhops = R->handles.ops.size();
         for (auto & d : R->blas) d->nops = d->nhops = d->ops.size();
+        if ((rc = check_ops(R))) return rc;
     }
     const auto t1 = clk::now();
     std::vector<Domain *> doms;
