@@ -300,3 +300,47 @@ def test_split_task_releases_successors_behind_all_its_units(torch_cuda, fan):
     for got, want in checks:
         np.testing.assert_array_equal(got.cpu().numpy(), want)
     sch.close(); res.close()
+
+
+def chains(torch, count, length, roots):
+    """`roots` heat tiles, then `count` chains of `length` tiles, spawned chain by chain; every chain
+    follows one of the roots, if there are any. Returns the graph, the descriptors, what keeps them
+    alive, and each chain's grids with the seed of its initial one."""
+    side, grids, descs, edges = 128, [], [], []
+    for k in range(roots + count):
+        g = O.heat_init(side, side, seed=k)
+        a, b = torch.from_numpy(g).cuda(), torch.from_numpy(g).cuda()
+        grids.append((k, a, b))
+        descs.append(xk.heat_task_descs((a.data_ptr(), b.data_ptr()), side, side, side, side, side, 1 if k < roots else length, C))
+        if k >= roots:
+            first = roots + (k - roots) * length
+            edges += [(first + i, first + i + 1) for i in range(length - 1)]
+            if roots:
+                edges.append((k % roots, first))
+    descs = np.concatenate(descs)
+    edges = np.array(sorted(edges), dtype=np.int64)
+    ptr = np.concatenate([[0], np.cumsum(np.bincount(edges[:, 0], minlength=len(descs)))])
+    keep = [torch.from_numpy(v.astype(np.int32)).cuda() for v in (ptr, edges[:, 1], np.bincount(edges[:, 1], minlength=len(descs)))]
+    return xk.TaskGraph(len(descs), len(edges), *(v.data_ptr() for v in keep)), descs, keep, grids[roots:]
+
+
+@pytest.mark.parametrize("roots", [1, 2])
+def test_chains_behind_common_roots_run_side_by_side(torch_cuda, roots):
+    """Chains spawned one after the other behind a first task or two that all of them follow: taken in
+    spawn order they would run one after another. They take about as long as without the roots (a
+    small part of what one after another takes), and every grid is the oracle's."""
+    torch = torch_cuda
+    ms = {}
+    for r in (0, roots):
+        graph, descs, keep, grids = chains(torch, 64, 100, r)
+        sch = xk.Scheduler(); sch.set_tasks(descs)
+        sch.run(graph)
+        assert sch.wait() == len(descs)
+        for seed, a, b in grids:
+            np.testing.assert_array_equal(a.cpu().numpy(), O.heat_run(O.heat_init(128, 128, seed=seed), 128, 128, 100, C))
+        ms[r] = []
+        for _ in range(5):
+            sch.run(graph); sch.wait()
+            ms[r].append(sch.kernel_ms())
+        sch.close()
+    assert min(ms[roots]) < 2 * min(ms[0]), ms

@@ -310,14 +310,16 @@ __device__ __forceinline__ int run_split_log2(const SchedArgs & a, unsigned warp
 }
 
 // Chooses the order of the run. Let W be the number of tasks ready at the start. The run goes in
-// order when those are tasks 0 .. W-1 and every edge leads from one block of W consecutive tasks to
-// a later one: then the tasks of a block are independent of one another, so taking them in spawn
-// order keeps W tasks runnable at a time and no warp waits behind a task that a later one could have
-// overtaken by more than a block. (A chain spawned before the next chain fails the test and takes
-// the queue.) In order, nothing is published, a warp knows its task -- descriptor and successors --
-// before it may run, and every unit decrements its successors itself, without waiting for the
-// answer: 15.6 us per step of the 2048^2 FP64 graph against 19.6 through the queue with the same
-// units, and 174 against 180 for 8192^2.
+// order when those are tasks 0 .. W-1, every edge leads from one block of W consecutive tasks to a
+// later one, and every task t is a predecessor of task t + W (a heat tile, of the same tile a step
+// later). Then the graph is W chains that advance side by side: no more than W tasks are ever ready at a
+// time, and the tasks of a block are independent of one another, so spawn order keeps as many tasks
+// runnable as the queue could. (Without the last condition a graph with one root passes whatever
+// follows: 64 chains of 100 tiles behind a common first task, spawned chain by chain, ran one after
+// another, 10.4 ms against 5.7 through the queue.) In order, nothing is published, a warp knows its
+// task -- descriptor and successors -- before it may run, and every unit decrements its successors
+// itself, without waiting for the answer: 15.6 us per step of the 2048^2 FP64 graph against 19.6
+// through the queue with the same units, and 174 against 180 for 8192^2.
 // In order, a counter starts at the task's number of predecessors n and every one of their 2^k units
 // takes one off, so the task may run at n - n * 2^k.
 constexpr unsigned INORDER_MAX_NPRED = 1u << 20;      // keeps that inside an int
@@ -338,7 +340,17 @@ __global__ void sched_plan_kernel(SchedArgs a, unsigned warps)
     if (ok)
     {
         ok = a.npred_first[t] < INORDER_MAX_NPRED && a.npred_next[t] < INORDER_MAX_NPRED;
-        for (uint32_t i = a.succ_ptr[t], e = a.succ_ptr[t + 1], b = t / W; i < e; ++i) ok = ok && a.succ[i] / W > b;
+        const uint64_t next = (uint64_t) t + W;                // the task a block later: in this window, or in the one after it
+        bool chained = next >= a.ntasks;
+        for (uint32_t i = a.succ_ptr[t], e = a.succ_ptr[t + 1], b = t / W; i < e; ++i)
+        {
+            const uint32_t s = a.succ[i];
+            ok = ok && s / W > b;
+            chained = chained || s == next;
+        }
+        if (!chained && next >= a.period && a.xsucc_ptr)
+            for (uint32_t i = a.xsucc_ptr[t], e = a.xsucc_ptr[t + 1]; i < e; ++i) chained = chained || a.xsucc[i] + (uint64_t) a.period == next;
+        ok = ok && chained;
     }
     if (!ok && *(volatile unsigned *) (a.ctr + CTR_QUEUE) == 0) atomicExch(a.ctr + CTR_QUEUE, 1u);
     // the first place among the ready tasks where the tiles' rows change (block_order); ~ so that 0 is none
