@@ -337,9 +337,9 @@ XKB_API int xkb_sched_set_grid(xkb_sched_t * sched, int ctas);
  * 16384^2 FP64 graph the register body moves 6.5 TB/s and the bulk-staged one 4.1 TB/s. Tiles
  * whose rows are not 16-byte aligned always use the register body. */
 XKB_API int xkb_sched_set_staging(xkb_sched_t * sched, int bulk);
-/* Warps that execute one task in the persistent kernel at least (1, 2, 4 or 8; default 1): a task
- * is split into that many units, each run by one warp, or into more where the graph has too few
- * tasks side by side to fill the device, or its axpby ranges are long. */
+/* Warps that execute one task in the persistent kernel (1, 2, 4 or 8): every task is split into that
+ * many units, each run by one warp. Without a call the scheduler chooses for each run: one, or more
+ * where the graph has too few tasks side by side to fill the device, or its axpby ranges are long. */
 XKB_API int xkb_sched_set_team(xkb_sched_t * sched, int warps_per_task);
 /* Distance, in columns, of the L2 bulk prefetch ahead of a heat tile's sweep (0 = off; default 4). */
 XKB_API int xkb_sched_set_prefetch(xkb_sched_t * sched, int columns);
@@ -369,7 +369,8 @@ XKB_API int xkb_sched_run_periodic(xkb_sched_t * sched, const xkb_periodic_graph
  * tasks; larger graphs get XKB_ERANGE. `tasks` is a DEVICE array of descriptors, `graph` the
  * resolver's device CSR. The call waits for the run to finish and returns XKB_ETIMEDOUT if a
  * device wait gave up after timeout_s seconds (finite, above 0, at most 3600 s); *executed
- * (optional) = tasks run.
+ * (optional) = tasks run. warps_per_task (1, 2, 4 or 8) warps run a task at least; more where the
+ * graph has too few tasks side by side to fill the device, or its axpby ranges are long.
  *
  * Set-up: the array and the kernels are device memory that the CUDA driver creates when the
  * library's module is first used on a device (modules load lazily), and the first call in each

@@ -344,3 +344,36 @@ def test_chains_behind_common_roots_run_side_by_side(torch_cuda, roots):
             ms[r].append(sch.kernel_ms())
         sch.close()
     assert min(ms[roots]) < 2 * min(ms[0]), ms
+
+
+def one_axpby_task(torch, n):
+    x, y = torch.rand(n, dtype=torch.float64, device="cuda"), torch.rand(n, dtype=torch.float64, device="cuda")
+    d = np.zeros(1, dtype=xk.axpby_desc_dtype())
+    d["kind"], d["x"], d["y"], d["hi"], d["a"], d["b"] = xk.TASK_AXPBY, x.data_ptr(), y.data_ptr(), n, 0.5, 0.25
+    keep = [torch.zeros(k, dtype=torch.int32, device="cuda") for k in (2, 1, 1)]
+    return xk.TaskGraph(1, 0, *(v.data_ptr() for v in keep)), d, [x, y, keep]
+
+
+def best_ms(sch, graph, reps=5):
+    sch.run(graph); sch.wait()
+    ms = []
+    for _ in range(reps):
+        sch.run(graph); sch.wait()
+        ms.append(sch.kernel_ms())
+    return min(ms)
+
+
+def test_team_is_what_the_caller_sets(torch_cuda):
+    """A caller that sets the warps per task gets that many: an axpby task of 512 pieces takes one warp
+    several times as long as eight, and these several times as long as the split that the
+    scheduler chooses by itself (256 warps)."""
+    torch = torch_cuda
+    graph, d, keep = one_axpby_task(torch, 512 * 8192)
+    ms = {}
+    for team in (None, 8, 1):
+        sch = xk.Scheduler(); sch.set_tasks(d)
+        if team:
+            sch.set_team(team)
+        ms[team] = best_ms(sch, graph)
+        sch.close()
+    assert ms[1] > 3 * ms[8] and ms[8] > 3 * ms[None], ms

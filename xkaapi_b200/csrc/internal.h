@@ -80,6 +80,8 @@ typedef struct xkb_edge_mark_t { size_t seg, off; uint32_t ntasks; } xkb_edge_ma
 int xkb_internal_resolver_edge_mark(xkb_resolver_t * R, xkb_edge_mark_t * m);
 // Reserve the working memory of a batch of about nops ops up front.
 int xkb_internal_resolver_prepare(xkb_resolver_t * R, size_t nops);
+// Units (1, 2, 4 or 8) a task is split into at least where the scheduler chooses their number itself.
+void xkb_internal_sched_min_units(xkb_sched_t * S, int units);
 // Reserve the device buffers of runs of up to ntasks tasks up front.
 int xkb_internal_sched_reserve(xkb_sched_t * S, size_t ntasks);
 // Unique edges stored so far (no graph build).

@@ -215,7 +215,8 @@ struct SchedArgs {
     uint64_t timeout_ns;
     int pfd;                   // L2 prefetch distance of the tile bodies, in columns
     int allow_team;            // narrow graphs may go to sched_team_kernel
-    int min_units;             // the caller's warps per task (xkb_sched_set_team): at least this many units
+    int units;                 // the caller's warps per task (xkb_sched_set_team): this many units; 0: chosen here,
+    int min_units;             // at least this many
 };
 
 __global__ void sched_init_kernel(SchedArgs a)
@@ -302,6 +303,7 @@ __host__ __device__ __forceinline__ int split_log2(unsigned width, bool heat, un
 __device__ __forceinline__ int run_split_log2(const SchedArgs & a, unsigned warps)
 {
     if (!a.units_done) return 0;
+    if (a.units) return a.units == 8 ? 3 : a.units / 2;
     const unsigned seeds = a.ctr[CTR_SEEDS], deg = a.ctr[CTR_SEED_DEG];
     const unsigned pieces = seeds ? (a.ctr[CTR_SEED_PIECES] + seeds - 1) / seeds : 0;
     int k = split_log2(max(seeds, deg / 8), a.ctr[CTR_SEED_HEAT] > 0, pieces, warps, a.min_units);
@@ -766,7 +768,8 @@ struct xkb_sched {
     const void * graph_key = nullptr;
     int last_form = -1;
     int grid = 0;
-    int team_warps = 1;                       // at least this many units (warps) per task
+    int team_warps = 0;                       // units (warps) per task, if the caller has set them
+    int min_units = 1;                        // else at least this many
     int bulk = 0;                             // 1: bulk-staged heat tile body (measured slower; opt-in)
     int pfd = SCHED_PFD_DEFAULT;              // L2 prefetch distance in columns
     uint64_t last_total = 0;                  // tasks of the last run
@@ -885,6 +888,8 @@ extern "C" int xkb_sched_set_team(xkb_sched_t * S, int warps_per_task)
     return XKB_OK;
 }
 
+void xkb_internal_sched_min_units(xkb_sched_t * S, int units) { S->min_units = units; }
+
 extern "C" int xkb_sched_set_staging(xkb_sched_t * S, int bulk)
 {
     if (!S || bulk < 0 || bulk > 1) return xkb_set_error(XKB_EINVAL, "sched_set_staging: 0 (register body) or 1 (bulk-staged body)");
@@ -916,7 +921,7 @@ static SchedArgs run_args(xkb_sched * S, uint32_t ntasks, uint32_t period)
     SchedArgs a;
     a.tasks = S->tasks.p; a.ntasks = ntasks; a.period = period;
     a.wc = S->wc.p; a.units_done = S->wc.p + ntasks; a.queue = S->queue.p; a.ctr = S->ctr.p;
-    a.timeout_ns = S->timeout_ns; a.pfd = S->pfd; a.min_units = S->team_warps;
+    a.timeout_ns = S->timeout_ns; a.pfd = S->pfd; a.units = S->team_warps; a.min_units = S->min_units;
     a.allow_team = !S->bulk;
     return a;
 }
@@ -1275,7 +1280,7 @@ extern "C" int xkb_sched_run_noalloc(const xkb_task_desc_t * tasks, const xkb_ta
     // a larger graph runs with one warp per task
     a.wc = scratch; a.queue = scratch + XKB_NOALLOC_MAX_TASKS;
     a.units_done = n <= XKB_NOALLOC_MAX_TASKS / 2 ? scratch + n : nullptr;
-    a.min_units = warps_per_task;
+    a.units = 0; a.min_units = warps_per_task;
     a.allow_team = 1;
     a.ctr = (unsigned *) (scratch + 2 * XKB_NOALLOC_MAX_TASKS);
     a.timeout_ns = (uint64_t) (timeout_s * 1e9);

@@ -253,7 +253,8 @@ extern "C" int xkb_server_create(xkb_server_t ** out, const xkb_server_cfg_t * c
         // step: 3.1 TB/s capacity and p99 155 ms at 80 % load on 1000 graphs; two warps per tile
         // and 8 columns ahead: 1.9 TB/s; a CTA per four or eight tasks: higher closed-loop
         // capacity that the open-loop trace then overloads)
-        if ((rc = xkb_sched_set_team(sl.sch, XKB_SERVE_TEAM)) || (rc = xkb_sched_set_prefetch(sl.sch, XKB_SERVE_PFD))) return rc;
+        xkb_internal_sched_min_units(sl.sch, XKB_SERVE_TEAM);
+        if ((rc = xkb_sched_set_prefetch(sl.sch, XKB_SERVE_PFD))) return rc;
     }
     int sms = 148, per = 2;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S->dev);

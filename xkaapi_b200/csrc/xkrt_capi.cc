@@ -2207,13 +2207,14 @@ static int translate_descs(xkb_runtime * R, size_t t0, size_t t1, std::vector<xk
     return XKB_OK;
 }
 
-// Warps per task: heat tiles (one warp strip covers 128 rows in FP64 and FP32) run best one warp
-// per task, axpby slices two (measured on the 16384^2 graphs and the axpby chains).
-static int team_for(xkb_runtime * R, const xkb_task_desc_t * d, size_t n)
+// Warps per task at least: heat tiles (one warp strip covers 128 rows in FP64 and FP32) run best one
+// warp per task where they fill the device, axpby slices two (measured on the 16384^2 graphs and the
+// axpby chains).
+static void team_for(xkb_runtime * R, const xkb_task_desc_t * d, size_t n)
 {
     bool heat = true;
     for (size_t t = 0; t < n && heat; t += 1 + n / 64) heat = d[t].kind == XKB_TASK_HEAT_F32 || d[t].kind == XKB_TASK_HEAT_F64;
-    return xkb_sched_set_team(R->sched, heat ? 1 : 2);
+    xkb_internal_sched_min_units(R->sched, heat ? 1 : 2);
 }
 
 // Make the new distinct records of accesses [a0, a1) coherent on the device (copies issued on the
@@ -2293,7 +2294,7 @@ static int stream_prepare(xkb_runtime * R, size_t t0, size_t t1, size_t a0, size
     unsigned bodies = 0;
     if (rc == XKB_OK) rc = translate_descs(R, t0, t1, copy, &descs, &longa, &bodies, sl.p);
     const double d_ms = ms_since(w0) - f_ms;
-    if (rc == XKB_OK) rc = team_for(R, descs, n);
+    if (rc == XKB_OK) team_for(R, descs, n);
     if (rc == XKB_OK) rc = xkb_internal_sched_upload_window(R->sched, descs, n, bodies);
     if (rc == XKB_OK && cudaEventRecord(sl.ev, R->stream) != cudaSuccess) rc = xkb_set_error(XKB_ECUDA, "xkrt: event");
     if (trace)
@@ -2387,7 +2388,7 @@ static int wait_batch(xkb_runtime * R)
         const xkb_task_graph_t & run_g = split ? sg.g : g;
         const xkb_task_desc_t * run_d = split ? sg.descs.data() : descs;
         const size_t run_n = split ? sg.descs.size() : nt;
-        if (rc == XKB_OK) rc = team_for(R, run_d, run_n);
+        if (rc == XKB_OK) team_for(R, run_d, run_n);
         if (P == 0)
         {
             if (rc == XKB_OK) rc = xkb_internal_sched_set_tasks_device(R->sched, run_d, run_n, bodies);
