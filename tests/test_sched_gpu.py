@@ -377,3 +377,51 @@ def test_team_is_what_the_caller_sets(torch_cuda):
         ms[team] = best_ms(sch, graph)
         sch.close()
     assert ms[1] > 3 * ms[8] and ms[8] > 3 * ms[None], ms
+
+
+@pytest.mark.parametrize("first", ["long axpby", "heat tile"])
+def test_split_fits_the_tasks_behind_the_first(torch_cuda, first):
+    """The one task that is ready at the start does not choose the split for what follows: a long axpby
+    task before 60,000 short ones, and a single tile before 4,096 tiles a step. The automatic split is
+    not slower than one warp per task (to a margin of a half), and the results are the oracle's."""
+    torch = torch_cuda
+    rng = np.random.default_rng(4)
+    if first == "long axpby":
+        n, short, m = 64 * 8192, 60_000, 64
+        host = [rng.uniform(-1, 1, n), rng.uniform(-1, 1, n), rng.uniform(-1, 1, short * m), rng.uniform(-1, 1, short * m)]
+        x, y, u, v = dev = [torch.from_numpy(h).cuda() for h in host]
+        d = np.zeros(1 + short, dtype=xk.axpby_desc_dtype())
+        d["kind"], d["a"], d["b"] = xk.TASK_AXPBY, 0.5, 0.25
+        d["x"], d["y"], d["lo"] = u.data_ptr(), v.data_ptr(), (np.arange(1 + short) - 1) * m
+        d["hi"] = d["lo"] + m
+        d["x"][0], d["y"][0], d["lo"][0], d["hi"][0] = x.data_ptr(), y.data_ptr(), 0, n
+        edges = np.stack([np.zeros(short, np.int64), 1 + np.arange(short)], axis=1)
+    else:
+        side, ts, steps = 2048, 32, 6
+        g = O.heat_init(side, side, seed=8)
+        small = O.heat_init(64, 64, seed=9)
+        a, b, p, q = dev = [torch.from_numpy(h).cuda() for h in (g, g, small, small)]
+        d = np.concatenate([xk.heat_task_descs((p.data_ptr(), q.data_ptr()), 64, 64, 64, 64, 64, 1, C),
+                            xk.heat_task_descs((a.data_ptr(), b.data_ptr()), side, side, side, ts, ts, steps, C)])
+        per = (side // ts) ** 2
+        r = xk.Resolver()
+        r.add(xk.heat_access_records(side, side, ts, ts, 0, steps, a.data_ptr(), b.data_ptr()))
+        e = r.edges().astype(np.int64)
+        r.close()
+        edges = np.concatenate([np.stack([np.zeros(per, np.int64), 1 + np.arange(per)], axis=1), e + 1])
+    edges = edges[np.lexsort((edges[:, 1], edges[:, 0]))]
+    ptr = np.concatenate([[0], np.cumsum(np.bincount(edges[:, 0], minlength=len(d)))])
+    keep = [torch.from_numpy(w.astype(np.int32)).cuda() for w in (ptr, edges[:, 1], np.bincount(edges[:, 1], minlength=len(d)))]
+    graph = xk.TaskGraph(len(d), len(edges), *(w.data_ptr() for w in keep))
+    sch = xk.Scheduler(); sch.set_tasks(d); sch.run(graph)
+    assert sch.wait() == len(d)
+    if first == "long axpby":
+        np.testing.assert_array_equal(y.cpu().numpy(), O.axpby(0.5, host[0], 0.25, host[1]))
+        np.testing.assert_array_equal(v.cpu().numpy(), O.axpby(0.5, host[2], 0.25, host[3]))
+    else:
+        np.testing.assert_array_equal(a.cpu().numpy(), O.heat_run(g, side, side, steps, C))
+    auto = best_ms(sch, graph)
+    sch.set_team(1)
+    one = best_ms(sch, graph)
+    sch.close()
+    assert auto < 1.5 * one, (auto, one)

@@ -189,11 +189,13 @@ __device__ __forceinline__ int atom_add_acq_rel(int * p, int v)
 }
 
 // Counters of a run (device memory): ready-queue tickets and tasks published, status, tasks
-// executed; then what the seed kernel learnt about the tasks that are ready at the start.
+// executed; then what the seed kernel learnt about the tasks that are ready at the start, and of the kinds
+// of all tasks (CTR_PIECES: 64 bits).
 // Head and tail have cache lines of their own: every warp's ticket and every release is an atomic there.
 // CTR_EXECUTED counts units of an in-order run, tasks of a queue run (executed_tasks).
-enum { CTR_HEAD = 0, CTR_TAIL = 32, CTR_STATUS = 48, CTR_EXECUTED, CTR_BAD_TASK, CTR_SEEDS, CTR_SEED_LAST, CTR_SEED_DEG, CTR_SEED_PIECES,
-       CTR_SEED_HEAT, CTR_QUEUE, CTR_SPLIT, CTR_TEAM, CTR_RUN, CTR_COUNT = 64 };
+enum { CTR_HEAD = 0, CTR_TAIL = 32, CTR_STATUS = 48, CTR_EXECUTED, CTR_BAD_TASK, CTR_SEEDS, CTR_SEED_LAST, CTR_SEED_WIDTH, CTR_SEED_HEAT,
+       CTR_HEAT, CTR_PIECES, CTR_PIECES_HI, CTR_AXPBY, CTR_QUEUE, CTR_SPLIT, CTR_TEAM, CTR_RUN, CTR_COUNT = 64 };
+static_assert(CTR_PIECES % 2 == 0, "64 bits");
 
 // A run covers `ntasks` tasks numbered w * period + t (window w, task t of the window's
 // `period` descriptors). A plain graph is one window (period = ntasks); a periodic graph adds
@@ -229,36 +231,59 @@ __global__ void sched_init_kernel(SchedArgs a)
     a.wc[t] = (int) (w == 0 ? a.npred_first[l] : a.npred_next[l]);
 }
 
-__global__ void sched_seed_kernel(SchedArgs a)
+// Eighths of the tasks that seed l releases, as far as its successors show: each counts for its share of
+// their predecessors, estimated on up to 16 of them. Few successors count an eighth each (a tile task has about
+// eight that each wait for as many tasks), without a look at them.
+__device__ __forceinline__ unsigned seed_width(const SchedArgs & a, uint32_t l)
+{
+    constexpr unsigned SAMPLE = 16;
+    const uint32_t b = a.succ_ptr[l], deg = a.succ_ptr[l + 1] - b;
+    if (deg <= SAMPLE) return deg;
+    float share = 0;
+#pragma unroll 8
+    for (unsigned i = 0; i < SAMPLE; ++i)
+    {
+        const uint32_t s = a.succ[b + (uint64_t) deg * i / SAMPLE];
+        if (s < a.period) share += 1.0f / (float) max(a.npred_first[s], 1u);
+    }
+    return (unsigned) fminf(8.0f / SAMPLE * share * (float) deg, 65536.0f);
+}
+
+__global__ void __launch_bounds__(256) sched_seed_kernel(SchedArgs a)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31;
     const bool ok = *(volatile unsigned *) (a.ctr + CTR_STATUS) == 0;   // a check before the run failed: nothing becomes ready
     const uint32_t w = t / a.period, l = t - w * a.period;
+    bool heat = false;
+    unsigned pieces = 0;
+    if (t < a.period && t < a.ntasks)
+    {
+        const xkb_task_desc_t & d = a.tasks[t];
+        heat = d.kind == XKB_TASK_HEAT_F64 || d.kind == XKB_TASK_HEAT_F32;
+        if (d.kind == XKB_TASK_AXPBY) pieces = (unsigned) max(min((d.u.axpby.hi - d.u.axpby.lo + AXPBY_PIECE - 1) / AXPBY_PIECE, (int64_t) 65536), (int64_t) 1);
+    }
+    if (__syncthreads_or(heat) && threadIdx.x == 0 && *(volatile unsigned *) (a.ctr + CTR_HEAT) == 0) atomicExch(a.ctr + CTR_HEAT, 1u);
+    const int naxpby = __syncthreads_count(pieces > 0);
+    if (naxpby)
+    {
+        const unsigned sum = __reduce_add_sync(0xffffffffu, pieces);
+        if (lane == 0 && sum) atomicAdd((unsigned long long *) (a.ctr + CTR_PIECES), (unsigned long long) sum);
+        if (threadIdx.x == 0) atomicAdd(a.ctr + CTR_AXPBY, (unsigned) naxpby);
+    }
     const bool seed = ok && t < a.ntasks && (w == 0 ? a.npred_first[l] : a.npred_next[l]) == 0;
     const unsigned m = __ballot_sync(0xffffffffu, seed);
     if (!m) return;
-    unsigned deg = 0, pieces = 0;
-    bool heat = false;
-    if (seed)
-    {
-        deg = min(a.succ_ptr[l + 1] - a.succ_ptr[l], 1u << 16);
-        const xkb_task_desc_t & d = a.tasks[l];
-        heat = d.kind == XKB_TASK_HEAT_F64 || d.kind == XKB_TASK_HEAT_F32;
-        if (d.kind == XKB_TASK_AXPBY) pieces = (unsigned) min((d.u.axpby.hi - d.u.axpby.lo + AXPBY_PIECE - 1) / AXPBY_PIECE, (int64_t) 4096);
-    }
-    deg = __reduce_add_sync(0xffffffffu, deg);
-    pieces = __reduce_add_sync(0xffffffffu, pieces);
+    const unsigned width = __reduce_add_sync(0xffffffffu, seed ? seed_width(a, l) : 0u);
     const unsigned last = __reduce_max_sync(0xffffffffu, seed ? t + 1 : 0u);
-    const unsigned nheat = __popc(__ballot_sync(0xffffffffu, heat));
+    const unsigned nheat = __popc(__ballot_sync(0xffffffffu, seed && heat));
     unsigned pos = 0;
     if (lane == 0)
     {
         pos = atomicAdd(a.ctr + CTR_TAIL, (unsigned) __popc(m));
         atomicAdd(a.ctr + CTR_SEEDS, (unsigned) __popc(m));
         atomicMax(a.ctr + CTR_SEED_LAST, last);
-        if (deg) atomicAdd(a.ctr + CTR_SEED_DEG, deg);
-        if (pieces) atomicAdd(a.ctr + CTR_SEED_PIECES, pieces);
+        if (width) atomicAdd(a.ctr + CTR_SEED_WIDTH, width);
         if (nheat) atomicAdd(a.ctr + CTR_SEED_HEAT, nheat);
     }
     pos = __shfl_sync(0xffffffffu, pos, 0);
@@ -266,8 +291,8 @@ __global__ void sched_seed_kernel(SchedArgs a)
 }
 
 // log2 of the units a run's tasks are split into, from `width` = how many tasks the graph runs side
-// by side, `heat` whether they are heat tiles, `pieces` the mean number of AXPBY_PIECE pieces per
-// task, `warps` the run's workers, and the caller's least.
+// by side, `heat` whether there are heat tiles among them, its `tasks`, the axpby ones' number `naxpby`
+// and AXPBY_PIECE `pieces`, `warps` the run's workers, and the caller's least.
 //  * heat tiles, few: as many units as there are warps, 32 at most (128^2 FP64 tiles, us per step:
 //    64 tiles, 32 units of 4 columns 5.4, 16 units 7.6, one warp per tile 59; 256 tiles, 8 units
 //    12.3, one warp 62);
@@ -275,11 +300,15 @@ __global__ void sched_seed_kernel(SchedArgs a)
 //    a warp alone does not keep its memory requests in flight (576 tiles: 28.5 with 8 units, 40.5
 //    with 4, 70 with one; 1024 tiles: 45.3 with 4, 49.3 with 2, 49.7 with 8); a tile per warp or
 //    more is not split (4096 tiles: 174 with one or two units);
-//  * axpby: units of about AXPBY_PIECE elements, twice as many as the mean task needs, so that the
-//    largest chunk of a mixed graph spreads too (10 passes over 2^26 elements in chunks of 64 KiB
-//    to 16 MiB: 2.5 ms against 142 ms with one warp per chunk).
-constexpr int SPLIT_MAX_HEAT = 5, SPLIT_MAX = 8;
-__host__ __device__ __forceinline__ int split_log2(unsigned width, bool heat, unsigned pieces, unsigned warps, int min_units)
+//  * axpby: units of about AXPBY_PIECE elements, twice as many as the mean axpby task needs, so that
+//    the largest chunk of a mixed graph spreads too (10 passes over 2^26 elements in chunks of 64 KiB
+//    to 16 MiB: 2.5 ms against 142 ms with one warp per chunk). Every task gets as many units, empty ones
+//    where it has no work for them, so where most tasks are not long axpby ones (more than four units per piece) the
+//    units are fewer: until what they cost, about a sixteenth of a piece each, is no more than the pieces that
+//    one unit of the mean axpby task runs.
+constexpr int SPLIT_MAX_HEAT = 5, SPLIT_MAX = 8, PIECE_UNITS = 16;
+__host__ __device__ __forceinline__ int split_log2(unsigned width, bool heat, uint64_t tasks, unsigned naxpby, uint64_t pieces,
+                                                   unsigned warps, int min_units)
 {
     int k = 0;
     if (heat)
@@ -287,10 +316,12 @@ __host__ __device__ __forceinline__ int split_log2(unsigned width, bool heat, un
         while (k < SPLIT_MAX_HEAT && ((uint64_t) width << (k + 1)) <= warps) ++k;
         if (k < TEAM_LOG2) while (k < TEAM_LOG2 && ((uint64_t) width << (k + 1)) <= 2 * (uint64_t) warps) ++k;
     }
-    if (pieces > 1)
+    if (pieces > naxpby)
     {
+        const uint64_t mean = (pieces + naxpby - 1) / naxpby;
         int q = 0;
-        while (q < SPLIT_MAX && (1u << q) < 2 * pieces) ++q;
+        while (q < SPLIT_MAX && (1ull << q) < 2 * mean) ++q;
+        while (q > 0 && (tasks << q) > 4 * pieces && (tasks << 2 * q) > PIECE_UNITS * mean * warps) --q;
         if (q > k) k = q;
     }
     while ((1 << k) < min_units) ++k;
@@ -298,15 +329,13 @@ __host__ __device__ __forceinline__ int split_log2(unsigned width, bool heat, un
 }
 
 // The split of a run, from the seed kernel's counters. The width is the number of tasks ready at the
-// start, or what those release if that is more (a graph with one root and a wide second level; a
-// tile task has about eight successors that each wait for as many tasks).
+// start, or what those release if that is more (a graph with one root and a wide second level).
 __device__ __forceinline__ int run_split_log2(const SchedArgs & a, unsigned warps)
 {
     if (!a.units_done) return 0;
     if (a.units) return a.units == 8 ? 3 : a.units / 2;
-    const unsigned seeds = a.ctr[CTR_SEEDS], deg = a.ctr[CTR_SEED_DEG];
-    const unsigned pieces = seeds ? (a.ctr[CTR_SEED_PIECES] + seeds - 1) / seeds : 0;
-    int k = split_log2(max(seeds, deg / 8), a.ctr[CTR_SEED_HEAT] > 0, pieces, warps, a.min_units);
+    int k = split_log2(max(a.ctr[CTR_SEEDS], a.ctr[CTR_SEED_WIDTH] / 8), a.ctr[CTR_HEAT] != 0, min(a.period, a.ntasks), a.ctr[CTR_AXPBY],
+                       *(unsigned long long *) (a.ctr + CTR_PIECES), warps, a.min_units);
     while (k > 0 && ((uint64_t) a.ntasks << k) > 0xf0000000ull) --k;      // tickets are 32-bit
     return k;
 }
@@ -334,7 +363,7 @@ __global__ void sched_plan_kernel(SchedArgs a, unsigned warps)
     {
         const int k = run_split_log2(a, warps);
         a.ctr[CTR_SPLIT] = (unsigned) k;
-        a.ctr[CTR_TEAM] = a.allow_team && a.ctr[CTR_SEED_HEAT] > 0 && a.ctr[CTR_SEED_PIECES] == 0 && k >= TEAM_LOG2 &&
+        a.ctr[CTR_TEAM] = a.allow_team && a.ctr[CTR_SEED_HEAT] > 0 && a.ctr[CTR_AXPBY] == 0 && k >= TEAM_LOG2 &&
                           ((uint64_t) a.ctr[CTR_SEEDS] << k) <= warps;
     }
     const uint32_t W = a.ctr[CTR_SEEDS];
@@ -1601,7 +1630,7 @@ int xkb_internal_server_launch(const XkbSrvArgs & a, int grid, cudaStream_t stre
 
 int xkb_internal_split_log2(uint64_t width, uint64_t warps)
 {
-    return split_log2((unsigned) std::min<uint64_t>(width, 1u << 30), true, 0, (unsigned) warps, 1);
+    return split_log2((unsigned) std::min<uint64_t>(width, 1u << 30), true, 0, 0, 0, (unsigned) warps, 1);
 }
 
 int xkb_internal_launch_task(const xkb_task_desc_t * d, cudaStream_t stream)
