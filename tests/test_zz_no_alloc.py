@@ -111,3 +111,37 @@ def test_noalloc_rejects_unusable_time_limits(limit):
     rc = xk.lib().xkb_sched_run_noalloc(None, ctypes.byref(graph), 2, limit, None, None)
     assert rc == xk.XKB_EINVAL
     assert b"time limit" in xk.lib().xkb_last_error()
+
+
+def test_noalloc_splits_tasks_of_any_graph(torch_cuda):
+    """Tasks are split, and the caller's warps per task kept, in graphs of more than half the capacity
+    too: one axpby task over 2^26 elements before the most no-op tasks a run may have takes about as
+    long as before half as many (one warp for all of it takes many times as long)."""
+    torch = torch_cuda
+    _setup_call(torch)
+    n, ms = 1 << 26, {}
+    x = torch.rand(n, dtype=torch.float64, device="cuda") - 0.5
+    y = torch.rand(n, dtype=torch.float64, device="cuda") - 0.5
+    for ntasks in (1 << 19, 1 << 20):
+        descs = np.zeros(ntasks, dtype=xk.axpby_desc_dtype())               # no-op tasks but the first
+        for name, v in (("kind", xk.TASK_AXPBY), ("x", x.data_ptr()), ("y", y.data_ptr()), ("hi", n), ("a", 0.5), ("b", -0.25)):
+            descs[name][0] = v
+        dev = torch.from_numpy(descs.view(np.uint8).copy()).cuda()
+        # every other task follows the one before it, so the run goes through the queue
+        ptr = (torch.arange(ntasks + 1, dtype=torch.int32, device="cuda") + 1) // 2
+        succ = 2 * torch.arange(ntasks // 2, dtype=torch.int32, device="cuda") + 1
+        npred = torch.arange(ntasks, dtype=torch.int32, device="cuda") % 2
+        graph = xk.TaskGraph(ntasks, ntasks // 2, ptr.data_ptr(), succ.data_ptr(), npred.data_ptr())
+        ms[ntasks] = []
+        for _ in range(3):
+            want = (0.5 * x) + (-0.25 * y)
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            executed = ctypes.c_uint64()
+            e[0].record()
+            xk.check(xk.lib().xkb_sched_run_noalloc(dev.data_ptr(), ctypes.byref(graph), 8, 10.0,
+                                                    torch.cuda.current_stream().cuda_stream, ctypes.byref(executed)))
+            e[1].record(); e[1].synchronize()
+            assert executed.value == ntasks
+            assert torch.equal(y, want)
+            ms[ntasks].append(e[0].elapsed_time(e[1]))
+    assert min(ms[1 << 20]) < 3 * min(ms[1 << 19]), ms

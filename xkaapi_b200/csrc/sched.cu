@@ -210,8 +210,7 @@ struct SchedArgs {
     const uint32_t * xsucc;
     const uint32_t * npred_first;
     const uint32_t * npred_next;
-    int * wc;                  // wait counters
-    int * units_done;          // units of each task that ended (null: tasks are not split)
+    int * wc;                  // wait counters; in a queue run, below 0: units of the task that ended
     int * queue;
     unsigned * ctr;            // CTR_*
     uint64_t timeout_ns;
@@ -226,7 +225,6 @@ __global__ void sched_init_kernel(SchedArgs a)
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= a.ntasks) return;
     a.queue[t] = -1;
-    if (a.units_done) a.units_done[t] = 0;
     const uint32_t w = t / a.period, l = t - w * a.period;
     a.wc[t] = (int) (w == 0 ? a.npred_first[l] : a.npred_next[l]);
 }
@@ -332,7 +330,6 @@ __host__ __device__ __forceinline__ int split_log2(unsigned width, bool heat, ui
 // start, or what those release if that is more (a graph with one root and a wide second level).
 __device__ __forceinline__ int run_split_log2(const SchedArgs & a, unsigned warps)
 {
-    if (!a.units_done) return 0;
     if (a.units) return a.units == 8 ? 3 : a.units / 2;
     int k = split_log2(max(a.ctr[CTR_SEEDS], a.ctr[CTR_SEED_WIDTH] / 8), a.ctr[CTR_HEAT] != 0, min(a.period, a.ntasks), a.ctr[CTR_AXPBY],
                        *(unsigned long long *) (a.ctr + CTR_PIECES), warps, a.min_units);
@@ -644,8 +641,9 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_persisten
         {
             if (k > 0)
             {
+                // (the counter of a published task stands at 0, and counts its units from there on)
                 int last = 0;
-                if (lane == 0) last = atom_add_relaxed(a.units_done + t, 1) == nunits - 1;
+                if (lane == 0) last = atom_add_relaxed(a.wc + t, -1) == 1 - nunits;
                 if (!__shfl_sync(0xffffffffu, last, 0)) continue;
                 __syncwarp();
                 // every lane decrements counters below, so every lane fences: the other units' writes, which
@@ -789,7 +787,7 @@ struct xkb_sched {
     size_t ntasks = 0;                        // descriptors set
     unsigned bodies = XKB_BODY_ALL;           // the bodies they need
     Dev<xkb_task_desc_t> tasks;
-    Dev<int> wc, queue;                       // wc: wait counters, then the units done of each task
+    Dev<int> wc, queue;
     Dev<unsigned> ctr;
     Dev<unsigned long long> wsum;             // windows run without waiting: [0] first status, [1] executed
     cudaGraphExec_t gexec = nullptr;
@@ -936,12 +934,12 @@ static int launch_bulk(xkb_sched * S, SchedArgs & a)
     return XKB_OK;
 }
 
-// Working memory of runs of up to n tasks: wait counters and units done, queue slots, counters.
+// Working memory of runs of up to n tasks: wait counters, queue slots, counters.
 static int reserve_run(xkb_sched * S, size_t n)
 {
     if (n < 1) n = 1;
     int rc;
-    if ((rc = S->wc.reserve(2 * n)) || (rc = S->queue.reserve(n)) || (rc = S->ctr.reserve(CTR_COUNT))) return rc;
+    if ((rc = S->wc.reserve(n)) || (rc = S->queue.reserve(n)) || (rc = S->ctr.reserve(CTR_COUNT))) return rc;
     return XKB_OK;
 }
 
@@ -949,7 +947,7 @@ static SchedArgs run_args(xkb_sched * S, uint32_t ntasks, uint32_t period)
 {
     SchedArgs a;
     a.tasks = S->tasks.p; a.ntasks = ntasks; a.period = period;
-    a.wc = S->wc.p; a.units_done = S->wc.p + ntasks; a.queue = S->queue.p; a.ctr = S->ctr.p;
+    a.wc = S->wc.p; a.queue = S->queue.p; a.ctr = S->ctr.p;
     a.timeout_ns = S->timeout_ns; a.pfd = S->pfd; a.units = S->team_warps; a.min_units = S->min_units;
     a.allow_team = !S->bulk;
     return a;
@@ -1118,7 +1116,7 @@ int xkb_internal_sched_upload_window(xkb_sched_t * S, const xkb_task_desc_t * ta
 {
     if (!S || (ntasks && !tasks) || ntasks >= (size_t(1) << 31)) return xkb_set_error(XKB_EINVAL, "sched_upload_window: bad arguments");
     int rc;
-    if (ntasks > S->tasks.cap || 2 * ntasks > S->wc.cap || ntasks > S->queue.cap)
+    if (ntasks > S->tasks.cap || ntasks > S->wc.cap || ntasks > S->queue.cap)
     {
         // earlier windows may still be reading these buffers
         XKB_CUDA_TRY(cudaStreamSynchronize(S->stream));
@@ -1305,10 +1303,7 @@ extern "C" int xkb_sched_run_noalloc(const xkb_task_desc_t * tasks, const xkb_ta
     SchedArgs a;
     a.tasks = tasks; a.ntasks = n; a.period = n ? n : 1; a.succ_ptr = graph->succ_ptr; a.succ = graph->succ;
     a.xsucc_ptr = nullptr; a.xsucc = nullptr; a.npred_first = graph->npred; a.npred_next = graph->npred;
-    // the units done stand behind the wait counters where these fill half of their room at most;
-    // a larger graph runs with one warp per task
     a.wc = scratch; a.queue = scratch + XKB_NOALLOC_MAX_TASKS;
-    a.units_done = n <= XKB_NOALLOC_MAX_TASKS / 2 ? scratch + n : nullptr;
     a.units = 0; a.min_units = warps_per_task;
     a.allow_team = 1;
     a.ctr = (unsigned *) (scratch + 2 * XKB_NOALLOC_MAX_TASKS);
