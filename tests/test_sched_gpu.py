@@ -425,3 +425,37 @@ def test_split_fits_the_tasks_behind_the_first(torch_cuda, first):
     one = best_ms(sch, graph)
     sch.close()
     assert auto < 1.5 * one, (auto, one)
+
+
+@pytest.mark.parametrize("group", [20, 33, 70, 200])
+def test_many_successors_in_this_window_and_the_next(torch_cuda, group):
+    """A periodic graph whose hub task has `group` successors in its own window and as many in the
+    next one (its first `group` tasks), over a partial last window: the oracle's vectors."""
+    torch = torch_cuda
+    rng = np.random.default_rng(group)
+    m, windows, tail = 40, 7, group + 1
+    n = group * m
+    y, z, u, v = (rng.uniform(-1, 1, n) for _ in range(4))
+    dy, dz, du, dv = (torch.from_numpy(h).cuda() for h in (y, z, u, v))
+    # u += y by slices, the hub y += z, v += y by slices
+    window = [(dy, du, k * m, (k + 1) * m, 0.5, 0.75) for k in range(group)] + [(dz, dy, 0, n, -0.5, 0.75)] + \
+             [(dy, dv, k * m, (k + 1) * m, 0.25, -0.75) for k in range(group)]
+    d = np.zeros(len(window), dtype=xk.axpby_desc_dtype())
+    d["kind"] = xk.TASK_AXPBY
+    tasks = []
+    for i, (src, dst, lo, hi, a, b) in enumerate(window):
+        for name, val in (("x", src.data_ptr()), ("y", dst.data_ptr()), ("lo", lo), ("hi", hi), ("a", a), ("b", b)):
+            d[name][i] = val
+        tasks.append([("s", S.R, src.data_ptr() + 8 * lo, src.data_ptr() + 8 * hi), ("s", S.RW, dst.data_ptr() + 8 * lo, dst.data_ptr() + 8 * hi)])
+    res = xk.Resolver(); res.add(S.from_tuples(tasks * 3))
+    sch = xk.Scheduler(); sch.set_tasks(d)
+    sch.run_periodic(res.periodic(len(window)), windows, tail)
+    assert sch.wait() == (windows - 1) * len(window) + tail
+    for w in range(windows):
+        u = O.axpby(0.5, y, 0.75, u)
+        y = O.axpby(-0.5, z, 0.75, y)
+        if w + 1 < windows:
+            v = O.axpby(0.25, y, -0.75, v)
+    for got, want in ((du, u), (dy, y), (dv, v)):
+        np.testing.assert_array_equal(got.cpu().numpy(), want)
+    sch.close(); res.close()
