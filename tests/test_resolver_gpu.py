@@ -303,3 +303,25 @@ def test_region_lists_sorted_over_several_bitmaps(torch_cuda):
     n = 870 * 800
     t = np.arange(n - 870)
     np.testing.assert_array_equal(gpu_edges(diagonal(870, 0, 870, 800)), np.stack([t, t + 870], axis=1))
+
+
+@pytest.mark.parametrize("cache,blocks,passes", [("0", 40, 3), ("1", 870, 7900)])
+def test_blocks_that_are_not_kept_stay_with_their_resolver(torch_cuda, tmp_path, cache, blocks, passes):
+    """Page-locked blocks that would be unlocked when a batch gives them back -- all of them where none
+    is kept, those over 256 MB (6.9 M rects) otherwise -- serve the resolver's next batch, and
+    go with the resolver."""
+    log = run_logged(tmp_path, f"""
+r = xk.Resolver()
+for k in range(2):
+    r.add(diagonal({blocks}, k * {blocks * passes}, {blocks}, {passes}))
+    mark("added")
+assert r.graph().nedges == {blocks * (2 * passes - 1)}
+r.close()
+mark("closed")
+""", XKB_POOL_CACHE=cache)
+    added = [k for k, ln in enumerate(log) if ln == ["added"]]
+    assert any(ln[0] == "lock" for ln in log[:added[0]])
+    assert not [ln for ln in log[added[0]:added[1]] if ln[0] in ("lock", "unlock")], log
+    freed = {ln[1] for ln in log[added[1]:log.index(["closed"])] if ln[0] == "unlock"}
+    largest = max((int(ln[2]), ln[1]) for ln in log if ln[0] == "lock")
+    assert largest[1] in freed, log
