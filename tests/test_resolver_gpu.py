@@ -325,3 +325,26 @@ mark("closed")
     freed = {ln[1] for ln in log[added[1]:log.index(["closed"])] if ln[0] == "unlock"}
     largest = max((int(ln[2]), ln[1]) for ln in log if ln[0] == "lock")
     assert largest[1] in freed, log
+
+
+def test_memory_kept_for_the_next_resolver_ends_with_its_context(torch_cuda, tmp_path):
+    """The page-locked blocks and the device pool kept for the next resolver are not handed out after
+    cudaDeviceReset has ended their context: the next resolver locks blocks of its own, and works."""
+    log = run_logged(tmp_path, """
+cudart = ctypes.CDLL("libcudart.so.12")
+for k in range(3):
+    r = xk.Resolver()
+    r.add(diagonal(40, 0, 40, 500))
+    assert r.graph().nedges == 40 * 499
+    e = r.edges()
+    np.testing.assert_array_equal(e, np.stack([np.arange(len(e)), np.arange(len(e)) + 40], axis=1))
+    r.close()
+    mark("closed")
+    if k == 1:
+        assert cudart.cudaDeviceReset() == 0
+""")
+    closed = [k for k, ln in enumerate(log) if ln == ["closed"]]
+    locks = [sorted(int(ln[2]) for ln in part if ln[0] == "lock")
+             for part in (log[:closed[0]], log[closed[0]:closed[1]], log[closed[1]:])]
+    assert locks[0] and locks[1] == [] and locks[2] == locks[0], log
+    assert not [ln for ln in log[closed[1]:] if ln[0] == "unlock"], log

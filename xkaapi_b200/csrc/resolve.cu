@@ -38,6 +38,8 @@
 #include <emmintrin.h>
 #endif
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <climits>
 #include <chrono>
@@ -656,24 +658,46 @@ static inline void stream_fence()
 
 static size_t g_realloc_bytes = 0;               // device bytes allocated by reserve (trace)
 
+// Number of the CUDA context current on this thread (the device's own is made so if there is none): never
+// used twice in a process, unlike a context's address. 0: the driver cannot tell.
+static uint64_t context_id()
+{
+    typedef CUresult (*get_id_t)(CUcontext, unsigned long long *);
+    static const get_id_t get_id = [] {
+        cudaDriverEntryPointQueryResult q;
+        void * f = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            return (get_id_t) f;
+        cudaGetLastError();
+        return (get_id_t) nullptr;
+    }();
+    unsigned long long id = 0;
+    if (!get_id || get_id(nullptr, &id) == CUDA_SUCCESS) return id;
+    return cudaFree(nullptr) == cudaSuccess && get_id(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 // Device memory pool of the resolver's work buffers on the current device (made on first use).
 // Buffers only the resolver's own stream touches are allocated from it in stream order, so
 // growing one neither waits for the whole device (as cudaFree does) nor asks the driver for
 // memory while copies and kernels of other streams run: a runtime streaming windows of tasks
 // had its resolution stall for up to 0.3 s in cudaMalloc / cudaFree of a domain's cell states.
 // Freed memory stays in the pool for the next resolver of the process, up to 4 GiB
-// (XKB_POOL_CACHE=0: none).
+// (XKB_POOL_CACHE=0: none). A pool ends with its context (cudaDeviceReset), and the next context of the
+// device gets one of its own.
 static cudaMemPool_t resolver_pool()
 {
     static std::mutex mu;
     static cudaMemPool_t pools[256];
     static bool made[256];
+    static uint64_t ctx[256];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 256) { cudaGetLastError(); return nullptr; }
+    const uint64_t now = context_id();
     std::lock_guard<std::mutex> lk(mu);
-    if (!made[dev])
+    if (!made[dev] || ctx[dev] != now)
     {
         made[dev] = true;
+        ctx[dev] = now;
         cudaMemPoolProps props;
         memset(&props, 0, sizeof(props));
         props.allocType = cudaMemAllocationTypePinned;
@@ -699,25 +723,33 @@ static cudaMemPool_t resolver_pool()
 // stream of batches finds its blocks again whatever an earlier one left: unlocking and locking 64 MB
 // behind a running window costs 35 to 90 ms a batch (16384^2 x 500 heat graph spawned through the C API:
 // 1.6 to 2.7 s to the end of the wait when a 128 MB block no batch asked for filled the room, 0.63 s now).
+// Blocks end with the context they were made in (cudaDeviceReset), so each context has its own, and those of
+// one that ended are neither handed out nor unlocked again.
 class PinnedBlocks {
 public:
     static constexpr size_t PINNED_KEEP = size_t(256) << 20, MIN_BLOCK = size_t(1) << 18;
 
-    static int take(size_t bytes, void ** p, size_t * cap)
+    static int take(size_t bytes, void ** p, size_t * cap, uint64_t * ctx)
     {
         size_t c = MIN_BLOCK;
         while (c < bytes) c *= 2;
+        *ctx = context_id();
+        std::vector<void *> due;
         {
             std::lock_guard<std::mutex> lk(mu());
-            auto it = free_blocks().lower_bound(c);
-            if (it != free_blocks().end() && it->first <= 4 * c)
+            Kept & k = kept(*ctx);
+            due.swap(k.due);
+            auto it = k.blocks.lower_bound(c);
+            if (it != k.blocks.end() && it->first <= 4 * c)
             {
                 *p = it->second; *cap = it->first;
-                kept() -= it->first;
-                free_blocks().erase(it);
-                return XKB_OK;
+                k.bytes -= it->first;
+                k.blocks.erase(it);
             }
+            else *p = nullptr;
         }
+        unlock(due);
+        if (*p) return XKB_OK;
         cudaError_t e = cudaHostAlloc(p, c, cudaHostAllocPortable);
         if (e != cudaSuccess) { *p = nullptr; return xkb_set_cuda_error(e); }
         *cap = c;
@@ -729,32 +761,38 @@ public:
         static const bool none = getenv("XKB_POOL_CACHE") && atoi(getenv("XKB_POOL_CACHE")) == 0;
         return !none && cap <= PINNED_KEEP;
     }
-    static void give(void * p, size_t cap)
+    static void give(void * p, size_t cap, uint64_t ctx)
     {
         if (!p) return;
-        std::vector<void *> out;
-        if (!keeps(cap)) out.push_back(p);
-        else
+        const bool current = ctx == context_id();
+        std::vector<void *> due;
         {
             std::lock_guard<std::mutex> lk(mu());
-            free_blocks().emplace(cap, p);
-            kept() += cap;
-            while (kept() > PINNED_KEEP)                         // (the block just given is the last to go)
+            Kept & k = kept(ctx);
+            if (!keeps(cap)) k.due.push_back(p);
+            else
             {
-                auto it = std::prev(free_blocks().end());
-                if (it->second == p) --it;
-                kept() -= it->first;
-                out.push_back(it->second);
-                free_blocks().erase(it);
+                k.blocks.emplace(cap, p);
+                k.bytes += cap;
+                while (k.bytes > PINNED_KEEP)                    // (the block just given is the last to go)
+                {
+                    auto it = std::prev(k.blocks.end());
+                    if (it->second == p) --it;
+                    k.bytes -= it->first;
+                    k.due.push_back(it->second);
+                    k.blocks.erase(it);
+                }
             }
+            if (current) due.swap(k.due);                        // (else when the context is current again)
         }
-        for (void * q : out) cudaFreeHost(q);
+        unlock(due);
     }
 
 private:                                        // (never destroyed: resolvers may outlive static objects)
+    struct Kept { std::multimap<size_t, void *> blocks; size_t bytes = 0; std::vector<void *> due; };
     static std::mutex & mu() { static std::mutex * m = new std::mutex; return *m; }
-    static std::multimap<size_t, void *> & free_blocks() { static auto * f = new std::multimap<size_t, void *>; return *f; }
-    static size_t & kept() { static size_t k = 0; return k; }
+    static void unlock(const std::vector<void *> & due) { for (void * q : due) cudaFreeHost(q); }     // (may wait for the device)
+    static Kept & kept(uint64_t ctx) { static auto * k = new std::map<uint64_t, Kept>; return (*k)[ctx]; }
 };
 
 template <typename T>
@@ -911,18 +949,19 @@ struct Domain {
 struct PinnedBlock {
     uint8_t * p = nullptr;
     size_t cap = 0;
+    uint64_t ctx = 0;
     PinnedBlock() = default;
     PinnedBlock(const PinnedBlock &) = delete;
     PinnedBlock & operator=(const PinnedBlock &) = delete;
     ~PinnedBlock() { drop(); }
-    void drop() { PinnedBlocks::give(p, cap); p = nullptr; cap = 0; }
+    void drop() { PinnedBlocks::give(p, cap, ctx); p = nullptr; cap = 0; }
     void rest() { if (PinnedBlocks::keeps(cap)) drop(); }
     // at least n bytes; what the block held is gone
     int take(size_t n)
     {
         if (p && n <= cap) return XKB_OK;
         drop();
-        return PinnedBlocks::take(n, (void **) &p, &cap);
+        return PinnedBlocks::take(n, (void **) &p, &cap, &ctx);
     }
 };
 
