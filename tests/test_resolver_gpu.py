@@ -348,3 +348,22 @@ for k in range(3):
              for part in (log[:closed[0]], log[closed[0]:closed[1]], log[closed[1]:])]
     assert locks[0] and locks[1] == [] and locks[2] == locks[0], log
     assert not [ln for ln in log[closed[1]:] if ln[0] == "unlock"], log
+
+
+def test_page_locked_memory_is_given_back_with_the_last_resolver(torch_cuda, tmp_path):
+    """Blocks kept for the next batch are unlocked when the last resolver goes, all but 64 MB."""
+    log = run_logged(tmp_path, """
+first, second = xk.Resolver(), xk.Resolver()
+first.add(diagonal(870, 0, 870, 2000))             # 70 MB of rects: a block of 128 MB
+first.close()
+mark("one")
+second.add(diagonal(40, 0, 40, 3))
+second.close()
+mark("none")
+""")
+    sizes = {ln[1]: int(ln[2]) for ln in log if ln[0] == "lock"}
+    left = log.index(["one"])
+    assert max(sizes.values()) == 128 << 20
+    assert not [ln for ln in log[:left] if ln[0] == "unlock"], log
+    held = sum(sizes.values()) - sum(sizes[ln[1]] for ln in log if ln[0] == "unlock" and ln[1] in sizes)
+    assert held <= 64 << 20, log

@@ -718,7 +718,7 @@ static cudaMemPool_t resolver_pool()
 // its read-backs and gives them back when it has been waited for, so a resolver holds none between
 // batches and a new one finds them there (page-locking costs about 0.5 ms per MB and waits for the
 // device; a server keeps a resolver per graph shape). Given-back blocks are kept up to PINNED_KEEP
-// bytes (XKB_POOL_CACHE=0: none); a block in use belongs to one batch. A block up to four times the size
+// bytes while there are resolvers, and PINNED_REST once there is none (XKB_POOL_CACHE=0: none); a block in use belongs to one batch. A block up to four times the size
 // asked for will do, and a block given back displaces larger ones rather than being unlocked, so a
 // stream of batches finds its blocks again whatever an earlier one left: unlocking and locking 64 MB
 // behind a running window costs 35 to 90 ms a batch (16384^2 x 500 heat graph spawned through the C API:
@@ -727,7 +727,7 @@ static cudaMemPool_t resolver_pool()
 // one that ended are neither handed out nor unlocked again.
 class PinnedBlocks {
 public:
-    static constexpr size_t PINNED_KEEP = size_t(256) << 20, MIN_BLOCK = size_t(1) << 18;
+    static constexpr size_t PINNED_KEEP = size_t(256) << 20, PINNED_REST = size_t(64) << 20, MIN_BLOCK = size_t(1) << 18;
 
     static int take(size_t bytes, void ** p, size_t * cap, uint64_t * ctx)
     {
@@ -774,22 +774,46 @@ public:
             {
                 k.blocks.emplace(cap, p);
                 k.bytes += cap;
-                while (k.bytes > PINNED_KEEP)                    // (the block just given is the last to go)
-                {
-                    auto it = std::prev(k.blocks.end());
-                    if (it->second == p) --it;
-                    k.bytes -= it->first;
-                    k.due.push_back(it->second);
-                    k.blocks.erase(it);
-                }
+                k.keep(k.resolvers ? PINNED_KEEP : PINNED_REST, p);
             }
             if (current) due.swap(k.due);                        // (else when the context is current again)
         }
         unlock(due);
     }
 
+    // A resolver of context ctx begins, and ends.
+    static void enter(uint64_t ctx) { std::lock_guard<std::mutex> lk(mu()); ++kept(ctx).resolvers; }
+    static void leave(uint64_t ctx)
+    {
+        const bool current = ctx == context_id();
+        std::vector<void *> due;
+        {
+            std::lock_guard<std::mutex> lk(mu());
+            Kept & k = kept(ctx);
+            if (--k.resolvers == 0) k.keep(PINNED_REST, nullptr);
+            if (current) due.swap(k.due);
+        }
+        unlock(due);
+    }
+
 private:                                        // (never destroyed: resolvers may outlive static objects)
-    struct Kept { std::multimap<size_t, void *> blocks; size_t bytes = 0; std::vector<void *> due; };
+    struct Kept {
+        std::multimap<size_t, void *> blocks;
+        size_t bytes = 0, resolvers = 0;
+        std::vector<void *> due;                                 // to be unlocked
+        // the smallest blocks, `limit` bytes of them at most; `last` is the last to go
+        void keep(size_t limit, void * last)
+        {
+            while (bytes > limit)
+            {
+                auto it = std::prev(blocks.end());
+                if (it->second == last && it != blocks.begin()) --it;
+                bytes -= it->first;
+                due.push_back(it->second);
+                blocks.erase(it);
+            }
+        }
+    };
     static std::mutex & mu() { static std::mutex * m = new std::mutex; return *m; }
     static void unlock(const std::vector<void *> & due) { for (void * q : due) cudaFreeHost(q); }     // (may wait for the device)
     static Kept & kept(uint64_t ctx) { static auto * k = new std::map<uint64_t, Kept>; return (*k)[ctx]; }
@@ -972,6 +996,7 @@ struct HostStage {
     HOp * ops() { return (HOp *) block.p; }
     int take(size_t n) { return block.take(n * sizeof(HOp)); }
     void rest() { block.rest(); }
+    void drop() { block.drop(); }
 };
 
 // Page-locked host memory for what the device reports back and for the small arrays it is given, so
@@ -982,6 +1007,7 @@ struct HostScratch {
     PinnedBlock block;
     size_t used = 0;
     void rest() { block.rest(); }
+    void drop() { block.drop(); }
     uint64_t * results() { return (uint64_t *) block.p; }
     uint64_t * keys(int axis) { return (uint64_t *) (block.p + RESULTS) + axis * KEYS; }
     void release() { used = RESULTS + 2 * KEYS * sizeof(uint64_t); }
@@ -1052,7 +1078,14 @@ struct xkb_resolver {
     double uniq_per_op = 8.0;                   // unique-pair estimate per op
     HostScratch host;
     cudaEvent_t ev[2] = {nullptr, nullptr};     // around the last batch
-    ~xkb_resolver() { for (cudaEvent_t e : ev) if (e) cudaEventDestroy(e); }
+    const uint64_t ctx = context_id();
+    xkb_resolver() { PinnedBlocks::enter(ctx); }
+    ~xkb_resolver()
+    {
+        for (cudaEvent_t e : ev) if (e) cudaEventDestroy(e);
+        host.drop(); stage.drop();
+        PinnedBlocks::leave(ctx);
+    }
     // parallel host passes (validation, op build): the host team and the page-locked staging buffer
     std::unique_ptr<WorkPool> pool;
     HostStage stage;
