@@ -352,10 +352,15 @@ __device__ __forceinline__ int run_split_log2(const SchedArgs & a, unsigned warp
 // takes one off, so the task may run at n - n * 2^k.
 constexpr unsigned INORDER_MAX_NPRED = 1u << 20;      // keeps that inside an int
 
-__global__ void sched_plan_kernel(SchedArgs a, unsigned warps)
+// Successor lists are looked at by their task's thread up to PLAN_LIST entries, and past them by the
+// whole warp (60,000 successors of one task by one thread: 4 ms before the run).
+constexpr uint32_t PLAN_LIST = 32;
+
+__global__ void __launch_bounds__(256) sched_plan_kernel(SchedArgs a, unsigned warps)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= a.period) return;
+    const uint32_t lane = threadIdx.x & 31;
+    const bool mine = t < a.period;
     if (t == 0)
     {
         const int k = run_split_log2(a, warps);
@@ -364,22 +369,41 @@ __global__ void sched_plan_kernel(SchedArgs a, unsigned warps)
                           ((uint64_t) a.ctr[CTR_SEEDS] << k) <= warps;
     }
     const uint32_t W = a.ctr[CTR_SEEDS];
-    bool ok = W > 0 && a.ctr[CTR_SEED_LAST] == W && (a.xsucc_ptr == nullptr || a.period % W == 0);
-    if (ok)
+    const bool level = W > 0 && a.ctr[CTR_SEED_LAST] == W && (a.xsucc_ptr == nullptr || a.period % W == 0);   // (the same for every thread)
+    bool ok = level;
+    if (level)
     {
-        ok = a.npred_first[t] < INORDER_MAX_NPRED && a.npred_next[t] < INORDER_MAX_NPRED;
         const uint64_t next = (uint64_t) t + W;                // the task a block later: in this window, or in the one after it
         bool chained = next >= a.ntasks;
-        for (uint32_t i = a.succ_ptr[t], e = a.succ_ptr[t + 1], b = t / W; i < e; ++i)
+        const uint32_t b = mine ? a.succ_ptr[t] : 0u, e = mine ? a.succ_ptr[t + 1] : 0u;
+        if (mine) ok = a.npred_first[t] < INORDER_MAX_NPRED && a.npred_next[t] < INORDER_MAX_NPRED;
+        for (uint32_t i = b, n = min(e, b + PLAN_LIST), blk = t / W; i < n; ++i)
         {
             const uint32_t s = a.succ[i];
-            ok = ok && s / W > b;
+            ok = ok && s / W > blk;
             chained = chained || s == next;
         }
-        if (!chained && next >= a.period && a.xsucc_ptr)
-            for (uint32_t i = a.xsucc_ptr[t], e = a.xsucc_ptr[t + 1]; i < e; ++i) chained = chained || a.xsucc[i] + (uint64_t) a.period == next;
+        for (unsigned rest = __ballot_sync(0xffffffffu, e - b > PLAN_LIST); rest; rest &= rest - 1)
+        {
+            const int src = __ffs(rest) - 1;
+            const uint32_t lt = t - lane + (uint32_t) src, lb = __shfl_sync(0xffffffffu, b, src), le = __shfl_sync(0xffffffffu, e, src);
+            bool lok = true, lchained = false;
+#pragma unroll 4
+            for (uint32_t i = lb + PLAN_LIST + lane; i < le; i += 32)
+            {
+                const uint32_t s = a.succ[i];
+                lok = lok && s / W > lt / W;
+                lchained = lchained || s == (uint64_t) lt + W;
+            }
+            lok = __all_sync(0xffffffffu, lok);
+            lchained = __any_sync(0xffffffffu, lchained);
+            if ((int) lane == src) { ok = ok && lok; chained = chained || lchained; }
+        }
+        if (mine && !chained && next >= a.period && a.xsucc_ptr)
+            for (uint32_t i = a.xsucc_ptr[t], n = a.xsucc_ptr[t + 1]; i < n && !chained; ++i) chained = a.xsucc[i] + (uint64_t) a.period == next;
         ok = ok && chained;
     }
+    if (!mine) return;
     if (!ok && *(volatile unsigned *) (a.ctr + CTR_QUEUE) == 0) atomicExch(a.ctr + CTR_QUEUE, 1u);
     // the first place among the ready tasks where the tiles' rows change (block_order); ~ so that 0 is none
     if (ok && t + 1 < W && a.ctr[CTR_SEED_HEAT] == W && a.tasks[t].u.heat.x0 != a.tasks[t + 1].u.heat.x0)
