@@ -481,3 +481,43 @@ def test_many_successors_of_one_task(torch_cuda):
             ms.append(e[0].elapsed_time(e[1]))
     sch.close()
     assert min(ms[1:]) < 3.2, ms
+
+
+@pytest.mark.parametrize("skip", [0, 20, 61])
+def test_graphs_that_begin_inside_a_step_run_in_order(torch_cuda, skip):
+    """A heat graph without its first tasks, as a runtime hands it over in windows: where its first tasks are
+    the ones ready at the start (some of the second step's last tiles are too when the first step is nearly
+    done) it is taken in spawn order like the whole graph, about twice as fast as the queue (11 against 5
+    us a step), and it ends with the oracle's grids."""
+    torch = torch_cuda
+    n, ts, steps = 1024, 128, 60
+    g = O.heat_init(n, n, seed=3)
+    after = O.heat_run(g, n, n, 1, C)
+    r = xk.Resolver()
+    r.add(xk.heat_access_records(n, n, ts, ts, 0, steps, 1 << 40, 1 << 41))
+    e = r.edges().astype(np.int64)
+    r.close()
+    times = {}
+    for extra in (0, 1):                       # a no-op task more, ready at the start behind all others: the queue
+        a, b = torch.from_numpy(g).cuda(), torch.from_numpy(g).cuda()
+        d = xk.heat_task_descs((a.data_ptr(), b.data_ptr()), n, n, n, ts, ts, steps, C)[skip:]
+        d = np.concatenate([d, np.zeros(extra, dtype=d.dtype)])
+        for t in range(skip):                  # the skipped tiles are there already
+            x, y = t // 8 * ts, t % 8 * ts
+            b[y:y + ts, x:x + ts] = torch.from_numpy(np.ascontiguousarray(after[y:y + ts, x:x + ts])).cuda()
+        edges = e[(e >= skip).all(axis=1)] - skip
+        edges = edges[np.lexsort((edges[:, 1], edges[:, 0]))]
+        ptr = np.concatenate([[0], np.cumsum(np.bincount(edges[:, 0], minlength=len(d)))])
+        npred = np.bincount(edges[:, 1], minlength=len(d))
+        keep = [torch.from_numpy(w.astype(np.int32)).cuda() for w in (ptr, edges[:, 1], npred)]
+        graph = xk.TaskGraph(len(d), len(edges), *(w.data_ptr() for w in keep))
+        sch = xk.Scheduler(); sch.set_tasks(d); sch.run(graph)
+        assert sch.wait() == len(d)
+        np.testing.assert_array_equal(a.cpu().numpy(), O.heat_run(g, n, n, steps, C))
+        if not extra:
+            ready = np.flatnonzero(npred == 0)
+            first = np.array_equal(ready, np.arange(len(ready)))
+        times[extra] = best_ms(sch, graph)
+        sch.close()
+    assert first == (skip != 61)
+    assert not first or times[0] < 0.75 * times[1], times

@@ -192,9 +192,11 @@ __device__ __forceinline__ int atom_add_acq_rel(int * p, int v)
 // executed; then what the seed kernel learnt about the tasks that are ready at the start, and of the kinds
 // of all tasks (CTR_PIECES: 64 bits).
 // Head and tail have cache lines of their own: every warp's ticket and every release is an atomic there.
-// CTR_EXECUTED counts units of an in-order run, tasks of a queue run (executed_tasks).
+// CTR_EXECUTED counts units of an in-order run, tasks of a queue run (executed_tasks); a run goes in order
+// when the plan kernel has left CTR_QUEUE and CTR_NEAR at 0 (run_in_order).
 enum { CTR_HEAD = 0, CTR_TAIL = 32, CTR_STATUS = 48, CTR_EXECUTED, CTR_BAD_TASK, CTR_SEEDS, CTR_SEED_LAST, CTR_SEED_WIDTH, CTR_SEED_HEAT,
-       CTR_HEAT, CTR_PIECES, CTR_PIECES_HI, CTR_AXPBY, CTR_QUEUE, CTR_SPLIT, CTR_TEAM, CTR_RUN, CTR_COUNT = 64 };
+       CTR_HEAT, CTR_PIECES, CTR_PIECES_HI, CTR_AXPBY, CTR_QUEUE, CTR_NEAR, CTR_SPLIT, CTR_TEAM, CTR_RUN, CTR_COUNT };
+static_assert(CTR_COUNT <= 64, "the no-allocation run's array has 64");
 static_assert(CTR_PIECES % 2 == 0, "64 bits");
 
 // A run covers `ntasks` tasks numbered w * period + t (window w, task t of the window's
@@ -339,15 +341,15 @@ __device__ __forceinline__ int run_split_log2(const SchedArgs & a, unsigned warp
 
 // Chooses the order of the run. Let W be the number of tasks ready at the start. The run goes in
 // order when those are tasks 0 .. W-1, every edge leads from one block of W consecutive tasks to a
-// later one, and every task t is a predecessor of task t + W (a heat tile, of the same tile a step
-// later). Then the graph is W chains that advance side by side: no more than W tasks are ever ready at a
-// time, and the tasks of a block are independent of one another, so spawn order keeps as many tasks
-// runnable as the queue could. (Without the last condition a graph with one root passes whatever
-// follows: 64 chains of 100 tiles behind a common first task, spawned chain by chain, ran one after
-// another, 10.4 ms against 5.7 through the queue.) In order, nothing is published, a warp knows its
-// task -- descriptor and successors -- before it may run, and every unit decrements its successors
-// itself, without waiting for the answer: 15.6 us per step of the 2048^2 FP64 graph against 19.6
-// through the queue with the same units, and 174 against 180 for 8192^2.
+// later one, and every other task has a predecessor at most 2 W tasks before it (a heat tile, the same tile a
+// step earlier, in graphs that begin inside a step too). Then the tasks of a block are independent
+// of one another, and no task is ready more than 2 W tasks behind the last one taken, so spawn order keeps
+// about as many tasks runnable as the queue could. (Without the last condition a graph with one root
+// passes whatever follows: 64 chains of 100 tiles behind a common first task, spawned chain by chain,
+// ran one after another, 10.4 ms against 5.7 through the queue.) In order, nothing is published, a warp
+// knows its task -- descriptor and successors -- before it may run, and every unit decrements its
+// successors itself, without waiting for the answer: 13.0 us per step of the 2048^2 FP64 graph against
+// 18.5 through the queue with the same units, 176 against 187 for 8192^2, 661 against 725 for 16384^2.
 // In order, a counter starts at the task's number of predecessors n and every one of their 2^k units
 // takes one off, so the task may run at n - n * 2^k.
 constexpr unsigned INORDER_MAX_NPRED = 1u << 20;      // keeps that inside an int
@@ -373,35 +375,41 @@ __global__ void __launch_bounds__(256) sched_plan_kernel(SchedArgs a, unsigned w
     bool ok = level;
     if (level)
     {
-        const uint64_t next = (uint64_t) t + W;                // the task a block later: in this window, or in the one after it
-        bool chained = next >= a.ntasks;
+        // tasks found to have a near predecessor are marked in the queue, whose places from W on are still
+        // empty (anything below 0); CTR_NEAR ends at 0 when all of them were
+        __shared__ unsigned marked;
+        if (threadIdx.x == 0) marked = 0;
+        __syncthreads();
+        const uint32_t own = min(a.period, a.ntasks), ahead = a.ntasks > a.period ? min(W, a.ntasks - a.period) : 0u;
+        if (t == 0) atomicSub(a.ctr + CTR_NEAR, (own > W ? own - W : 0u) + ahead);
+        unsigned near = 0;
+        auto mark = [&](uint32_t from, uint32_t to) {
+            if (to - from <= 2 * (uint64_t) W && *(volatile int *) (a.queue + to) == -1 && atomicExch(a.queue + to, -2) == -1) ++near;
+        };
+        auto edge = [&](uint32_t from, uint32_t to) -> bool {
+            const bool later = to / W > from / W;
+            if (later && to < own) mark(from, to);
+            return later;
+        };
         const uint32_t b = mine ? a.succ_ptr[t] : 0u, e = mine ? a.succ_ptr[t + 1] : 0u;
         if (mine) ok = a.npred_first[t] < INORDER_MAX_NPRED && a.npred_next[t] < INORDER_MAX_NPRED;
-        for (uint32_t i = b, n = min(e, b + PLAN_LIST), blk = t / W; i < n; ++i)
-        {
-            const uint32_t s = a.succ[i];
-            ok = ok && s / W > blk;
-            chained = chained || s == next;
-        }
+        for (uint32_t i = b, n = min(e, b + PLAN_LIST); i < n; ++i) ok = edge(t, a.succ[i]) && ok;
         for (unsigned rest = __ballot_sync(0xffffffffu, e - b > PLAN_LIST); rest; rest &= rest - 1)
         {
             const int src = __ffs(rest) - 1;
             const uint32_t lt = t - lane + (uint32_t) src, lb = __shfl_sync(0xffffffffu, b, src), le = __shfl_sync(0xffffffffu, e, src);
-            bool lok = true, lchained = false;
-#pragma unroll 4
-            for (uint32_t i = lb + PLAN_LIST + lane; i < le; i += 32)
-            {
-                const uint32_t s = a.succ[i];
-                lok = lok && s / W > lt / W;
-                lchained = lchained || s == (uint64_t) lt + W;
-            }
+            bool lok = true;
+            for (uint32_t i = lb + PLAN_LIST + lane; i < le; i += 32) lok = edge(lt, a.succ[i]) && lok;
             lok = __all_sync(0xffffffffu, lok);
-            lchained = __any_sync(0xffffffffu, lchained);
-            if ((int) lane == src) { ok = ok && lok; chained = chained || lchained; }
+            if ((int) lane == src) ok = ok && lok;
         }
-        if (mine && !chained && next >= a.period && a.xsucc_ptr)
-            for (uint32_t i = a.xsucc_ptr[t], n = a.xsucc_ptr[t + 1]; i < n && !chained; ++i) chained = a.xsucc[i] + (uint64_t) a.period == next;
-        ok = ok && chained;
+        // into the next window: its first W tasks have no predecessor in their own
+        if (mine && a.xsucc_ptr && ahead && t + 2 * (uint64_t) W >= a.period)
+            for (uint32_t i = a.xsucc_ptr[t], n = a.xsucc_ptr[t + 1]; i < n; ++i)
+                if (a.xsucc[i] < ahead) mark(t, a.period + a.xsucc[i]);
+        if (near) atomicAdd(&marked, near);
+        __syncthreads();
+        if (threadIdx.x == 0 && marked) atomicAdd(a.ctr + CTR_NEAR, marked);
     }
     if (!mine) return;
     if (!ok && *(volatile unsigned *) (a.ctr + CTR_QUEUE) == 0) atomicExch(a.ctr + CTR_QUEUE, 1u);
@@ -437,13 +445,16 @@ struct BlockOrder {
     }
 };
 
+// Whether the run goes in order, from its counters.
+__host__ __device__ __forceinline__ bool run_in_order(const unsigned * ctr) { return ctr[CTR_QUEUE] == 0 && ctr[CTR_NEAR] == 0; }
+
 // Whether sched_team_kernel has the run.
-__device__ __forceinline__ bool team_run(const SchedArgs & a) { return a.ctr[CTR_TEAM] != 0 && a.ctr[CTR_QUEUE] == 0; }
+__device__ __forceinline__ bool team_run(const SchedArgs & a) { return a.ctr[CTR_TEAM] != 0 && run_in_order(a.ctr); }
 
 // Tasks run, from the counters of a run that ended.
 __host__ __device__ __forceinline__ unsigned executed_tasks(const unsigned * ctr)
 {
-    return ctr[CTR_QUEUE] ? ctr[CTR_EXECUTED] : ctr[CTR_EXECUTED] >> ctr[CTR_SPLIT];
+    return run_in_order(ctr) ? ctr[CTR_EXECUTED] >> ctr[CTR_SPLIT] : ctr[CTR_EXECUTED];
 }
 
 __device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
@@ -616,7 +627,7 @@ __global__ void __launch_bounds__(SCHED_THREADS, XKB_SCHED_MINB) sched_persisten
     constexpr int NWARPS = SCHED_THREADS / 32;
     extern __shared__ __align__(128) unsigned char bulk_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool inorder = a.ctr[CTR_QUEUE] == 0;
+    const bool inorder = run_in_order(a.ctr);
     const int k = (int) a.ctr[CTR_SPLIT];
     const int nunits = 1 << k;
     unsigned executed = 0;
