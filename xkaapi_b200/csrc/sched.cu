@@ -190,7 +190,7 @@ __device__ __forceinline__ int atom_add_acq_rel(int * p, int v)
 
 // Counters of a run (device memory): ready-queue tickets and tasks published, status, tasks
 // executed; then what the seed kernel learnt about the tasks that are ready at the start, and of the kinds
-// of all tasks (CTR_PIECES: 64 bits).
+// of all tasks (CTR_HEAT, CTR_AXPBY, CTR_PIECES of 64 bits; only where there may be axpby tasks).
 // Head and tail have cache lines of their own: every warp's ticket and every release is an atomic there.
 // CTR_EXECUTED counts units of an in-order run, tasks of a queue run (executed_tasks); a run goes in order
 // when the plan kernel has left CTR_QUEUE and CTR_NEAR at 0 (run_in_order).
@@ -218,6 +218,7 @@ struct SchedArgs {
     uint64_t timeout_ns;
     int pfd;                   // L2 prefetch distance of the tile bodies, in columns
     int allow_team;            // narrow graphs may go to sched_team_kernel
+    unsigned bodies;           // the bodies the tasks need (XKB_BODY_*), as far as the host knows
     int units;                 // the caller's warps per task (xkb_sched_set_team): this many units; 0: chosen here,
     int min_units;             // at least this many
 };
@@ -255,23 +256,28 @@ __global__ void __launch_bounds__(256) sched_seed_kernel(SchedArgs a)
     const uint32_t lane = threadIdx.x & 31;
     const bool ok = *(volatile unsigned *) (a.ctr + CTR_STATUS) == 0;   // a check before the run failed: nothing becomes ready
     const uint32_t w = t / a.period, l = t - w * a.period;
+    const bool seed = ok && t < a.ntasks && (w == 0 ? a.npred_first[l] : a.npred_next[l]) == 0;
+    const bool scan = a.bodies & XKB_BODY_AXPBY;           // (the host knows of heat tiles alone: no look at each task)
     bool heat = false;
     unsigned pieces = 0;
-    if (t < a.period && t < a.ntasks)
+    if (seed || (scan && t < a.period && t < a.ntasks))
     {
-        const xkb_task_desc_t & d = a.tasks[t];
+        const xkb_task_desc_t & d = a.tasks[l];
         heat = d.kind == XKB_TASK_HEAT_F64 || d.kind == XKB_TASK_HEAT_F32;
-        if (d.kind == XKB_TASK_AXPBY) pieces = (unsigned) max(min((d.u.axpby.hi - d.u.axpby.lo + AXPBY_PIECE - 1) / AXPBY_PIECE, (int64_t) 65536), (int64_t) 1);
+        if (scan && w == 0 && d.kind == XKB_TASK_AXPBY)
+            pieces = (unsigned) max(min((d.u.axpby.hi - d.u.axpby.lo + AXPBY_PIECE - 1) / AXPBY_PIECE, (int64_t) 65536), (int64_t) 1);
     }
-    if (__syncthreads_or(heat) && threadIdx.x == 0 && *(volatile unsigned *) (a.ctr + CTR_HEAT) == 0) atomicExch(a.ctr + CTR_HEAT, 1u);
-    const int naxpby = __syncthreads_count(pieces > 0);
-    if (naxpby)
+    if (scan)
     {
-        const unsigned sum = __reduce_add_sync(0xffffffffu, pieces);
-        if (lane == 0 && sum) atomicAdd((unsigned long long *) (a.ctr + CTR_PIECES), (unsigned long long) sum);
-        if (threadIdx.x == 0) atomicAdd(a.ctr + CTR_AXPBY, (unsigned) naxpby);
+        if (__syncthreads_or(heat) && threadIdx.x == 0 && *(volatile unsigned *) (a.ctr + CTR_HEAT) == 0) atomicExch(a.ctr + CTR_HEAT, 1u);
+        const int naxpby = __syncthreads_count(pieces > 0);
+        if (naxpby)
+        {
+            const unsigned sum = __reduce_add_sync(0xffffffffu, pieces);
+            if (lane == 0 && sum) atomicAdd((unsigned long long *) (a.ctr + CTR_PIECES), (unsigned long long) sum);
+            if (threadIdx.x == 0) atomicAdd(a.ctr + CTR_AXPBY, (unsigned) naxpby);
+        }
     }
-    const bool seed = ok && t < a.ntasks && (w == 0 ? a.npred_first[l] : a.npred_next[l]) == 0;
     const unsigned m = __ballot_sync(0xffffffffu, seed);
     if (!m) return;
     const unsigned width = __reduce_add_sync(0xffffffffu, seed ? seed_width(a, l) : 0u);
@@ -333,7 +339,8 @@ __host__ __device__ __forceinline__ int split_log2(unsigned width, bool heat, ui
 __device__ __forceinline__ int run_split_log2(const SchedArgs & a, unsigned warps)
 {
     if (a.units) return a.units == 8 ? 3 : a.units / 2;
-    int k = split_log2(max(a.ctr[CTR_SEEDS], a.ctr[CTR_SEED_WIDTH] / 8), a.ctr[CTR_HEAT] != 0, min(a.period, a.ntasks), a.ctr[CTR_AXPBY],
+    const bool heat = a.bodies & XKB_BODY_AXPBY ? a.ctr[CTR_HEAT] != 0 : (a.bodies & XKB_BODY_ALL) != 0;
+    int k = split_log2(max(a.ctr[CTR_SEEDS], a.ctr[CTR_SEED_WIDTH] / 8), heat, min(a.period, a.ntasks), a.ctr[CTR_AXPBY],
                        *(unsigned long long *) (a.ctr + CTR_PIECES), warps, a.min_units);
     while (k > 0 && ((uint64_t) a.ntasks << k) > 0xf0000000ull) --k;      // tickets are 32-bit
     return k;
@@ -357,6 +364,7 @@ constexpr unsigned INORDER_MAX_NPRED = 1u << 20;      // keeps that inside an in
 // Successor lists are looked at by their task's thread up to PLAN_LIST entries, and past them by the
 // whole warp (60,000 successors of one task by one thread: 4 ms before the run).
 constexpr uint32_t PLAN_LIST = 32;
+constexpr int PLAN_BATCH = 12;           // successors looked at together (a tile has 9)
 
 __global__ void __launch_bounds__(256) sched_plan_kernel(SchedArgs a, unsigned warps)
 {
@@ -383,30 +391,62 @@ __global__ void __launch_bounds__(256) sched_plan_kernel(SchedArgs a, unsigned w
         const uint32_t own = min(a.period, a.ntasks), ahead = a.ntasks > a.period ? min(W, a.ntasks - a.period) : 0u;
         if (t == 0) atomicSub(a.ctr + CTR_NEAR, (own > W ? own - W : 0u) + ahead);
         unsigned near = 0;
-        auto mark = [&](uint32_t from, uint32_t to) {
-            if (to - from <= 2 * (uint64_t) W && *(volatile int *) (a.queue + to) == -1 && atomicExch(a.queue + to, -2) == -1) ++near;
+        // marks the near ones among N tasks behind `from`; every load is under way before one is looked at, and so
+        // is every exchange (one edge after the other: 5 us more before each run)
+        auto mark = [&](uint32_t from, const uint32_t (&to)[PLAN_BATCH], unsigned which) {
+            int q[PLAN_BATCH];
+#pragma unroll
+            for (int j = 0; j < PLAN_BATCH; ++j) q[j] = which >> j & 1u && to[j] - from <= 2 * (uint64_t) W ? *(volatile int *) (a.queue + to[j]) : 0;
+#pragma unroll
+            for (int j = 0; j < PLAN_BATCH; ++j) q[j] = q[j] == -1 ? atomicExch(a.queue + to[j], -2) : 0;
+#pragma unroll
+            for (int j = 0; j < PLAN_BATCH; ++j) near += q[j] == -1;
         };
-        auto edge = [&](uint32_t from, uint32_t to) -> bool {
-            const bool later = to / W > from / W;
-            if (later && to < own) mark(from, to);
+        // the successors [i, n) of task `from` that are `step` apart: whether all of them are in later blocks
+        auto edges = [&](uint32_t from, uint32_t i, uint32_t n, uint32_t step) -> bool {
+            bool later = true;
+            for (; i < n; i += PLAN_BATCH * step)
+            {
+                uint32_t to[PLAN_BATCH];
+                unsigned which = 0;
+#pragma unroll
+                for (int j = 0; j < PLAN_BATCH; ++j) to[j] = i + j * (uint64_t) step < n ? a.succ[i + j * step] : 0xffffffffu;
+#pragma unroll
+                for (int j = 0; j < PLAN_BATCH; ++j)
+                {
+                    const bool there = to[j] != 0xffffffffu, ok = to[j] / W > from / W;
+                    later = later && (!there || ok);
+                    which |= (there && ok && to[j] < own) << j;
+                }
+                mark(from, to, which);
+            }
             return later;
         };
         const uint32_t b = mine ? a.succ_ptr[t] : 0u, e = mine ? a.succ_ptr[t + 1] : 0u;
         if (mine) ok = a.npred_first[t] < INORDER_MAX_NPRED && a.npred_next[t] < INORDER_MAX_NPRED;
-        for (uint32_t i = b, n = min(e, b + PLAN_LIST); i < n; ++i) ok = edge(t, a.succ[i]) && ok;
+        ok = edges(t, b, min(e, b + PLAN_LIST), 1) && ok;
         for (unsigned rest = __ballot_sync(0xffffffffu, e - b > PLAN_LIST); rest; rest &= rest - 1)
         {
             const int src = __ffs(rest) - 1;
-            const uint32_t lt = t - lane + (uint32_t) src, lb = __shfl_sync(0xffffffffu, b, src), le = __shfl_sync(0xffffffffu, e, src);
-            bool lok = true;
-            for (uint32_t i = lb + PLAN_LIST + lane; i < le; i += 32) lok = edge(lt, a.succ[i]) && lok;
-            lok = __all_sync(0xffffffffu, lok);
+            const uint32_t lb = __shfl_sync(0xffffffffu, b, src), le = __shfl_sync(0xffffffffu, e, src);
+            const bool lok = __all_sync(0xffffffffu, edges(t - lane + (uint32_t) src, lb + PLAN_LIST + lane, le, 32));
             if ((int) lane == src) ok = ok && lok;
         }
         // into the next window: its first W tasks have no predecessor in their own
         if (mine && a.xsucc_ptr && ahead && t + 2 * (uint64_t) W >= a.period)
-            for (uint32_t i = a.xsucc_ptr[t], n = a.xsucc_ptr[t + 1]; i < n; ++i)
-                if (a.xsucc[i] < ahead) mark(t, a.period + a.xsucc[i]);
+            for (uint32_t i = a.xsucc_ptr[t], n = a.xsucc_ptr[t + 1]; i < n; i += PLAN_BATCH)
+            {
+                uint32_t to[PLAN_BATCH];
+                unsigned which = 0;
+#pragma unroll
+                for (int j = 0; j < PLAN_BATCH; ++j)
+                {
+                    const uint32_t x = i + j < n ? a.xsucc[i + j] : ahead;
+                    to[j] = a.period + x;
+                    which |= (x < ahead) << j;
+                }
+                mark(t, to, which);
+            }
         if (near) atomicAdd(&marked, near);
         __syncthreads();
         if (threadIdx.x == 0 && marked) atomicAdd(a.ctr + CTR_NEAR, marked);
@@ -1012,7 +1052,7 @@ static SchedArgs run_args(xkb_sched * S, uint32_t ntasks, uint32_t period)
     a.tasks = S->tasks.p; a.ntasks = ntasks; a.period = period;
     a.wc = S->wc.p; a.queue = S->queue.p; a.ctr = S->ctr.p;
     a.timeout_ns = S->timeout_ns; a.pfd = S->pfd; a.units = S->team_warps; a.min_units = S->min_units;
-    a.allow_team = !S->bulk;
+    a.allow_team = !S->bulk; a.bodies = S->bodies;
     return a;
 }
 
@@ -1368,7 +1408,7 @@ extern "C" int xkb_sched_run_noalloc(const xkb_task_desc_t * tasks, const xkb_ta
     a.xsucc_ptr = nullptr; a.xsucc = nullptr; a.npred_first = graph->npred; a.npred_next = graph->npred;
     a.wc = scratch; a.queue = scratch + XKB_NOALLOC_MAX_TASKS;
     a.units = 0; a.min_units = warps_per_task;
-    a.allow_team = 1;
+    a.allow_team = 1; a.bodies = XKB_BODY_ALL;
     a.ctr = (unsigned *) (scratch + 2 * XKB_NOALLOC_MAX_TASKS);
     a.timeout_ns = (uint64_t) (timeout_s * 1e9);
     a.pfd = SCHED_PFD_DEFAULT;
