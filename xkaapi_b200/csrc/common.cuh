@@ -33,7 +33,3 @@ __device__ __forceinline__ int xkb_ld_acquire(const int * p)
     return v;
 }
 
-__device__ __forceinline__ void xkb_st_release(int * p, int v)
-{
-    asm volatile("st.release.gpu.global.s32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
-}

@@ -186,7 +186,7 @@ __device__ __forceinline__ void heat_strip_impl(const T * __restrict__ src, T * 
 
 // Edge strips (grid bottom rows, unaligned grids) take a checked path kept out of line so the
 // fast path's register allocation stays small.
-template <typename T, int VEC, int PF, bool CG>
+template <typename T, int VEC, bool CG>
 __device__ __noinline__ void heat_strip_edge(const T * __restrict__ src, T * __restrict__ dst, int64_t ld,
                                              int64_t nx, int64_t ny, int64_t rbase, int64_t rx0, int64_t rx1,
                                              int64_t cy0, int64_t cy1, double c, bool vec_ok, int pfd)
@@ -202,7 +202,7 @@ __device__ __forceinline__ void heat_strip(const T * __restrict__ src, T * __res
     if (vec_ok && rbase + StripGeom<VEC>::LOAD <= nx)
         heat_strip_impl<T, VEC, PF, CG, true>(src, dst, ld, nx, ny, rbase, rx0, rx1, cy0, cy1, c, vec_ok, pfd);
     else
-        heat_strip_edge<T, VEC, PF, CG>(src, dst, ld, nx, ny, rbase, rx0, rx1, cy0, cy1, c, vec_ok, pfd);
+        heat_strip_edge<T, VEC, CG>(src, dst, ld, nx, ny, rbase, rx0, rx1, cy0, cy1, c, vec_ok, pfd);
 }
 
 // Cells a tile task writes: its rows/cols clipped to the interior [1, n-1).

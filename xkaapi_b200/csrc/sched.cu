@@ -87,7 +87,7 @@ static_assert((1 << TEAM_LOG2) * 32 == SCHED_THREADS, "a team is a CTA");
 
 constexpr int SCHED_BULK_NBUF = 8;       // staged columns in flight per warp (bulk tile body)
 #ifndef XKB_TILE_PF
-#define XKB_TILE_PF 5                    // (4, 6, 8: 111, 108, 111 us per step of the 8192^2 graph; 5: 107) east columns an FP32 tile strip loads ahead into registers
+#define XKB_TILE_PF 5                    // east columns an FP32 tile strip loads ahead into registers (us per step of the 8192^2 graph: 3 104, 4 95, 5 95, 6 93, 8 93)
 #endif
 #ifndef XKB_F64_VEC
 #define XKB_F64_VEC 4                    // rows per lane of the FP64 tile body: one warp covers 128 rows
@@ -179,13 +179,6 @@ __device__ __forceinline__ void run_unit(const xkb_task_desc_t & d, int unit, in
             axpby_team<true>(lo, hi, a.a, (const double *) a.x, a.b, (double *) a.y, threadIdx.x & 31, 32);
         }
     // (XKB_TASK_NOOP: first-touch / placement tasks)
-}
-
-__device__ __forceinline__ int atom_add_acq_rel(int * p, int v)
-{
-    int old;
-    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    return old;
 }
 
 // Counters of a run (device memory): ready-queue tickets and tasks published, status, tasks
@@ -1018,7 +1011,7 @@ extern "C" int xkb_sched_set_team(xkb_sched_t * S, int warps_per_task)
     return XKB_OK;
 }
 
-void xkb_internal_sched_min_units(xkb_sched_t * S, int units) { S->min_units = units; }
+void xkb_internal_sched_min_units(xkb_sched_t * S, int units) { if (S) S->min_units = units; }
 
 extern "C" int xkb_sched_set_staging(xkb_sched_t * S, int bulk)
 {
@@ -1313,7 +1306,7 @@ extern "C" int xkb_sched_kernel_ms(xkb_sched_t * S, double * ms)
 // HBM for its device memory areas), or a serving loop whose device memory is already carved
 // into fixed pools, gets a failed or competing cudaMalloc; and cudaMalloc/cudaFree can
 // synchronise the device in the middle of a latency-critical loop. This entry point keeps the
-// scheduler's working set -- wait counters, queue slots and four counters -- in the file-scope
+// scheduler's working set -- wait counters, queue slots and the run's counters -- in the file-scope
 // array below instead, sized for at most XKB_NOALLOC_MAX_TASKS tasks (8 MiB + 256 B held by
 // every GPU that loads the library, until the process exits).
 static __device__ __align__(256) int g_sched_noalloc_scratch[2 * XKB_NOALLOC_MAX_TASKS + 64];   // + counters
