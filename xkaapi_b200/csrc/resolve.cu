@@ -687,42 +687,40 @@ static uint64_t context_id()
 static cudaMemPool_t resolver_pool()
 {
     static std::mutex mu;
-    static cudaMemPool_t pools[256];
-    static bool made[256];
-    static uint64_t ctx[256];
+    static auto * pools = new std::map<std::pair<int, uint64_t>, cudaMemPool_t>;       // by device and context
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 256) { cudaGetLastError(); return nullptr; }
-    const uint64_t now = context_id();
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    const uint64_t ctx = context_id();
     std::lock_guard<std::mutex> lk(mu);
-    if (!made[dev] || ctx[dev] != now)
+    const auto known = pools->find({dev, ctx});
+    if (known != pools->end()) return known->second;
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { cudaGetLastError(); pool = nullptr; }
+    else
     {
-        made[dev] = true;
-        ctx[dev] = now;
-        cudaMemPoolProps props;
-        memset(&props, 0, sizeof(props));
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        if (cudaMemPoolCreate(&pools[dev], &props) != cudaSuccess) { cudaGetLastError(); pools[dev] = nullptr; }
-        else
-        {
-            const char * e = getenv("XKB_POOL_CACHE");
-            uint64_t keep = (e && atoi(e) == 0) ? 0 : (uint64_t(4) << 30);
-            cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
-        }
+        const char * e = getenv("XKB_POOL_CACHE");
+        uint64_t keep = (e && atoi(e) == 0) ? 0 : (uint64_t(4) << 30);
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
-    return pools[dev];
+    (*pools)[{dev, ctx}] = pool;
+    return pool;
 }
 
 // Page-locked host memory the resolvers of the process share: a batch takes blocks for its staging and
 // its read-backs and gives them back when it has been waited for, so a resolver holds none between
 // batches and a new one finds them there (page-locking costs about 0.5 ms per MB and waits for the
 // device; a server keeps a resolver per graph shape). Given-back blocks are kept up to PINNED_KEEP
-// bytes while there are resolvers, and PINNED_REST once there is none (XKB_POOL_CACHE=0: none); a block in use belongs to one batch. A block up to four times the size
-// asked for will do, and a block given back displaces larger ones rather than being unlocked, so a
-// stream of batches finds its blocks again whatever an earlier one left: unlocking and locking 64 MB
-// behind a running window costs 35 to 90 ms a batch (16384^2 x 500 heat graph spawned through the C API:
-// 1.6 to 2.7 s to the end of the wait when a 128 MB block no batch asked for filled the room, 0.63 s now).
+// bytes while there are resolvers, and PINNED_REST once there is none (XKB_POOL_CACHE=0: none); a block
+// in use belongs to one batch. A block up to four times the size asked for will do, and a block given back
+// displaces larger ones rather than being unlocked, so a stream of batches finds its blocks again
+// whatever an earlier one left: unlocking and locking 64 MB behind a running window costs 35 to 90 ms a
+// batch (16384^2 x 500 heat graph spawned through the C API: 1.6 to 2.7 s to the end of the wait when a
+// 128 MB block no batch asked for filled the room, 0.63 s now).
 // Blocks end with the context they were made in (cudaDeviceReset), so each context has its own, and those of
 // one that ended are neither handed out nor unlocked again.
 class PinnedBlocks {
