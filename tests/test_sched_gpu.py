@@ -521,3 +521,18 @@ def test_graphs_that_begin_inside_a_step_run_in_order(torch_cuda, skip):
         sch.close()
     assert first == (skip != 61)
     assert not first or times[0] < 0.75 * times[1], times
+
+
+def test_units_of_the_longest_runs_are_numbered(torch_cuda):
+    """A run of 2^29 tasks and eight warps per task would need more unit numbers than there are: tasks are
+    split into fewer units there, whoever set their number, and every task runs once."""
+    torch = torch_cuda
+    period, windows = 1 << 16, (1 << 13) + 3
+    ptr = torch.zeros(period + 1, dtype=torch.int32, device="cuda")
+    each = torch.arange(period + 1, dtype=torch.int32, device="cuda")       # task t of a window follows task t of the one before
+    none, one = torch.zeros(period, dtype=torch.int32, device="cuda"), torch.ones(period, dtype=torch.int32, device="cuda")
+    graph = xk.PeriodicGraph(period, ptr.data_ptr(), none.data_ptr(), each.data_ptr(), each.data_ptr(), none.data_ptr(), one.data_ptr())
+    sch = xk.Scheduler(); sch.set_team(8); sch.set_tasks(np.zeros(period, dtype=xk.task_desc_dtype()))
+    sch.run_periodic(graph, windows)
+    assert sch.wait() == period * windows
+    sch.close()

@@ -331,10 +331,10 @@ __host__ __device__ __forceinline__ int split_log2(unsigned width, bool heat, ui
 // start, or what those release if that is more (a graph with one root and a wide second level).
 __device__ __forceinline__ int run_split_log2(const SchedArgs & a, unsigned warps)
 {
-    if (a.units) return a.units == 8 ? 3 : a.units / 2;
     const bool heat = a.bodies & XKB_BODY_AXPBY ? a.ctr[CTR_HEAT] != 0 : (a.bodies & XKB_BODY_ALL) != 0;
-    int k = split_log2(max(a.ctr[CTR_SEEDS], a.ctr[CTR_SEED_WIDTH] / 8), heat, min(a.period, a.ntasks), a.ctr[CTR_AXPBY],
-                       *(unsigned long long *) (a.ctr + CTR_PIECES), warps, a.min_units);
+    int k = a.units ? (a.units == 8 ? 3 : a.units / 2)
+                    : split_log2(max(a.ctr[CTR_SEEDS], a.ctr[CTR_SEED_WIDTH] / 8), heat, min(a.period, a.ntasks), a.ctr[CTR_AXPBY],
+                                 *(unsigned long long *) (a.ctr + CTR_PIECES), warps, a.min_units);
     while (k > 0 && ((uint64_t) a.ntasks << k) > 0xf0000000ull) --k;      // tickets are 32-bit
     return k;
 }
